@@ -94,6 +94,7 @@ struct gsofa_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // job scratch
     DevBuf queue, cnt, nxt, poff, gptr, lrow, snind, snlist, tiles, misc, pool, out, mats, ranges, stamp;
+    DevBuf snap;              // snapshots of finished traversals
     DevBuf gstate;            // visited bitmaps of the global-state kernels
     DevBuf blk;               // streaming: written entries per pool block
     DevBuf order;             // gsofa_order_rcm: symmetric structure, levels, sort space
@@ -124,8 +125,16 @@ struct gsofa_ctx {
             b.p = nullptr;
             b.bytes = 0;
         }
+        // snapshots only save time: they give way to what a job needs
+        if (held + bytes > budget && &b != &snap) release(snap);
         if (held + bytes > budget) throw CudaFail{cudaErrorMemoryAllocation};
-        GS_CUDA(cudaMalloc(&b.p, bytes));
+        cudaError_t e = cudaMalloc(&b.p, bytes);
+        if (e == cudaErrorMemoryAllocation && snap.p && &b != &snap) {
+            cudaGetLastError();
+            release(snap);
+            e = cudaMalloc(&b.p, bytes);
+        }
+        GS_CUDA(e);
         b.bytes = bytes;
         held += bytes;
         return b.p;
@@ -418,7 +427,9 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
     void *kfn = factor_kernel_for(block, paired, gbm, wide, want_pattern != 0);
     if (!kfn) return GSOFA_ERR_INVALID_INPUT;
     const int NS = paired ? 2 : 1;
-    int lanes = p.threads_per_source ? p.threads_per_source : 1;
+    // accepted as ever; a warp's lanes share its vertices' rows by their
+    // lengths, so the value chooses nothing any more
+    const int lanes = p.threads_per_source ? p.threads_per_source : 1;
     if (lanes != 1 && lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32)
         return GSOFA_ERR_INVALID_INPUT;
 
@@ -585,6 +596,24 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         if (want_pattern)
             d_stamp = (uint16_t *)ctx->grow(ctx->stamp, (size_t)grid * NS * stamp_stride * sizeof(uint16_t));
         uint32_t *d_gstate = gbm ? (uint32_t *)ctx->grow(ctx->gstate, (size_t)grid * NS * state_words * 4) : nullptr;
+        // Snapshots: paired passes with reuse, as many as a sixteenth of the
+        // budget holds, and none where the job leaves no room for them.
+        uint32_t *d_snap = nullptr;
+        int snap_k = 0;
+        if (paired && reuse) {
+            const size_t one = (size_t)grid * NS * bitmap_words * 4;
+            for (int k = SNAP_MAX; k >= 2 && !snap_k; k >>= 1) {
+                const size_t need = std::max<size_t>(one * k, 256);
+                if (need > ctx->budget / 16) continue;
+                if (ctx->snap.bytes < need && ctx->held - ctx->snap.bytes + need > ctx->budget) continue;
+                try {
+                    d_snap = (uint32_t *)ctx->grow(ctx->snap, need);
+                    snap_k = k;
+                } catch (CudaFail &) {
+                    cudaGetLastError();
+                }
+            }
+        }
         MatDesc *d_mats = (MatDesc *)ctx->grow(ctx->mats, md.size() * sizeof(MatDesc));
         int64_t *d_minfo = (int64_t *)ctx->grow(ctx->matinfo, (size_t)3 * count * sizeof(int64_t));
         Range *d_ranges = (Range *)ctx->grow(ctx->ranges, std::max<size_t>(ranges.size(), 1) * sizeof(Range));
@@ -602,7 +631,8 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         a.bitmap_words = bitmap_words;
         a.state_words = state_words;
         a.ring_size = ring;
-        a.lanes = lanes;
+        a.snap = d_snap;
+        a.snap_k = snap_k;
         a.reuse = reuse;
         a.want_pattern = pattern_form;
         a.max_sn = p.max_supernode_size;
@@ -950,7 +980,7 @@ void gsofa_destroy(gsofa_ctx *c)
     DevBuf *bufs[] = {&c->queue, &c->cnt, &c->nxt, &c->poff, &c->gptr, &c->lrow, &c->snind,
                       &c->snlist, &c->tiles, &c->misc, &c->pool, &c->out, &c->mats, &c->ranges,
                       &c->st_beg, &c->st_end, &c->st_adj, &c->st_tmp, &c->matinfo, &c->stamp,
-                      &c->sn_head, &c->sn_data, &c->gstate, &c->blk, &c->order};
+                      &c->sn_head, &c->sn_data, &c->gstate, &c->blk, &c->order, &c->snap};
     for (DevBuf *b : bufs) c->release(*b);
     for (DevBuf &b : c->slabs) cudaFree(b.p);
     c->slabs.clear();
@@ -2159,7 +2189,8 @@ extern "C" gsofa_status gsofa_symbfact_counts_noalloc(int device, void *cuda_str
         a.bitmap_words = bitmap_words;
         a.state_words = state_words;
         a.ring_size = ring;
-        a.lanes = 1;
+        a.snap = nullptr;
+        a.snap_k = 0;
         a.reuse = 1;
         a.want_pattern = 0;
         a.max_sn = max_supernode_size;
@@ -2385,7 +2416,8 @@ gsofa_status server_launch_if_idle_impl(gsofa_server *s)
     a.state_words = s->state_words;
     a.ring_size = s->ring;
     a.gbm = s->d_gstate;
-    a.lanes = 1;
+    a.snap = nullptr;
+    a.snap_k = 0;
     a.reuse = 1;
     a.want_pattern = 0;
     a.L = s->lmax;

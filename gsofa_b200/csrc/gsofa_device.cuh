@@ -108,8 +108,7 @@ struct JobArgs {
     int32_t bitmap_words;      // shared-memory bitmap size (>= max n / 32, multiple of 128)
     int32_t state_words;       // bitmap + its two summary levels
     int32_t ring_size;         // shared-memory frontier ring entries (power of two)
-    int32_t lanes;             // lanes per frontier vertex: 1 (thread per vertex,
-                               // warp for long rows) or 4..32
+    int32_t snap_k;            // snapshots a traversal slot keeps (0: none)
     int32_t reuse;
     int32_t want_pattern;
     int32_t max_sn;
@@ -136,13 +135,15 @@ struct JobArgs {
     unsigned long long *counters; // [0] edges inspected, [1] sources, [2] sn total,
                                   // [3] pass-G expansions, [4] pass-G input degrees,
                                   // [5] levels, [6] sources that reused state,
-                                  // [7..13] cycles: seeding, levels, fold, count,
-                                  // list output, clearing, pair wait;
+                                  // [7..13] cycles: the sources' own steps, their
+                                  // levels, snapshots, (unused), list output,
+                                  // clearing, pair wait;
                                   // [14] ns until the traversals ended,
                                   // [15] CTAs' traversal ns, summed
     uint32_t *status;
     uint16_t *stamp;           // pattern mode: per traversal, stamp_stride entries:
     int64_t stamp_stride;      // the chain index at which each vertex was first set
+    uint32_t *snap;            // snapshots: snap_k bitmaps per traversal slot
     uint32_t *gbm;             // global-state kernels: per traversal, state_words
                                // words (bitmap and its summaries) in global memory
     unsigned int *blk_done;    // ranges form, streamed: entries written into each
@@ -251,27 +252,45 @@ __device__ __forceinline__ int bm_summary_words(const uint32_t *bm, const uint32
     return (int)(summ - bm) >> 5;
 }
 
-// Bit test-and-set in the shared-memory bitmap; true when this call set it.
-// summ holds one bit per bitmap word, set when that word first becomes
-// nonzero, so output scans can skip empty stretches 32 words at a time.
-// summ is followed by a second level (one bit per summary word, i.e. per
-// 32K vertices) at summ + summary_words; SUMM2_OFF gives that offset.
-// GBM: the bitmap lives in global memory (L2), where a read before the
-// atomic would cost as much as the atomic itself, so the atomic goes first.
-template <bool GBM>
-__device__ __forceinline__ bool test_and_set(uint32_t *bm, uint32_t *summ, int32_t m)
+// Enters bitmap word wi, which just became nonzero, in both summary levels.
+__device__ __forceinline__ void mark_word(const uint32_t *bm, uint32_t *summ, int wi)
 {
-    const uint32_t bit = 1u << (m & 31);
-    const int wi = m >> 5;
-    uint32_t *w = bm + wi;
-    if (!GBM && (*reinterpret_cast<volatile uint32_t *>(w) & bit)) return false;
-    const uint32_t old = atomicOr(w, bit);
-    if (old == 0u) {
-        const int si = wi >> 5;
-        const uint32_t olds = atomicOr(summ + si, 1u << (wi & 31));
-        if (olds == 0u) atomicOr(summ + (bm_summary_words(bm, summ)) + (si >> 5), 1u << (si & 31));
+    atomicOr(summ + (wi >> 5), 1u << (wi & 31));
+    atomicOr(summ + bm_summary_words(bm, summ) + (wi >> 10), 1u << ((wi >> 5) & 31));
+}
+
+// Sets the bits m >= 0 of a traversal's bitmap, one per lane and u, all of
+// them in flight together: the words' reads first, then the atomics of those
+// that look unset, then the summaries of words that became nonzero.  Returns a
+// mask over u of the bits that this call set.  summ holds one bit per bitmap
+// word and is followed by a second level, one bit per summary word (per 32K
+// vertices); a summary bit is only ever added, so neither level is read back.
+// GBM: the bitmap lives in global memory (L2), where a read before the atomic
+// would cost as much as the atomic itself, so the atomics go first.
+template <int U, bool GBM>
+__device__ __forceinline__ unsigned set_bits(uint32_t *bm, uint32_t *summ, const int32_t (&m)[U])
+{
+    unsigned todo = 0u, fresh = 0u;
+    uint32_t w[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        w[u] = 0u;
+        if (!GBM && m[u] >= 0) w[u] = *reinterpret_cast<volatile uint32_t *>(bm + (m[u] >> 5));
     }
-    return !(old & bit);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        if (m[u] >= 0 && !((w[u] >> (m[u] & 31)) & 1u)) todo |= 1u << u;
+    if (todo == 0u) return 0u;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        if ((todo >> u) & 1u) w[u] = atomicOr(bm + (m[u] >> 5), 1u << (m[u] & 31));
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        if (((todo >> u) & 1u) && !((w[u] >> (m[u] & 31)) & 1u)) {
+            fresh |= 1u << u;
+            if (w[u] == 0u) mark_word(bm, summ, m[u] >> 5);
+        }
+    return fresh;
 }
 
 // Reads a word of a traversal's state: from shared memory, or (GBM) from
@@ -311,18 +330,6 @@ __device__ __forceinline__ int32_t fr_get(const Frontier &f, int p, int w0)
     return (p - w0 < f.ring_size) ? f.ring[p & (f.ring_size - 1)] : f.spill[p];
 }
 
-// Appends m to the next level; one shared atomic per coalesced group of lanes
-// (warp-aggregated enqueue).  base: first position of the next level;
-// w0: first position of the current level.
-__device__ __forceinline__ void push(const Frontier &f, int *tail, int base, int w0, int32_t m)
-{
-    cg::coalesced_group g = cg::coalesced_threads();
-    int b = 0;
-    if (g.thread_rank() == 0) b = atomicAdd(tail, (int)g.size());
-    b = g.shfl(b, 0);
-    fr_put(f, base + b + (int)g.thread_rank(), w0, m);
-}
-
 // Seeding window: the rows of up to SEED_WIN consecutive sources (SEED_ADJ
 // ids at most), loaded together -- consecutive rows are one stretch of the
 // adjacency array -- so a source's seeding reads shared memory instead of
@@ -330,58 +337,80 @@ __device__ __forceinline__ void push(const Frontier &f, int *tail, int base, int
 constexpr int SEED_WIN = 32;
 constexpr int SEED_ADJ = 512;
 
+// Snapshots of finished traversals (paired passes): at most SNAP_MAX a
+// traversal slot, each usable by the sources of the SNAP_REACH words of lines
+// from its own source on.
+constexpr int SNAP_MAX = 8;
+constexpr int SNAP_REACH = 16;
+
+// Levels of at most this many vertices are run by a traversal's leader alone.
+constexpr int SOLO_MAX = 32;
+
+// Work that a traversal's first warp (its leader) hands to all of its warps.
+enum : int { OP_EXIT = 0, OP_LEVELS, OP_CLEAR, OP_LISTS, OP_SAVE, OP_MERGE };
+
+// One traversal's shared state.  The leader warp runs the piece's sources and
+// alone touches the fields marked L; the other warps wait at the traversal's
+// barrier for an op, and the fields marked O are its arguments and results.
 struct SharedState {
-    long long piece;
-    int flag;
-    int tailc[3];     // level entry counts by phase (barrier-synchronised levels)
-    int fetch[3];     // dynamic fetch counters by phase
-    int chain_lo;     // lowest vertex set in the bitmap since the last clear
-    int chain_hi;     // highest vertex set since the last clear
-    int seg[2];       // piece boundaries after chain alignment
-    int stail;        // entries of the next level, counted while warp 0 runs levels alone
-    int solo_start, solo_wstart, solo_count;   // where such a run ended
-    int64_t warp[32]; // per-warp entry counts of a chain's last list (list output)
-    int64_t last_off; // pool offset of a chain's last list (-1: pool short)
-    int last_cnt;     // its entries
-    // tallies kept by the half's first thread only: levels, then cycles of
-    // seeding, level loop, range fold, count and link flag, list output (per
-    // chain), bitmap clearing, wait for the other pass; sources; reused
-    // sources
+    int op;                 // O: OP_*
+    int src, cidx;          // O: the source, its index in its chain
+    int lv_start, lv_end, lv_wstart;   // O: OP_LEVELS: the level to start from
+    int snap, lo, hi, t;    // O: OP_SAVE / OP_MERGE: slot, its bitmap words, its source
+    int tailc[3];           // level entry counts by phase
+    int fetch[3];           // dynamic fetch counters by phase
+    int nh;                 // O: new vertices above the source that an op found
+    int npush;              // O: queue entries that OP_MERGE made
+    int seg[2];             // piece boundaries after chain alignment
+    // list output (pattern mode): the chain -- consecutive sources sharing one
+    // bitmap -- whose lists are written when it ends
+    uint16_t *stamp;        // this traversal's stamp row, or null (counts only)
+    int chain_s0;           // its first source
+    int chain_len;          // its sources
+    int chain_hi;           // no vertex above is set
+    int64_t chain_total;    // entries of its lists
+    int64_t warp[32];       // per-warp entry counts of a chain's last list
+    int64_t last_off;       // pool offset of a chain's last list (-1: pool short)
+    int last_cnt;           // its entries
+    // tallies, kept by the leader's first lane: levels, then cycles of the
+    // sources' own steps, their levels, list output, clearing, snapshots, wait
+    // for the other pass; sources; reused sources
     unsigned long long prof[8];
     unsigned long long nsrc, nreuse;
-    int hcount;        // set bits above the current source (|hi(s)| once done)
-    // the current chain -- consecutive sources sharing one bitmap -- whose
-    // lists are written when it ends (pattern mode)
-    uint16_t *stamp;   // this traversal's stamp row, or null (counts only)
-    int chain_s0;      // its first source
-    int chain_len;     // its sources so far (the current one included)
-    int64_t chain_total;  // entries of its lists
-    // the seeding window: sources [win_lo, win_hi) of the current piece
-    int win_lo, win_hi;
-    int32_t win_ptr[SEED_WIN + 1];   // their row bounds in adj
-    int32_t win_raw[SEED_WIN];       // their input degrees (work counters)
-    int32_t win_adj[SEED_ADJ];       // adj[win_ptr[0] .. win_ptr[win_hi - win_lo])
+    uint32_t reach[2][SNAP_REACH];            // by source parity: this bitmap's words from the source's on
+    uint32_t snap_reach[SNAP_MAX][SNAP_REACH];  // L: the other pass's words when the snapshot was taken
+    int32_t win_adj[SEED_ADJ];                // L: the window's rows
 };
 
-// Records that v was first set while the chain's source `idx` ran (sources
-// of a chain are consecutive, so idx = s - chain_s0).  Only vertices above
-// the chain's first source can appear in its lists.
-__device__ __forceinline__ void stamp_set(const SharedState &sh, int32_t v, int idx, int32_t chain_s0)
+// Snapshots that a CTA saves ahead of taking any over (each one taken over
+// earns eight more).
+constexpr int SNAP_CREDIT = 24;
+
+__device__ __forceinline__ void init_state(SharedState &sh)
 {
-    uint16_t *st = sh.stamp;
-    if (st != nullptr && v > chain_s0) st[v] = (uint16_t)idx;
+    sh.stamp = nullptr;
+    sh.nh = 0;
+    for (int q = 0; q < 8; q++) sh.prof[q] = 0;
+    sh.nsrc = sh.nreuse = 0;
+    sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
+    sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
 }
 
-// Clears the bitmap words covering vertices [lo, hi]; gtid/GT: the calling
-// thread's index and the size of the thread group that shares the bitmap.
+// Barrier of the GT threads that work on one traversal: the whole CTA or one
+// half of it, through the named barrier `bar` (1 or 2).
 template <int GT>
-__device__ __forceinline__ void clear_range(uint32_t *bm, uint32_t *summ, int lo, int hi, int gtid)
+__device__ __forceinline__ void gsync(int bar)
 {
-    if (hi < lo) return;
-    for (int w = (lo >> 5) + gtid; w <= (hi >> 5); w += GT) bm[w] = 0u;
-    for (int w = (lo >> 10) + gtid; w <= (hi >> 10); w += GT) summ[w] = 0u;
-    uint32_t *summ2 = summ + bm_summary_words(bm, summ);
-    for (int w = (lo >> 15) + gtid; w <= (hi >> 15); w += GT) summ2[w] = 0u;
+    if (GT == 32) __syncwarp();
+    else if (bar == 1) asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
+}
+
+// Barrier of the two leader warps of a CTA that runs both passes of a source.
+__device__ __forceinline__ void pair_sync()
+{
+    __syncwarp();
+    asm volatile("bar.sync 3, 64;" ::: "memory");
 }
 
 // Visits the nonzero chunks c in [c0, c1) (chunk = 32 bitmap words = one
@@ -404,16 +433,6 @@ __device__ __forceinline__ void for_nonzero_chunks(const uint32_t *summ2, int c0
     }
 }
 
-// Barrier of the GT threads that work on one traversal: the whole CTA
-// (bar == 0) or one half of it (named barrier `bar`).
-template <int GT>
-__device__ __forceinline__ void gsync(int bar)
-{
-    if (bar == 0) __syncthreads();
-    else if (bar == 1) asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
-    else asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
-}
-
 // True when x-1 is in adj(x); evaluated by one whole warp.
 __device__ __forceinline__ bool warp_has_prev(const PassGraph &g, int32_t x)
 {
@@ -426,7 +445,7 @@ __device__ __forceinline__ bool warp_has_prev(const PassGraph &g, int32_t x)
 
 // The chain start at or below x: the lowest y with y+1 .. x each holding its
 // predecessor, searched at most `limit - 1` steps down; x itself when the
-// chain reaches further (then the cut is not aligned).  Warp 0 only.
+// chain reaches further (then the cut is not aligned).  One warp.
 __device__ __forceinline__ int32_t chain_start(const PassGraph &g, int32_t x, int32_t limit)
 {
     int32_t y = x;
@@ -437,349 +456,264 @@ __device__ __forceinline__ int32_t chain_start(const PassGraph &g, int32_t x, in
     return (y == 0 || !warp_has_prev(g, y)) ? y : x;
 }
 
-// Visits neighbour m of a frontier vertex: marks it, and queues it for the
-// next level when it lies below the source, else counts it in nh (new
-// vertices above the source).
-#define GSOFA_VISIT(m)                                                          \
-    do {                                                                        \
-        const int32_t _m = (m);                                                 \
-        if (test_and_set<GBM>(bm, summ, _m)) {                                        \
-            t_lo = min(t_lo, _m);                                               \
-            t_hi = max(t_hi, _m);                                               \
-            stamp_set(sh, _m, cidx, s - cidx);                                            \
-            if (_m < s) push(f, tailp, end, start, _m);                         \
-            else nh++;                                                          \
-        }                                                                       \
-    } while (0)
+// What every warp of a traversal knows about it for one work piece.
+struct Trav {
+    PassGraph g;
+    const int32_t *rawdeg;
+    int pass;
+    uint32_t *bm, *summ;
+    Frontier f;
+    uint16_t *stamp;       // or null
+    uint32_t *snaps;       // this traversal's snapshots
+};
 
-// One source s of one pass: seeds from adj(s), expands the frontier level by
-// level through vertices < s, then records |hi(s)| and the s+1 link flag (the
-// list itself is written when the chain of sources ends, output_chain).
-// When the caller reuses state, the bitmap still holds the finished traversal
-// of s-1, which is valid whenever s-1 is in X(s): then X(s-1) u {s-1} is inside
-// X(s) and hi(s-1) minus {s} is inside hi(s).
-// END_SYNC: finish with a barrier of the traversal's threads (not needed when
-// the caller's next step is a barrier of the whole CTA).
-//
-// The level counters (tailc, fetch) are zero on entry: the previous source
-// left them so.  s_end: the end of the piece (the seeding window stays within
-// it); stride: the distance between the piece's sources; cidx: the index of
-// s in its chain (every thread tracks it; a chain's sources are consecutive,
-// so it starts at s - cidx).
-template <int GT, bool CG, bool END_SYNC, bool GBM>
-__device__ void process_source(const JobArgs &a, const PassGraph g, int32_t n,
-                               int64_t line, int pass, int32_t s, int32_t s_end, int32_t stride,
-                               int cidx, uint32_t *bm, uint32_t *summ,
-                               const Frontier &f, SharedState &sh,
-                               unsigned long long &edges, const int32_t *rawdeg,
-                               unsigned long long &xcnt, unsigned long long &einsp,
-                               unsigned long long *prof, const int gtid, const int bar)
+// Per-thread tallies of one CTA's traversals (summed over the CTA at the
+// end); the per-source ones live in SharedState, kept by one thread.
+struct Tally {
+    unsigned long long edges = 0, xcnt = 0, einsp = 0;
+};
+
+// New vertices of one warp step: those below s are queued for the next level
+// (alloc(k) hands out k positions, warp-uniformly; w0 is the first position of
+// the level whose vertices found them), those above s are counted (the return
+// value, warp-uniform).  Every new vertex above the chain's first source gets
+// the chain index of s as its stamp (pattern mode).
+template <int U, bool GBM, class Alloc>
+__device__ __forceinline__ int visit(const Trav &t, const int32_t (&m)[U], int32_t s, int cidx, int w0, Alloc alloc)
 {
-    const int tid = gtid;
-    const int lane = tid & 31;
-    const int lanes = a.lanes;
-    const int lane_in_group = tid & (lanes - 1);
-    int t_lo = INT32_MAX, t_hi = -1;
-
-    long long c0 = 0;
-    if (tid == 0) c0 = clock64();
-    // a new seeding window when s is past the current one (consecutive
-    // sources only): row bounds, then the rows themselves, all threads
-    int wlo = sh.win_lo, whi = sh.win_hi;   // stable: set behind earlier barriers
-    if (stride == 1 && (s < wlo || s >= whi)) {
-        const int hi0 = min(s_end, s + SEED_WIN);
-        for (int i = tid; i <= hi0 - s; i += GT) {
-            sh.win_ptr[i] = ld<CG>(g.ptr + s + i);
-            if (i < hi0 - s) sh.win_raw[i] = ld<CG>(rawdeg + s + i);
-        }
-        gsync<GT>(bar);
-        int k = hi0 - s;   // rows that fit
-        while (k > 0 && sh.win_ptr[k] - sh.win_ptr[0] > SEED_ADJ) k--;
-        const int32_t a0 = sh.win_ptr[0], na = sh.win_ptr[k] - a0;
-        for (int i = tid; i < na; i += GT) sh.win_adj[i] = ld<CG>(g.adj + a0 + i);
-        gsync<GT>(bar);
-        wlo = s;
-        whi = s + k;
-        if (tid == 0) { sh.win_lo = wlo; sh.win_hi = whi; }   // read by later sources
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned fresh = set_bits<U, GBM>(t.bm, t.summ, m);
+    if (!__any_sync(0xffffffffu, fresh != 0u)) return 0;
+    if (t.stamp != nullptr) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (((fresh >> u) & 1u) && m[u] > s - cidx) t.stamp[m[u]] = (uint16_t)cidx;
     }
-    const bool in_win = stride == 1 && s >= wlo && s < whi;
-    if (tid == 0) {
-        sh.chain_len = cidx + 1;
-        if (test_and_set<GBM>(bm, summ, s)) { t_lo = s; t_hi = s; stamp_set(sh, s, cidx, s - cidx); }
-        else atomicAdd(&sh.hcount, -1);   // s was in hi(s-1): counted, but not above s
+    unsigned low[U];
+    int nlow = 0, nnew = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const bool f = (fresh >> u) & 1u;
+        low[u] = __ballot_sync(0xffffffffu, f && m[u] < s);
+        nnew += __popc(__ballot_sync(0xffffffffu, f));
+        nlow += __popc(low[u]);
     }
-    // No barrier here: seeding pushes onto the zeroed level-0 counter, the
-    // stamps take the thread's own cidx, and s itself (which no neighbour of
-    // s is) is set before the level loop's first barrier.
-
-    // seeding: every neighbour of s is structure of line s; level-0 items
-    {
-        int32_t b0, e0;
-        if (in_win) {
-            b0 = sh.win_ptr[s - wlo];
-            e0 = sh.win_ptr[s - wlo + 1];
-        } else {
-            b0 = ld<CG>(g.ptr + s);
-            e0 = ld<CG>(g.ptr + s + 1);
+    if (nlow) {
+        int pos = alloc(nlow);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if ((low[u] >> lane) & 1u) fr_put(t.f, pos + __popc(low[u] & below), w0, m[u]);
+            pos += __popc(low[u]);
         }
-        if (tid == 0) {
-            edges += (unsigned long long)(e0 - b0);
-            if (pass == 0) einsp += (unsigned long long)(in_win ? sh.win_raw[s - wlo] : ld<CG>(rawdeg + s));
-        }
-        int *tailp = &sh.tailc[0];
-        const int end = 0, start = 0;
-        int nh = 0;
-        if (in_win) {
-            const int32_t *wa = sh.win_adj - sh.win_ptr[0];
-            for (int32_t k = b0 + tid; k < e0; k += GT) GSOFA_VISIT(wa[k]);
-        } else {
-            for (int32_t k = b0 + tid; k < e0; k += GT) GSOFA_VISIT(ld<CG>(g.adj + k));
-        }
-        nh = (int)__reduce_add_sync(0xffffffffu, (unsigned)nh);
-        if (lane == 0 && nh) atomicAdd(&sh.hcount, nh);
     }
-    long long cs = 0;
-    if (tid == 0) { cs = clock64(); prof[1] += (unsigned long long)(cs - c0); }
+    return nnew - nlow;
+}
 
-    // One warp's step of a level (one thread per vertex): items base ..
-    // base + 31 of the level [start, end), whose entries were written while
-    // the level starting at wstart ran; new vertices below s go to the next
-    // level through tailp.  Each lane loads its row bounds and then up to
-    // eight adjacency ids at once (independent loads in flight hide the L2
-    // latency).  The id loop runs to the warp's longest light row so every
-    // step is warp-uniform and new vertices below s are enqueued with one
-    // ballot and one shared atomic.  Rows longer than HEAVY_ROW are expanded
-    // by the whole warp.
-    auto warp_step = [&](const int base, const int start, const int end, const int wstart, int *const tailp) {
-        const int it = base + lane;
-        int32_t b = 0, d = 0;
-        int4 sl0 = make_int4(0, 0, -1, -1), sl1 = make_int4(-1, -1, -1, -1);
-        if (it < end) {
-            const int32_t v = fr_get(f, it, wstart);
-            if (g.slot != nullptr) {   // degree, offset and short rows in one 32-byte load
-                sl0 = ld4<CG>(g.slot + 2 * (int64_t)v);
-                sl1 = ld4<CG>(g.slot + 2 * (int64_t)v + 1);
-                d = sl0.x;
-                b = sl0.y;
-            } else {
-                b = ld<CG>(g.ptr + v);
-                d = ld<CG>(g.ptr + v + 1) - b;
-            }
-            edges += (unsigned long long)d;
-            if (pass == 0) { xcnt++; einsp += (unsigned long long)ld<CG>(rawdeg + v); }
-        }
-        // the row's ids are in the slot (first step of the id loop)
-        const bool in_slot = g.slot != nullptr && d <= SLOT_NB;
-        unsigned heavy = __ballot_sync(0xffffffffu, d > HEAVY_ROW);
-        while (heavy) {
-            const int src = __ffs(heavy) - 1;
-            heavy &= heavy - 1u;
-            const int32_t hb = __shfl_sync(0xffffffffu, b, src);
-            const int32_t hd = __shfl_sync(0xffffffffu, d, src);
-            for (int32_t k0 = 0; k0 < hd; k0 += 32) {
-                const bool on = k0 + lane < hd;
-                const int32_t m = on ? ld<CG>(g.adj + hb + k0 + lane) : 0;
-                const bool fresh = on && test_and_set<GBM>(bm, summ, m);
-                if (fresh) { t_lo = min(t_lo, m); t_hi = max(t_hi, m); stamp_set(sh, m, cidx, s - cidx); }
-                const bool low = fresh && m < s;
-                const unsigned bal = __ballot_sync(0xffffffffu, low);
-                const unsigned bhi = __ballot_sync(0xffffffffu, fresh) & ~bal;
-                if (lane == 0 && bhi) atomicAdd(&sh.hcount, __popc(bhi));
-                if (bal) {
-                    int pb = 0;
-                    if (lane == 0) pb = atomicAdd(tailp, __popc(bal));
-                    pb = __shfl_sync(0xffffffffu, pb, 0);
-                    if (low) fr_put(f, end + pb + __popc(bal & ((1u << lane) - 1u)), start, m);
-                }
+// Expands up to 32 frontier vertices, one per lane (v, or -1).  Rows that
+// their 32-byte slot holds whole are visited lane by lane, six ids at once.
+// The others are read edge by edge: the lanes share the rows' ids by a prefix
+// sum of their lengths, 128 consecutive ids in flight, so a warp's loads touch
+// the rows' own sectors once.  (One lane per row, eight ids at a time, fetched
+// a sector per id -- 32 rows' lines do not stay in the L1 that the bitmaps
+// leave -- and ran the 200,003-line power-law counts at 0.31 edges per SM
+// cycle.)
+template <bool CG, bool GBM, class Alloc>
+__device__ __forceinline__ int expand(const Trav &t, int32_t v, int32_t s, int cidx, int w0, Tally &acc, Alloc alloc)
+{
+    const int lane = threadIdx.x & 31;
+    int32_t b = 0, d = 0;
+    int nh = 0;
+    if (t.g.slot != nullptr) {
+        int32_t m[SLOT_NB] = {-1, -1, -1, -1, -1, -1};
+        if (v >= 0) {   // degree, offset and short rows in one 32-byte load
+            const int4 sl0 = ld4<CG>(t.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(t.g.slot + 2 * (int64_t)v + 1);
+            d = sl0.x;
+            b = sl0.y;
+            acc.edges += (unsigned)d;
+            if (t.pass == 0) { acc.xcnt++; acc.einsp += (unsigned)ld<CG>(t.rawdeg + v); }
+            if (d <= SLOT_NB) {   // ids past the degree are -1 in the slot
+                m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
+                d = 0;
             }
         }
-        const int dl = d > HEAVY_ROW ? 0 : d;
-        const int dmax = __reduce_max_sync(0xffffffffu, dl);
-        for (int k0 = 0; k0 < dmax; k0 += 8) {
-            int32_t buf[8];
-            if (in_slot) {   // d <= 6 < 8: only this first step has ids
-                const int32_t sv[SLOT_NB] = {sl0.z, sl0.w, sl1.x, sl1.y, sl1.z, sl1.w};
+        nh = visit<SLOT_NB, GBM>(t, m, s, cidx, w0, alloc);
+        if (!__any_sync(0xffffffffu, d != 0)) return nh;
+    } else if (v >= 0) {
+        b = ld<CG>(t.g.ptr + v);
+        d = ld<CG>(t.g.ptr + v + 1) - b;
+        acc.edges += (unsigned)d;
+        if (t.pass == 0) { acc.xcnt++; acc.einsp += (unsigned)ld<CG>(t.rawdeg + v); }
+    }
+    int incl = d;   // a warp's rows hold at most nnz < 2^31 ids together: distinct vertices
 #pragma unroll
-                for (int u = 0; u < 8; u++) buf[u] = (u < SLOT_NB && k0 + u < dl) ? sv[u < SLOT_NB ? u : 0] : -1;
-            } else {
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int32_t from = b - (incl - d);   // id e of the warp's edges is adj[from + e] of its owner
+    constexpr int U = 4;
+    for (int e0 = 0; e0 < total; e0 += 32 * U) {
+        int32_t m[U];
 #pragma unroll
-                for (int u = 0; u < 8; u++) buf[u] = (k0 + u < dl) ? ld<CG>(g.adj + b + k0 + u) : -1;
-            }
-            // independent bit tests and sets first, then one enqueue
-            // (warp scan + one shared atomic) for all new low vertices
-            unsigned fresh = 0u;
+        for (int u = 0; u < U; u++) {
+            const int e = e0 + 32 * u + lane;
+            int o = 0;     // the first lane whose inclusive sum passes e
 #pragma unroll
-            for (int u = 0; u < 8; u++)
-                if (buf[u] >= 0 && test_and_set<GBM>(bm, summ, buf[u])) fresh |= 1u << u;
-            // new vertices below s in the low 16 bits, above s in
-            // the high ones (a warp step finds at most 256)
-            int nlh = 0;
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-                if ((fresh >> u) & 1u) {
-                    t_lo = min(t_lo, buf[u]);
-                    t_hi = max(t_hi, buf[u]);
-                    nlh += buf[u] < s ? 1 : 0x10000;
-                }
-            if (fresh && sh.stamp != nullptr) {
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if ((fresh >> u) & 1u) stamp_set(sh, buf[u], cidx, s - cidx);
-            }
-            int incl = nlh;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const int wsum = __shfl_sync(0xffffffffu, incl, 31);
-            const int wtot = wsum & 0xffff;
-            if (lane == 0 && (wsum >> 16)) atomicAdd(&sh.hcount, wsum >> 16);
-            if (wtot) {
-                int pb = 0;
-                if (lane == 0) pb = atomicAdd(tailp, wtot);
-                pb = __shfl_sync(0xffffffffu, pb, 0) + ((incl - nlh) & 0xffff);
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    if (((fresh >> u) & 1u) && buf[u] < s) fr_put(f, end + pb++, start, buf[u]);
-            }
+            for (int h = 16; h; h >>= 1)
+                if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= e) o += h;
+            const int32_t at = __shfl_sync(0xffffffffu, from, o & 31) + e;
+            m[u] = e < total ? ld<CG>(t.g.adj + at) : -1;
         }
-    };
+        nh += visit<U, GBM>(t, m, s, cidx, w0, alloc);
+    }
+    return nh;
+}
 
-    // level-synchronous expansion through vertices < s, one barrier a level.
-    // A level of at most 32 vertices (one per lane) is run by warp 0 alone
-    // (solo), and so are the small levels after it, with warp barriers only,
-    // while the traversal's other warps wait at the next barrier.  The
-    // barrier-synchronised levels count their entries in tailc[] by phase c:
-    // the current level's count in tailc[c % 3], the next level's in
-    // tailc[(c + 1) % 3] (zero when the level starts), fetch counter
-    // fetch[c % 3] (zero too).  Solo levels count in sh.stail only, touched by
-    // lane 0 alone, and hand over through sh.solo_* after the next barrier:
-    // the phase and its counters are then as they were when the run began.
-    int start = 0, wstart = 0, c = 0;
-    bool relay = false;   // warp 0 ran levels alone: take up its position
+// All warps of a traversal: levels from [start, end) on (entries written while
+// the level starting at wstart ran) until one is small enough for the leader
+// alone.  One barrier a level.  The level counters rotate through three phases
+// that run on from call to call (every warp counts them in `phase`): a level
+// counts the next one's entries in tailc[phase] and its own dynamic fetches in
+// fetch[phase]; the counters of the phase after next are cleared behind the
+// level's barrier, when every warp is done with them.
+template <int GT, bool CG, bool GBM>
+__device__ __forceinline__ void run_levels(const Trav &t, SharedState &sh, int gtid, int bar, int &phase,
+                                           Tally &acc)
+{
+    constexpr int NW = GT / 32;
+    const int lane = gtid & 31, wid = gtid >> 5;
+    const int32_t s = sh.src;
+    const int cidx = sh.cidx;
+    int start = sh.lv_start, end = sh.lv_end, wstart = sh.lv_wstart;
+    int nlev = 0;
     for (;;) {
+        int *const tailp = &sh.tailc[phase], *const fetchp = &sh.fetch[phase];
+        const int cnt = end - start;
+        // vertices a warp takes at a time: all its lanes', or, where lanes
+        // share the rows' ids, fewer while that keeps every warp busy
+        const int take = t.g.slot != nullptr ? 32 : min(32, max(4, (cnt + NW - 1) / NW));
+        auto alloc = [&](int k) {
+            int p = 0;
+            if (lane == 0) p = atomicAdd(tailp, k);
+            return end + __shfl_sync(0xffffffffu, p, 0);
+        };
+        int nh = 0;
+        int base = wid * take;   // the first one by position, the others by demand
+        while (base < cnt) {
+            const int32_t v = (lane < take && base + lane < cnt) ? fr_get(t.f, start + base + lane, wstart) : -1;
+            nh += expand<CG, GBM>(t, v, s, cidx, start, acc, alloc);
+            if (cnt <= NW * take) break;
+            if (lane == 0) base = atomicAdd(fetchp, take);
+            base = __shfl_sync(0xffffffffu, base, 0) + NW * take;
+        }
+        if (lane == 0 && nh) atomicAdd(&sh.nh, nh);
         gsync<GT>(bar);
-        int end;
-        if (relay) {
-            start = sh.solo_start;
-            wstart = sh.solo_wstart;
-            end = start + sh.solo_count;
-            relay = false;
-        } else {
-            end = start + sh.tailc[c % 3];
-        }
-        if (end == start) break;
-        const bool solo = lanes == 1 && end - start <= 32;
-        if (solo && tid >= 32) {
-            relay = true;
-            continue;
-        }
-        if (tid == 0) prof[0]++;   // levels
-        if (!solo && tid == 0) { sh.tailc[(c + 2) % 3] = 0; sh.fetch[(c + 1) % 3] = 0; }
-        int *const tailp = solo ? &sh.stail : &sh.tailc[(c + 1) % 3];
-        int *const fetchp = &sh.fetch[c % 3];
-        if (lanes == 1) {
-            // a warp takes 32 queue items with one shared atomic; solo, warp
-            // 0 takes the whole level, then the next while it is small
-            for (;;) {
-                int base = start;
-                if (solo) {
-                    if (lane == 0) sh.stail = 0;
-                } else {
-                    if (lane == 0) base = atomicAdd(fetchp, 32);
-                    base = __shfl_sync(0xffffffffu, base, 0) + start;
-                    if (base >= end) break;
-                }
-                warp_step(base, start, end, wstart, tailp);
-                if (solo) {
-                    __syncwarp();   // the level's queue entries, for every lane
-                    int nn = 0;
-                    if (lane == 0) nn = sh.stail;
-                    nn = __shfl_sync(0xffffffffu, nn, 0);
-                    wstart = start;
-                    start = end;
-                    end += nn;
-                    if (nn == 0 || nn > 32) {
-                        if (lane == 0) {
-                            sh.solo_start = start;
-                            sh.solo_wstart = wstart;
-                            sh.solo_count = nn;
-                        }
-                        break;
-                    }
-                    if (lane == 0) prof[0]++;
-                }
-            }
-            if (solo) {
-                relay = true;
-                continue;
-            }
-        } else {
-            // groups of `lanes` threads per vertex
-            const unsigned gmask = (lanes == 32)
-                                       ? 0xffffffffu
-                                       : (((1u << lanes) - 1u) << (lane & ~(lanes - 1)));
-            int nh = 0;
-            for (;;) {
-                int it = 0;
-                if (lane_in_group == 0) it = atomicAdd(fetchp, 1);
-                it = __shfl_sync(gmask, it, 0, lanes) + start;
-                if (it >= end) break;
-                const int32_t v = fr_get(f, it, wstart);
-                const int32_t b = ld<CG>(g.ptr + v), e = ld<CG>(g.ptr + v + 1);
-                if (lane_in_group == 0) {
-                    edges += (unsigned long long)(e - b);
-                    if (pass == 0) { xcnt++; einsp += (unsigned long long)ld<CG>(rawdeg + v); }
-                }
-                for (int32_t k = b + lane_in_group; k < e; k += lanes) GSOFA_VISIT(ld<CG>(g.adj + k));
-            }
-            nh = (int)__reduce_add_sync(0xffffffffu, (unsigned)nh);
-            if (lane == 0 && nh) atomicAdd(&sh.hcount, nh);
-        }
+        const int nn = sh.tailc[phase];
+        nlev++;
         wstart = start;
         start = end;
-        c++;
+        end += nn;
+        const int next = phase == 2 ? 0 : phase + 1;
+        if (gtid == 0) {
+            const int clr = next == 2 ? 0 : next + 1;
+            sh.tailc[clr] = 0;
+            sh.fetch[clr] = 0;
+        }
+        phase = next;
+        if (nn <= SOLO_MAX) break;
     }
-    long long ce = 0;
-    if (tid == 0) { ce = clock64(); prof[2] += (unsigned long long)(ce - cs); }
+    if (gtid == 0) {   // for the leader's own lanes
+        sh.lv_start = start;
+        sh.lv_end = end;
+        sh.lv_wstart = wstart;
+        sh.prof[0] += (unsigned long long)nlev;
+    }
+}
 
-    // fold the touched range into the chain range (warp reduce + shared
-    // atomics; it is read only when the bitmap is cleared, after later
-    // barriers)
-    {
-        const int wl = __reduce_min_sync(0xffffffffu, t_lo);
-        const int wh = __reduce_max_sync(0xffffffffu, t_hi);
-        if (lane == 0) {
-            if (wl != INT32_MAX) atomicMin(&sh.chain_lo, wl);
-            if (wh >= 0) atomicMax(&sh.chain_hi, wh);
+// Warps wid, wid + nw, ... clear the nonzero chunks of a traversal's bitmap and
+// their summaries.  The summaries say where the set bits are, so a state that
+// touches a few stretches of a large matrix costs those stretches only.
+template <bool GBM>
+__device__ __forceinline__ void clear_state(uint32_t *bm, uint32_t *summ, int wid, int nw, int lane)
+{
+    const int sw = bm_summary_words(bm, summ);
+    uint32_t *summ2 = summ + sw;
+    for (int i = wid; i < (sw + 31) >> 5; i += nw) {
+        uint32_t m = bm_word<GBM>(summ2 + i);
+        if (m == 0u) continue;
+        for (; m; m &= m - 1u) bm[(((i << 5) + __ffs(m) - 1) << 5) + lane] = 0u;
+        if ((i << 5) + lane < sw) summ[(i << 5) + lane] = 0u;
+        if (lane == 0) summ2[i] = 0u;
+    }
+}
+
+// All threads of a traversal copy bitmap words [lo, hi) into a snapshot.
+template <int GT, bool GBM>
+__device__ __forceinline__ void save_state(const uint32_t *bm, uint32_t *snap, int lo, int hi, int gtid)
+{
+    const uint4 *src = reinterpret_cast<const uint4 *>(bm);
+    uint4 *dst = reinterpret_cast<uint4 *>(snap);
+    for (int i = (lo >> 2) + gtid; i < (hi >> 2); i += GT) dst[i] = GBM ? __ldcg(src + i) : src[i];
+}
+
+// All threads of a traversal add the snapshot of source st (words [lo, hi)) to
+// the bitmap of source s, st < s: the new vertices between the two join the
+// first level (they were above st, so nothing was expanded from them), those
+// above s are counted in sh.nh.
+template <int GT, bool GBM>
+__device__ __forceinline__ void merge_state(const Trav &t, const uint32_t *snap, int lo, int hi, int st, int s, int cidx,
+                                            SharedState &sh, int gtid)
+{
+    const int lane = gtid & 31;
+    const uint4 *src = reinterpret_cast<const uint4 *>(snap);
+    uint4 *dst = reinterpret_cast<uint4 *>(t.bm);
+    const int ws = s >> 5;
+    const uint32_t above_s = ~1u << (s & 31);   // in word ws
+    int cnt = 0;
+    const int hi4 = hi >> 2;
+    for (int i0 = lo >> 2; i0 < hi4; i0 += GT) {   // warp-uniform trips
+        const int i = i0 + gtid;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u), c = v;
+        if (i < hi4) {
+            v = __ldcg(src + i);
+            c = GBM ? __ldcg(dst + i) : dst[i];
+        }
+        const uint32_t nb[4] = {v.x & ~c.x, v.y & ~c.y, v.z & ~c.z, v.w & ~c.w};
+        const uint32_t old[4] = {c.x, c.y, c.z, c.w};
+        if (nb[0] | nb[1] | nb[2] | nb[3]) {
+            dst[i] = make_uint4(c.x | v.x, c.y | v.y, c.z | v.z, c.w | v.w);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int w = 4 * i + q;
+                if (nb[q] == 0u) continue;
+                if (old[q] == 0u) mark_word(t.bm, t.summ, w);
+                cnt += w > ws ? __popc(nb[q]) : (w == ws ? __popc(nb[q] & above_s) : 0);
+                if (w <= ws && w >= (st >> 5)) {   // the few words between the two sources
+                    uint32_t x = nb[q];
+                    if (w == ws) x &= (1u << (s & 31)) - 1u;
+                    if (w == (st >> 5)) x &= ~1u << (st & 31);
+                    for (; x; x &= x - 1u) fr_put(t.f, atomicAdd(&sh.npush, 1), 0, (w << 5) + __ffs(x) - 1);
+                }
+            }
+        }
+        if (t.stamp != nullptr) {   // a word at a time across the warp (lane = bit)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                unsigned any = __ballot_sync(0xffffffffu, nb[q] != 0u);
+                for (; any; any &= any - 1u) {
+                    const int j = __ffs(any) - 1;
+                    const uint32_t x = __shfl_sync(0xffffffffu, nb[q], j);
+                    const int32_t m = ((4 * (i - lane + j) + q) << 5) + lane;
+                    if (((x >> lane) & 1u) && m > s - cidx) t.stamp[m] = (uint16_t)cidx;
+                }
+            }
         }
     }
-    long long c1 = 0;
-    if (tid == 0) { c1 = clock64(); prof[3] += (unsigned long long)(c1 - ce); }
-
-    // |hi(s)| = the bits above s: the traversal's running count, complete
-    // since the level loop's last barrier.  The lists themselves are written
-    // when the chain ends (output_chain); here only the count and the link
-    // flag.
-    if (tid == 0) {
-        // the next source starts from zeroed level counters (every thread
-        // read this one's last, empty level before leaving the loop; the
-        // counters of that level are zero already)
-        sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
-        sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
-        const int total = sh.hcount;
-        const int64_t slot = (int64_t)pass * a.L + line;
-        a.cnt[slot] = (int32_t)total;
-        const int nx = (s + 1 < n) && ((bm_word<GBM>(bm + ((s + 1) >> 5)) >> ((s + 1) & 31)) & 1u);
-        a.nxt[slot] = (uint8_t)nx;
-        sh.flag = nx;
-        sh.chain_total += total;
-    }
-    if (END_SYNC) gsync<GT>(bar);
-    if (tid == 0) prof[4] += (unsigned long long)(clock64() - c1);
+    cnt = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+    if (lane == 0 && cnt) atomicAdd(&sh.nh, cnt);
 }
-#undef GSOFA_VISIT
 
 // Lane's bitmap word of chunk cc, without the bits below word w0 and below
 // first_mask in word w0.
@@ -1010,85 +944,362 @@ __device__ void output_chain(const JobArgs &a, int64_t line_base, int pass, cons
     }
 }
 
-// Per-thread tallies of one CTA's traversals (summed over the CTA at the
-// end); the per-source ones live in SharedState, kept by one thread.
-struct Tally {
-    unsigned long long edges = 0, xcnt = 0, einsp = 0;
-};
+// One op of the leader's, run by all threads of the traversal after its
+// barrier.
+template <int GT, bool CG, bool GBM, bool LISTS>
+__device__ __forceinline__ void run_op(const JobArgs &a, int64_t line_base, const Trav &t, SharedState &sh, int op,
+                                       int gtid, int bar, int &phase, Tally &acc)
+{
+    if (op == OP_LEVELS) {
+        run_levels<GT, CG, GBM>(t, sh, gtid, bar, phase, acc);
+        return;
+    }
+    if (op == OP_CLEAR) {
+        clear_state<GBM>(t.bm, t.summ, gtid >> 5, GT / 32, gtid & 31);
+    } else if (op == OP_SAVE) {
+        save_state<GT, GBM>(t.bm, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, gtid);
+    } else if (op == OP_MERGE) {
+        merge_state<GT, GBM>(t, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, sh.t, sh.src, sh.cidx, sh,
+                             gtid);
+    } else if (LISTS && op == OP_LISTS) {
+        output_chain<GT, GBM>(a, line_base, t.pass, t.bm, t.summ, sh, t.f.spill, gtid, bar);
+    }
+    gsync<GT>(bar);
+}
+
+// Nonzero stretch of a bitmap as words [lo, hi), whole chunks, and its number
+// of nonzero chunks; one warp.
+template <bool GBM>
+__device__ __forceinline__ int state_extent(const uint32_t *bm, const uint32_t *summ, int lane, int &lo, int &hi)
+{
+    const int sw = bm_summary_words(bm, summ);
+    int first = INT32_MAX, last = -1, chunks = 0;
+    for (int i = lane; i < (sw + 31) >> 5; i += 32) {
+        const uint32_t m = bm_word<GBM>(summ + sw + i);
+        if (m) {
+            first = min(first, (i << 5) + __ffs(m) - 1);
+            last = (i << 5) + 31 - __clz(m);
+            chunks += __popc(m);
+        }
+    }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    lo = last < 0 ? 0 : first << 5;
+    hi = (last + 1) << 5;
+    return (int)__reduce_add_sync(0xffffffffu, (unsigned)chunks);
+}
 
 // The sources s_lo, s_lo + stride, ... < s_hi of one work piece, in order,
 // each starting from the previous source's state whenever that is valid.
+//
+// A traversal's first warp, its leader, runs the sources by itself: nine of
+// ten on nested-dissection matrices add no vertex below the source and need no
+// other warp.  The other warps wait at the traversal's barrier and join only
+// for large steps: a level of more than 32 vertices (and the levels after it
+// while they stay large), clearing or copying a wide bitmap, a chain's list
+// output.  With all warps at a barrier two or three times a source, the 80^3
+// counts spent 4,600 cycles a source and pass.
+//
+// PAIRED: the leaders of the two passes exchange "s+1 reached" flags after
+// every source (pair_sync).  s-1 is in X_G(s) exactly when s is in
+// hi_{G^T}(s-1), and then X(s-1) u {s-1} is inside X(s) and hi(s-1) minus {s}
+// inside hi(s), so the bitmap can be kept.  The same holds for every earlier
+// source t: when s is in hi_{G^T}(t), the state that pass G had after t is
+// inside that of s.  States that took a long traversal to build are copied to
+// global memory (snapshots, the SNAP_MAX latest of a piece) with the other
+// pass's bits for the sources after t, and each later source takes over the
+// snapshots that it provably contains.  On power-law matrices nearly half of
+// the sources do not contain s-1 but do contain some t a few lines below, whose
+// closure is most of the matrix: the 20,000-line one inspects 2.4e7 edges
+// instead of 2.7e8.  Where snapshots are saved but not taken over (meshes),
+// the piece's CTA stops saving them.
 template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
-__device__ void run_piece(const JobArgs &a, const MatDesc &md, const PassGraph &g, int pass,
-                          int32_t s_lo, int32_t s_hi, int32_t stride, uint32_t *bm, uint32_t *summ,
-                          const Frontier &fr, SharedState &sh, int (*pair_flag)[2], int half,
-                          int gtid, int bar, Tally &acc)
+__device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, int32_t s_lo, int32_t s_hi,
+                           int32_t stride, SharedState *shs, volatile int (*pair_flag)[2], int half, int bar,
+                           int &phase, int &snap_credit, Tally &acc)
 {
     constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
-    const int tid = threadIdx.x;
-    int prev = -2;
-    int idx = 0;
-    // the current chain, tracked by every thread alike (decisions never read
-    // state another thread may be changing): index of the last source in it
-    // (-1: none yet)
-    int cidx = -1;
+    constexpr int NW = GT / 32;
+    SharedState &sh = shs[half];
+    const int lane = threadIdx.x & 31;
+    const int pass = t.pass;
+    const int nsnap = PAIRED ? a.snap_k : 0;
+    auto collective = [&](int op) {   // arguments are in place
+        if (lane == 0) sh.op = op;
+        __syncwarp();
+        gsync<GT>(bar);
+        run_op<GT, CG, GBM, LISTS>(a, md.line_base, t, sh, op, lane, bar, phase, acc);
+        __syncwarp();
+    };
+    auto take_nh = [&]() {   // what the last op counted
+        const int v = sh.nh;
+        __syncwarp();
+        if (lane == 0) sh.nh = 0;
+        return v;
+    };
+    unsigned long long n_levels = 0, n_src = 0, n_reuse = 0, cy_lev = 0, cy_lists = 0, cy_clear = 0, cy_snap = 0,
+                       cy_wait = 0;
+    const long long c_begin = clock64();
+
+    int prev = -2, idx = 0;
+    int cidx = -1;            // index of the last source in its chain (-1: none yet)
+    int hc = 0;               // set bits above the last source
+    int other = 0;            // the other pass reached s
+    long long total = 0;      // entries of the chain's lists
+    // the seeding window: lane i holds row bounds and degree of source wlo + i
+    int wlo = 0, whi = 0, wb = 0, we = 0, wraw = 0, wadj0 = 0;
+    // snapshots: lane k < nsnap holds slot k's source (-1: empty), words and weight
+    int sn_t = -1, sn_lo = 0, sn_hi = 0, sn_w = 0, sn_next = 0;
+    int weight = 0;           // vertices below the source in the state's traversals
+    const int heavy = max(64, a.bitmap_words >> 3);   // worth a copy of the bitmap
+
+    auto end_chain = [&]() {
+        int lo, hi;
+        if (LISTS && a.want_pattern && cidx >= 0) {
+            const long long c0 = clock64();
+            state_extent<GBM>(t.bm, t.summ, lane, lo, hi);
+            if (lane == 0) {
+                sh.chain_s0 = prev - cidx;
+                sh.chain_len = cidx + 1;
+                sh.chain_total = total;
+                sh.chain_hi = min(hi << 5, md.n) - 1;
+            }
+            collective(OP_LISTS);
+            cy_lists += (unsigned long long)(clock64() - c0);
+        }
+        const long long c0 = clock64();
+        const int chunks = state_extent<GBM>(t.bm, t.summ, lane, lo, hi);
+        if (NW == 1 || chunks <= 48) {
+            clear_state<GBM>(t.bm, t.summ, 0, 1, lane);
+            __syncwarp();
+            if (GBM) __threadfence_block();
+        } else {
+            collective(OP_CLEAR);
+        }
+        cy_clear += (unsigned long long)(clock64() - c0);
+    };
+
     for (int32_t s = s_lo; s < s_hi; s += stride, idx++) {
-        int reuse = 0;
-        // chain indices are 16-bit stamps: a chain ends after 65535 sources
+        // a new seeding window when s is past the current one (consecutive
+        // sources only): row bounds, then the rows themselves
+        if (stride == 1 && s >= whi) {
+            const int cnt = min(s_hi - s, SEED_WIN);
+            const int i = min(lane, cnt - 1);
+            wb = ld<CG>(t.g.ptr + s + i);
+            we = ld<CG>(t.g.ptr + s + i + 1);
+            if (pass == 0) wraw = ld<CG>(t.rawdeg + s + i);
+            wadj0 = __shfl_sync(0xffffffffu, wb, 0);
+            const int k = __popc(__ballot_sync(0xffffffffu, lane < cnt && we - wadj0 <= SEED_ADJ));   // rows that fit
+            const int na = k ? __shfl_sync(0xffffffffu, we, k - 1) - wadj0 : 0;
+            __syncwarp();
+            for (int q = lane; q < na; q += 32) sh.win_adj[q] = ld<CG>(t.g.adj + wadj0 + q);
+            __syncwarp();
+            wlo = s;
+            whi = s + k;   // k == 0: a row too long for the window, read where it lies
+        }
+        const bool in_win = stride == 1 && s < whi;
+        int32_t b0, d0;
+        if (in_win) {
+            b0 = __shfl_sync(0xffffffffu, wb, s - wlo);
+            d0 = __shfl_sync(0xffffffffu, we, s - wlo) - b0;
+        } else {
+            b0 = ld<CG>(t.g.ptr + s);
+            d0 = ld<CG>(t.g.ptr + s + 1) - b0;
+        }
+
+        // take over the previous source's state, or end its chain; chain
+        // indices are 16-bit stamps: a chain ends after 65535 sources
+        bool reuse = false;
         if (a.reuse && prev == s - 1 && !(a.want_pattern && cidx + 1 >= 65535)) {
             if (PAIRED) {
-                reuse = pair_flag[(idx - 1) & 1][1 - half];
+                reuse = other != 0;
             } else {
-                if (tid < 32) {
-                    const bool h = warp_has_prev(g, s);
-                    if (tid == 0) sh.flag = h ? 1 : 0;
-                }
-                __syncthreads();
-                reuse = sh.flag;
+                bool hit = false;
+                for (int k = lane; k < d0; k += 32)
+                    hit |= (in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(t.g.adj + b0 + k)) == s - 1;
+                reuse = __any_sync(0xffffffffu, hit);
             }
         }
-        if (!reuse) {
-            if (LISTS && a.want_pattern && cidx >= 0) {
-                const long long co = clock64();
-                output_chain<GT, GBM>(a, md.line_base, pass, bm, summ, sh, fr.spill, gtid, bar);
-                if (gtid == 0) sh.prof[5] += (unsigned long long)(clock64() - co);
-            }
-            const long long cc = clock64();
-            const int clo = sh.chain_lo, chi = sh.chain_hi;
-            clear_range<GT>(bm, summ, clo, chi, gtid);
-            // the new chain's counters, in place before the barrier that
-            // precedes its first seeding (which adds to hcount)
-            if (gtid == 0) { sh.hcount = 0; sh.chain_s0 = s; sh.chain_len = 0; sh.chain_total = 0; }
-            gsync<GT>(bar);
-            if (gtid == 0) {
-                sh.chain_lo = INT32_MAX; sh.chain_hi = -1;
-                sh.prof[6] += (unsigned long long)(clock64() - cc);
-            }
-            cidx = 0;
-        } else {
+        if (reuse) {
             cidx++;
-            if (gtid == 0) sh.nreuse++;
+            n_reuse++;
+        } else {
+            if (cidx >= 0) end_chain();
+            cidx = 0;
+            hc = 0;
+            total = 0;
+            weight = 0;
         }
-        // paired: the pass-flag exchange below is a barrier of the whole CTA
-        process_source<GT, CG, !PAIRED, GBM>(a, g, md.n, md.line_base + s, pass, s, s_hi, stride, cidx,
-                                             bm, summ, fr, sh, acc.edges, md.rawdeg, acc.xcnt, acc.einsp,
-                                             sh.prof, gtid, bar);
-        if (PAIRED) {
-            if (gtid == 0) pair_flag[idx & 1][half] = sh.flag;
-            const long long cw = clock64();
-            __syncthreads();
-            if (gtid == 0) sh.prof[7] += (unsigned long long)(clock64() - cw);
+
+        // Seeding: s itself and its neighbours; those below s are the first
+        // level.  nh counts new vertices above s, and s when it is new: a
+        // source that was set already was counted by the sources before it.
+        int tail = 0, nh = 0;
+        bool self = false;   // s is set
+        auto alloc = [&](int k) { const int p = tail; tail += k; return p; };
+        if (lane == 0) acc.edges += (unsigned)d0;
+        if (pass == 0) {
+            const int r = in_win ? __shfl_sync(0xffffffffu, wraw, s - wlo) : ld<CG>(t.rawdeg + s);
+            if (lane == 0) acc.einsp += (unsigned)r;
+        }
+        if (nsnap > 0 && __any_sync(0xffffffffu, sn_t >= 0)) {
+            // the newest snapshot that s contains and its state does not yet,
+            // until there is none (bit t set: t and all of its state are in)
+            for (;;) {
+                bool use = false;
+                if (lane < nsnap && sn_t >= 0) {
+                    const int w = (s >> 5) - (sn_t >> 5);
+                    use = w < SNAP_REACH && ((sh.snap_reach[lane][w] >> (s & 31)) & 1u) &&
+                          !((bm_word<GBM>(t.bm + (sn_t >> 5)) >> (sn_t & 31)) & 1u);
+                }
+                const int best = __reduce_max_sync(0xffffffffu, use ? sn_t : -1);
+                if (best < 0) break;
+                const long long c0 = clock64();
+                if (!self) {   // before the merge, which leaves it out
+                    const int32_t m[1] = {lane == 0 ? s : -1};
+                    nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
+                    self = true;
+                }
+                const int k = __ffs(__ballot_sync(0xffffffffu, use && sn_t == best)) - 1;
+                const int lo = __shfl_sync(0xffffffffu, sn_lo, k), hi = __shfl_sync(0xffffffffu, sn_hi, k);
+                weight += __shfl_sync(0xffffffffu, sn_w, k);
+                if (lane == 0) {
+                    sh.src = s;
+                    sh.cidx = cidx;
+                    sh.snap = k;
+                    sh.t = best;
+                    sh.lo = lo;
+                    sh.hi = hi;
+                    sh.npush = tail;
+                }
+                collective(OP_MERGE);
+                tail = sh.npush;
+                nh += take_nh();
+                snap_credit += 8;
+                cy_snap += (unsigned long long)(clock64() - c0);
+            }
+        }
+        {
+            auto id = [&](int k) { return in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(t.g.adj + b0 + k); };
+            const int32_t m[1] = {lane == 31 ? (self ? -1 : s) : (lane < d0 ? id(lane) : -1)};
+            nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
+            for (int k0 = 31; k0 < d0; k0 += 128) {
+                int32_t x[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) x[u] = k0 + 32 * u + lane < d0 ? id(k0 + 32 * u + lane) : -1;
+                nh += visit<4, GBM>(t, x, s, cidx, 0, alloc);
+            }
+        }
+
+        // level-synchronous expansion through vertices < s
+        int start = 0, end = tail, wstart = 0;
+        if (end > 0) {
+            const long long c0 = clock64();
+            do {
+                if (NW == 1 || end - start <= SOLO_MAX) {
+                    __syncwarp();   // the level's queue entries, for every lane
+                    n_levels++;
+                    for (int base = start; base < end; base += 32) {
+                        const int32_t v = base + lane < end ? fr_get(t.f, base + lane, wstart) : -1;
+                        nh += expand<CG, GBM>(t, v, s, cidx, start, acc, alloc);
+                    }
+                    wstart = start;
+                    start = end;
+                    end = tail;
+                } else {
+                    if (lane == 0) {
+                        sh.src = s;
+                        sh.cidx = cidx;
+                        sh.lv_start = start;
+                        sh.lv_end = end;
+                        sh.lv_wstart = wstart;
+                    }
+                    collective(OP_LEVELS);
+                    start = sh.lv_start;
+                    end = sh.lv_end;
+                    wstart = sh.lv_wstart;
+                    tail = end;
+                    nh += take_nh();
+                }
+            } while (end > start);
+            cy_lev += (unsigned long long)(clock64() - c0);
+        }
+
+        // |hi(s)|: the bits above s; the link flag; both passes' exchange
+        hc += nh - 1;
+        total += hc;
+        weight += end;
+        n_src++;
+        __syncwarp();
+        const int nx = s + 1 < md.n ? (int)((bm_word<GBM>(t.bm + ((s + 1) >> 5)) >> ((s + 1) & 31)) & 1u) : 0;
+        if (lane == 0) {
+            const int64_t slot = (int64_t)pass * a.L + md.line_base + s;
+            a.cnt[slot] = hc;
+            a.nxt[slot] = (uint8_t)nx;
         }
         prev = s;
-        if (gtid == 0) sh.nsrc++;
+        if (PAIRED) {
+            const int par = idx & 1;
+            if (lane == 0) pair_flag[par][half] = nx;
+            if (nsnap > 0 && lane < SNAP_REACH)
+                sh.reach[par][lane] = (s >> 5) + lane < a.bitmap_words ? bm_word<GBM>(t.bm + (s >> 5) + lane) : 0u;
+            if ((idx & 15) == 0) {   // the wait, sampled
+                const long long c0 = clock64();
+                pair_sync();
+                cy_wait += 16ull * (unsigned long long)(clock64() - c0);
+            } else {
+                pair_sync();
+            }
+            other = pair_flag[par][1 - half];
+            if (nsnap > 0 && end > 0 && weight >= heavy && snap_credit > 0) {
+                const long long c0 = clock64();
+                int lo, hi;
+                state_extent<GBM>(t.bm, t.summ, lane, lo, hi);
+                const int k = sn_next;
+                sn_next = k + 1 == nsnap ? 0 : k + 1;
+                if (lane == k) { sn_t = s; sn_lo = lo; sn_hi = hi; sn_w = weight; }
+                if (lane < SNAP_REACH) sh.snap_reach[k][lane] = shs[1 - half].reach[par][lane];
+                if (lane == 0) { sh.snap = k; sh.lo = lo; sh.hi = hi; }
+                collective(OP_SAVE);
+                snap_credit--;
+                cy_snap += (unsigned long long)(clock64() - c0);
+            }
+        }
     }
-    // the piece's last chain
-    if (LISTS && a.want_pattern && cidx >= 0) {
-        const long long co = clock64();
-        output_chain<GT, GBM>(a, md.line_base, pass, bm, summ, sh, fr.spill, gtid, bar);
-        if (gtid == 0) {
-            sh.prof[5] += (unsigned long long)(clock64() - co);
-            sh.chain_len = 0;
+    if (cidx >= 0) end_chain();   // the next piece starts from an empty bitmap
+    if (lane == 0) {
+        sh.nsrc += n_src;
+        sh.nreuse += n_reuse;
+        sh.prof[0] += n_levels;
+        sh.prof[1] += (unsigned long long)(clock64() - c_begin) - cy_lev - cy_lists - cy_clear - cy_snap - cy_wait;
+        sh.prof[2] += cy_lev;
+        sh.prof[3] += cy_snap;
+        sh.prof[5] += cy_lists;
+        sh.prof[6] += cy_clear;
+        sh.prof[7] += cy_wait;
+        sh.op = OP_EXIT;
+    }
+    __syncwarp();
+    gsync<GT>(bar);
+}
+
+// One work piece: the first warp of every traversal leads, the others help.
+template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
+__device__ __forceinline__ void run_piece(const JobArgs &a, const MatDesc &md, const Trav &t, int32_t s_lo,
+                                          int32_t s_hi, int32_t stride, SharedState *shs,
+                                          volatile int (*pair_flag)[2], int half, int gtid, int bar, int &phase,
+                                          int &snap_credit, Tally &acc)
+{
+    constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
+    if (gtid < 32) {
+        lead_piece<BLOCK, PAIRED, CG, GBM, LISTS>(a, md, t, s_lo, s_hi, stride, shs, pair_flag, half, bar, phase,
+                                                  snap_credit, acc);
+    } else {
+        for (;;) {
+            gsync<GT>(bar);
+            const int op = shs[half].op;
+            if (op == OP_EXIT) break;
+            run_op<GT, CG, GBM, LISTS>(a, md.line_base, t, shs[half], op, gtid, bar, phase, acc);
         }
     }
 }
@@ -1123,14 +1334,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
     constexpr int NS = PAIRED ? 2 : 1;
     extern __shared__ __align__(16) uint32_t smem_dyn[];
     __shared__ SharedState shs[NS];
-    __shared__ int pair_flag[2][2];   // [source parity][pass]: s+1 in hi(s)
+    __shared__ volatile int pair_flag[2][2];   // [source parity][pass]: s+1 in hi(s)
     __shared__ long long s_piece;
     cg::grid_group grid = cg::this_grid();
     const int tid = threadIdx.x;
     const int half = PAIRED ? tid / GT : 0;
     const int gtid = PAIRED ? tid % GT : tid;
-    const int bar = PAIRED ? 1 + half : 0;
+    const int bar = 1 + half;
     SharedState &sh = shs[half];
+    const int64_t trav = (int64_t)blockIdx.x * NS + half;
     uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * NS) * a.state_words : smem_dyn;
     uint32_t *bm = state + (size_t)half * a.state_words;
     uint32_t *summ = bm + a.bitmap_words;
@@ -1140,19 +1352,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
     unsigned long long t_start = 0;
     if (tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
     for (int w = tid; w < NS * a.state_words; w += BLOCK) state[w] = 0u;
-    if (gtid == 0) {
-        sh.chain_lo = INT32_MAX; sh.chain_hi = -1; sh.hcount = 0;
-        sh.stamp = a.want_pattern ? a.stamp + ((int64_t)blockIdx.x * NS + half) * a.stamp_stride : nullptr;
-        sh.chain_s0 = 0; sh.chain_len = 0; sh.chain_total = 0;
-        for (int q = 0; q < 8; q++) sh.prof[q] = 0;
-        sh.nsrc = sh.nreuse = 0;
-        sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
-        sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
-        sh.win_lo = sh.win_hi = 0;
-    }
-    const Frontier fr{ring, a.queue + ((int64_t)blockIdx.x * NS + half) * a.qcap, a.qcap, a.status,
-                      a.ring_size};
+    if (gtid == 0) init_state(sh);
+    Trav t{};
+    t.bm = bm;
+    t.summ = summ;
+    t.f = Frontier{ring, a.queue + trav * a.qcap, a.qcap, a.status, a.ring_size};
+    t.stamp = LISTS && a.want_pattern ? a.stamp + trav * a.stamp_stride : nullptr;
+    t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
+    if (gtid == 0) sh.stamp = t.stamp;
     Tally acc;
+    int phase = 0, snap_credit = SNAP_CREDIT, last_mat = -1;
     __syncthreads();
     for (;;) {
         if (tid == 0) s_piece = (long long)atomicAdd(a.piece_counter, 1ull);
@@ -1190,17 +1399,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
             s_lo = sh.seg[0];
             s_hi = sh.seg[1];
         }
-        run_piece<BLOCK, PAIRED, false, GBM, LISTS>(a, md, g, pass, s_lo, s_hi, rg.stride, bm, summ, fr, sh, pair_flag,
-                                        half, gtid, bar, acc);
-        // the next piece starts from an empty bitmap
-        {
-            const int clo = sh.chain_lo, chi = sh.chain_hi;
-            clear_range<GT>(bm, summ, clo, chi, gtid);
-            __syncthreads();
-            // the next piece may be another matrix: no seeding window yet
-            if (gtid == 0) { sh.chain_lo = INT32_MAX; sh.chain_hi = -1; sh.hcount = 0; sh.win_lo = sh.win_hi = 0; }
-            __syncthreads();
-        }
+        if (rg.mat != last_mat) snap_credit = SNAP_CREDIT;
+        last_mat = rg.mat;
+        t.g = g;
+        t.rawdeg = md.rawdeg;
+        t.pass = pass;
+        run_piece<BLOCK, PAIRED, false, GBM, LISTS>(a, md, t, s_lo, s_hi, rg.stride, shs, pair_flag, half, gtid, bar,
+                                                    phase, snap_credit, acc);
+        __syncthreads();   // every thread is done with s_piece
     }
     {
         if (tid == 0) {   // this CTA's busy time, summed over CTAs (load balance)

@@ -73,7 +73,7 @@ __global__ void __maxnreg__(64) serve_kernel(ServeArgs sa)
     const JobArgs &a = sa.job;
     extern __shared__ __align__(16) uint32_t smem_dyn[];
     __shared__ SharedState shs[2];
-    __shared__ int pair_flag[2][2];
+    __shared__ volatile int pair_flag[2][2];
     __shared__ long long s_piece;
     const int tid = threadIdx.x;
     const int half = tid / GT;
@@ -85,19 +85,16 @@ __global__ void __maxnreg__(64) serve_kernel(ServeArgs sa)
     uint32_t *summ = bm + a.bitmap_words;
     int32_t *ring = (int32_t *)(GBM ? smem_dyn : smem_dyn + (size_t)2 * a.state_words) + (size_t)half * a.ring_size;
     for (int w = tid; w < 2 * a.state_words; w += BLOCK) state[w] = 0u;
-    if (gtid == 0) {
-        sh.chain_lo = INT32_MAX; sh.chain_hi = -1; sh.hcount = 0;
-        sh.stamp = nullptr;   // counts only: no lists, no stamps
-        sh.chain_s0 = 0; sh.chain_len = 0; sh.chain_total = 0;
-        for (int q = 0; q < 8; q++) sh.prof[q] = 0;
-        sh.nsrc = sh.nreuse = 0;
-        sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
-        sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
-        sh.win_lo = sh.win_hi = 0;
-    }
-    const Frontier fr{ring, a.queue + ((int64_t)blockIdx.x * 2 + half) * a.qcap, a.qcap, a.status,
-                      a.ring_size};
+    if (gtid == 0) init_state(sh);   // counts only: no lists, no stamps
+    const int64_t trav = (int64_t)blockIdx.x * 2 + half;
+    Trav t{};
+    t.bm = bm;
+    t.summ = summ;
+    t.f = Frontier{ring, a.queue + trav * a.qcap, a.qcap, a.status, a.ring_size};
+    t.stamp = nullptr;
+    t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
     Tally acc;
+    int phase = 0, snap_credit = SNAP_CREDIT;
     __shared__ int s_class;
     __syncthreads();
     for (;;) {
@@ -128,15 +125,13 @@ __global__ void __maxnreg__(64) serve_kernel(ServeArgs sa)
         const ServePiece piece =
             load_cg(sa.pieces + (unsigned long long)s_class * sa.piece_cap + (pc % (long long)sa.piece_cap));
         const MatDesc md = load_cg(sa.slots + piece.slot);
-        run_piece<BLOCK, true, true, GBM, false>(a, md, md.g[half], half, piece.s_lo, piece.s_hi, 1, bm, summ, fr, sh,
-                                     pair_flag, half, gtid, bar, acc);
-        {
-            const int clo = sh.chain_lo, chi = sh.chain_hi;
-            clear_range<GT>(bm, summ, clo, chi, gtid);
-            __syncthreads();
-            // the next piece may be another request: no seeding window yet
-            if (gtid == 0) { sh.chain_lo = INT32_MAX; sh.chain_hi = -1; sh.hcount = 0; sh.win_lo = sh.win_hi = 0; }
-        }
+        t.g = md.g[half];
+        t.rawdeg = md.rawdeg;
+        t.pass = half;
+        snap_credit = SNAP_CREDIT;   // the piece may be another request's
+        run_piece<BLOCK, true, true, GBM, false>(a, md, t, piece.s_lo, piece.s_hi, 1, shs, pair_flag, half, gtid, bar,
+                                                 phase, snap_credit, acc);
+        __syncthreads();
         if (tid == 0) {
             __threadfence();
             atomicAdd(sa.slot_done + piece.slot, 1u);

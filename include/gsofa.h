@@ -67,9 +67,9 @@ typedef struct gsofa_params {
                                    512, about eight pieces per resident CTA  */
     int32_t block_size;         /* threads per CTA: 128, 256, 512, 768 (the
                                    two passes side by side only) or 1024      */
-    int32_t threads_per_source; /* lanes expanding one frontier vertex:
-                                   1 (default: one thread per vertex, a warp
-                                   for rows longer than 32), 4, 8, 16 or 32   */
+    int32_t threads_per_source; /* 0, 1, 4, 8, 16 or 32; chooses nothing any
+                                   more (the lanes of a warp share its
+                                   vertices' rows by their lengths)           */
     int32_t ctas_per_sm;        /* resident CTAs per SM                       */
     int64_t queue_capacity;     /* frontier entries per CTA (>= n, else n)    */
     int64_t pool_capacity;      /* pattern entries kept on the device         */
@@ -143,11 +143,10 @@ typedef struct gsofa_result {
                                 duplicates included)                      */
     uint64_t levels;         /* frontier levels summed over the traversals  */
     uint64_t reused_sources; /* traversals that started from s-1's state    */
-    uint64_t cycles[7];      /* SM cycles summed over traversals: seeding,
-                                level loop, range fold, count and link
-                                flag, list output (once per chain of
-                                sources), bitmap clearing, waiting for the
-                                other pass                                  */
+    uint64_t cycles[7];      /* SM cycles summed over traversals: the
+                                sources' own steps, their levels, snapshots,
+                                (unused), list output, bitmap clearing,
+                                waiting for the other pass                */
     uint64_t ctas;           /* CTAs of the persistent launch               */
     double kernel_ms;        /* factorization kernel time on the device     */
     /* per-line arrays (host, library-owned; NULL with NO_DOWNLOAD) */
