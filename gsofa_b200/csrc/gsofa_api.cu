@@ -94,6 +94,7 @@ struct gsofa_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // job scratch
     DevBuf queue, cnt, nxt, poff, gptr, lrow, snind, snlist, tiles, misc, pool, out, mats, ranges, stamp;
+    DevBuf lists;             // list output: a chain's vertices, per traversal
     DevBuf snap;              // snapshots of finished traversals
     DevBuf gstate;            // visited bitmaps of the global-state kernels
     DevBuf blk;               // streaming: written entries per pool block
@@ -229,6 +230,15 @@ struct ExtPool {
     int64_t nblk = 0;
     std::function<void()> while_running;
 };
+
+// Static shared memory of the factorization kernel, with some slack: a
+// SharedState per traversal and, for the list output, a row of 32 counters per
+// helper warp.
+constexpr int kMinRing = 512;
+size_t static_shared(int block, int ns, bool lists)
+{
+    return sizeof(SharedState) * ns + (lists ? (size_t)(block / 32 - ns) * 128 : 0) + 512;
+}
 
 int pick_block(int32_t max_n)
 {
@@ -395,9 +405,9 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
     // paired kernel) up to ~850K lines and one up to ~1.7M; global memory
     // holds any number of any size.  GSOFA_FLAG_GLOBAL_STATE /
     // GSOFA_FLAG_SHARED_STATE choose; else shared memory while the pair fits.
-    const size_t pair_smem = (size_t)2 * state_needed * 4 + 2 * 1024 * 4 + sizeof(SharedState) * 2 + 1024;
+    const size_t pair_smem = (size_t)2 * state_needed * 4 + 2 * kMinRing * 4 + static_shared(768, 2, want_pattern);
     if ((p.flags & GSOFA_FLAG_GLOBAL_STATE) && (p.flags & GSOFA_FLAG_SHARED_STATE)) return GSOFA_ERR_INVALID_INPUT;
-    const size_t single_smem = (size_t)state_needed * 4 + 1024 * 4 + sizeof(SharedState) + 1024;
+    const size_t single_smem = (size_t)state_needed * 4 + kMinRing * 4 + static_shared(512, 1, want_pattern);
     const bool want_pair = reuse && p.reuse != 2;
     const bool gbm = (p.flags & GSOFA_FLAG_GLOBAL_STATE) ||
                      (!(p.flags & GSOFA_FLAG_SHARED_STATE) &&
@@ -435,12 +445,12 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
 
     const int32_t bitmap_words = words_needed;
     const int32_t state_words = state_needed;
-    const size_t static_smem = sizeof(SharedState) * NS + 1024;
+    const size_t static_smem = static_shared(block, NS, true);
     // shared memory per traversal: its bitmap and summaries (unless in global
     // memory) and its frontier ring
     const size_t smem_state = gbm ? 0 : (size_t)state_words * 4;
-    if ((size_t)NS * (smem_state + 1024 * 4) + static_smem > ctx->smem_optin) return GSOFA_ERR_UNSUPPORTED;
-    // frontier ring: the largest of 8K/4K/2K/1K entries that keeps the most
+    if ((size_t)NS * (smem_state + kMinRing * 4) + static_smem > ctx->smem_optin) return GSOFA_ERR_UNSUPPORTED;
+    // frontier ring: the largest of 8K down to 512 entries that keeps the most
     // CTAs (each with its own bitmap) resident on an SM; sized once per shape
     int ring = 0, occ = 0;
     size_t smem = 0;
@@ -454,7 +464,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         smem = (size_t)NS * (smem_state + (size_t)ring * 4);
     } else {
         std::lock_guard<std::mutex> lk(kernel_attr_mutex());
-        for (int cand = 8192; cand >= 1024; cand >>= 1) {
+        for (int cand = 8192; cand >= kMinRing; cand >>= 1) {
             const size_t sm = (size_t)NS * (smem_state + (size_t)cand * 4);
             if (sm + static_smem > ctx->smem_optin) continue;
             GS_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -471,17 +481,18 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         // Concurrent traversals within the memory budget (the reference
         // shrinks its sources per pass until the state fits its pool,
         // with_space_optimization/symbfact.cuh:1465-1507): every traversal
-        // holds a frontier queue of n entries and, with the pattern, a row of
-        // n chain stamps; the per-line arrays and a minimal pool come first.
+        // holds a frontier queue of n entries and, with the pattern, two rows
+        // of n chain stamps and n entries of list scratch; the per-line arrays
+        // and a minimal pool come first.
         const int64_t q = std::max<int64_t>(p.queue_capacity, max_n);
-        const int64_t per_cta = (int64_t)NS * (q * 4 + (want_pattern ? (int64_t)words_needed * 32 * 2 : 0) +
+        const int64_t per_cta = (int64_t)NS * (q * 4 + (want_pattern ? (int64_t)words_needed * 32 * 4 + q * 4 : 0) +
                                                (gbm ? (int64_t)state_words * 4 : 0));
         // cnt, nxt, poff, gptr, lrow, snind, sn_list
         const int64_t per_line = 2 * 4 + 2 + 2 * 8 + 2 * 8 + 4 + 1 + 4;
         const int64_t fixed = L * per_line + ((L + TILE - 1) / TILE) * 32 + 64 * 1024 +
                               (want_pattern ? (int64_t)2 * 4 * (1 << 20) : 0);
         const int64_t others = (int64_t)ctx->held - (int64_t)ctx->queue.bytes - (int64_t)ctx->stamp.bytes -
-                               (int64_t)ctx->gstate.bytes;
+                               (int64_t)ctx->gstate.bytes - (int64_t)ctx->lists.bytes - (int64_t)ctx->snap.bytes;
         const int64_t room = (int64_t)ctx->budget - others - fixed;
         if (room < per_cta) return GSOFA_ERR_OOM;
         grid = (int)std::min<int64_t>(grid, room / per_cta);
@@ -593,8 +604,11 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         } else if (pattern_form == 2) {
             d_pool = ext->dev;
         }
-        if (want_pattern)
-            d_stamp = (uint16_t *)ctx->grow(ctx->stamp, (size_t)grid * NS * stamp_stride * sizeof(uint16_t));
+        int32_t *d_lists = nullptr;
+        if (want_pattern) {
+            d_stamp = (uint16_t *)ctx->grow(ctx->stamp, (size_t)grid * NS * 2 * stamp_stride * sizeof(uint16_t));
+            d_lists = (int32_t *)ctx->grow(ctx->lists, (size_t)grid * NS * qcap * sizeof(int32_t));
+        }
         uint32_t *d_gstate = gbm ? (uint32_t *)ctx->grow(ctx->gstate, (size_t)grid * NS * state_words * 4) : nullptr;
         // Snapshots: paired passes with reuse, as many as a sixteenth of the
         // budget holds, and none where the job leaves no room for them.
@@ -662,6 +676,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         a.status = d_status;
         a.stamp = d_stamp;
         a.stamp_stride = stamp_stride;
+        a.lists = d_lists;
         a.gbm = d_gstate;
         a.blk_done = ext ? ext->blk_done : nullptr;
         a.blk_shift = ext ? ext->blk_shift : 0;
@@ -679,7 +694,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
                 GS_CUDA(cudaMemcpyAsync(d_ranges, rg_src, ranges.size() * sizeof(Range),
                                         cudaMemcpyHostToDevice, st));
             GS_CUDA(cudaMemsetAsync(d_misc, 0, 256, st));
-            GS_CUDA(cudaMemsetAsync(d_lrow, 0, (size_t)L * sizeof(int32_t), st));
+            if (a.want_pattern) GS_CUDA(cudaMemsetAsync(d_lrow, 0, (size_t)L * sizeof(int32_t), st));
             if (a.blk_done) GS_CUDA(cudaMemsetAsync(a.blk_done, 0, (size_t)ext->nblk * 4, st));
             if (subset) {
                 GS_CUDA(cudaMemsetAsync(d_cnt, 0, (size_t)2 * L * sizeof(int32_t), st));
@@ -765,7 +780,6 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         const unsigned long long xtot = h_misc[5], einsp = h_misc[6];
         const unsigned long long levels = h_misc[7], reused = h_misc[8];
 
-        if (status & ERR_QUEUE_OVERFLOW) return GSOFA_ERR_QUEUE_OVERFLOW;
         // a list's count and its pattern disagree: an internal fault, never
         // a property of the input
         if (status & ERR_COUNT_MISMATCH) return GSOFA_ERR_CUDA;
@@ -980,7 +994,7 @@ void gsofa_destroy(gsofa_ctx *c)
     DevBuf *bufs[] = {&c->queue, &c->cnt, &c->nxt, &c->poff, &c->gptr, &c->lrow, &c->snind,
                       &c->snlist, &c->tiles, &c->misc, &c->pool, &c->out, &c->mats, &c->ranges,
                       &c->st_beg, &c->st_end, &c->st_adj, &c->st_tmp, &c->matinfo, &c->stamp,
-                      &c->sn_head, &c->sn_data, &c->gstate, &c->blk, &c->order, &c->snap};
+                      &c->sn_head, &c->sn_data, &c->gstate, &c->blk, &c->order, &c->snap, &c->lists};
     for (DevBuf *b : bufs) c->release(*b);
     for (DevBuf &b : c->slabs) cudaFree(b.p);
     c->slabs.clear();
@@ -1231,8 +1245,8 @@ gsofa_status gsofa_upload(gsofa_ctx *c, int32_t n, int64_t nnz, const int32_t *b
             GS_CUDA(cudaGetLastError());
             if (m->d_gslot != nullptr) {
                 const int sgrid = (int)std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)c->sm_count * 8);
-                slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, m->d_gptr, m->d_gadj, m->d_gslot);
-                slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, m->d_tptr, m->d_tadj, m->d_tslot);
+                slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, m->d_gptr, m->d_gadj, m->d_rawdeg, m->d_gslot);
+                slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, m->d_tptr, m->d_tadj, nullptr, m->d_tslot);
                 GS_CUDA(cudaGetLastError());
             }
         }
@@ -1737,8 +1751,8 @@ size_t gsofa_predict_scratch_bytes(const gsofa_ctx *c, int32_t n, int64_t nnz,
     b += 2 * (L + 1) * 8;                       // gptr
     b += (size_t)(n + 1) * 8 + (size_t)nnz * 8; // G and G^T
     b += (size_t)n * 64;                        // their 32-byte row slots
-    if (p.want_pattern)                         // chain stamps, two traversals a CTA
-        b += grid * 2 * ((size_t)(n + 4095) / 4096 * 4096) * 2;
+    if (p.want_pattern)                         // chain stamps and list scratch, two traversals a CTA
+        b += grid * 2 * ((size_t)(n + 4095) / 4096 * 4096) * 4 + grid * 2 * qcap * 4;
     return b;
 }
 
@@ -2153,8 +2167,8 @@ extern "C" gsofa_status gsofa_symbfact_counts_noalloc(int device, void *cuda_str
         if ((int64_t)hc[2] > nnz || (int64_t)hc[3] > nnz) return GSOFA_ERR_INVALID_INPUT;
         GS_CUDA(cudaMemcpyAsync(tcur, tptr, (size_t)(n + 1) * 4, cudaMemcpyDeviceToDevice, st));
         upload_fill_kernel<<<ugrid, 256, 0, st>>>(u, gptr_g, gadj, tcur, tadj);
-        slot_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, gptr_g, gadj, gslot);
-        slot_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, tptr, tadj, tslot);
+        slot_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, gptr_g, gadj, rawdeg, gslot);
+        slot_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, tptr, tadj, nullptr, tslot);
         GS_CUDA(cudaGetLastError());
 
         // ---- factorization (counts only) ----
@@ -2231,8 +2245,7 @@ extern "C" gsofa_status gsofa_symbfact_counts_noalloc(int device, void *cuda_str
         GS_CUDA(cudaMemcpyAsync(&tot[1], gp + (L + 1) + L, 8, cudaMemcpyDeviceToHost, st));
         GS_CUDA(cudaStreamSynchronize(st));
         const uint32_t kst = (uint32_t)(hm[24] & 0xffffffffu);
-        if (kst & ERR_QUEUE_OVERFLOW) return GSOFA_ERR_QUEUE_OVERFLOW;
-        // any other status bit is an internal fault: no result is returned
+        // any status bit is an internal fault: no result is returned
         if (kst != 0u) return GSOFA_ERR_CUDA;
         summary[0] = (uint64_t)(tot[0] + tot[1]) - hc[0] - hc[1];
         summary[1] = (uint64_t)(tot[0] + tot[1] + n);
@@ -2716,8 +2729,8 @@ gsofa_status gsofa_server_submit(gsofa_server *s, int32_t n, int64_t nnz, const 
         upload_fill_kernel<<<ugrid, 256, 0, st>>>(u, gptr, gadj, tcur, tadj);
         {
             const int sgrid = (int)std::min<int64_t>(((int64_t)n + 255) / 256, (int64_t)s->sms * 8);
-            slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, gptr, gadj, gslot);
-            slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, tptr, tadj, tslot);
+            slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, gptr, gadj, rawdeg, gslot);
+            slot_fill_kernel<<<sgrid, 256, 0, st>>>(n, tptr, tadj, nullptr, tslot);
         }
         GS_CUDA(cudaGetLastError());
 

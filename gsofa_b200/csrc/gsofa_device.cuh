@@ -27,9 +27,9 @@ namespace dev {
 namespace cg = cooperative_groups;
 
 // Rows of at most SLOT_NB ids are also kept whole in a 32-byte slot per
-// vertex -- {degree, row offset, up to six ids} -- so expanding a frontier
+// vertex -- {degree, input degree, up to six ids} -- so expanding a frontier
 // vertex is one L2 round trip instead of two (row bounds, then ids); longer
-// rows take their ids from adj at the slot's offset.  Matrices whose mean
+// rows' slots hold their offset instead and their ids are taken from adj.  Matrices whose mean
 // off-diagonal degree is above SLOT_NB have no slots (slot == nullptr): most
 // of their rows would pay the 32-byte slot load and still read adj.
 constexpr int SLOT_NB = 6;
@@ -92,7 +92,6 @@ __host__ __device__ inline int64_t pieces_per_pass(const Range &rg)
 // Error bits reported through JobArgs::status.
 enum : uint32_t {
     ERR_POOL_OVERFLOW = 1u,
-    ERR_QUEUE_OVERFLOW = 2u,
     ERR_COUNT_MISMATCH = 4u,   // a list's running count and its bitmap disagree
 };
 
@@ -141,8 +140,9 @@ struct JobArgs {
                                   // [14] ns until the traversals ended,
                                   // [15] CTAs' traversal ns, summed
     uint32_t *status;
-    uint16_t *stamp;           // pattern mode: per traversal, stamp_stride entries:
-    int64_t stamp_stride;      // the chain index at which each vertex was first set
+    uint16_t *stamp;           // pattern mode: per traversal, two rows of stamp_stride
+    int64_t stamp_stride;      // entries: the chain index at which each vertex was first set
+    int32_t *lists;            // pattern mode: qcap entries per traversal
     uint32_t *snap;            // snapshots: snap_k bitmaps per traversal slot
     uint32_t *gbm;             // global-state kernels: per traversal, state_words
                                // words (bitmap and its summaries) in global memory
@@ -245,89 +245,143 @@ __device__ __forceinline__ int4 ld4(const int4 *p)
     return *p;
 }
 
-// Words of a bitmap's first summary level (the bitmap is followed directly by
-// its summary, so their distance is the bitmap size).
-__device__ __forceinline__ int bm_summary_words(const uint32_t *bm, const uint32_t *summ)
+// The visited set of one traversal: a bitmap of `words` words (a multiple of
+// 128) followed by its summaries, one bit per bitmap word and then one bit per
+// summary word (per 32K vertices), so that output, clearing and copying skip
+// empty stretches.  Words are numbered through all three.  A summary bit is
+// only ever added while a state grows, so neither level is read back then.
+//
+// In shared memory the words are addressed in the shared window (one register,
+// and no generic loads or atomics whatever the code around them).
+template <bool GBM>
+struct Bits;
+
+template <>
+struct Bits<false> {
+    uint32_t base;   // shared-window address
+    int words;
+    __device__ __forceinline__ uint32_t get(int i) const
+    {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(base + 4u * (uint32_t)i));
+        return v;
+    }
+    __device__ __forceinline__ uint4 get4(int i4) const
+    {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(base + 16u * (uint32_t)i4));
+        return v;
+    }
+    __device__ __forceinline__ void put(int i, uint32_t v) const
+    {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + 4u * (uint32_t)i), "r"(v) : "memory");
+    }
+    __device__ __forceinline__ void put4(int i4, uint4 v) const
+    {
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(base + 16u * (uint32_t)i4), "r"(v.x), "r"(v.y),
+                     "r"(v.z), "r"(v.w)
+                     : "memory");
+    }
+    // The old word where `on`, else `was`: predicated, not branched round.
+    __device__ __forceinline__ uint32_t fetch_or(int i, uint32_t m, bool on, uint32_t was) const
+    {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
+            : "+r"(was)
+            : "r"(base + 4u * (uint32_t)i), "r"(m), "r"((uint32_t)on));
+        return was;
+    }
+    __device__ __forceinline__ void add_or(int i, uint32_t m, bool on) const
+    {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.shared.or.b32 [%0], %1;\n\t}" ::"r"(
+                         base + 4u * (uint32_t)i),
+                     "r"(m), "r"((uint32_t)on));
+    }
+};
+
+// In global memory (resident in L2 at the sizes that matter) the words change
+// by atomics in L2 and are cleared by plain stores, so they are read through
+// L2 only: an L1 copy could be stale.
+template <>
+struct Bits<true> {
+    uint32_t *base;
+    int words;
+    __device__ __forceinline__ uint32_t get(int i) const { return __ldcg(base + i); }
+    __device__ __forceinline__ uint4 get4(int i4) const { return __ldcg(reinterpret_cast<const uint4 *>(base) + i4); }
+    __device__ __forceinline__ void put(int i, uint32_t v) const { base[i] = v; }
+    __device__ __forceinline__ void put4(int i4, uint4 v) const { reinterpret_cast<uint4 *>(base)[i4] = v; }
+    __device__ __forceinline__ uint32_t fetch_or(int i, uint32_t m, bool on, uint32_t was) const
+    {
+        return on ? atomicOr(base + i, m) : was;
+    }
+    __device__ __forceinline__ void add_or(int i, uint32_t m, bool on) const
+    {
+        if (on) atomicOr(base + i, m);
+    }
+};
+
+template <bool GBM>
+__device__ __forceinline__ Bits<GBM> bits_at(uint32_t *p, int words)
 {
-    return (int)(summ - bm) >> 5;
+    if constexpr (GBM) return Bits<GBM>{p, words};
+    else return Bits<GBM>{(uint32_t)__cvta_generic_to_shared(p), words};
 }
+
+// First words of the two summary levels, and the second one's length.
+template <bool GBM>
+__device__ __forceinline__ int summ1(const Bits<GBM> &b) { return b.words; }
+template <bool GBM>
+__device__ __forceinline__ int summ2(const Bits<GBM> &b) { return b.words + (b.words >> 5); }
+template <bool GBM>
+__device__ __forceinline__ int summ2_words(const Bits<GBM> &b) { return ((b.words >> 5) + 31) >> 5; }
 
 // Enters bitmap word wi, which just became nonzero, in both summary levels.
-__device__ __forceinline__ void mark_word(const uint32_t *bm, uint32_t *summ, int wi)
-{
-    atomicOr(summ + (wi >> 5), 1u << (wi & 31));
-    atomicOr(summ + bm_summary_words(bm, summ) + (wi >> 10), 1u << ((wi >> 5) & 31));
-}
-
-// Sets the bits m >= 0 of a traversal's bitmap, one per lane and u, all of
-// them in flight together: the words' reads first, then the atomics of those
-// that look unset, then the summaries of words that became nonzero.  Returns a
-// mask over u of the bits that this call set.  summ holds one bit per bitmap
-// word and is followed by a second level, one bit per summary word (per 32K
-// vertices); a summary bit is only ever added, so neither level is read back.
-// GBM: the bitmap lives in global memory (L2), where a read before the atomic
-// would cost as much as the atomic itself, so the atomics go first.
-template <int U, bool GBM>
-__device__ __forceinline__ unsigned set_bits(uint32_t *bm, uint32_t *summ, const int32_t (&m)[U])
-{
-    unsigned todo = 0u, fresh = 0u;
-    uint32_t w[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        w[u] = 0u;
-        if (!GBM && m[u] >= 0) w[u] = *reinterpret_cast<volatile uint32_t *>(bm + (m[u] >> 5));
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++)
-        if (m[u] >= 0 && !((w[u] >> (m[u] & 31)) & 1u)) todo |= 1u << u;
-    if (todo == 0u) return 0u;
-#pragma unroll
-    for (int u = 0; u < U; u++)
-        if ((todo >> u) & 1u) w[u] = atomicOr(bm + (m[u] >> 5), 1u << (m[u] & 31));
-#pragma unroll
-    for (int u = 0; u < U; u++)
-        if (((todo >> u) & 1u) && !((w[u] >> (m[u] & 31)) & 1u)) {
-            fresh |= 1u << u;
-            if (w[u] == 0u) mark_word(bm, summ, m[u] >> 5);
-        }
-    return fresh;
-}
-
-// Reads a word of a traversal's state: from shared memory, or (GBM) from
-// global memory through L2 only -- its words change by atomics in L2 and are
-// cleared by plain stores, so an L1 copy could be stale.
 template <bool GBM>
-__device__ __forceinline__ uint32_t bm_word(const uint32_t *p)
+__device__ __forceinline__ void mark_word(const Bits<GBM> &b, int wi, bool on)
 {
-    if (GBM) return __ldcg(p);
-    return *p;
+    b.add_or(summ1(b) + (wi >> 5), 1u << (wi & 31), on);
+    b.add_or(summ2(b) + (wi >> 10), 1u << ((wi >> 5) & 31), on);
 }
 
 // Frontier queue of one source: absolute positions 0, 1, 2, ... in BFS order.
 // A position p written while the writer's level started at w0 lives in the
-// shared-memory ring (ring_size entries, a power of two) when
-// p - w0 < ring_size and in the CTA's global spill array otherwise; readers
-// apply the same rule with the same w0.  Ring entries of one level and of the
-// level it feeds always lie within ring_size consecutive positions, so live
-// ring slots never collide.
+// shared-memory ring (a power of two of entries) when p - w0 < ring_size and in
+// the traversal's global spill array otherwise; readers apply the same rule
+// with the same w0.  Ring entries of one level and of the level it feeds always
+// lie within ring_size consecutive positions, so live ring slots never collide.
+// A vertex enters at most once per source, so positions stay below n.
 struct Frontier {
-    int32_t *ring;    // shared memory
-    int32_t *spill;   // global memory, qcap entries (this CTA's slice)
-    int64_t qcap;
-    uint32_t *status;
+    uint32_t ring;    // shared-window address
     int ring_size;
+    int32_t *spill;   // global memory, at least n entries
 };
 
-__device__ __forceinline__ void fr_put(const Frontier &f, int p, int w0, int32_t m)
+__device__ __forceinline__ void ring_put(const Frontier &f, int p, int32_t m, bool on)
 {
-    if (p - w0 < f.ring_size) f.ring[p & (f.ring_size - 1)] = m;
-    else if ((int64_t)p < f.qcap) f.spill[p] = m;
-    else atomicOr(f.status, ERR_QUEUE_OVERFLOW);  // cannot happen: p < n <= qcap
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(
+                     f.ring + 4u * (uint32_t)(p & (f.ring_size - 1))),
+                 "r"(m), "r"((uint32_t)on));
+}
+
+__device__ __forceinline__ int32_t ring_get(const Frontier &f, int p)
+{
+    int32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(f.ring + 4u * (uint32_t)(p & (f.ring_size - 1))));
+    return v;
+}
+
+__device__ __forceinline__ void fr_put(const Frontier &f, int p, int w0, int32_t m, bool on)
+{
+    const bool in = p - w0 < f.ring_size;
+    ring_put(f, p, m, on && in);
+    if (on && !in) f.spill[p] = m;
 }
 
 __device__ __forceinline__ int32_t fr_get(const Frontier &f, int p, int w0)
 {
-    return (p - w0 < f.ring_size) ? f.ring[p & (f.ring_size - 1)] : f.spill[p];
+    return p - w0 < f.ring_size ? ring_get(f, p) : f.spill[p];
 }
 
 // Seeding window: the rows of up to SEED_WIN consecutive sources (SEED_ADJ
@@ -346,7 +400,8 @@ constexpr int SNAP_REACH = 16;
 // Levels of at most this many vertices are run by a traversal's leader alone.
 constexpr int SOLO_MAX = 32;
 
-// Work that a traversal's first warp (its leader) hands to all of its warps.
+// Work that a traversal's first warp (its leader) hands to its other warps, the
+// helpers.
 enum : int { OP_EXIT = 0, OP_LEVELS, OP_CLEAR, OP_LISTS, OP_SAVE, OP_MERGE };
 
 // One traversal's shared state.  The leader warp runs the piece's sources and
@@ -365,19 +420,22 @@ struct SharedState {
     int seg[2];             // piece boundaries after chain alignment
     // list output (pattern mode): the chain -- consecutive sources sharing one
     // bitmap -- whose lists are written when it ends
-    uint16_t *stamp;        // this traversal's stamp row, or null (counts only)
+    uint16_t *stamp;        // the chain's stamp row, or null (counts only)
     int chain_s0;           // its first source
     int chain_len;          // its sources
     int chain_hi;           // no vertex above is set
     int64_t chain_total;    // entries of its lists
-    int64_t warp[32];       // per-warp entry counts of a chain's last list
-    int64_t last_off;       // pool offset of a chain's last list (-1: pool short)
-    int last_cnt;           // its entries
+    int64_t warp[32];       // per-warp counts of a chain's vertices
+    long long pool_base;    // the chain's pool range (-1: pool short)
     // tallies, kept by the leader's first lane: levels, then cycles of the
     // sources' own steps, their levels, list output, clearing, snapshots, wait
     // for the other pass; sources; reused sources
     unsigned long long prof[8];
     unsigned long long nsrc, nreuse;
+    unsigned long long work[3];   // edges, pass-G expansions, pass-G input degrees
+    int snaps;              // L: snapshots taken in this piece
+    int snap_credit;        // L: how many more may be saved
+    int weight;             // L: vertices queued by the state's traversals
     uint32_t reach[2][SNAP_REACH];            // by exchange: this bitmap's words from the source's on
     uint32_t snap_reach[SNAP_MAX][SNAP_REACH];  // L: the other pass's words when the snapshot was taken
     int snap_t[SNAP_MAX], snap_lo[SNAP_MAX], snap_hi[SNAP_MAX], snap_w[SNAP_MAX];   // L: source (-1: empty),
@@ -396,6 +454,7 @@ __device__ __forceinline__ void init_state(SharedState &sh)
     sh.nh = 0;
     for (int q = 0; q < 8; q++) sh.prof[q] = 0;
     sh.nsrc = sh.nreuse = 0;
+    sh.work[0] = sh.work[1] = sh.work[2] = 0;
     sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
     sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
 }
@@ -405,9 +464,17 @@ __device__ __forceinline__ void init_state(SharedState &sh)
 template <int GT>
 __device__ __forceinline__ void gsync(int bar)
 {
-    if (GT == 32) __syncwarp();
-    else if (bar == 1) asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
+    if (bar == 1) asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
     else asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
+}
+
+// Barrier of a traversal's helper warps (all but its leader).
+template <int GT>
+__device__ __forceinline__ void helper_sync(int bar)
+{
+    if (GT == 64) __syncwarp();
+    else if (bar == 1) asm volatile("bar.sync 4, %0;" ::"n"(GT - 32) : "memory");
+    else asm volatile("bar.sync 5, %0;" ::"n"(GT - 32) : "memory");
 }
 
 // Barrier of the two leader warps of a CTA that runs both passes of a source.
@@ -421,17 +488,17 @@ __device__ __forceinline__ void pair_sync()
 // summary word) in increasing order, using the second summary level to skip
 // empty stretches; fn(c) runs warp-uniformly.
 template <bool GBM, class F>
-__device__ __forceinline__ void for_nonzero_chunks(const uint32_t *summ2, int c0, int c1, F fn)
+__device__ __forceinline__ void for_nonzero_chunks(const Bits<GBM> &b, int c0, int c1, F fn)
 {
     int c = c0;
     while (c < c1) {
         const int wb = c & ~31;
-        uint32_t m = bm_word<GBM>(summ2 + (wb >> 5)) & (~0u << (c & 31));
+        uint32_t m = b.get(summ2(b) + (wb >> 5)) & (~0u << (c & 31));
         if (c1 - wb < 32) m &= (1u << (c1 - wb)) - 1u;
         while (m) {
-            const int b = __ffs(m) - 1;
+            const int k = __ffs(m) - 1;
             m &= m - 1u;
-            fn(wb + b);
+            fn(wb + k);
         }
         c = wb + 32;
     }
@@ -461,54 +528,105 @@ __device__ __forceinline__ int32_t chain_start(const PassGraph &g, int32_t x, in
 }
 
 // What every warp of a traversal knows about it for one work piece.
+template <bool GBM>
 struct Trav {
     PassGraph g;
     const int32_t *rawdeg;
     int pass;
-    uint32_t *bm, *summ;
+    Bits<GBM> bits;
     Frontier f;
-    uint16_t *stamp;       // or null
+    uint16_t *stamp;       // the chain's stamps (pattern mode, else null)
+    uint16_t *stamps;      // this traversal's two stamp rows
+    int32_t *lists;        // pattern mode: a chain's vertices while its lists are written
     uint32_t *snaps;       // this traversal's snapshots
 };
 
-// Per-thread tallies of one CTA's traversals (summed over the CTA at the
-// end); the per-source ones live in SharedState, kept by one thread.
+// Per-thread tallies of one work piece (folded into SharedState::work when it
+// ends); the per-source ones live in SharedState, kept by one thread.
 struct Tally {
-    unsigned long long edges = 0, xcnt = 0, einsp = 0;
+    uint32_t edges = 0, xcnt = 0, einsp = 0;
 };
 
-// New vertices of one warp step: those below s are queued for the next level
-// (alloc(k) hands out k positions, warp-uniformly; w0 is the first position of
-// the level whose vertices found them), those above s are counted (the return
-// value, warp-uniform).  Every new vertex above the chain's first source gets
-// the chain index of s as its stamp (pattern mode).
+// The sum of a 32-bit tally over a warp, and its addition to a 64-bit counter.
+__device__ __forceinline__ void fold_tally(unsigned long long *to, uint32_t v, int lane)
+{
+    const unsigned long long lo = __reduce_add_sync(0xffffffffu, v & 0xffffu);
+    const unsigned long long hi = __reduce_add_sync(0xffffffffu, v >> 16);
+    if (lane == 0) atomicAdd(to, lo + (hi << 16));
+}
+
+__device__ __forceinline__ void fold_work(SharedState &sh, const Tally &acc, int pass, int lane)
+{
+    fold_tally(&sh.work[0], acc.edges, lane);
+    if (pass) return;
+    fold_tally(&sh.work[1], acc.xcnt, lane);
+    fold_tally(&sh.work[2], acc.einsp, lane);
+}
+
+// One warp step: sets the bits m, one per lane and u, all of them in flight
+// together and without branches -- the words' reads first (not in global
+// memory, where a read would cost as much as the atomic), then the atomics of
+// those that look unset, then the summaries of words that became nonzero.  A
+// lane without an id holds s, which is set (or is to be: seeding).  New vertices
+// below s are queued for the next level (alloc(k) hands out k positions,
+// warp-uniformly; w0 is the first position of the level whose vertices found
+// them); the others, s itself included, are counted (the return value,
+// warp-uniform).  Every new vertex above the chain's first source gets the
+// chain index of s as its stamp (pattern mode).
 template <int U, bool GBM, class Alloc>
-__device__ __forceinline__ int visit(const Trav &t, const int32_t (&m)[U], int32_t s, int cidx, int w0, Alloc alloc)
+__device__ __forceinline__ int visit(const Trav<GBM> &t, const int32_t (&m)[U], int32_t s, int cidx, int w0,
+                                     Alloc alloc)
 {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const unsigned fresh = set_bits<U, GBM>(t.bm, t.summ, m);
-    if (!__any_sync(0xffffffffu, fresh != 0u)) return 0;
+    uint32_t w[U], bit[U];
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        bit[u] = 1u << (m[u] & 31);
+        // GBM: of the lanes without an id, the last one sees to s
+        w[u] = GBM ? (m[u] == s && lane != 31 ? ~0u : 0u) : t.bits.get(m[u] >> 5);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) any |= !(w[u] & bit[u]);
+    if (!__any_sync(0xffffffffu, any)) return 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) w[u] = t.bits.fetch_or(m[u] >> 5, bit[u], !(w[u] & bit[u]), w[u]);
+    any = false;
+#pragma unroll
+    for (int u = 0; u < U; u++) any |= w[u] == 0u;
+    if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+        for (int u = 0; u < U; u++) mark_word(t.bits, m[u] >> 5, w[u] == 0u);
+    }
     if (t.stamp != nullptr) {
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (((fresh >> u) & 1u) && m[u] > s - cidx) t.stamp[m[u]] = (uint16_t)cidx;
+            if (!(w[u] & bit[u]) && m[u] > s - cidx) t.stamp[m[u]] = (uint16_t)cidx;
     }
     unsigned low[U];
     int nlow = 0, nnew = 0;
 #pragma unroll
     for (int u = 0; u < U; u++) {
-        const bool f = (fresh >> u) & 1u;
-        low[u] = __ballot_sync(0xffffffffu, f && m[u] < s);
-        nnew += __popc(__ballot_sync(0xffffffffu, f));
+        const unsigned f = __ballot_sync(0xffffffffu, !(w[u] & bit[u]));
+        low[u] = f & __ballot_sync(0xffffffffu, m[u] < s);
+        nnew += __popc(f);
         nlow += __popc(low[u]);
     }
     if (nlow) {
         int pos = alloc(nlow);
+        if (pos + nlow - w0 <= t.f.ring_size) {
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            if ((low[u] >> lane) & 1u) fr_put(t.f, pos + __popc(low[u] & below), w0, m[u]);
-            pos += __popc(low[u]);
+            for (int u = 0; u < U; u++) {
+                ring_put(t.f, pos + __popc(low[u] & below), m[u], (low[u] >> lane) & 1u);
+                pos += __popc(low[u]);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                fr_put(t.f, pos + __popc(low[u] & below), w0, m[u], (low[u] >> lane) & 1u);
+                pos += __popc(low[u]);
+            }
         }
     }
     return nnew - nlow;
@@ -521,11 +639,21 @@ __device__ __forceinline__ int visit(const Trav &t, const int32_t (&m)[U], int32
 // id -- 32 rows' lines do not stay in the L1 that the bitmaps leave -- and ran
 // the 200,003-line power-law counts at 0.31 edges per SM cycle.)
 template <bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand_edges(const Trav &t, int32_t b, int32_t d, int32_t s, int cidx, int w0,
+__device__ __forceinline__ int expand_edges(const Trav<GBM> &t, int32_t b, int32_t d, int32_t s, int cidx, int w0,
                                             Alloc alloc)
 {
     const int lane = threadIdx.x & 31;
+    const unsigned upto = ~0u >> (31 - lane);   // lanes 0 .. lane
     int nh = 0;
+    // the rows with ids first
+    const unsigned some = __ballot_sync(0xffffffffu, d > 0);
+    const int rows = __popc(some);
+    if (some & (some + 1u)) {
+        const int from = __fns(some, 0, lane + 1) & 31;   // the lane of row `lane`
+        b = __shfl_sync(0xffffffffu, b, from);
+        d = __shfl_sync(0xffffffffu, d, from);
+        if (lane >= rows) d = 0;
+    }
     int incl = d;   // distinct vertices: their rows hold at most nnz < 2^31 ids together
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -533,144 +661,143 @@ __device__ __forceinline__ int expand_edges(const Trav &t, int32_t b, int32_t d,
         if (lane >= o) incl += y;
     }
     const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int32_t from = b - (incl - d);   // id e of the warp's edges is adj[from + e] of its owner
-    auto id = [&](int e) {
-        int o = 0;     // the first lane whose inclusive sum passes e
-#pragma unroll
-        for (int h = 16; h; h >>= 1)
-            if (__shfl_sync(0xffffffffu, incl, o + h - 1) <= e) o += h;
-        const int32_t at = __shfl_sync(0xffffffffu, from, o) + e;
-        return e < total ? ld<CG>(t.g.adj + at) : -1;
+    const int excl = lane < rows ? incl - d : INT32_MAX;   // where row `lane` begins among the warp's ids
+    const int32_t from = b - excl;                         // id e is adj[from + e] of its row
+    // ids e0 .. e0 + 31, one a lane: a lane's row is the last one that begins
+    // at or before its id
+    auto id = [&](int e0) {
+        const int before = __popc(__ballot_sync(0xffffffffu, excl < e0));
+        const unsigned begins =
+            __reduce_or_sync(0xffffffffu, (unsigned)(excl - e0) < 32u ? 1u << (excl - e0) : 0u);
+        const int row = before + __popc(begins & upto) - 1;
+        const int32_t at = __shfl_sync(0xffffffffu, from, row & 31) + e0 + lane;
+        return e0 + lane < total ? ld<CG>(t.g.adj + at) : s;
     };
     int e0 = 0;
     for (; total - e0 > 32; e0 += 128) {   // 128 ids in flight
         int32_t m[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) m[u] = id(e0 + 32 * u + lane);
+        for (int u = 0; u < 4; u++) m[u] = id(e0 + 32 * u);
         nh += visit<4, GBM>(t, m, s, cidx, w0, alloc);
     }
     if (e0 < total) {
-        const int32_t m[1] = {id(e0 + lane)};
+        const int32_t m[1] = {id(e0)};
         nh += visit<1, GBM>(t, m, s, cidx, w0, alloc);
     }
     return nh;
 }
 
-// Expands the frontier's entries [first, first + cnt), cnt <= 4 * U, of a graph
-// with row slots: eight lanes take a vertex: lane j reads word j of its 32-byte slot
-// {degree, offset, six ids}, four vertices to a load and U loads in flight, so
-// a level of few vertices is one short chain of dependent steps: ring, slot,
-// bitmap, atomic, ring.  (One lane a vertex, six ids a lane, took 3,500 cycles
-// for a level of a few vertices on the 80^3 matrix.)
+// Expands the frontier's entries [first, first + cnt), 0 < cnt <= 4 * U, of a
+// graph with row slots: eight lanes take a vertex: lane j reads word j of its
+// 32-byte slot, four vertices to a load and U loads in flight, so a level of
+// few vertices is one short chain of dependent steps: ring, slot, bitmap,
+// atomic, ring.  (One lane a vertex, six ids a lane, took 3,500 cycles for a
+// level of a few vertices on the 80^3 matrix.)  Rows longer than a slot are
+// left to the caller: lane i gets the bounds (b, d) of vertex i, or d = 0.
 template <int U, bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand_slots(const Trav &t, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
-                                            Tally &acc, Alloc alloc)
+__device__ __forceinline__ int expand_slots(const Trav<GBM> &t, int first, int cnt, bool in_ring, int wstart, int32_t s,
+                                            int cidx, int w0, Tally &acc, Alloc alloc, int32_t &b, int32_t &d)
 {
     const int lane = threadIdx.x & 31;
     const int j = lane & 7;
     int32_t v[U], m[U];
-    unsigned lng = 0u;     // this lane's vertices with rows longer than the slot (j == 0)
+#pragma unroll
+    for (int u = 0; u < U; u++) {   // lanes past the last vertex read its slot again
+        const int p = first + min(4 * u + (lane >> 3), cnt - 1);
+        v[u] = in_ring ? ring_get(t.f, p) : fr_get(t.f, p, wstart);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) m[u] = ld<CG>(reinterpret_cast<const int32_t *>(t.g.slot) + 8 * (int64_t)v[u] + j);
+    bool lng = false;
 #pragma unroll
     for (int u = 0; u < U; u++) {
-        const int i = 4 * u + (lane >> 3);
-        v[u] = i < cnt ? fr_get(t.f, first + i, wstart) : -1;
+        const bool on = 4 * u + (lane >> 3) < cnt;
+        if (on && j == 0) acc.edges += (unsigned)m[u];
+        if (on && j == 1) acc.einsp += (unsigned)m[u];
+        lng |= j == 0 && m[u] > SLOT_NB;
+    }
+    b = d = 0;
+    if (__any_sync(0xffffffffu, lng)) {   // those rows are read from adj: nothing from their slots
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int own = __shfl_sync(0xffffffffu, m[u], lane & 24);
+            const int deg = __shfl_sync(0xffffffffu, m[u], (lane & 3) << 3);
+            const int off = __shfl_sync(0xffffffffu, m[u], ((lane & 3) << 3) + 1);
+            if ((lane >> 2) == u && lane < cnt && deg > SLOT_NB) { d = deg; b = off; }
+            if (own > SLOT_NB) {
+                if (j == 1 && 4 * u + (lane >> 3) < cnt) acc.einsp += (unsigned)(ld<CG>(t.rawdeg + v[u]) - m[u]);
+                m[u] = -1;
+            }
+        }
     }
 #pragma unroll
     for (int u = 0; u < U; u++)
-        m[u] = v[u] >= 0 ? ld<CG>(reinterpret_cast<const int32_t *>(t.g.slot) + 8 * (int64_t)v[u] + j) : -1;
-    if (t.pass == 0 && j == 0) {
-#pragma unroll
-        for (int u = 0; u < U; u++)
-            if (v[u] >= 0) { acc.xcnt++; acc.einsp += (unsigned)ld<CG>(t.rawdeg + v[u]); }
-    }
-    int32_t off[U], deg[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-        deg[u] = j == 0 && v[u] >= 0 ? m[u] : 0;
-        off[u] = m[u];
-        acc.edges += (unsigned)deg[u];
-        if (deg[u] > SLOT_NB) lng |= 1u << u;
-        if (j < 2) m[u] = -1;
-    }
-    const unsigned any_long = __ballot_sync(0xffffffffu, lng != 0u);
-    if (any_long) {   // those rows are read from adj: nothing from their slots
-#pragma unroll
-        for (int u = 0; u < U; u++)
-            if ((__shfl_sync(0xffffffffu, lng, lane & ~7) >> u) & 1u) m[u] = -1;
-    }
-    int nh = visit<U, GBM>(t, m, s, cidx, w0, alloc);
-    if (any_long) {
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int32_t b = __shfl_down_sync(0xffffffffu, off[u], 1);
-            nh += expand_edges<CG, GBM>(t, b, ((lng >> u) & 1u) ? deg[u] : 0, s, cidx, w0, alloc);
-        }
-    }
-    return nh;
+        if (j < 2 || m[u] < 0) m[u] = s;   // ids past the degree are -1
+    return visit<U, GBM>(t, m, s, cidx, w0, alloc);
 }
 
-// The same with a lane a vertex (cnt <= 32), six ids a lane: fewer instructions
-// a vertex, for levels that keep every warp busy.
-template <bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand_lanes(const Trav &t, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
-                                            Tally &acc, Alloc alloc)
-{
-    const int lane = threadIdx.x & 31;
-    int32_t m[SLOT_NB] = {-1, -1, -1, -1, -1, -1};
-    int32_t b = 0, d = 0;
-    if (lane < cnt) {
-        const int32_t v = fr_get(t.f, first + lane, wstart);
-        const int4 sl0 = ld4<CG>(t.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(t.g.slot + 2 * (int64_t)v + 1);
-        d = sl0.x;
-        b = sl0.y;
-        acc.edges += (unsigned)d;
-        if (t.pass == 0) { acc.xcnt++; acc.einsp += (unsigned)ld<CG>(t.rawdeg + v); }
-        if (d <= SLOT_NB) {   // ids past the degree are -1 in the slot
-            m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
-            d = 0;
-        }
-    }
-    int nh = visit<SLOT_NB, GBM>(t, m, s, cidx, w0, alloc);
-    if (__any_sync(0xffffffffu, d != 0)) nh += expand_edges<CG, GBM>(t, b, d, s, cidx, w0, alloc);
-    return nh;
-}
-
-// Expands the frontier's entries [first, first + cnt), cnt <= 32, which were
+// Expands the frontier's entries [first, first + cnt), 0 < cnt <= 32, which were
 // written while the level starting at wstart ran.
 template <bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand(const Trav &t, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
+__device__ __forceinline__ int expand(const Trav<GBM> &t, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
                                       Tally &acc, Alloc alloc)
 {
-    if (t.g.slot != nullptr) {
-        if (cnt <= 4) return expand_slots<1, CG, GBM>(t, first, cnt, wstart, s, cidx, w0, acc, alloc);
-        if (cnt <= 16) return expand_slots<4, CG, GBM>(t, first, cnt, wstart, s, cidx, w0, acc, alloc);
-        return expand_lanes<CG, GBM>(t, first, cnt, wstart, s, cidx, w0, acc, alloc);
-    }
     const int lane = threadIdx.x & 31;
+    const bool in_ring = first + cnt - wstart <= t.f.ring_size;
     int32_t b = 0, d = 0;
-    if (lane < cnt) {
+    int nh = 0;
+    if (lane == 0) acc.xcnt += cnt;
+    if (t.g.slot != nullptr) {
+        if (cnt <= 4) {
+            nh = expand_slots<1, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
+        } else if (cnt <= 16) {
+            nh = expand_slots<4, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
+        } else {
+            // a lane a vertex, six ids a lane: fewer instructions a vertex,
+            // for levels that keep every warp busy
+            int32_t m[SLOT_NB] = {s, s, s, s, s, s};
+            if (lane < cnt) {
+                const int32_t v = fr_get(t.f, first + lane, wstart);
+                const int4 sl0 = ld4<CG>(t.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(t.g.slot + 2 * (int64_t)v + 1);
+                d = sl0.x;
+                b = sl0.y;
+                acc.edges += (unsigned)d;
+                if (d <= SLOT_NB) {   // ids past the degree are -1 in the slot
+                    acc.einsp += (unsigned)b;
+                    m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
+#pragma unroll
+                    for (int u = 0; u < SLOT_NB; u++) m[u] = m[u] < 0 ? s : m[u];
+                    d = 0;
+                } else if (t.pass == 0) {
+                    acc.einsp += (unsigned)ld<CG>(t.rawdeg + v);
+                }
+            }
+            nh = visit<SLOT_NB, GBM>(t, m, s, cidx, w0, alloc);
+        }
+        if (!__any_sync(0xffffffffu, d != 0)) return nh;
+    } else if (lane < cnt) {
         const int32_t v = fr_get(t.f, first + lane, wstart);
         b = ld<CG>(t.g.ptr + v);
         d = ld<CG>(t.g.ptr + v + 1) - b;
         acc.edges += (unsigned)d;
-        if (t.pass == 0) { acc.xcnt++; acc.einsp += (unsigned)ld<CG>(t.rawdeg + v); }
+        if (t.pass == 0) acc.einsp += (unsigned)ld<CG>(t.rawdeg + v);
     }
-    return expand_edges<CG, GBM>(t, b, d, s, cidx, w0, alloc);
+    return nh + expand_edges<CG, GBM>(t, b, d, s, cidx, w0, alloc);
 }
 
-// All warps of a traversal: levels from [start, end) on (entries written while
-// the level starting at wstart ran) until one is small enough for the leader
+// The helper warps: levels from [start, end) on (entries written while the
+// level starting at wstart ran) until one is small enough for the leader
 // alone.  One barrier a level.  The level counters rotate through three phases
 // that run on from call to call (every warp counts them in `phase`): a level
 // counts the next one's entries in tailc[phase] and its own dynamic fetches in
 // fetch[phase]; the counters of the phase after next are cleared behind the
 // level's barrier, when every warp is done with them.
 template <int GT, bool CG, bool GBM>
-__device__ __forceinline__ void run_levels(const Trav &t, SharedState &sh, int gtid, int bar, int &phase,
+__device__ __forceinline__ void run_levels(const Trav<GBM> &t, SharedState &sh, int htid, int bar, int &phase,
                                            Tally &acc)
 {
-    constexpr int NW = GT / 32;
-    const int lane = gtid & 31, wid = gtid >> 5;
+    constexpr int NW = GT / 32 - 1;
+    const int lane = htid & 31, wid = htid >> 5;
     const int32_t s = sh.src;
     const int cidx = sh.cidx;
     int start = sh.lv_start, end = sh.lv_end, wstart = sh.lv_wstart;
@@ -680,7 +807,7 @@ __device__ __forceinline__ void run_levels(const Trav &t, SharedState &sh, int g
         const int cnt = end - start;
         // vertices a warp takes at a time: fewer than its lanes could, while
         // that keeps every warp busy
-        const int take = min(32, max(4, (cnt + NW - 1) / NW));
+        const int take = cnt <= 4 * NW ? 4 : (cnt <= 16 * NW ? 16 : 32);
         auto alloc = [&](int k) {
             int p = 0;
             if (lane == 0) p = atomicAdd(tailp, k);
@@ -695,14 +822,14 @@ __device__ __forceinline__ void run_levels(const Trav &t, SharedState &sh, int g
             base = __shfl_sync(0xffffffffu, base, 0) + NW * take;
         }
         if (lane == 0 && nh) atomicAdd(&sh.nh, nh);
-        gsync<GT>(bar);
+        helper_sync<GT>(bar);
         const int nn = sh.tailc[phase];
         nlev++;
         wstart = start;
         start = end;
         end += nn;
         const int next = phase == 2 ? 0 : phase + 1;
-        if (gtid == 0) {
+        if (htid == 0) {
             const int clr = next == 2 ? 0 : next + 1;
             sh.tailc[clr] = 0;
             sh.fetch[clr] = 0;
@@ -710,7 +837,7 @@ __device__ __forceinline__ void run_levels(const Trav &t, SharedState &sh, int g
         phase = next;
         if (nn <= SOLO_MAX) break;
     }
-    if (gtid == 0) {   // for the leader's own lanes
+    if (htid == 0) {   // for the leader's own lanes
         sh.lv_start = start;
         sh.lv_end = end;
         sh.lv_wstart = wstart;
@@ -723,79 +850,74 @@ __device__ __forceinline__ void run_levels(const Trav &t, SharedState &sh, int g
 // touches a few stretches of a large matrix costs those stretches only; 32
 // second-level words are read at once.
 template <bool GBM>
-__device__ __forceinline__ void clear_state(uint32_t *bm, uint32_t *summ, int wid, int nw, int lane)
+__device__ __forceinline__ void clear_state(const Bits<GBM> &b, int wid, int nw, int lane)
 {
-    const int sw = bm_summary_words(bm, summ);
-    uint32_t *summ2 = summ + sw;
-    const int s2 = (sw + 31) >> 5;
+    const int s2 = summ2_words(b);
     for (int i0 = 0; i0 < s2; i0 += 32) {
-        const uint32_t mine = i0 + lane < s2 ? bm_word<GBM>(summ2 + i0 + lane) : 0u;
+        const uint32_t mine = i0 + lane < s2 ? b.get(summ2(b) + i0 + lane) : 0u;
         unsigned any = __ballot_sync(0xffffffffu, mine != 0u);
-        int k = 0;
-        for (; any; any &= any - 1u, k++) {
+        for (int k = 0; any; any &= any - 1u, k++) {
             const int j = __ffs(any) - 1;
             uint32_t m = __shfl_sync(0xffffffffu, mine, j);
             if (k % nw != wid) continue;
             const int i = i0 + j;
-            for (; m; m &= m - 1u) bm[(((i << 5) + __ffs(m) - 1) << 5) + lane] = 0u;
-            if ((i << 5) + lane < sw) summ[(i << 5) + lane] = 0u;
+            for (; m; m &= m - 1u) b.put((((i << 5) + __ffs(m) - 1) << 5) + lane, 0u);
+            if ((i << 5) + lane < (b.words >> 5)) b.put(summ1(b) + (i << 5) + lane, 0u);
         }
     }
 }
 
 // The second level, once every warp has read it.
-__device__ __forceinline__ void clear_summ2(uint32_t *bm, uint32_t *summ, int lane)
+template <bool GBM>
+__device__ __forceinline__ void clear_summ2(const Bits<GBM> &b, int lane)
 {
-    const int sw = bm_summary_words(bm, summ);
-    for (int i = lane; i < (sw + 31) >> 5; i += 32) summ[sw + i] = 0u;
+    for (int i = lane; i < summ2_words(b); i += 32) b.put(summ2(b) + i, 0u);
 }
 
-// All threads of a traversal copy bitmap words [lo, hi) into a snapshot.
+// The helper warps copy bitmap words [lo, hi) into a snapshot.
 template <int GT, bool GBM>
-__device__ __forceinline__ void save_state(const uint32_t *bm, uint32_t *snap, int lo, int hi, int gtid)
+__device__ __forceinline__ void save_state(const Bits<GBM> &b, uint32_t *snap, int lo, int hi, int htid)
 {
-    const uint4 *src = reinterpret_cast<const uint4 *>(bm);
     uint4 *dst = reinterpret_cast<uint4 *>(snap);
-    for (int i = (lo >> 2) + gtid; i < (hi >> 2); i += GT) dst[i] = GBM ? __ldcg(src + i) : src[i];
+    for (int i = (lo >> 2) + htid; i < (hi >> 2); i += GT - 32) dst[i] = b.get4(i);
 }
 
-// All threads of a traversal add the snapshot of source st (words [lo, hi)) to
+// The helper warps add the snapshot of source st (words [lo, hi)) to
 // the bitmap of source s, st < s: the new vertices between the two join the
 // first level (they were above st, so nothing was expanded from them), those
 // above s are counted in sh.nh.
 template <int GT, bool GBM>
-__device__ __forceinline__ void merge_state(const Trav &t, const uint32_t *snap, int lo, int hi, int st, int s, int cidx,
-                                            SharedState &sh, int gtid)
+__device__ __forceinline__ void merge_state(const Trav<GBM> &t, const uint32_t *snap, int lo, int hi, int st, int s, int cidx,
+                                            SharedState &sh, int htid)
 {
-    const int lane = gtid & 31;
+    const int lane = htid & 31;
     const uint4 *src = reinterpret_cast<const uint4 *>(snap);
-    uint4 *dst = reinterpret_cast<uint4 *>(t.bm);
     const int ws = s >> 5;
     const uint32_t above_s = ~1u << (s & 31);   // in word ws
     int cnt = 0;
     const int hi4 = hi >> 2;
-    for (int i0 = lo >> 2; i0 < hi4; i0 += GT) {   // warp-uniform trips
-        const int i = i0 + gtid;
+    for (int i0 = lo >> 2; i0 < hi4; i0 += GT - 32) {   // warp-uniform trips
+        const int i = i0 + htid;
         uint4 v = make_uint4(0u, 0u, 0u, 0u), c = v;
         if (i < hi4) {
             v = __ldcg(src + i);
-            c = GBM ? __ldcg(dst + i) : dst[i];
+            c = t.bits.get4(i);
         }
         const uint32_t nb[4] = {v.x & ~c.x, v.y & ~c.y, v.z & ~c.z, v.w & ~c.w};
         const uint32_t old[4] = {c.x, c.y, c.z, c.w};
         if (nb[0] | nb[1] | nb[2] | nb[3]) {
-            dst[i] = make_uint4(c.x | v.x, c.y | v.y, c.z | v.z, c.w | v.w);
+            t.bits.put4(i, make_uint4(c.x | v.x, c.y | v.y, c.z | v.z, c.w | v.w));
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int w = 4 * i + q;
                 if (nb[q] == 0u) continue;
-                if (old[q] == 0u) mark_word(t.bm, t.summ, w);
+                mark_word(t.bits, w, old[q] == 0u);
                 cnt += w > ws ? __popc(nb[q]) : (w == ws ? __popc(nb[q] & above_s) : 0);
                 if (w <= ws && w >= (st >> 5)) {   // the few words between the two sources
                     uint32_t x = nb[q];
                     if (w == ws) x &= (1u << (s & 31)) - 1u;
                     if (w == (st >> 5)) x &= ~1u << (st & 31);
-                    for (; x; x &= x - 1u) fr_put(t.f, atomicAdd(&sh.npush, 1), 0, (w << 5) + __ffs(x) - 1);
+                    for (; x; x &= x - 1u) fr_put(t.f, atomicAdd(&sh.npush, 1), 0, (w << 5) + __ffs(x) - 1, true);
                 }
             }
         }
@@ -816,254 +938,238 @@ __device__ __forceinline__ void merge_state(const Trav &t, const uint32_t *snap,
     if (lane == 0 && cnt) atomicAdd(&sh.nh, cnt);
 }
 
-// Lane's bitmap word of chunk cc, without the bits below word w0 and below
-// first_mask in word w0.
-template <bool GBM>
-__device__ __forceinline__ uint32_t last_word(const uint32_t *bm, const uint32_t *summ, int cc, int lane, int w0,
-                                              uint32_t first_mask)
-{
-    const int w = (cc << 5) + lane;
-    uint32_t x = ((bm_word<GBM>(summ + cc) >> lane) & 1u) ? bm_word<GBM>(bm + w) : 0u;
-    if (w < w0) x = 0u;
-    if (w == w0) x &= first_mask;
-    return x;
-}
-
-// Writes the lists of the chain that just ended -- sources chain_s0 ..
-// chain_s0 + chain_len - 1, which shared one bitmap -- while the bitmap still
-// holds the last source's traversal.  Bits are only ever added along a chain,
-// so the bits above source i of the chain that were set by the time it
-// finished are its list: hi(s_i) = { v > s_i : v set, stamp(v) <= i }.  One
-// pool range holds all of the chain's lists.
+// Writes the lists of the chain that just ended -- sources s0 .. s0 + len - 1,
+// which shared one bitmap -- by the helper warps, while the leader goes on with
+// the next sources: it waits only until the set vertices above s0 are out of
+// the bitmap (the barrier in the middle).  Bits are only ever added along a
+// chain, so list i is { v > s0 + i : v set, stamp(v) <= i }.  One exact pool
+// range holds all of the chain's lists (one global atomic per chain).
 //
-// The last source's list is every set bit above it: all warps write it at
-// once from the bitmap (each a share of its chunks, offsets from a count
-// pass), into the pool and into `scratch` (this traversal's frontier spill
-// array, free once the traversal is done).  Every earlier list i is then the
-// chain's own later sources that it reached, followed by the last list's
-// entries of stamp <= i: a warp streams the last list from scratch (several
-// coalesced loads and their stamps in flight at once) and keeps its entries
-// by ballot -- no per-list walk of the bitmap.  Lists of pass G^T (columns
-// of L) also count their entries into the L row histogram (fire-and-forget
-// reductions that overlap other traversals).
+// First each warp extracts its share of the bitmap's chunks, in order, into
+// `lists` (offsets from a count pass).  Then the lists go out 32 at a time:
+// every warp takes a block of the extracted vertices; a vertex belongs to the
+// lists [stamp, v - s0) of the chain, so two counters a vertex, summed, give
+// each warp its block's entries in each list and, over the warps, where they
+// start; then the block's vertices are read once more and, 32 at a time, go to
+// each of the lists by ballot -- where all 32 belong to all of the lists, as
+// most do, as one full store a list.  (A warp a list, filtering the last list
+// once per list with a dependent load of the stamp in every step, took 1,650
+// cycles a source on the 80^3 matrix with all warps waiting for it.)
+// Lists of pass G^T (columns of L) also count their entries into the L row
+// histogram, one reduction for the 32 lists.
 template <int GT, bool GBM>
-__device__ void output_chain(const JobArgs &a, int64_t line_base, int pass, const uint32_t *bm,
-                             const uint32_t *summ, SharedState &sh, int32_t *scratch, int gtid, int bar)
+__device__ __forceinline__ void write_lists(const JobArgs &a, int64_t line_base, const Trav<GBM> &t, SharedState &sh, int (*hist)[32],
+                            int htid, int bar)
 {
-    const int64_t line0 = line_base + sh.chain_s0;
-    int32_t *const lrow = pass ? a.lrow + line_base : nullptr;
-    constexpr int NWARP = GT / 32;
-    const int lane = gtid & 31, wid = gtid >> 5;
+    constexpr int NH = GT / 32 - 1;
+    constexpr int UNR = 4;
+    const int lane = htid & 31, wid = htid >> 5;
     const unsigned below = (1u << lane) - 1u;
-    const int s0 = sh.chain_s0, len = sh.chain_len;
-    const int64_t row0 = (int64_t)pass * a.L + line0;   // cnt / poff entry of s0
+    const int s0 = sh.chain_s0, len = sh.chain_len, chain_hi = sh.chain_hi;
+    const int64_t total = sh.chain_total;
+    const uint16_t *const stamp = sh.stamp;
+    int32_t *const scratch = t.lists;
+    const int64_t row0 = (int64_t)t.pass * a.L + line_base + s0;   // cnt / poff entry of s0
+    int32_t *const lrow = t.pass ? a.lrow + line_base : nullptr;
 
-    // The last source's list: set bits in words from w0 on (first_mask on
-    // w0), chunks [c_lo, c_hi) shared out among the warps.  Every warp counts
-    // its share (shared memory only) while warp 0 also takes the chain's pool
-    // range and writes every list's offset; one barrier then covers both.
-    const int s_last = s0 + len - 1;
-    const int chain_hi = sh.chain_hi;
-    const uint32_t *summ2 = summ + bm_summary_words(bm, summ);
-    const int w0 = (s_last + 1) >> 5;
-    const uint32_t first_mask = ~0u << ((s_last + 1) & 31);
-    const int c_lo = w0 >> 5;
-    const int c_hi = chain_hi > s_last ? (chain_hi >> 10) + 1 : c_lo;
-    const int share = (max(c_hi - c_lo, 0) + NWARP - 1) / NWARP;
-    const int my_lo = c_lo + wid * share, my_hi = min(c_hi, my_lo + share);
-    if (wid == 0) {
-        // one exact range per chain (one global atomic per chain of sources,
-        // so the pool holds the lists with no gaps); past the capacity the
-        // chain's lists are not written, the tail still advances, and its
-        // final value is the capacity the job needs
-        long long base = -1;
-        if (lane == 0) {
-            const int64_t total = sh.chain_total;
-            base = 0;
-            if (total > 0) {
-                const unsigned long long o = atomicAdd(a.pool_tail, (unsigned long long)total);
-                base = ((int64_t)o + total <= a.pool_cap) ? (long long)o : -1;
-            }
-            if (base < 0) atomicOr(a.status, ERR_POOL_OVERFLOW);
-        }
-        base = __shfl_sync(0xffffffffu, base, 0);
-        long long carry = 0;
-        for (int i0 = 0; i0 < len; i0 += 32) {
-            const int i = i0 + lane;
-            const long long c = i < len ? (long long)a.cnt[row0 + i] : 0;
-            long long incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const long long off = base >= 0 ? base + carry + incl - c : -1;
-            if (i < len) a.poff[row0 + i] = off;
-            if (i == len - 1) {
-                sh.last_off = off;
-                sh.last_cnt = (int)c;
-            }
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
+    // past the pool's capacity the chain's lists are not written, the tail
+    // still advances, and its final value is the capacity the job needs
+    long long base = 0;
+    if (wid == 0 && lane == 0 && total > 0) {
+        const unsigned long long o = atomicAdd(a.pool_tail, (unsigned long long)total);
+        base = (int64_t)o + total <= a.pool_cap ? (long long)o : -1;
+        if (base < 0) atomicOr(a.status, ERR_POOL_OVERFLOW);
     }
+
+    // set bits above s0: words from w0 on (first_mask on w0)
+    const int w0 = (s0 + 1) >> 5;
+    const uint32_t first_mask = ~0u << ((s0 + 1) & 31);
+    const int c_lo = w0 >> 5;
+    const int c_hi = chain_hi > s0 ? (chain_hi >> 10) + 1 : c_lo;
+    const int share = (max(c_hi - c_lo, 0) + NH - 1) / NH;
+    const int my_lo = c_lo + wid * share, my_hi = min(c_hi, my_lo + share);
+    auto word = [&](int cc) {
+        const int w = (cc << 5) + lane;
+        uint32_t x = t.bits.get(w);
+        if (w < w0) x = 0u;
+        if (w == w0) x &= first_mask;
+        return x;
+    };
     int mine = 0;
     if (my_lo < my_hi)
-        for_nonzero_chunks<GBM>(summ2, my_lo, my_hi, [&](int cc) {
-            mine += __popc(last_word<GBM>(bm, summ, cc, lane, w0, first_mask));
-        });
+        for_nonzero_chunks<GBM>(t.bits, my_lo, my_hi, [&](int cc) { mine += __popc(word(cc)); });
     mine = (int)__reduce_add_sync(0xffffffffu, (unsigned)mine);
     if (lane == 0) sh.warp[wid] = mine;
-    gsync<GT>(bar);
-    const int64_t off_last = sh.last_off;
-    const int cnt_last = sh.last_cnt;
-    const bool write = off_last >= 0;   // else the pool is short: nothing is written
-    if (write) {
-        int pos = 0, all = 0;
-        for (int k = 0; k < NWARP; k++) {
-            const int c = (int)sh.warp[k];
-            pos += k < wid ? c : 0;
-            all += c;
-        }
-        if (gtid == 0 && all != cnt_last) atomicOr(a.status, ERR_COUNT_MISMATCH);
-        int32_t *const out = a.pool + off_last;
-        if (my_lo < my_hi)
-            for_nonzero_chunks<GBM>(summ2, my_lo, my_hi, [&](int cc) {
-                uint32_t x = last_word<GBM>(bm, summ, cc, lane, w0, first_mask);
-                const int pc = __popc(x);
-                int incl = pc;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int excl = incl - pc;
-                const int wbase = cc << 5;
-                // at most two entries a word: a word per lane; denser chunks
-                // a word at a time across the warp (lane = bit), one
-                // coalesced run per store.  Nothing lands past the list's
-                // own cnt_last entries.
-                if (__reduce_max_sync(0xffffffffu, (unsigned)pc) <= 2u) {
-                    int at = pos + excl;
-                    while (x) {
-                        const int bit = __ffs(x) - 1;
-                        x &= x - 1u;
-                        const int32_t v = ((wbase + lane) << 5) + bit;
-                        if (at < cnt_last) {
-                            out[at] = v;
-                            scratch[at] = v;
-                            if (lrow) atomicAdd(lrow + v, 1);
-                        }
-                        at++;
-                    }
-                } else {
-                    unsigned nzw = __ballot_sync(0xffffffffu, x != 0u);
-                    while (nzw) {
-                        const int j = __ffs(nzw) - 1;
-                        nzw &= nzw - 1u;
-                        const uint32_t xj = __shfl_sync(0xffffffffu, x, j);
-                        const int pj = __shfl_sync(0xffffffffu, excl, j);
-                        const int at = pos + pj + __popc(xj & below);
-                        if (((xj >> lane) & 1u) && at < cnt_last) {
-                            const int32_t v = ((wbase + j) << 5) + lane;
-                            out[at] = v;
-                            scratch[at] = v;
-                            if (lrow) atomicAdd(lrow + v, 1);
-                        }
-                    }
-                }
-                pos += __shfl_sync(0xffffffffu, incl, 31);
-            });
+    helper_sync<GT>(bar);
+    int pos = 0, all = 0;
+    for (int k = 0; k < NH; k++) {
+        const int c = (int)sh.warp[k];
+        pos += k < wid ? c : 0;
+        all += c;
     }
-    gsync<GT>(bar);
+    if (my_lo < my_hi)
+        for_nonzero_chunks<GBM>(t.bits, my_lo, my_hi, [&](int cc) {
+            uint32_t x = word(cc);
+            const int pc = __popc(x);
+            int incl = pc;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const int excl = incl - pc;
+            // at most two entries a word: a word per lane; denser chunks a
+            // word at a time across the warp (lane = bit)
+            if (__reduce_max_sync(0xffffffffu, (unsigned)pc) <= 2u) {
+                for (int at = pos + excl; x; x &= x - 1u, at++) scratch[at] = (((cc << 5) + lane) << 5) + __ffs(x) - 1;
+            } else {
+                for (unsigned nzw = __ballot_sync(0xffffffffu, x != 0u); nzw; nzw &= nzw - 1u) {
+                    const int j = __ffs(nzw) - 1;
+                    const uint32_t xj = __shfl_sync(0xffffffffu, x, j);
+                    const int pj = __shfl_sync(0xffffffffu, excl, j);
+                    if ((xj >> lane) & 1u) scratch[pos + pj + __popc(xj & below)] = (((cc << 5) + j) << 5) + lane;
+                }
+            }
+            pos += __shfl_sync(0xffffffffu, incl, 31);
+        });
+    if (wid == 0 && lane == 0) sh.pool_base = base;
+    gsync<GT>(bar);   // the bitmap is free, the vertices are out
+    base = sh.pool_base;
 
-    // every earlier list i: its later chain sources (s_i, s_last] that were
-    // reached by then, then the last list's entries of stamp <= i (all above
-    // s_last, so the list stays sorted)
-    const uint16_t *stamp = sh.stamp;
-    for (int i = wid; write && i < len - 1; i += NWARP) {
-        const int s = s0 + i;
-        const int64_t off = a.poff[row0 + i];
-        const int cnt = a.cnt[row0 + i];
-        if (cnt == 0) continue;
-        int32_t *const out = a.pool + off;
-        int pos = 0;
-        for (int k0 = s + 1; k0 <= s_last; k0 += 32) {
-            const int v = k0 + lane;
-            const bool in = v <= s_last && ((bm_word<GBM>(bm + (v >> 5)) >> (v & 31)) & 1u) && (int)stamp[v] <= i;
-            const unsigned bal = __ballot_sync(0xffffffffu, in);
-            const int at = pos + __popc(bal & below);
-            if (in && at < cnt) {
-                out[at] = v;
-                if (lrow) atomicAdd(lrow + v, 1);
-            }
-            pos += __popc(bal);
+    const int steps = (all + 31) >> 5, per = (steps + NH - 1) / NH;
+    const int k_lo = min(all, wid * per * 32), k_hi = min(all, k_lo + per * 32);
+    long long carry = 0;
+    for (int i0 = 0; i0 < len; i0 += 32) {
+        const int nl = min(32, len - i0);
+        // lane l: list i0 + l, its entries and its place
+        const int c = lane < nl ? a.cnt[row0 + i0 + lane] : 0;
+        long long incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
         }
-        // UNR loads of the last list and their stamps in flight at once (two
-        // where 64 registers a thread must do)
-        constexpr int UNR = GT > 384 ? 2 : 4;
-        for (int k0 = 0; k0 < cnt_last; k0 += 32 * UNR) {
-            int32_t e[UNR];
-            int t[UNR];
+        long long p = base + carry + incl - c;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+        if (wid == 0 && lane < nl) a.poff[row0 + i0 + lane] = base >= 0 ? p : -1;
+        if (base < 0) continue;
+        // the lists [lo, hi) of the 32 that vertex v belongs to
+        auto lists_of = [&](int32_t v, int st, int &lo, int &hi) {
+            lo = max(st - i0, 0);
+            hi = v - s0 - i0;
+        };
+        hist[wid][lane] = 0;
+        __syncwarp();
+        int whole = 0;   // vertices that belong to all 32
+        for (int k0 = k_lo; k0 < k_hi; k0 += 32 * UNR) {
+            int32_t v[UNR];
+            int st[UNR];
+#pragma unroll
+            for (int u = 0; u < UNR; u++) v[u] = k0 + 32 * u + lane < k_hi ? __ldcg(scratch + k0 + 32 * u + lane) : -1;
+#pragma unroll
+            for (int u = 0; u < UNR; u++) st[u] = v[u] > s0 && v[u] <= chain_hi ? (int)stamp[v[u]] : INT32_MAX;
 #pragma unroll
             for (int u = 0; u < UNR; u++) {
-                const int k = k0 + 32 * u + lane;
-                e[u] = k < cnt_last ? __ldcg(scratch + k) : -1;
-            }
-#pragma unroll
-            for (int u = 0; u < UNR; u++)   // only vertices of the last list (s_last, chain_hi] are read
-                t[u] = (e[u] > s_last && e[u] <= chain_hi) ? (int)stamp[e[u]] : INT32_MAX;
-#pragma unroll
-            for (int u = 0; u < UNR; u++) {
-                const bool in = t[u] <= i;
-                const unsigned bal = __ballot_sync(0xffffffffu, in);
-                const int at = pos + __popc(bal & below);
-                if (in && at < cnt) {
-                    out[at] = e[u];
-                    if (lrow) atomicAdd(lrow + e[u], 1);
+                int lo, hi;
+                lists_of(v[u], min(st[u], 1 << 20), lo, hi);
+                const bool full = lo == 0 && hi >= 32;
+                whole += __popc(__ballot_sync(0xffffffffu, full));
+                if (!full && lo < 32 && hi > lo) {
+                    atomicAdd(&hist[wid][lo], 1);
+                    if (hi < 32) atomicAdd(&hist[wid][hi], -1);
                 }
-                pos += __popc(bal);
             }
         }
-        if (lane == 0 && pos != cnt) atomicOr(a.status, ERR_COUNT_MISMATCH);
+        __syncwarp();
+        int n = hist[wid][lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, n, o);
+            if (lane >= o) n += y;
+        }
+        n += whole;
+        __syncwarp();
+        hist[wid][lane] = n;
+        helper_sync<GT>(bar);
+        int sum = 0;
+        for (int k = 0; k < NH; k++) {
+            const int x = hist[k][lane];
+            p += k < wid ? x : 0;
+            sum += x;
+        }
+        // a list's running count and its vertices disagree: an internal fault,
+        // and nothing is written
+        const bool bad = __any_sync(0xffffffffu, lane < nl && sum != c);
+        if (bad && lane == 0) atomicOr(a.status, ERR_COUNT_MISMATCH);
+        for (int k0 = bad ? k_hi : k_lo; k0 < k_hi; k0 += 32 * UNR) {
+            int32_t v[UNR];
+            int st[UNR];
+#pragma unroll
+            for (int u = 0; u < UNR; u++) v[u] = k0 + 32 * u + lane < k_hi ? __ldcg(scratch + k0 + 32 * u + lane) : -1;
+#pragma unroll
+            for (int u = 0; u < UNR; u++) st[u] = v[u] > s0 && v[u] <= chain_hi ? (int)stamp[v[u]] : INT32_MAX;
+#pragma unroll
+            for (int u = 0; u < UNR; u++) {
+                int lo, hi;
+                lists_of(v[u], min(st[u], 1 << 20), lo, hi);
+                if (lrow && lo < nl) {
+                    const int k = min(hi, nl) - lo;
+                    if (k > 0) atomicAdd(lrow + v[u], k);
+                }
+                if (__all_sync(0xffffffffu, lo == 0 && hi >= nl)) {
+#pragma unroll 4
+                    for (int l = 0; l < nl; l++) a.pool[__shfl_sync(0xffffffffu, p, l) + lane] = v[u];
+                    p += 32;
+                } else {
+                    int got = 0;
+                    for (int l = 0; l < nl; l++) {
+                        const bool in = lo <= l && l < hi;
+                        const unsigned bal = __ballot_sync(0xffffffffu, in);
+                        const long long q = __shfl_sync(0xffffffffu, p, l);
+                        if (in) a.pool[q + __popc(bal & below)] = v[u];
+                        if (lane == l) got = __popc(bal);
+                    }
+                    p += got;
+                }
+            }
+        }
+        helper_sync<GT>(bar);   // the counters are free again
     }
-    gsync<GT>(bar);
     // Streaming: count the chain's entries into the pool blocks they fill.
     // Every list of the chain is written (the barrier above); one fence makes
     // those writes visible device-wide before the counts that let the host
     // copy a full block out while the traversals go on.
-    if (a.blk_done != nullptr && gtid == 0 && sh.chain_total > 0) {
-        const int64_t base = a.poff[row0];
-        if (base >= 0) {
-            __threadfence();
-            const int64_t end = base + sh.chain_total;
-            const int64_t bsz = (int64_t)1 << a.blk_shift;
-            for (int64_t b = base >> a.blk_shift; b <= (end - 1) >> a.blk_shift; b++) {
-                const int64_t lo = max(base, b * bsz), hi = min(end, (b + 1) * bsz);
-                atomicAdd(a.blk_done + b, (unsigned int)(hi - lo));
-            }
+    if (a.blk_done != nullptr && wid == 0 && lane == 0 && total > 0 && base >= 0) {
+        __threadfence();
+        const int64_t end = base + total;
+        const int64_t bsz = (int64_t)1 << a.blk_shift;
+        for (int64_t b = base >> a.blk_shift; b <= (end - 1) >> a.blk_shift; b++) {
+            const int64_t lo = max(base, (long long)(b * bsz)), hi = min(end, (b + 1) * bsz);
+            atomicAdd(a.blk_done + b, (unsigned int)(hi - lo));
         }
     }
 }
 
-// One op of the leader's, run by all threads of the traversal after its
-// barrier.
+// One op of the leader's, run by the helper warps (htid: the thread among
+// them) behind the traversal's barrier; a second one tells the leader that it
+// is done.
 template <int GT, bool CG, bool GBM, bool LISTS>
-__device__ __forceinline__ void run_op(const JobArgs &a, int64_t line_base, const Trav &t, SharedState &sh, int op,
-                                       int gtid, int bar, int &phase, Tally &acc)
+__device__ __forceinline__ void run_op(const JobArgs &a, int64_t line_base, Trav<GBM> &t, SharedState &sh,
+                                       int (*hist)[32], int op, int htid, int bar, int &phase, Tally &acc)
 {
+    if (LISTS) t.stamp = sh.stamp;
     if (op == OP_LEVELS) {
-        run_levels<GT, CG, GBM>(t, sh, gtid, bar, phase, acc);
-        return;
-    }
-    if (op == OP_CLEAR) {
-        clear_state<GBM>(t.bm, t.summ, gtid >> 5, GT / 32, gtid & 31);
+        run_levels<GT, CG, GBM>(t, sh, htid, bar, phase, acc);
+    } else if (op == OP_CLEAR) {
+        clear_state<GBM>(t.bits, htid >> 5, GT / 32 - 1, htid & 31);
     } else if (op == OP_SAVE) {
-        save_state<GT, GBM>(t.bm, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, gtid);
+        save_state<GT, GBM>(t.bits, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, htid);
     } else if (op == OP_MERGE) {
         merge_state<GT, GBM>(t, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, sh.t, sh.src, sh.cidx, sh,
-                             gtid);
+                             htid);
     } else if (LISTS && op == OP_LISTS) {
-        output_chain<GT, GBM>(a, line_base, t.pass, t.bm, t.summ, sh, t.f.spill, gtid, bar);
+        write_lists<GT, GBM>(a, line_base, t, sh, hist, htid, bar);   // the leader goes on from its middle
+        return;
     }
     gsync<GT>(bar);
 }
@@ -1071,12 +1177,11 @@ __device__ __forceinline__ void run_op(const JobArgs &a, int64_t line_base, cons
 // Nonzero stretch of a bitmap as words [lo, hi), whole chunks, and its number
 // of nonzero chunks; one warp.
 template <bool GBM>
-__device__ __forceinline__ int state_extent(const uint32_t *bm, const uint32_t *summ, int lane, int &lo, int &hi)
+__device__ __forceinline__ int state_extent(const Bits<GBM> &b, int lane, int &lo, int &hi)
 {
-    const int sw = bm_summary_words(bm, summ);
     int first = INT32_MAX, last = -1, chunks = 0;
-    for (int i = lane; i < (sw + 31) >> 5; i += 32) {
-        const uint32_t m = bm_word<GBM>(summ + sw + i);
+    for (int i = lane; i < summ2_words(b); i += 32) {
+        const uint32_t m = b.get(summ2(b) + i);
         if (m) {
             first = min(first, (i << 5) + __ffs(m) - 1);
             last = (i << 5) + 31 - __clz(m);
@@ -1115,23 +1220,26 @@ __device__ __forceinline__ int state_extent(const uint32_t *bm, const uint32_t *
 // instead of 2.7e8.  Where snapshots are saved but not taken over (meshes),
 // the piece's CTA stops saving them.
 template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
-__device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, int32_t s_lo, int32_t s_hi,
-                           int32_t stride, SharedState *shs, volatile int (*pair_flag)[2], int half, int bar,
-                           int &phase, int &snap_credit, Tally &acc)
+__device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, Trav<GBM> &t, int32_t s_lo, int32_t s_hi,
+                           int32_t stride, SharedState *shs, volatile int (*pair_flag)[2], int half,
+                           int bar)
 {
     constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
-    constexpr int NW = GT / 32;
+    static_assert(GT >= 64, "a leader and at least one helper");
     SharedState &sh = shs[half];
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     const int pass = t.pass;
+    Tally acc;
     const int nsnap = PAIRED ? a.snap_k : 0;
     auto collective = [&](int op) {   // arguments are in place
-        if (lane == 0) sh.op = op;
+        if (lane == 0) {
+            sh.op = op;
+            if (LISTS) sh.stamp = t.stamp;
+        }
         __syncwarp();
-        gsync<GT>(bar);
-        run_op<GT, CG, GBM, LISTS>(a, md.line_base, t, sh, op, lane, bar, phase, acc);
-        __syncwarp();
+        gsync<GT>(bar);   // the helpers have the op
+        gsync<GT>(bar);   // they are done
     };
     auto take_nh = [&]() {   // what the last op counted
         const int v = sh.nh;
@@ -1141,13 +1249,12 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
     };
     // tallies: the first lane's, in shared memory
     auto tally = [&](unsigned long long &x, unsigned long long v) { if (lane == 0) x += v; };
-    const long long c_begin = clock64();
-    unsigned long long c_ops = 0;   // cycles tallied elsewhere
-    auto spent = [&](int q, long long c0) {
+    auto spent = [&](int q, long long c0) {   // cycles of one kind, none of the sources' own
         const unsigned long long c = (unsigned long long)(clock64() - c0);
         tally(sh.prof[q], c);
-        c_ops += c;
+        tally(sh.prof[1], 0ull - c);
     };
+    tally(sh.prof[1], 0ull - (unsigned long long)clock64());
 
     int prev = -2;
     int cidx = -1;            // index of the last source in its chain (-1: none yet)
@@ -1158,16 +1265,16 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
     long long total = 0;      // entries of the chain's lists
     // the seeding window: lane i holds row bounds and degree of source wlo + i
     int wlo = 0, whi = 0, wb = 0, we = 0, wraw = 0, wadj0 = 0;
-    int snaps = 0;            // snapshots taken in this piece
     if (lane < SNAP_MAX) sh.snap_t[lane] = -1;
-    int weight = 0;           // vertices queued by the state's traversals
+    if (lane == 0) sh.snaps = sh.weight = 0;
+    __syncwarp();
     const int heavy = max(64, a.bitmap_words >> 3);   // worth a copy of the bitmap
 
     auto end_chain = [&]() {
         int lo, hi;
         if (LISTS && a.want_pattern && cidx >= 0) {
             const long long c0 = clock64();
-            state_extent<GBM>(t.bm, t.summ, lane, lo, hi);
+            state_extent<GBM>(t.bits, lane, lo, hi);
             if (lane == 0) {
                 sh.chain_s0 = prev - cidx;
                 sh.chain_len = cidx + 1;
@@ -1175,26 +1282,30 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
                 sh.chain_hi = min(hi << 5, md.n) - 1;
             }
             collective(OP_LISTS);
+            // the helpers read this chain's stamps on: the next chain takes
+            // the traversal's other row
+            t.stamp = t.stamp == t.stamps ? t.stamps + a.stamp_stride : t.stamps;
             spent(5, c0);
         }
         const long long c0 = clock64();
-        const int chunks = state_extent<GBM>(t.bm, t.summ, lane, lo, hi);
-        if (NW == 1 || chunks <= 48) {
-            clear_state<GBM>(t.bm, t.summ, 0, 1, lane);
+        const int chunks = state_extent<GBM>(t.bits, lane, lo, hi);
+        if (chunks <= 48) {
+            clear_state<GBM>(t.bits, 0, 1, lane);
             __syncwarp();
         } else {
             collective(OP_CLEAR);
         }
-        clear_summ2(t.bm, t.summ, lane);
+        clear_summ2(t.bits, lane);
         __syncwarp();
         if (GBM) __threadfence_block();
         spent(6, c0);
     };
 
-    for (int32_t s = s_lo; s < s_hi;) {
+    for (int32_t s = s_lo;;) {
+        const bool more = s < s_hi;   // else: end the piece's last chain
         // a new seeding window when s is past the current one (consecutive
         // sources only): row bounds, then the rows themselves
-        if (stride == 1 && s >= whi) {
+        if (more && stride == 1 && s >= whi) {
             const int cnt = min(s_hi - s, SEED_WIN);
             const int i = min(lane, cnt - 1);
             wb = ld<CG>(t.g.ptr + s + i);
@@ -1224,13 +1335,13 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
         // takes (counts 8.9 ms to 5.2 ms).
         // Both passes come here or neither does; one that cannot run (a row too
         // long for its window, a chain near its last stamp) says k = 0.
-        if (PAIRED && mine && other && !step) {
+        if (PAIRED && more && mine && other && !step) {
             const bool can = in_win && !(a.want_pattern && cidx + 32 >= 65535);
             int k = can ? min(whi - s, 31) : 0;
             const int i0 = can ? s - wlo : 0;
             const int p0 = __shfl_sync(0xffffffffu, wb, i0) - wadj0;
             const int p1 = can ? __shfl_sync(0xffffffffu, we, i0 + k - 1) - wadj0 : p0;
-            const uint32_t ws = s + lane < md.n ? bm_word<GBM>(t.bm + ((s + lane) >> 5)) : 0u;
+            const uint32_t ws = s + lane < md.n ? t.bits.get((s + lane) >> 5) : 0u;
             unsigned run_set = __ballot_sync(0xffffffffu, (ws >> ((s + lane) & 31)) & 1u);
             int ne = 0;
             for (int q0 = p0; q0 < p1 && ne <= 32; q0 += 128) {
@@ -1239,7 +1350,7 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
 #pragma unroll
                 for (int u = 0; u < 4; u++) x[u] = q0 + 32 * u + lane < p1 ? sh.win_adj[q0 + 32 * u + lane] : -1;
 #pragma unroll
-                for (int u = 0; u < 4; u++) w[u] = x[u] >= 0 ? bm_word<GBM>(t.bm + (x[u] >> 5)) : ~0u;
+                for (int u = 0; u < 4; u++) w[u] = x[u] >= 0 ? t.bits.get(x[u] >> 5) : ~0u;
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const bool isnew = !((w[u] >> (x[u] & 31)) & 1u);
@@ -1292,11 +1403,8 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
             if (~both) cut = min(cut, __ffs(~both) - 1);
             if (cut > 0) {
                 win = win && ei < cut;
-                if (win) {
-                    const uint32_t old = atomicOr(t.bm + (x >> 5), 1u << (x & 31));
-                    if (old == 0u) mark_word(t.bm, t.summ, x >> 5);
-                    if (t.stamp != nullptr) t.stamp[x] = (uint16_t)(cidx + 1 + ei);
-                }
+                mark_word(t.bits, x >> 5, t.bits.fetch_or(x >> 5, 1u << (x & 31), win, ~0u) == 0u);
+                if (win && t.stamp != nullptr) t.stamp[x] = (uint16_t)(cidx + 1 + ei);
                 // lane i: source s + i; events are in row order
                 const unsigned wins = __ballot_sync(0xffffffffu, win);
                 int upto = 0;   // events of rows 0 .. lane
@@ -1336,11 +1444,11 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
             if (cut > 0) continue;
         }
         step = false;
-        int32_t b0, d0;
+        int32_t b0 = 0, d0 = 0;
         if (in_win) {
             b0 = __shfl_sync(0xffffffffu, wb, s - wlo);
             d0 = __shfl_sync(0xffffffffu, we, s - wlo) - b0;
-        } else {
+        } else if (more) {
             b0 = ld<CG>(t.g.ptr + s);
             d0 = ld<CG>(t.g.ptr + s + 1) - b0;
         }
@@ -1348,7 +1456,7 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
         // take over the previous source's state, or end its chain; chain
         // indices are 16-bit stamps: a chain ends after 65535 sources
         bool reuse = false;
-        if (a.reuse && prev == s - 1 && !(a.want_pattern && cidx + 1 >= 65535)) {
+        if (more && a.reuse && prev == s - 1 && !(a.want_pattern && cidx + 1 >= 65535)) {
             if (PAIRED) {
                 reuse = other;
             } else {
@@ -1363,24 +1471,26 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
             tally(sh.nreuse, 1u);
         } else {
             if (cidx >= 0) end_chain();
+            if (!more) break;   // the next piece starts from an empty bitmap
             cidx = 0;
             hc = 0;
             total = 0;
-            weight = 0;
+            if (nsnap > 0 && lane == 0) sh.weight = 0;
         }
 
-        // Seeding: s itself and its neighbours; those below s are the first
+        // Seeding: s itself (in the lanes that the row leaves) and its neighbours;
+        // those below s are the first
         // level.  nh counts new vertices above s, and s when it is new: a
         // source that was set already was counted by the sources before it.
         int tail = 0, nh = 0;
         bool self = false;   // s is set
         auto alloc = [&](int k) { const int p = tail; tail += k; return p; };
-        if (lane == 0) acc.edges += (unsigned)d0;
-        if (pass == 0) {
-            const int r = in_win ? __shfl_sync(0xffffffffu, wraw, s - wlo) : ld<CG>(t.rawdeg + s);
-            if (lane == 0) acc.einsp += (unsigned)r;
+        if (lane == 0) {
+            acc.edges += (unsigned)d0;
+            if (pass == 0 && !in_win) acc.einsp += (unsigned)ld<CG>(t.rawdeg + s);
         }
-        if (snaps > 0) {
+        if (in_win && lane == s - wlo) acc.einsp += (unsigned)wraw;
+        if (nsnap > 0 && sh.snaps > 0) {
             // the newest snapshot that s contains and its state does not yet,
             // until there is none (bit t set: t and all of its state are in)
             for (;;) {
@@ -1389,20 +1499,21 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
                 if (st >= 0) {
                     const int w = (s >> 5) - (st >> 5);
                     if (!(w < SNAP_REACH && ((sh.snap_reach[lane][w] >> (s & 31)) & 1u) &&
-                          !((bm_word<GBM>(t.bm + (st >> 5)) >> (st & 31)) & 1u)))
+                          !((t.bits.get(st >> 5) >> (st & 31)) & 1u)))
                         st = -1;
                 }
                 const int best = __reduce_max_sync(0xffffffffu, st);
                 if (best < 0) break;
                 const long long c0 = clock64();
                 if (!self) {   // before the merge, which leaves it out
-                    const int32_t m[1] = {lane == 0 ? s : -1};
+                    const int32_t m[1] = {s};
                     nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
                     self = true;
                 }
                 const int k = __ffs(__ballot_sync(0xffffffffu, st == best)) - 1;
-                weight += sh.snap_w[k];
                 if (lane == 0) {
+                    sh.weight += sh.snap_w[k];
+                    sh.snap_credit += 8;
                     sh.src = s;
                     sh.cidx = cidx;
                     sh.snap = k;
@@ -1414,19 +1525,23 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
                 collective(OP_MERGE);
                 tail = sh.npush;
                 nh += take_nh();
-                snap_credit += 8;
                 spent(3, c0);
             }
         }
         {
             auto id = [&](int k) { return in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(t.g.adj + b0 + k); };
-            const int32_t m[1] = {lane == 31 ? (self ? -1 : s) : (lane < d0 ? id(lane) : -1)};
+            const int32_t m[1] = {lane < d0 ? id(lane) : s};
             nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
-            for (int k0 = 31; k0 < d0; k0 += 128) {
+            for (int k0 = 32; k0 < d0; k0 += 128) {
                 int32_t x[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) x[u] = k0 + 32 * u + lane < d0 ? id(k0 + 32 * u + lane) : -1;
+                for (int u = 0; u < 4; u++) x[u] = k0 + 32 * u + lane < d0 ? id(k0 + 32 * u + lane) : s;
                 nh += visit<4, GBM>(t, x, s, cidx, 0, alloc);
+            }
+            // s where the row filled every lane
+            if (d0 >= 32 && !self) {
+                const int32_t m1[1] = {s};
+                nh += visit<1, GBM>(t, m1, s, cidx, 0, alloc);
             }
         }
 
@@ -1435,11 +1550,10 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
         if (end > 0) {
             const long long c0 = clock64();
             do {
-                if (NW == 1 || end - start <= SOLO_MAX) {
+                if (end - start <= SOLO_MAX) {
                     __syncwarp();   // the level's queue entries, for every lane
                     tally(sh.prof[0], 1u);
-                    for (int base = start; base < end; base += 32)
-                        nh += expand<CG, GBM>(t, base, min(32, end - base), wstart, s, cidx, start, acc, alloc);
+                    nh += expand<CG, GBM>(t, start, end - start, wstart, s, cidx, start, acc, alloc);
                     wstart = start;
                     start = end;
                     end = tail;
@@ -1465,10 +1579,10 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
         // |hi(s)|: the bits above s; the link flag; both passes' exchange
         hc += nh - 1;
         total += hc;
-        weight += end;
+        if (nsnap > 0 && end > 0 && lane == 0) sh.weight += end;
         tally(sh.nsrc, 1u);
         __syncwarp();
-        mine = s + 1 < md.n && ((bm_word<GBM>(t.bm + ((s + 1) >> 5)) >> ((s + 1) & 31)) & 1u);
+        mine = s + 1 < md.n && ((t.bits.get((s + 1) >> 5) >> ((s + 1) & 31)) & 1u);
         if (lane == 0) {
             const int64_t slot = (int64_t)pass * a.L + md.line_base + s;
             a.cnt[slot] = hc;
@@ -1480,34 +1594,36 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
             xch++;
             if (lane == 0) pair_flag[par][half] = mine;
             if (nsnap > 0 && lane < SNAP_REACH)
-                sh.reach[par][lane] = (s >> 5) + lane < a.bitmap_words ? bm_word<GBM>(t.bm + (s >> 5) + lane) : 0u;
+                sh.reach[par][lane] = (s >> 5) + lane < a.bitmap_words ? t.bits.get((s >> 5) + lane) : 0u;
             const long long c0 = clock64();
             pair_sync();
             other = pair_flag[par][1 - half] != 0;
             spent(7, c0);
-            if (nsnap > 0 && end > 0 && weight >= heavy && snap_credit > 0) {
+            if (nsnap > 0 && end > 0 && sh.weight >= heavy && sh.snap_credit > 0) {
                 const long long c0 = clock64();
                 int lo, hi;
-                state_extent<GBM>(t.bm, t.summ, lane, lo, hi);
-                const int k = snaps++ & (nsnap - 1);   // nsnap is a power of two
+                state_extent<GBM>(t.bits, lane, lo, hi);
+                const int k = sh.snaps & (nsnap - 1);   // nsnap is a power of two
+                __syncwarp();
                 if (lane < SNAP_REACH) sh.snap_reach[k][lane] = shs[1 - half].reach[par][lane];
                 if (lane == 0) {
                     sh.snap_t[k] = s;
-                    sh.snap_w[k] = weight;
+                    sh.snaps++;
+                    sh.snap_credit--;
+                    sh.snap_w[k] = sh.weight;
                     sh.snap = k;
                     sh.snap_lo[k] = sh.lo = lo;
                     sh.snap_hi[k] = sh.hi = hi;
                 }
                 collective(OP_SAVE);
-                snap_credit--;
                 spent(3, c0);
             }
         }
         s += stride;
     }
-    if (cidx >= 0) end_chain();   // the next piece starts from an empty bitmap
+    fold_work(sh, acc, pass, lane);
     if (lane == 0) {
-        sh.prof[1] += (unsigned long long)(clock64() - c_begin) - c_ops;
+        sh.prof[1] += (unsigned long long)clock64();
         sh.op = OP_EXIT;
     }
     __syncwarp();
@@ -1516,22 +1632,22 @@ __device__ void lead_piece(const JobArgs &a, const MatDesc &md, const Trav &t, i
 
 // One work piece: the first warp of every traversal leads, the others help.
 template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
-__device__ __forceinline__ void run_piece(const JobArgs &a, const MatDesc &md, const Trav &t, int32_t s_lo,
-                                          int32_t s_hi, int32_t stride, SharedState *shs,
-                                          volatile int (*pair_flag)[2], int half, int gtid, int bar, int &phase,
-                                          int &snap_credit, Tally &acc)
+__device__ __forceinline__ void run_piece(const JobArgs &a, const MatDesc &md, Trav<GBM> &t, int32_t s_lo,
+                                          int32_t s_hi, int32_t stride, SharedState *shs, int (*hist)[32],
+                                          volatile int (*pair_flag)[2], int half, int gtid, int bar, int &phase)
 {
     constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
     if (gtid < 32) {
-        lead_piece<BLOCK, PAIRED, CG, GBM, LISTS>(a, md, t, s_lo, s_hi, stride, shs, pair_flag, half, bar, phase,
-                                                  snap_credit, acc);
+        lead_piece<BLOCK, PAIRED, CG, GBM, LISTS>(a, md, t, s_lo, s_hi, stride, shs, pair_flag, half, bar);
     } else {
+        Tally acc;
         for (;;) {
             gsync<GT>(bar);
             const int op = shs[half].op;
             if (op == OP_EXIT) break;
-            run_op<GT, CG, GBM, LISTS>(a, md.line_base, t, shs[half], op, gtid, bar, phase, acc);
+            run_op<GT, CG, GBM, LISTS>(a, md.line_base, t, shs[half], hist, op, gtid - 32, bar, phase, acc);
         }
+        fold_work(shs[half], acc, t.pass, gtid & 31);
     }
 }
 
@@ -1559,7 +1675,7 @@ __device__ __forceinline__ void run_piece(const JobArgs &a, const MatDesc &md, c
 // LISTS: the list output is compiled in; counts-only jobs run an
 // instantiation without it, whose registers go to the traversal alone.
 template <int BLOCK, bool PAIRED, bool GBM, int MINB = (BLOCK >= 1024 ? 1 : 1024 / BLOCK), bool LISTS = true>
-__global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
+__global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_constant__ JobArgs a)
 {
     constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
     constexpr int NS = PAIRED ? 2 : 1;
@@ -1567,6 +1683,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
     __shared__ SharedState shs[NS];
     __shared__ volatile int pair_flag[2][2];   // [source parity][pass]: s+1 in hi(s)
     __shared__ long long s_piece;
+    __shared__ int s_hist[LISTS ? NS * (GT / 32 - 1) : 1][32];   // list output: a row a helper warp
+    int (*const hist)[32] = s_hist + (LISTS ? (int)threadIdx.x / GT * (GT / 32 - 1) : 0);
     cg::grid_group grid = cg::this_grid();
     const int tid = threadIdx.x;
     const int half = PAIRED ? tid / GT : 0;
@@ -1575,24 +1693,22 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
     SharedState &sh = shs[half];
     const int64_t trav = (int64_t)blockIdx.x * NS + half;
     uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * NS) * a.state_words : smem_dyn;
-    uint32_t *bm = state + (size_t)half * a.state_words;
-    uint32_t *summ = bm + a.bitmap_words;
-    int32_t *ring = (int32_t *)(GBM ? smem_dyn : smem_dyn + (size_t)NS * a.state_words) + (size_t)half * a.ring_size;
+    uint32_t *const ring = (GBM ? smem_dyn : smem_dyn + (size_t)NS * a.state_words) + (size_t)half * a.ring_size;
 
     // ---- phase 1: traversals ------------------------------------------------
     unsigned long long t_start = 0;
     if (tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
     for (int w = tid; w < NS * a.state_words; w += BLOCK) state[w] = 0u;
     if (gtid == 0) init_state(sh);
-    Trav t{};
-    t.bm = bm;
-    t.summ = summ;
-    t.f = Frontier{ring, a.queue + trav * a.qcap, a.qcap, a.status, a.ring_size};
-    t.stamp = LISTS && a.want_pattern ? a.stamp + trav * a.stamp_stride : nullptr;
+    Trav<GBM> t{};
+    t.bits = bits_at<GBM>(state + (size_t)half * a.state_words, a.bitmap_words);
+    t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size, a.queue + trav * a.qcap};
+    if (LISTS && a.want_pattern) {
+        t.stamp = t.stamps = a.stamp + 2 * trav * a.stamp_stride;
+        t.lists = a.lists + trav * a.qcap;
+    }
     t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
-    if (gtid == 0) sh.stamp = t.stamp;
-    Tally acc;
-    int phase = 0, snap_credit = SNAP_CREDIT, last_mat = -1;
+    int phase = 0, last_mat = -1;
     __syncthreads();
     for (;;) {
         if (tid == 0) s_piece = (long long)atomicAdd(a.piece_counter, 1ull);
@@ -1630,13 +1746,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
             s_lo = sh.seg[0];
             s_hi = sh.seg[1];
         }
-        if (rg.mat != last_mat) snap_credit = SNAP_CREDIT;
+        if (rg.mat != last_mat && gtid == 0) sh.snap_credit = SNAP_CREDIT;
         last_mat = rg.mat;
         t.g = g;
         t.rawdeg = md.rawdeg;
         t.pass = pass;
-        run_piece<BLOCK, PAIRED, false, GBM, LISTS>(a, md, t, s_lo, s_hi, rg.stride, shs, pair_flag, half, gtid, bar,
-                                                    phase, snap_credit, acc);
+        run_piece<BLOCK, PAIRED, false, GBM, LISTS>(a, md, t, s_lo, s_hi, rg.stride, shs, hist, pair_flag, half, gtid,
+                                                    bar, phase);
         __syncthreads();   // every thread is done with s_piece
     }
     {
@@ -1645,21 +1761,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(JobArgs a)
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_done));
             atomicAdd(&a.counters[15], t_done - t_start);
         }
-        int64_t *wsum = shs[0].warp;
-        const int64_t e = block_sum<BLOCK>((int64_t)acc.edges, wsum);
-        const int64_t x = block_sum<BLOCK>((int64_t)acc.xcnt, wsum);
-        const int64_t ei = block_sum<BLOCK>((int64_t)acc.einsp, wsum);
         if (tid == 0) {
-            unsigned long long ns = 0, nr = 0, pv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            unsigned long long ns = 0, nr = 0, wk[3] = {0, 0, 0}, pv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int h = 0; h < NS; h++) {
+                for (int q = 0; q < 3; q++) wk[q] += shs[h].work[q];
                 ns += shs[h].nsrc;
                 nr += shs[h].nreuse;
                 for (int q = 0; q < 8; q++) pv[q] += shs[h].prof[q];
             }
-            atomicAdd(&a.counters[0], (unsigned long long)e);
+            atomicAdd(&a.counters[0], wk[0]);
             atomicAdd(&a.counters[1], (unsigned long long)ns);
-            atomicAdd(&a.counters[3], (unsigned long long)x);
-            atomicAdd(&a.counters[4], (unsigned long long)ei);
+            atomicAdd(&a.counters[3], wk[1]);
+            atomicAdd(&a.counters[4], wk[2]);
             atomicAdd(&a.counters[5], (unsigned long long)pv[0]);
             atomicAdd(&a.counters[6], (unsigned long long)nr);
             for (int q = 1; q < 8; q++) atomicAdd(&a.counters[6 + q], (unsigned long long)pv[q]);
@@ -1954,16 +2067,17 @@ __global__ void upload_fill_kernel(UploadArgs u, const int32_t *gptr, int32_t *g
     }
 }
 
-// Fills the 32-byte slot of every vertex of one pass graph: {degree, row
-// offset, the first SLOT_NB ids (-1 past the degree)}.
-__global__ void slot_fill_kernel(int32_t n, const int32_t *ptr, const int32_t *adj, int4 *slot)
+// Fills the 32-byte slot of every vertex of one pass graph: {degree, input
+// degree (pass G) or, of rows longer than SLOT_NB, the row's offset, the first
+// SLOT_NB ids (-1 past the degree)}.
+__global__ void slot_fill_kernel(int32_t n, const int32_t *ptr, const int32_t *adj, const int32_t *rawdeg, int4 *slot)
 {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t b = ptr[v], d = ptr[v + 1] - b;
         int32_t x[SLOT_NB];
 #pragma unroll
         for (int u = 0; u < SLOT_NB; u++) x[u] = u < d ? adj[b + u] : -1;
-        slot[2 * v] = make_int4(d, b, x[0], x[1]);
+        slot[2 * v] = make_int4(d, d > SLOT_NB ? b : (rawdeg ? rawdeg[v] : 0), x[0], x[1]);
         slot[2 * v + 1] = make_int4(x[2], x[3], x[4], x[5]);
     }
 }

@@ -67,7 +67,7 @@ __device__ __forceinline__ T load_cg(const T *p)
 // bitmaps in shared memory); the global-state form (GBM, bitmaps in global
 // memory) three 256-thread CTAs per SM, six traversals of four warps each.
 template <int BLOCK, bool GBM>
-__global__ void __maxnreg__(64) serve_kernel(ServeArgs sa)
+__global__ void __maxnreg__(64) serve_kernel(const __grid_constant__ ServeArgs sa)
 {
     constexpr int GT = BLOCK / 2;
     const JobArgs &a = sa.job;
@@ -81,20 +81,16 @@ __global__ void __maxnreg__(64) serve_kernel(ServeArgs sa)
     const int bar = 1 + half;
     SharedState &sh = shs[half];
     uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * 2) * a.state_words : smem_dyn;
-    uint32_t *bm = state + (size_t)half * a.state_words;
-    uint32_t *summ = bm + a.bitmap_words;
-    int32_t *ring = (int32_t *)(GBM ? smem_dyn : smem_dyn + (size_t)2 * a.state_words) + (size_t)half * a.ring_size;
+    uint32_t *const ring = (GBM ? smem_dyn : smem_dyn + (size_t)2 * a.state_words) + (size_t)half * a.ring_size;
     for (int w = tid; w < 2 * a.state_words; w += BLOCK) state[w] = 0u;
     if (gtid == 0) init_state(sh);   // counts only: no lists, no stamps
     const int64_t trav = (int64_t)blockIdx.x * 2 + half;
-    Trav t{};
-    t.bm = bm;
-    t.summ = summ;
-    t.f = Frontier{ring, a.queue + trav * a.qcap, a.qcap, a.status, a.ring_size};
+    Trav<GBM> t{};
+    t.bits = bits_at<GBM>(state + (size_t)half * a.state_words, a.bitmap_words);
+    t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size, a.queue + trav * a.qcap};
     t.stamp = nullptr;
     t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
-    Tally acc;
-    int phase = 0, snap_credit = SNAP_CREDIT;
+    int phase = 0;
     __shared__ int s_class;
     __syncthreads();
     for (;;) {
@@ -128,9 +124,9 @@ __global__ void __maxnreg__(64) serve_kernel(ServeArgs sa)
         t.g = md.g[half];
         t.rawdeg = md.rawdeg;
         t.pass = half;
-        snap_credit = SNAP_CREDIT;   // the piece may be another request's
-        run_piece<BLOCK, true, true, GBM, false>(a, md, t, piece.s_lo, piece.s_hi, 1, shs, pair_flag, half, gtid, bar,
-                                                 phase, snap_credit, acc);
+        if (gtid == 0) sh.snap_credit = SNAP_CREDIT;   // the piece may be another request's
+        run_piece<BLOCK, true, true, GBM, false>(a, md, t, piece.s_lo, piece.s_hi, 1, shs, nullptr, pair_flag, half, gtid,
+                                                 bar, phase);
         __syncthreads();
         if (tid == 0) {
             __threadfence();
