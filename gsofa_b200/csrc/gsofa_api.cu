@@ -400,7 +400,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
     // bitmap words rounded to 128 so its summary (one bit per word) is a
     // whole number of 16-byte groups
     const int32_t words_needed = ((max_n + 31) / 32 + 127) / 128 * 128;
-    const int32_t state_needed = words_needed + words_needed / 32 + ((words_needed / 32 + 31) / 32 + 3) / 4 * 4;
+    const int32_t state_needed = STATE_PAD + words_needed + words_needed / 32 + ((words_needed / 32 + 31) / 32 + 3) / 4 * 4;
     // Where the visited bitmaps live: shared memory holds two of them (the
     // paired kernel) up to ~850K lines and one up to ~1.7M; global memory
     // holds any number of any size.  GSOFA_FLAG_GLOBAL_STATE /
@@ -1164,7 +1164,7 @@ gsofa_status gsofa_upload(gsofa_ctx *c, int32_t n, int64_t nnz, const int32_t *b
             // row slots only where most rows fit one (mean off-diagonal
             // degree of the input at most SLOT_NB)
             const bool slots = nnz - (int64_t)n <= (int64_t)SLOT_NB * n;
-            const size_t sb = slots ? al((size_t)std::max<int32_t>(n, 1) * 32) : 0;
+            const size_t sb = slots ? al(((size_t)n + 1) * 32) : 0;
             const size_t total = 2 * pb + 3 * lb + 2 * ab + 2 * sb;
             char *q = (char *)c->slab_take(total, &m->slab_bytes);
             m->slab = q;
@@ -2084,7 +2084,7 @@ extern "C" gsofa_status gsofa_symbfact_counts_noalloc(int device, void *cuda_str
         constexpr int BLOCK = 256;
         void *kfn = factor_kernel_for(BLOCK, false);
         const int32_t bitmap_words = ((n + 31) / 32 + 127) / 128 * 128;
-        const int32_t state_words = bitmap_words + bitmap_words / 32 + ((bitmap_words / 32 + 31) / 32 + 3) / 4 * 4;
+        const int32_t state_words = STATE_PAD + bitmap_words + bitmap_words / 32 + ((bitmap_words / 32 + 31) / 32 + 3) / 4 * 4;
         const int ring = 4096;
         const size_t smem = (size_t)state_words * 4 + (size_t)ring * 4;
         int occ = 0;
@@ -2112,8 +2112,8 @@ extern "C" gsofa_status gsofa_symbfact_counts_noalloc(int device, void *cuda_str
         int32_t *orig_up = lay.take<int32_t>(n);
         int32_t *orig_lo = lay.take<int32_t>(n);
         int32_t *rawdeg = lay.take<int32_t>(n);
-        int4 *gslot = lay.take<int4>((size_t)2 * n);
-        int4 *tslot = lay.take<int4>((size_t)2 * n);
+        int4 *gslot = lay.take<int4>((size_t)2 * n + 2);
+        int4 *tslot = lay.take<int4>((size_t)2 * n + 2);
         int64_t *tsum = lay.take<int64_t>(2 * scan_tiles);
         unsigned long long *ucounts = lay.take<unsigned long long>(8);
         int32_t *cnt = lay.take<int32_t>(2 * L);
@@ -2369,7 +2369,7 @@ int64_t server_graph_bytes(int32_t n, int64_t nnz)
     const int64_t a = 256;
     auto r = [&](int64_t b) { return (b + a - 1) / a * a; };
     return 2 * r(4 * ((int64_t)n + 1)) + 2 * r(4 * std::max<int64_t>(nnz, 1)) + 3 * r(4 * std::max<int32_t>(n, 1)) +
-           2 * r(32 * std::max<int32_t>(n, 1));
+           2 * r(32 * ((int64_t)n + 1));
 }
 
 // Upload staging: input copy, degree arrays, scan partials, counters.
@@ -2504,7 +2504,7 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         s->max_slots = cfg->max_requests > 0 ? cfg->max_requests : 4096;
         s->idle_spins = std::max(1, (cfg->idle_exit_us > 0 ? cfg->idle_exit_us : 30000000) / 2);
         s->bitmap_words = ((s->max_n + 31) / 32 + 127) / 128 * 128;
-        s->state_words = s->bitmap_words + s->bitmap_words / 32 + ((s->bitmap_words / 32 + 31) / 32 + 3) / 4 * 4;
+        s->state_words = STATE_PAD + s->bitmap_words + s->bitmap_words / 32 + ((s->bitmap_words / 32 + 31) / 32 + 3) / 4 * 4;
         // frontier ring: the largest that fits beside the two bitmaps (shared
         // state), or beside two more CTAs' rings (global state)
         void *kfn = s->gbm ? (void *)serve_kernel<kServeBlockG, true> : (void *)serve_kernel<kServeBlock, false>;
@@ -2673,8 +2673,8 @@ gsofa_status gsofa_server_submit(gsofa_server *s, int32_t n, int64_t nnz, const 
         int32_t *orig_up = (int32_t *)take(gb, 4 * (int64_t)n);
         int32_t *orig_lo = (int32_t *)take(gb, 4 * (int64_t)n);
         int32_t *rawdeg = (int32_t *)take(gb, 4 * (int64_t)n);
-        int4 *gslot = (int4 *)take(gb, 32 * (int64_t)n);
-        int4 *tslot = (int4 *)take(gb, 32 * (int64_t)n);
+        int4 *gslot = (int4 *)take(gb, 32 * ((int64_t)n + 1));
+        int4 *tslot = (int4 *)take(gb, 32 * ((int64_t)n + 1));
         const int64_t scan_tiles = ((int64_t)n + 1 + 255) / 256 + 1;
         int32_t *d_beg = (int32_t *)take(sb, 4 * (int64_t)n);
         int32_t *d_end = (int32_t *)take(sb, 4 * (int64_t)n);

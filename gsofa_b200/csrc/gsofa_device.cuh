@@ -37,7 +37,7 @@ constexpr int SLOT_NB = 6;
 struct PassGraph {
     const int32_t *ptr;  // [n+1]
     const int32_t *adj;  // [ptr[n]]
-    const int4 *slot;    // [2n]: vertex v at slot[2v], slot[2v+1] (or null)
+    const int4 *slot;    // [2n + 2]: vertex v at slot[2v], slot[2v+1], then an empty slot (or null)
 };
 
 struct MatDesc {
@@ -105,7 +105,7 @@ struct JobArgs {
     int32_t *queue;            // gridDim.x * qcap
     int64_t qcap;
     int32_t bitmap_words;      // shared-memory bitmap size (>= max n / 32, multiple of 128)
-    int32_t state_words;       // bitmap + its two summary levels
+    int32_t state_words;       // STATE_PAD, bitmap, its two summary levels
     int32_t ring_size;         // shared-memory frontier ring entries (power of two)
     int32_t snap_k;            // snapshots a traversal slot keeps (0: none)
     int32_t reuse;
@@ -245,6 +245,9 @@ __device__ __forceinline__ int4 ld4(const int4 *p)
     return *p;
 }
 
+// Words of ones before a traversal's bitmap (a 16-byte group; id -1 has the last).
+constexpr int STATE_PAD = 4;
+
 // The visited set of one traversal: a bitmap of `words` words (a multiple of
 // 128) followed by its summaries, one bit per bitmap word and then one bit per
 // summary word (per 32K vertices), so that output, clearing and copying skip
@@ -284,14 +287,24 @@ struct Bits<false> {
                      "r"(v.z), "r"(v.w)
                      : "memory");
     }
-    // The old word where `on`, else `was`: predicated, not branched round.
-    __device__ __forceinline__ uint32_t fetch_or(int i, uint32_t m, bool on, uint32_t was) const
+    // Where vertex m's word is; m = -1 (no vertex) has the word before the
+    // first, which is all ones.
+    typedef uint32_t Place;
+    __device__ __forceinline__ Place place(int32_t m) const { return base + (uint32_t)((m >> 3) & ~3); }
+    __device__ __forceinline__ uint32_t peek(Place at, int32_t) const
+    {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
+        return v;
+    }
+    // Adds `bit` where it is not in w; w becomes the word as it was.
+    __device__ __forceinline__ void add(Place at, uint32_t bit, uint32_t &w) const
     {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
-            : "+r"(was)
-            : "r"(base + 4u * (uint32_t)i), "r"(m), "r"((uint32_t)on));
-        return was;
+            "{\n\t.reg .pred p;\n\t.reg .b32 x;\n\tand.b32 x, %0, %2;\n\tsetp.eq.u32 p, x, 0;\n\t"
+            "@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
+            : "+r"(w)
+            : "r"(at), "r"(bit));
     }
     __device__ __forceinline__ void add_or(int i, uint32_t m, bool on) const
     {
@@ -312,9 +325,14 @@ struct Bits<true> {
     __device__ __forceinline__ uint4 get4(int i4) const { return __ldcg(reinterpret_cast<const uint4 *>(base) + i4); }
     __device__ __forceinline__ void put(int i, uint32_t v) const { base[i] = v; }
     __device__ __forceinline__ void put4(int i4, uint4 v) const { reinterpret_cast<uint4 *>(base)[i4] = v; }
-    __device__ __forceinline__ uint32_t fetch_or(int i, uint32_t m, bool on, uint32_t was) const
+    // A read before the atomic would cost as much as the atomic itself: `peek`
+    // only tells vertices from -1.
+    typedef int Place;
+    __device__ __forceinline__ Place place(int32_t m) const { return m >> 5; }
+    __device__ __forceinline__ uint32_t peek(Place, int32_t m) const { return m < 0 ? ~0u : 0u; }
+    __device__ __forceinline__ void add(Place at, uint32_t bit, uint32_t &w) const
     {
-        return on ? atomicOr(base + i, m) : was;
+        if (!(w & bit)) w = atomicOr(base + at, bit);
     }
     __device__ __forceinline__ void add_or(int i, uint32_t m, bool on) const
     {
@@ -358,11 +376,14 @@ struct Frontier {
     int32_t *spill;   // global memory, at least n entries
 };
 
-__device__ __forceinline__ void ring_put(const Frontier &f, int p, int32_t m, bool on)
+// Queues m at p where the bit was not in w and m < s.
+__device__ __forceinline__ void ring_put(const Frontier &f, int p, int32_t m, uint32_t w, uint32_t bit, int32_t s)
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(
-                     f.ring + 4u * (uint32_t)(p & (f.ring_size - 1))),
-                 "r"(m), "r"((uint32_t)on));
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 x;\n\tand.b32 x, %2, %3;\n\tsetp.eq.u32 p, x, 0;\n\t"
+        "setp.lt.and.s32 q, %1, %4, p;\n\t@q st.shared.u32 [%0], %1;\n\t}" ::"r"(
+            f.ring + 4u * (uint32_t)(p & (f.ring_size - 1))),
+        "r"(m), "r"(w), "r"(bit), "r"(s));
 }
 
 __device__ __forceinline__ int32_t ring_get(const Frontier &f, int p)
@@ -375,8 +396,17 @@ __device__ __forceinline__ int32_t ring_get(const Frontier &f, int p)
 __device__ __forceinline__ void fr_put(const Frontier &f, int p, int w0, int32_t m, bool on)
 {
     const bool in = p - w0 < f.ring_size;
-    ring_put(f, p, m, on && in);
+    ring_put(f, p, m, on && in ? 0u : 1u, 1u, INT32_MAX);
     if (on && !in) f.spill[p] = m;
+}
+
+// The ring's entry at p where p < end, else `none`.
+__device__ __forceinline__ int32_t ring_get(const Frontier &f, int p, int end, int32_t none)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\t@p ld.shared.u32 %0, [%1];\n\t}"
+                 : "+r"(none)
+                 : "r"(f.ring + 4u * (uint32_t)(p & (f.ring_size - 1))), "r"(p), "r"(end));
+    return none;
 }
 
 __device__ __forceinline__ int32_t fr_get(const Frontier &f, int p, int w0)
@@ -429,9 +459,9 @@ struct SharedState {
     long long pool_base;    // the chain's pool range (-1: pool short)
     // tallies, kept by the leader's first lane: levels, then cycles of the
     // sources' own steps, their levels, list output, clearing, snapshots, wait
-    // for the other pass; sources; reused sources
+    // for the other pass; sources; those that started afresh
     unsigned long long prof[8];
-    unsigned long long nsrc, nreuse;
+    unsigned long long nsrc, nfresh;
     unsigned long long work[3];   // edges, pass-G expansions, pass-G input degrees
     int snaps;              // L: snapshots taken in this piece
     int snap_credit;        // L: how many more may be saved
@@ -453,7 +483,7 @@ __device__ __forceinline__ void init_state(SharedState &sh)
     sh.stamp = nullptr;
     sh.nh = 0;
     for (int q = 0; q < 8; q++) sh.prof[q] = 0;
-    sh.nsrc = sh.nreuse = 0;
+    sh.nsrc = sh.nfresh = 0;
     sh.work[0] = sh.work[1] = sh.work[2] = 0;
     sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
     sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
@@ -475,6 +505,13 @@ __device__ __forceinline__ void helper_sync(int bar)
     if (GT == 64) __syncwarp();
     else if (bar == 1) asm volatile("bar.sync 4, %0;" ::"n"(GT - 32) : "memory");
     else asm volatile("bar.sync 5, %0;" ::"n"(GT - 32) : "memory");
+}
+
+__device__ __forceinline__ uint32_t clock32()
+{
+    uint32_t c;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+    return c;
 }
 
 // Barrier of the two leader warps of a CTA that runs both passes of a source.
@@ -533,6 +570,7 @@ struct Trav {
     PassGraph g;
     const int32_t *rawdeg;
     int pass;
+    int32_t n;
     Bits<GBM> bits;
     Frontier f;
     uint16_t *stamp;       // the chain's stamps (pattern mode, else null)
@@ -545,6 +583,7 @@ struct Trav {
 // ends); the per-source ones live in SharedState, kept by one thread.
 struct Tally {
     uint32_t edges = 0, xcnt = 0, einsp = 0;
+    uint32_t slot = 0;   // sums of slot words: lanes 0, 8, .. degrees, lanes 1, 9, .. input degrees
 };
 
 // The sum of a 32-bit tally over a warp, and its addition to a 64-bit counter.
@@ -557,41 +596,43 @@ __device__ __forceinline__ void fold_tally(unsigned long long *to, uint32_t v, i
 
 __device__ __forceinline__ void fold_work(SharedState &sh, const Tally &acc, int pass, int lane)
 {
-    fold_tally(&sh.work[0], acc.edges, lane);
+    fold_tally(&sh.work[0], acc.edges + ((lane & 7) == 0 ? acc.slot : 0u), lane);
     if (pass) return;
     fold_tally(&sh.work[1], acc.xcnt, lane);
-    fold_tally(&sh.work[2], acc.einsp, lane);
+    fold_tally(&sh.work[2], acc.einsp + ((lane & 7) == 1 ? acc.slot : 0u), lane);
 }
 
-// One warp step: sets the bits m, one per lane and u, all of them in flight
-// together and without branches -- the words' reads first (not in global
-// memory, where a read would cost as much as the atomic), then the atomics of
-// those that look unset, then the summaries of words that became nonzero.  A
-// lane without an id holds s, which is set (or is to be: seeding).  New vertices
-// below s are queued for the next level (alloc(k) hands out k positions,
-// warp-uniformly; w0 is the first position of the level whose vertices found
-// them); the others, s itself included, are counted (the return value,
-// warp-uniform).  Every new vertex above the chain's first source gets the
-// chain index of s as its stamp (pattern mode).
+// One warp step: sets the bits m, one per lane and u (-1: none), all of them in
+// flight together and without branches -- the words' reads first (not in global
+// memory), then the atomics of those that look unset, then the summaries of
+// words that became nonzero.  New vertices below s are queued for the next
+// level (alloc(k) hands out k positions, warp-uniformly; w0 is the first
+// position of the level whose vertices found them); the others, s itself
+// included, are counted (the return value, warp-uniform).  Every new vertex
+// above the chain's first source gets the chain index of s as its stamp
+// (pattern mode).  The integer pipe bounds this code (it issues every other
+// cycle, and ran at 80% of that on the 300 x 300 grid), so every instruction
+// here is counted: predicates are formed inside the memory operations, and a
+// lane without an id needs no test of its own.
 template <int U, bool GBM, class Alloc>
 __device__ __forceinline__ int visit(const Trav<GBM> &t, const int32_t (&m)[U], int32_t s, int cidx, int w0,
                                      Alloc alloc)
 {
-    const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
     uint32_t w[U], bit[U];
+    typename Bits<GBM>::Place at[U];
     bool any = false;
 #pragma unroll
     for (int u = 0; u < U; u++) {
         bit[u] = 1u << (m[u] & 31);
-        // GBM: of the lanes without an id, the last one sees to s
-        w[u] = GBM ? (m[u] == s && lane != 31 ? ~0u : 0u) : t.bits.get(m[u] >> 5);
+        at[u] = t.bits.place(m[u]);
+        w[u] = t.bits.peek(at[u], m[u]);
     }
 #pragma unroll
     for (int u = 0; u < U; u++) any |= !(w[u] & bit[u]);
     if (!__any_sync(0xffffffffu, any)) return 0;
 #pragma unroll
-    for (int u = 0; u < U; u++) w[u] = t.bits.fetch_or(m[u] >> 5, bit[u], !(w[u] & bit[u]), w[u]);
+    for (int u = 0; u < U; u++) t.bits.add(at[u], bit[u], w[u]);
     any = false;
 #pragma unroll
     for (int u = 0; u < U; u++) any |= w[u] == 0u;
@@ -605,31 +646,34 @@ __device__ __forceinline__ int visit(const Trav<GBM> &t, const int32_t (&m)[U], 
             if (!(w[u] & bit[u]) && m[u] > s - cidx) t.stamp[m[u]] = (uint16_t)cidx;
     }
     unsigned low[U];
-    int nlow = 0, nnew = 0;
+    int nlow = 0, nhigh = 0;
 #pragma unroll
     for (int u = 0; u < U; u++) {
-        const unsigned f = __ballot_sync(0xffffffffu, !(w[u] & bit[u]));
-        low[u] = f & __ballot_sync(0xffffffffu, m[u] < s);
-        nnew += __popc(f);
+        low[u] = __ballot_sync(0xffffffffu, !(w[u] & bit[u]) && m[u] < s);
         nlow += __popc(low[u]);
+        nhigh += __popc(__ballot_sync(0xffffffffu, !(w[u] & bit[u]) && m[u] >= s));
     }
     if (nlow) {
         int pos = alloc(nlow);
         if (pos + nlow - w0 <= t.f.ring_size) {
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                ring_put(t.f, pos + __popc(low[u] & below), m[u], (low[u] >> lane) & 1u);
+                ring_put(t.f, pos + __popc(low[u] & below), m[u], w[u], bit[u], s);
                 pos += __popc(low[u]);
             }
         } else {
-#pragma unroll
+#pragma unroll 1
             for (int u = 0; u < U; u++) {
-                fr_put(t.f, pos + __popc(low[u] & below), w0, m[u], (low[u] >> lane) & 1u);
-                pos += __popc(low[u]);
+                int32_t mu = m[0], lu = low[0];
+#pragma unroll
+                for (int k = 1; k < U; k++)
+                    if (u == k) { mu = m[k]; lu = low[k]; }
+                fr_put(t.f, pos + __popc(lu & below), w0, mu, (lu >> (threadIdx.x & 31)) & 1u);
+                pos += __popc(lu);
             }
         }
     }
-    return nnew - nlow;
+    return nhigh;
 }
 
 // The rows of up to 32 frontier vertices -- each lane holds the bounds of one,
@@ -671,7 +715,7 @@ __device__ __forceinline__ int expand_edges(const Trav<GBM> &t, int32_t b, int32
             __reduce_or_sync(0xffffffffu, (unsigned)(excl - e0) < 32u ? 1u << (excl - e0) : 0u);
         const int row = before + __popc(begins & upto) - 1;
         const int32_t at = __shfl_sync(0xffffffffu, from, row & 31) + e0 + lane;
-        return e0 + lane < total ? ld<CG>(t.g.adj + at) : s;
+        return e0 + lane < total ? ld<CG>(t.g.adj + at) : -1;
     };
     int e0 = 0;
     for (; total - e0 > 32; e0 += 128) {   // 128 ids in flight
@@ -700,39 +744,40 @@ __device__ __forceinline__ int expand_slots(const Trav<GBM> &t, int first, int c
 {
     const int lane = threadIdx.x & 31;
     const int j = lane & 7;
+    const int32_t *const word = reinterpret_cast<const int32_t *>(t.g.slot) + j;
     int32_t v[U], m[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) {   // lanes past the last vertex read its slot again
-        const int p = first + min(4 * u + (lane >> 3), cnt - 1);
-        v[u] = in_ring ? ring_get(t.f, p) : fr_get(t.f, p, wstart);
+    for (int u = 0; u < U; u++) {   // past the last vertex: the empty slot behind the others
+        const int p = first + 4 * u + (lane >> 3);
+        v[u] = t.n;
+        if (in_ring) v[u] = ring_get(t.f, p, first + cnt, t.n);
+        else if (p < first + cnt) v[u] = fr_get(t.f, p, wstart);
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) m[u] = ld<CG>(reinterpret_cast<const int32_t *>(t.g.slot) + 8 * (int64_t)v[u] + j);
-    bool lng = false;
+    for (int u = 0; u < U; u++) m[u] = ld<CG>(word + 8 * (int64_t)v[u]);
+    int32_t most = 0;
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-        const bool on = 4 * u + (lane >> 3) < cnt;
-        if (on && j == 0) acc.edges += (unsigned)m[u];
-        if (on && j == 1) acc.einsp += (unsigned)m[u];
-        lng |= j == 0 && m[u] > SLOT_NB;
+    for (int u = 0; u < U; u++) {   // lane j = 0 sums degrees, j = 1 input degrees
+        acc.slot += (uint32_t)m[u];
+        most = max(most, m[u]);
     }
     b = d = 0;
-    if (__any_sync(0xffffffffu, lng)) {   // those rows are read from adj: nothing from their slots
+    if (__any_sync(0xffffffffu, j == 0 && most > SLOT_NB)) {   // long rows are read from adj
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int own = __shfl_sync(0xffffffffu, m[u], lane & 24);
             const int deg = __shfl_sync(0xffffffffu, m[u], (lane & 3) << 3);
             const int off = __shfl_sync(0xffffffffu, m[u], ((lane & 3) << 3) + 1);
-            if ((lane >> 2) == u && lane < cnt && deg > SLOT_NB) { d = deg; b = off; }
+            if ((lane >> 2) == u && deg > SLOT_NB) { d = deg; b = off; }
             if (own > SLOT_NB) {
-                if (j == 1 && 4 * u + (lane >> 3) < cnt) acc.einsp += (unsigned)(ld<CG>(t.rawdeg + v[u]) - m[u]);
+                if (j == 1) acc.slot += (uint32_t)(ld<CG>(t.rawdeg + v[u]) - m[u]);
                 m[u] = -1;
             }
         }
     }
 #pragma unroll
     for (int u = 0; u < U; u++)
-        if (j < 2 || m[u] < 0) m[u] = s;   // ids past the degree are -1
+        if (j < 2) m[u] = -1;
     return visit<U, GBM>(t, m, s, cidx, w0, alloc);
 }
 
@@ -750,12 +795,14 @@ __device__ __forceinline__ int expand(const Trav<GBM> &t, int first, int cnt, in
     if (t.g.slot != nullptr) {
         if (cnt <= 4) {
             nh = expand_slots<1, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
+        } else if (cnt <= 8) {
+            nh = expand_slots<2, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         } else if (cnt <= 16) {
             nh = expand_slots<4, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         } else {
             // a lane a vertex, six ids a lane: fewer instructions a vertex,
             // for levels that keep every warp busy
-            int32_t m[SLOT_NB] = {s, s, s, s, s, s};
+            int32_t m[SLOT_NB] = {-1, -1, -1, -1, -1, -1};
             if (lane < cnt) {
                 const int32_t v = fr_get(t.f, first + lane, wstart);
                 const int4 sl0 = ld4<CG>(t.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(t.g.slot + 2 * (int64_t)v + 1);
@@ -765,8 +812,6 @@ __device__ __forceinline__ int expand(const Trav<GBM> &t, int first, int cnt, in
                 if (d <= SLOT_NB) {   // ids past the degree are -1 in the slot
                     acc.einsp += (unsigned)b;
                     m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
-#pragma unroll
-                    for (int u = 0; u < SLOT_NB; u++) m[u] = m[u] < 0 ? s : m[u];
                     d = 0;
                 } else if (t.pass == 0) {
                     acc.einsp += (unsigned)ld<CG>(t.rawdeg + v);
@@ -807,7 +852,11 @@ __device__ __forceinline__ void run_levels(const Trav<GBM> &t, SharedState &sh, 
         const int cnt = end - start;
         // vertices a warp takes at a time: fewer than its lanes could, while
         // that keeps every warp busy
-        const int take = cnt <= 4 * NW ? 4 : (cnt <= 16 * NW ? 16 : 32);
+        const int take = t.g.slot == nullptr ? min(32, max(1, (cnt + NW - 1) / NW))
+                         : cnt <= 4 * NW     ? 4
+                         : cnt <= 8 * NW     ? 8
+                         : cnt <= 32 * NW    ? 16
+                                             : 32;
         auto alloc = [&](int k) {
             int p = 0;
             if (lane == 0) p = atomicAdd(tailp, k);
@@ -1255,6 +1304,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         tally(sh.prof[1], 0ull - c);
     };
     tally(sh.prof[1], 0ull - (unsigned long long)clock64());
+    uint32_t n_levels = 0, c_levels = 0, c_wait = 0;
 
     int prev = -2;
     int cidx = -1;            // index of the last source in its chain (-1: none yet)
@@ -1403,7 +1453,9 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             if (~both) cut = min(cut, __ffs(~both) - 1);
             if (cut > 0) {
                 win = win && ei < cut;
-                mark_word(t.bits, x >> 5, t.bits.fetch_or(x >> 5, 1u << (x & 31), win, ~0u) == 0u);
+                uint32_t w = win ? 0u : ~0u;
+                t.bits.add(t.bits.place(x), 1u << (x & 31), w);
+                mark_word(t.bits, x >> 5, w == 0u);
                 if (win && t.stamp != nullptr) t.stamp[x] = (uint16_t)(cidx + 1 + ei);
                 // lane i: source s + i; events are in row order
                 const unsigned wins = __ballot_sync(0xffffffffu, win);
@@ -1431,8 +1483,6 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 hc = __shfl_sync(0xffffffffu, c, cut - 1);
                 cidx += cut;
                 prev = s + cut - 1;
-                tally(sh.nsrc, (unsigned)cut);
-                tally(sh.nreuse, (unsigned)cut);
                 mine = (run_set >> cut) & 1u;
                 other = (oset >> cut) & 1u;
                 s += cut;
@@ -1468,17 +1518,17 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         }
         if (reuse) {
             cidx++;
-            tally(sh.nreuse, 1u);
         } else {
             if (cidx >= 0) end_chain();
             if (!more) break;   // the next piece starts from an empty bitmap
+            tally(sh.nfresh, 1u);
             cidx = 0;
             hc = 0;
             total = 0;
             if (nsnap > 0 && lane == 0) sh.weight = 0;
         }
 
-        // Seeding: s itself (in the lanes that the row leaves) and its neighbours;
+        // Seeding: s itself (in the lane after its row) and its neighbours;
         // those below s are the first
         // level.  nh counts new vertices above s, and s when it is new: a
         // source that was set already was counted by the sources before it.
@@ -1506,7 +1556,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 if (best < 0) break;
                 const long long c0 = clock64();
                 if (!self) {   // before the merge, which leaves it out
-                    const int32_t m[1] = {s};
+                    const int32_t m[1] = {lane == 0 ? s : -1};
                     nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
                     self = true;
                 }
@@ -1530,17 +1580,16 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         }
         {
             auto id = [&](int k) { return in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(t.g.adj + b0 + k); };
-            const int32_t m[1] = {lane < d0 ? id(lane) : s};
+            const int32_t m[1] = {lane < d0 ? id(lane) : (lane == d0 && !self ? s : -1)};
             nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
             for (int k0 = 32; k0 < d0; k0 += 128) {
                 int32_t x[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) x[u] = k0 + 32 * u + lane < d0 ? id(k0 + 32 * u + lane) : s;
+                for (int u = 0; u < 4; u++) x[u] = k0 + 32 * u + lane < d0 ? id(k0 + 32 * u + lane) : -1;
                 nh += visit<4, GBM>(t, x, s, cidx, 0, alloc);
             }
-            // s where the row filled every lane
-            if (d0 >= 32 && !self) {
-                const int32_t m1[1] = {s};
+            if (d0 >= 32 && !self) {   // the row left no lane for s
+                const int32_t m1[1] = {lane == 0 ? s : -1};
                 nh += visit<1, GBM>(t, m1, s, cidx, 0, alloc);
             }
         }
@@ -1548,11 +1597,11 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         // level-synchronous expansion through vertices < s
         int start = 0, end = tail, wstart = 0;
         if (end > 0) {
-            const long long c0 = clock64();
+            const uint32_t c0 = clock32();
             do {
                 if (end - start <= SOLO_MAX) {
                     __syncwarp();   // the level's queue entries, for every lane
-                    tally(sh.prof[0], 1u);
+                    n_levels++;
                     nh += expand<CG, GBM>(t, start, end - start, wstart, s, cidx, start, acc, alloc);
                     wstart = start;
                     start = end;
@@ -1573,14 +1622,13 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                     nh += take_nh();
                 }
             } while (end > start);
-            spent(2, c0);
+            c_levels += clock32() - c0;
         }
 
         // |hi(s)|: the bits above s; the link flag; both passes' exchange
         hc += nh - 1;
         total += hc;
         if (nsnap > 0 && end > 0 && lane == 0) sh.weight += end;
-        tally(sh.nsrc, 1u);
         __syncwarp();
         mine = s + 1 < md.n && ((t.bits.get((s + 1) >> 5) >> ((s + 1) & 31)) & 1u);
         if (lane == 0) {
@@ -1595,10 +1643,10 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             if (lane == 0) pair_flag[par][half] = mine;
             if (nsnap > 0 && lane < SNAP_REACH)
                 sh.reach[par][lane] = (s >> 5) + lane < a.bitmap_words ? t.bits.get((s >> 5) + lane) : 0u;
-            const long long c0 = clock64();
+            const uint32_t c0 = clock32();
             pair_sync();
             other = pair_flag[par][1 - half] != 0;
-            spent(7, c0);
+            c_wait += clock32() - c0;
             if (nsnap > 0 && end > 0 && sh.weight >= heavy && sh.snap_credit > 0) {
                 const long long c0 = clock64();
                 int lo, hi;
@@ -1623,7 +1671,11 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     }
     fold_work(sh, acc, pass, lane);
     if (lane == 0) {
-        sh.prof[1] += (unsigned long long)clock64();
+        sh.nsrc += (unsigned)((s_hi - s_lo + stride - 1) / stride);
+        sh.prof[0] += n_levels;
+        sh.prof[2] += c_levels;
+        sh.prof[7] += c_wait;
+        sh.prof[1] += (unsigned long long)clock64() - c_levels - c_wait;
         sh.op = OP_EXIT;
     }
     __syncwarp();
@@ -1698,10 +1750,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
     // ---- phase 1: traversals ------------------------------------------------
     unsigned long long t_start = 0;
     if (tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
-    for (int w = tid; w < NS * a.state_words; w += BLOCK) state[w] = 0u;
+    for (int w = tid; w < NS * a.state_words; w += BLOCK) state[w] = w % a.state_words < STATE_PAD ? ~0u : 0u;
     if (gtid == 0) init_state(sh);
     Trav<GBM> t{};
-    t.bits = bits_at<GBM>(state + (size_t)half * a.state_words, a.bitmap_words);
+    t.bits = bits_at<GBM>(state + (size_t)half * a.state_words + STATE_PAD, a.bitmap_words);
     t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size, a.queue + trav * a.qcap};
     if (LISTS && a.want_pattern) {
         t.stamp = t.stamps = a.stamp + 2 * trav * a.stamp_stride;
@@ -1751,6 +1803,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
         t.g = g;
         t.rawdeg = md.rawdeg;
         t.pass = pass;
+        t.n = md.n;
         run_piece<BLOCK, PAIRED, false, GBM, LISTS>(a, md, t, s_lo, s_hi, rg.stride, shs, hist, pair_flag, half, gtid,
                                                     bar, phase);
         __syncthreads();   // every thread is done with s_piece
@@ -1766,7 +1819,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
             for (int h = 0; h < NS; h++) {
                 for (int q = 0; q < 3; q++) wk[q] += shs[h].work[q];
                 ns += shs[h].nsrc;
-                nr += shs[h].nreuse;
+                nr += shs[h].nsrc - shs[h].nfresh;
                 for (int q = 0; q < 8; q++) pv[q] += shs[h].prof[q];
             }
             atomicAdd(&a.counters[0], wk[0]);
@@ -2069,10 +2122,15 @@ __global__ void upload_fill_kernel(UploadArgs u, const int32_t *gptr, int32_t *g
 
 // Fills the 32-byte slot of every vertex of one pass graph: {degree, input
 // degree (pass G) or, of rows longer than SLOT_NB, the row's offset, the first
-// SLOT_NB ids (-1 past the degree)}.
+// SLOT_NB ids (-1 past the degree)}; one empty slot follows the last.
 __global__ void slot_fill_kernel(int32_t n, const int32_t *ptr, const int32_t *adj, const int32_t *rawdeg, int4 *slot)
 {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += (int64_t)gridDim.x * blockDim.x) {
+        if (v == n) {
+            slot[2 * v] = make_int4(0, 0, -1, -1);
+            slot[2 * v + 1] = make_int4(-1, -1, -1, -1);
+            break;
+        }
         const int32_t b = ptr[v], d = ptr[v + 1] - b;
         int32_t x[SLOT_NB];
 #pragma unroll

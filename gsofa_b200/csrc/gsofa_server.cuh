@@ -82,11 +82,11 @@ __global__ void __maxnreg__(64) serve_kernel(const __grid_constant__ ServeArgs s
     SharedState &sh = shs[half];
     uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * 2) * a.state_words : smem_dyn;
     uint32_t *const ring = (GBM ? smem_dyn : smem_dyn + (size_t)2 * a.state_words) + (size_t)half * a.ring_size;
-    for (int w = tid; w < 2 * a.state_words; w += BLOCK) state[w] = 0u;
+    for (int w = tid; w < 2 * a.state_words; w += BLOCK) state[w] = w % a.state_words < STATE_PAD ? ~0u : 0u;
     if (gtid == 0) init_state(sh);   // counts only: no lists, no stamps
     const int64_t trav = (int64_t)blockIdx.x * 2 + half;
     Trav<GBM> t{};
-    t.bits = bits_at<GBM>(state + (size_t)half * a.state_words, a.bitmap_words);
+    t.bits = bits_at<GBM>(state + (size_t)half * a.state_words + STATE_PAD, a.bitmap_words);
     t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size, a.queue + trav * a.qcap};
     t.stamp = nullptr;
     t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
@@ -124,6 +124,7 @@ __global__ void __maxnreg__(64) serve_kernel(const __grid_constant__ ServeArgs s
         t.g = md.g[half];
         t.rawdeg = md.rawdeg;
         t.pass = half;
+        t.n = md.n;
         if (gtid == 0) sh.snap_credit = SNAP_CREDIT;   // the piece may be another request's
         run_piece<BLOCK, true, true, GBM, false>(a, md, t, piece.s_lo, piece.s_hi, 1, shs, nullptr, pair_flag, half, gtid,
                                                  bar, phase);
