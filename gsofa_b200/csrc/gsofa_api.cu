@@ -261,7 +261,7 @@ void *factor_fn()
 void *factor_kernel_for(int block, bool paired, bool gbm = false, bool wide = false, bool lists = true)
 {
     if (!lists && paired) {
-        if (gbm && block == 256) return factor_fn<256, true, true, 4, false>();
+        if (gbm && block == 512) return factor_fn<512, true, true, 2, false>();
         if (wide && block == 512) return factor_fn<512, true, false, 1, false>();
         if (!gbm && !wide && block == 768) return factor_fn<768, true, false, 1, false>();
         if (!gbm && !wide && block == 1024) return factor_fn<1024, true, false, 1, false>();
@@ -429,7 +429,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
     int block = p.block_size;
     if (wide) block = 512;
     if (!block) {
-        if (gbm) block = paired ? 256 : 128;
+        if (gbm) block = paired ? 512 : 128;
         else if (paired && max_n > 8192) block = (!want_pattern && long_rows) ? 1024 : 768;
         else block = pick_block(max_n) * (paired ? 2 : 1);
     }
@@ -2336,6 +2336,8 @@ struct gsofa_server {
     int block = kServeBlock, ring = 1024, grid = 0;
     bool gbm = false;               // bitmaps in global memory (d_gstate)
     uint32_t *d_gstate = nullptr;
+    uint32_t *d_snap = nullptr;     // snapshots of finished traversals, snap_k a traversal slot
+    int snap_k = 0;
     int32_t bitmap_words = 0, state_words = 0;
     size_t smem = 0;
     cudaStream_t run = nullptr, io = nullptr;
@@ -2429,8 +2431,8 @@ gsofa_status server_launch_if_idle_impl(gsofa_server *s)
     a.state_words = s->state_words;
     a.ring_size = s->ring;
     a.gbm = s->d_gstate;
-    a.snap = nullptr;
-    a.snap_k = 0;
+    a.snap = s->d_snap;
+    a.snap_k = s->snap_k;
     a.reuse = 1;
     a.want_pattern = 0;
     a.L = s->lmax;
@@ -2540,7 +2542,19 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         const int64_t fixed = (int64_t)s->grid * 2 * s->max_n * 4 + gstate_bytes +
                               (int64_t)kServeClasses * s->piece_cap * sizeof(ServePiece) +
                               (int64_t)s->max_slots * (sizeof(MatDesc) + 4) + s->lmax * 10 + 4096;
-        s->arena_units = (budget - fixed) / kArenaUnit;
+        // snapshots: as many as a sixteenth of the budget holds
+        int64_t snap_bytes = 0;
+        for (int k = SNAP_MAX; k >= 2 && !s->snap_k; k >>= 1) {
+            snap_bytes = (int64_t)s->grid * 2 * s->bitmap_words * 4 * k;
+            if (snap_bytes <= budget / 16) s->snap_k = k;
+        }
+        if (!s->snap_k) snap_bytes = 0;
+        const int64_t least = units(server_graph_bytes(s->max_n, 8 * (int64_t)s->max_n)) * kArenaUnit;
+        if (budget - fixed - snap_bytes < least) {   // they only save time
+            s->snap_k = 0;
+            snap_bytes = 0;
+        }
+        s->arena_units = (budget - fixed - snap_bytes) / kArenaUnit;
         if (s->arena_units < units(server_graph_bytes(s->max_n, 8 * (int64_t)s->max_n))) {
             gsofa_server_destroy(s);
             return GSOFA_ERR_OOM;
@@ -2554,6 +2568,7 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         GS_CUDA(cudaMalloc(&s->d_nxt, (size_t)2 * s->lmax));
         GS_CUDA(cudaMalloc(&s->d_queue, (size_t)s->grid * 2 * s->max_n * 4));
         if (s->gbm) GS_CUDA(cudaMalloc(&s->d_gstate, (size_t)gstate_bytes));
+        if (s->snap_k) GS_CUDA(cudaMalloc(&s->d_snap, (size_t)snap_bytes));
         GS_CUDA(cudaMalloc(&s->d_arena, (size_t)s->arena_units * kArenaUnit));
         GS_CUDA(cudaMemsetAsync(s->d_ctl, 0, sizeof(ServeCtl) + 64, s->io));
         GS_CUDA(cudaMemsetAsync(s->d_done, 0, (size_t)s->max_slots * 4, s->io));
@@ -2608,6 +2623,7 @@ void gsofa_server_destroy(gsofa_server *s)
     cudaFree(s->d_nxt);
     cudaFree(s->d_queue);
     cudaFree(s->d_gstate);
+    cudaFree(s->d_snap);
     cudaFree(s->d_arena);
     if (s->run) cudaStreamDestroy(s->run);
     if (s->io) cudaStreamDestroy(s->io);

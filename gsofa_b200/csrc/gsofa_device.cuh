@@ -1318,7 +1318,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     if (lane < SNAP_MAX) sh.snap_t[lane] = -1;
     if (lane == 0) sh.snaps = sh.weight = 0;
     __syncwarp();
-    const int heavy = max(64, a.bitmap_words >> 3);   // worth a copy of the bitmap
+    const int heavy = max(64, md.n >> 8);   // worth a copy of the bitmap: an eighth of its words
 
     auto end_chain = [&]() {
         int lo, hi;
