@@ -464,7 +464,7 @@ struct SharedState {
     unsigned long long nsrc, nfresh;
     unsigned long long work[3];   // edges, pass-G expansions, pass-G input degrees
     int snaps;              // L: snapshots taken in this piece
-    int snap_credit;        // L: how many more may be saved
+    int snap_credit;        // L: what traversals and snapshots taken over have earned, in vertices (-1: none yet)
     int weight;             // L: vertices queued by the state's traversals
     uint32_t reach[2][SNAP_REACH];            // by exchange: this bitmap's words from the source's on
     uint32_t snap_reach[SNAP_MAX][SNAP_REACH];  // L: the other pass's words when the snapshot was taken
@@ -473,10 +473,6 @@ struct SharedState {
     int32_t win_adj[SEED_ADJ];                // L: the window's rows
     int32_t ev_x[33], ev_p[33];               // L: a run's new ids and their places in the window
 };
-
-// Snapshots that a CTA saves ahead of taking any over (each one taken over
-// earns eight more).
-constexpr int SNAP_CREDIT = 24;
 
 __device__ __forceinline__ void init_state(SharedState &sh)
 {
@@ -1266,8 +1262,7 @@ __device__ __forceinline__ int state_extent(const Bits<GBM> &b, int lane, int &l
 // snapshots that it provably contains.  On power-law matrices nearly half of
 // the sources do not contain s-1 but do contain some t a few lines below, whose
 // closure is most of the matrix: the 20,000-line one inspects 2.4e7 edges
-// instead of 2.7e8.  Where snapshots are saved but not taken over (meshes),
-// the piece's CTA stops saving them.
+// instead of 2.7e8.
 template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
 __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, Trav<GBM> &t, int32_t s_lo, int32_t s_hi,
                            int32_t stride, SharedState *shs, volatile int (*pair_flag)[2], int half,
@@ -1316,9 +1311,16 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     // the seeding window: lane i holds row bounds and degree of source wlo + i
     int wlo = 0, whi = 0, wb = 0, we = 0, wraw = 0, wadj0 = 0;
     if (lane < SNAP_MAX) sh.snap_t[lane] = -1;
-    if (lane == 0) sh.snaps = sh.weight = 0;
+    // A state of this many vertices is worth a copy of the bitmap (an eighth of
+    // its words), and a copy is paid with as many vertices traversed or taken
+    // over: where snapshots help, long traversals pay for them at once, and
+    // where traversals are short they cost next to nothing.
+    const int heavy = max(64, md.n >> 8);
+    if (lane == 0) {
+        sh.snaps = sh.weight = 0;
+        if (sh.snap_credit < 0) sh.snap_credit = 4 * heavy;
+    }
     __syncwarp();
-    const int heavy = max(64, md.n >> 8);   // worth a copy of the bitmap: an eighth of its words
 
     auto end_chain = [&]() {
         int lo, hi;
@@ -1562,8 +1564,8 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 }
                 const int k = __ffs(__ballot_sync(0xffffffffu, st == best)) - 1;
                 if (lane == 0) {
-                    sh.weight += sh.snap_w[k];
-                    sh.snap_credit += 8;
+                    sh.weight = min(sh.weight + sh.snap_w[k], 1 << 28);
+                    sh.snap_credit = min(sh.snap_credit + sh.snap_w[k], 1 << 28);
                     sh.src = s;
                     sh.cidx = cidx;
                     sh.snap = k;
@@ -1628,7 +1630,10 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         // |hi(s)|: the bits above s; the link flag; both passes' exchange
         hc += nh - 1;
         total += hc;
-        if (nsnap > 0 && end > 0 && lane == 0) sh.weight += end;
+        if (nsnap > 0 && end > 0 && lane == 0) {
+            sh.weight = min(sh.weight + end, 1 << 28);
+            sh.snap_credit = min(sh.snap_credit + end, 1 << 28);
+        }
         __syncwarp();
         mine = s + 1 < md.n && ((t.bits.get((s + 1) >> 5) >> ((s + 1) & 31)) & 1u);
         if (lane == 0) {
@@ -1647,7 +1652,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             pair_sync();
             other = pair_flag[par][1 - half] != 0;
             c_wait += clock32() - c0;
-            if (nsnap > 0 && end > 0 && sh.weight >= heavy && sh.snap_credit > 0) {
+            if (nsnap > 0 && end > 0 && sh.weight >= heavy && sh.snap_credit >= heavy) {
                 const long long c0 = clock64();
                 int lo, hi;
                 state_extent<GBM>(t.bits, lane, lo, hi);
@@ -1657,7 +1662,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 if (lane == 0) {
                     sh.snap_t[k] = s;
                     sh.snaps++;
-                    sh.snap_credit--;
+                    sh.snap_credit -= heavy;
                     sh.snap_w[k] = sh.weight;
                     sh.snap = k;
                     sh.snap_lo[k] = sh.lo = lo;
@@ -1798,7 +1803,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
             s_lo = sh.seg[0];
             s_hi = sh.seg[1];
         }
-        if (rg.mat != last_mat && gtid == 0) sh.snap_credit = SNAP_CREDIT;
+        if (rg.mat != last_mat && gtid == 0) sh.snap_credit = -1;
         last_mat = rg.mat;
         t.g = g;
         t.rawdeg = md.rawdeg;

@@ -125,7 +125,7 @@ __global__ void __maxnreg__(64) serve_kernel(const __grid_constant__ ServeArgs s
         t.rawdeg = md.rawdeg;
         t.pass = half;
         t.n = md.n;
-        if (gtid == 0) sh.snap_credit = SNAP_CREDIT;   // the piece may be another request's
+        if (gtid == 0) sh.snap_credit = -1;   // the piece may be another request's
         run_piece<BLOCK, true, true, GBM, false>(a, md, t, piece.s_lo, piece.s_hi, 1, shs, nullptr, pair_flag, half, gtid,
                                                  bar, phase);
         __syncthreads();
