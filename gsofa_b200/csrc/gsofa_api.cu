@@ -231,13 +231,19 @@ struct ExtPool {
     std::function<void()> while_running;
 };
 
-// Static shared memory of the factorization kernel, with some slack: a
-// SharedState per traversal and, for the list output, a row of 32 counters per
-// helper warp.
+// Shared memory of the factorization kernel beside bitmaps and rings.
+// lists: the instance has the list output (factor_kernel_for).
 constexpr int kMinRing = 512;
-size_t static_shared(int block, int ns, bool lists)
+constexpr size_t kStaticShared = 1024;   // the runtime's own and some slack
+size_t cta_shared(int block, int ns, bool lists) { return cta_bytes(ns, lists ? block / 32 - ns : 1); }
+
+// Launch shapes whose counts-only jobs run an instantiation without the list
+// output (fewer registers for the traversal).
+bool has_counts_form(int block, bool paired, bool gbm, bool wide)
 {
-    return sizeof(SharedState) * ns + (lists ? (size_t)(block / 32 - ns) * 128 : 0) + 512;
+    if (!paired) return false;
+    if (gbm || wide) return block == 512;
+    return block == 768 || block == 1024;
 }
 
 int pick_block(int32_t max_n)
@@ -260,11 +266,10 @@ void *factor_fn()
 // registers: no spills where the list output's code would cause them).
 void *factor_kernel_for(int block, bool paired, bool gbm = false, bool wide = false, bool lists = true)
 {
-    if (!lists && paired) {
-        if (gbm && block == 512) return factor_fn<512, true, true, 2, false>();
-        if (wide && block == 512) return factor_fn<512, true, false, 1, false>();
-        if (!gbm && !wide && block == 768) return factor_fn<768, true, false, 1, false>();
-        if (!gbm && !wide && block == 1024) return factor_fn<1024, true, false, 1, false>();
+    if (!lists && has_counts_form(block, paired, gbm, wide)) {
+        if (gbm) return factor_fn<512, true, true, 2, false>();
+        if (wide) return factor_fn<512, true, false, 1, false>();
+        return block == 768 ? factor_fn<768, true, false, 1, false>() : factor_fn<1024, true, false, 1, false>();
     }
     if (gbm) {
         switch (block) {
@@ -329,8 +334,9 @@ double now_ms()
     return duration<double, std::milli>(steady_clock::now().time_since_epoch()).count();
 }
 
-gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
-                     const gsofa_params *pin, gsofa_result *out, const ExtPool *ext = nullptr)
+// On at most *grid_io CTAs (returns how many it asked for).
+gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
+                        const gsofa_params *pin, gsofa_result *out, const ExtPool *ext, int *grid_io)
 {
     static const bool host_timing = std::getenv("GSOFA_HOST_TIMING") != nullptr;
     const double t_enter = now_ms();
@@ -405,9 +411,9 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
     // paired kernel) up to ~850K lines and one up to ~1.7M; global memory
     // holds any number of any size.  GSOFA_FLAG_GLOBAL_STATE /
     // GSOFA_FLAG_SHARED_STATE choose; else shared memory while the pair fits.
-    const size_t pair_smem = (size_t)2 * state_needed * 4 + 2 * kMinRing * 4 + static_shared(768, 2, want_pattern);
+    const size_t pair_smem = (size_t)2 * state_needed * 4 + 2 * kMinRing * 4 + cta_shared(768, 2, want_pattern) + kStaticShared;
     if ((p.flags & GSOFA_FLAG_GLOBAL_STATE) && (p.flags & GSOFA_FLAG_SHARED_STATE)) return GSOFA_ERR_INVALID_INPUT;
-    const size_t single_smem = (size_t)state_needed * 4 + kMinRing * 4 + static_shared(512, 1, want_pattern);
+    const size_t single_smem = (size_t)state_needed * 4 + kMinRing * 4 + cta_shared(512, 1, true) + kStaticShared;
     const bool want_pair = reuse && p.reuse != 2;
     const bool gbm = (p.flags & GSOFA_FLAG_GLOBAL_STATE) ||
                      (!(p.flags & GSOFA_FLAG_SHARED_STATE) &&
@@ -445,11 +451,11 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
 
     const int32_t bitmap_words = words_needed;
     const int32_t state_words = state_needed;
-    const size_t static_smem = static_shared(block, NS, true);
+    const size_t fixed_smem = cta_shared(block, NS, want_pattern || !has_counts_form(block, paired, gbm, wide));
     // shared memory per traversal: its bitmap and summaries (unless in global
     // memory) and its frontier ring
     const size_t smem_state = gbm ? 0 : (size_t)state_words * 4;
-    if ((size_t)NS * (smem_state + kMinRing * 4) + static_smem > ctx->smem_optin) return GSOFA_ERR_UNSUPPORTED;
+    if ((size_t)NS * (smem_state + kMinRing * 4) + fixed_smem + kStaticShared > ctx->smem_optin) return GSOFA_ERR_UNSUPPORTED;
     // frontier ring: the largest of 8K down to 512 entries that keeps the most
     // CTAs (each with its own bitmap) resident on an SM; sized once per shape
     int ring = 0, occ = 0;
@@ -461,12 +467,12 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
             ring = sh.ring; occ = sh.occ; cached = true;
         }
     if (cached) {
-        smem = (size_t)NS * (smem_state + (size_t)ring * 4);
+        smem = fixed_smem + (size_t)NS * (smem_state + (size_t)ring * 4);
     } else {
         std::lock_guard<std::mutex> lk(kernel_attr_mutex());
         for (int cand = 8192; cand >= kMinRing; cand >>= 1) {
-            const size_t sm = (size_t)NS * (smem_state + (size_t)cand * 4);
-            if (sm + static_smem > ctx->smem_optin) continue;
+            const size_t sm = fixed_smem + (size_t)NS * (smem_state + (size_t)cand * 4);
+            if (sm + kStaticShared > ctx->smem_optin) continue;
             GS_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             int o = 0;
             GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kfn, block, sm));
@@ -495,21 +501,32 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
                                (int64_t)ctx->gstate.bytes - (int64_t)ctx->lists.bytes - (int64_t)ctx->snap.bytes;
         const int64_t room = (int64_t)ctx->budget - others - fixed;
         if (room < per_cta) return GSOFA_ERR_OOM;
-        grid = (int)std::min<int64_t>(grid, room / per_cta);
+        grid = (int)std::min<int64_t>(std::min(grid, *grid_io), room / per_cta);
+        *grid_io = grid;
     }
-    // sources per work piece: a piece's first source cannot reuse state, so
-    // pieces are long (up to 512 sources) while there are still about eight
-    // per concurrent traversal -- the last pieces handed out are the light,
-    // low-numbered sources, so the launch's tail stays short
+    // Sources per work piece.  A piece's first source cannot reuse state, and
+    // its traversal from nothing costs as much as hundreds of later ones, so
+    // pieces should be few and long, and yet the launch must not wait for the
+    // last one.  Paired passes with reuse share their pieces: a CTA that has
+    // run out takes part of another's.  Two a CTA for counts (the 200K-line
+    // power-law matrix takes 19.4 ms, and 20.3 with three; 300^2 grid 2.57 and
+    // 3.04; the 80^3 stencil 4.24 and 4.35; fixed pieces, eight a CTA, took
+    // 23.2, 7.1 and 4.6), two and a half with lists, which weigh more beside
+    // the fresh starts (80^3: 8.5 ms with two, 7.7 with two and a half).
     int chunk = p.src_chunk;
-    if (chunk <= 0) {
+    const int64_t mult = paired ? 1 : 2;
+    const int64_t lines = line_range ? (int64_t)(range_hi - range_lo) : L;
+    const bool share = paired && reuse && chunk <= 0 && max_n <= (int32_t)(UNIT << UNIT_BITS) - UNIT &&
+                       count < (1 << (64 - 2 * UNIT_BITS));
+    if (share) {
+        const int64_t per = 2 * lines / ((int64_t)(want_pattern ? 5 : 4) * grid) + 1;
+        chunk = (int)std::max<int64_t>(32, (std::min<int64_t>(per, 1 << 20) + UNIT - 1) / UNIT * UNIT);
+    } else if (chunk <= 0) {
         // a line range keeps the pieces the whole matrix would have (smaller
         // ones start more traversals afresh, and a fresh start costs most in
         // the separator lines a range of the last lines holds) while every
         // CTA still gets about four pieces; shorter ranges take the length
         // that gives every CTA four, or eight, pieces
-        const int64_t mult = paired ? 1 : 2;
-        const int64_t lines = line_range ? (int64_t)(range_hi - range_lo) : L;
         const int64_t per = std::max(mult * lines / ((int64_t)8 * grid),
                                      std::min(mult * L / ((int64_t)8 * grid), mult * lines / ((int64_t)4 * grid)));
         chunk = reuse ? (int)std::min<int64_t>(512, std::max<int64_t>(32, per)) : 1;
@@ -538,7 +555,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         }
         r.piece_base = npieces;
         // the bottom eighth in quarter-length pieces (the last handed out)
-        r.tail = (reuse && chunk >= 64) ? r.nj / 8 : 0;
+        r.tail = (reuse && chunk >= 64 && !share) ? r.nj / 8 : 0;
         r.small = r.tail ? std::max(32, chunk / 4) : chunk;
         r.npieces = (paired ? 1 : 2) * pieces_per_pass(r);
         npieces += r.npieces;
@@ -588,7 +605,9 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         int32_t *d_sn = (int32_t *)ctx->grow(ctx->snlist, (size_t)L * sizeof(int32_t));
         int64_t *d_tiles = (int64_t *)ctx->grow(ctx->tiles, (size_t)4 * ntiles * sizeof(int64_t));
         // misc: piece counter, pool tail, counters[4], status
-        char *d_misc = (char *)ctx->grow(ctx->misc, 256);
+        // and shared pieces: two words a CTA, the costs of pieces' beginnings
+        const size_t misc_bytes = 256 + (share ? (size_t)grid * 16 + FRESH_BUCKETS * 4 : 0);
+        char *d_misc = (char *)ctx->grow(ctx->misc, misc_bytes);
         unsigned long long *d_piece = (unsigned long long *)d_misc;
         unsigned long long *d_tail = (unsigned long long *)(d_misc + 8);
         unsigned long long *d_counters = (unsigned long long *)(d_misc + 16);   // 16 counters
@@ -640,6 +659,9 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         a.ranges = d_ranges;
         a.npieces = npieces;
         a.piece_counter = d_piece;
+        a.shared_piece = share ? (unsigned long long *)(d_misc + 256) : nullptr;
+        a.shared_cost = share ? a.shared_piece + grid : nullptr;
+        a.fresh_cost = share ? (unsigned *)(a.shared_cost + grid) : nullptr;
         a.queue = d_queue;
         a.qcap = qcap;
         a.bitmap_words = bitmap_words;
@@ -693,7 +715,7 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
             if (!ranges.empty())
                 GS_CUDA(cudaMemcpyAsync(d_ranges, rg_src, ranges.size() * sizeof(Range),
                                         cudaMemcpyHostToDevice, st));
-            GS_CUDA(cudaMemsetAsync(d_misc, 0, 256, st));
+            GS_CUDA(cudaMemsetAsync(d_misc, 0, misc_bytes, st));
             if (a.want_pattern) GS_CUDA(cudaMemsetAsync(d_lrow, 0, (size_t)L * sizeof(int32_t), st));
             if (a.blk_done) GS_CUDA(cudaMemsetAsync(a.blk_done, 0, (size_t)ext->nblk * 4, st));
             if (subset) {
@@ -898,6 +920,29 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         return GSOFA_OK;
     }
     return GSOFA_ERR_QUEUE_OVERFLOW;
+}
+
+// The job on as many CTAs as the budget holds: where it runs out of memory (the
+// lists' pool comes after the traversals' scratch), it is tried again on three
+// quarters of them.
+gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
+                     const gsofa_params *pin, gsofa_result *out, const ExtPool *ext = nullptr)
+{
+    int grid = INT32_MAX;
+    for (;;) {
+        gsofa_status s;
+        try {
+            s = run_job_on(ctx, count, mats, pin, out, ext, &grid);
+        } catch (CudaFail &f) {
+            if (f.e != cudaErrorMemoryAllocation || grid <= 1 || grid == INT32_MAX) throw;
+            cudaGetLastError();
+            s = GSOFA_ERR_OOM;
+        }
+        if (s != GSOFA_ERR_OOM || grid <= 1 || grid == INT32_MAX) return s;
+        for (int i = 0; i < count; i++) free_result_arrays(&out[i]);
+        for (DevBuf *b : {&ctx->queue, &ctx->stamp, &ctx->lists, &ctx->gstate, &ctx->snap}) ctx->release(*b);
+        grid = grid * 3 / 4;
+    }
 }
 
 }  // namespace
@@ -1751,8 +1796,8 @@ size_t gsofa_predict_scratch_bytes(const gsofa_ctx *c, int32_t n, int64_t nnz,
     b += 2 * (L + 1) * 8;                       // gptr
     b += (size_t)(n + 1) * 8 + (size_t)nnz * 8; // G and G^T
     b += (size_t)n * 64;                        // their 32-byte row slots
-    if (p.want_pattern)                         // chain stamps and list scratch, two traversals a CTA
-        b += grid * 2 * ((size_t)(n + 4095) / 4096 * 4096) * 4 + grid * 2 * qcap * 4;
+    if (p.want_pattern)                         // chain stamps, two traversals a CTA
+        b += grid * 2 * ((size_t)(n + 4095) / 4096 * 4096) * 2;
     return b;
 }
 
@@ -2086,7 +2131,7 @@ extern "C" gsofa_status gsofa_symbfact_counts_noalloc(int device, void *cuda_str
         const int32_t bitmap_words = ((n + 31) / 32 + 127) / 128 * 128;
         const int32_t state_words = STATE_PAD + bitmap_words + bitmap_words / 32 + ((bitmap_words / 32 + 31) / 32 + 3) / 4 * 4;
         const int ring = 4096;
-        const size_t smem = (size_t)state_words * 4 + (size_t)ring * 4;
+        const size_t smem = cta_shared(BLOCK, 1, true) + (size_t)state_words * 4 + (size_t)ring * 4;
         int occ = 0;
         {
             std::lock_guard<std::mutex> lk(kernel_attr_mutex());
@@ -2336,7 +2381,8 @@ struct gsofa_server {
     int block = kServeBlock, ring = 1024, grid = 0;
     bool gbm = false;               // bitmaps in global memory (d_gstate)
     uint32_t *d_gstate = nullptr;
-    uint32_t *d_snap = nullptr;     // snapshots of finished traversals, snap_k a traversal slot
+    uint32_t *d_snap = nullptr;     // snapshots of finished traversals, snap_k a traversal slot,
+    int64_t snap_units = 0;         // behind the arena
     int snap_k = 0;
     int32_t bitmap_words = 0, state_words = 0;
     size_t smem = 0;
@@ -2487,7 +2533,8 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         // runtime's memset kernels) of new requests run beside the serving
         // kernel instead of waiting for it to exit.
         const size_t reserve = 12 * 1024;
-        const size_t static_smem = 2 * sizeof(SharedState) + 1024 + reserve;
+        const size_t fixed_smem = cta_bytes(2, 1);
+        const size_t static_smem = kStaticShared + reserve;
         if ((cfg->flags & GSOFA_FLAG_GLOBAL_STATE) && (cfg->flags & GSOFA_FLAG_SHARED_STATE)) {
             delete s;
             return GSOFA_ERR_INVALID_INPUT;
@@ -2495,7 +2542,7 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         // the global-state form unless shared memory is asked for
         s->gbm = !(cfg->flags & GSOFA_FLAG_SHARED_STATE);
         s->block = s->gbm ? kServeBlockG : kServeBlock;
-        const int64_t per_half_words = ((int64_t)(s->optin - static_smem) / 2 - 1024 * 4) / 4;
+        const int64_t per_half_words = ((int64_t)(s->optin - static_smem - fixed_smem) / 2 - 1024 * 4) / 4;
         const int32_t limit_n =
             s->gbm ? (int32_t)(1 << 26)
                    : (int32_t)std::min<int64_t>((per_half_words - 64) * 32 / 33 / 128 * 128 * 32, INT32_MAX);
@@ -2514,7 +2561,7 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         const size_t smem_state = s->gbm ? 0 : (size_t)s->state_words * 4;
         s->ring = 0;
         for (int cand = 8192; cand >= 1024; cand >>= 1) {
-            const size_t sm = 2 * (smem_state + (size_t)cand * 4);
+            const size_t sm = fixed_smem + 2 * (smem_state + (size_t)cand * 4);
             if ((sm + static_smem - reserve) * per_sm + reserve <= (size_t)prop.sharedMemPerMultiprocessor &&
                 sm + static_smem <= s->optin) {
                 s->ring = cand;
@@ -2542,10 +2589,11 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         const int64_t fixed = (int64_t)s->grid * 2 * s->max_n * 4 + gstate_bytes +
                               (int64_t)kServeClasses * s->piece_cap * sizeof(ServePiece) +
                               (int64_t)s->max_slots * (sizeof(MatDesc) + 4) + s->lmax * 10 + 4096;
-        // snapshots: as many as a sixteenth of the budget holds
+        // snapshots: as many as a sixteenth of the budget holds, behind the
+        // arena, which takes their room when a request needs it (submit)
         int64_t snap_bytes = 0;
         for (int k = SNAP_MAX; k >= 2 && !s->snap_k; k >>= 1) {
-            snap_bytes = (int64_t)s->grid * 2 * s->bitmap_words * 4 * k;
+            snap_bytes = units((int64_t)s->grid * 2 * s->bitmap_words * 4 * k) * kArenaUnit;
             if (snap_bytes <= budget / 16) s->snap_k = k;
         }
         if (!s->snap_k) snap_bytes = 0;
@@ -2568,8 +2616,9 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         GS_CUDA(cudaMalloc(&s->d_nxt, (size_t)2 * s->lmax));
         GS_CUDA(cudaMalloc(&s->d_queue, (size_t)s->grid * 2 * s->max_n * 4));
         if (s->gbm) GS_CUDA(cudaMalloc(&s->d_gstate, (size_t)gstate_bytes));
-        if (s->snap_k) GS_CUDA(cudaMalloc(&s->d_snap, (size_t)snap_bytes));
-        GS_CUDA(cudaMalloc(&s->d_arena, (size_t)s->arena_units * kArenaUnit));
+        s->snap_units = snap_bytes / kArenaUnit;
+        GS_CUDA(cudaMalloc(&s->d_arena, (size_t)(s->arena_units + s->snap_units) * kArenaUnit));
+        if (s->snap_k) s->d_snap = (uint32_t *)(s->d_arena + s->arena_units * kArenaUnit);
         GS_CUDA(cudaMemsetAsync(s->d_ctl, 0, sizeof(ServeCtl) + 64, s->io));
         GS_CUDA(cudaMemsetAsync(s->d_done, 0, (size_t)s->max_slots * 4, s->io));
         GS_CUDA(cudaStreamSynchronize(s->io));
@@ -2623,7 +2672,6 @@ void gsofa_server_destroy(gsofa_server *s)
     cudaFree(s->d_nxt);
     cudaFree(s->d_queue);
     cudaFree(s->d_gstate);
-    cudaFree(s->d_snap);
     cudaFree(s->d_arena);
     if (s->run) cudaStreamDestroy(s->run);
     if (s->io) cudaStreamDestroy(s->io);
@@ -2659,6 +2707,19 @@ gsofa_status gsofa_server_submit(gsofa_server *s, int32_t n, int64_t nnz, const 
     const int64_t st_units = units(server_staging_bytes(n, nnz));
     r.g_units = units(server_graph_bytes(n, nnz));
     if (!s->lines.alloc(n, &r.lb)) return GSOFA_ERR_BUSY;
+    if (s->snap_k && s->reqs.empty() && r.g_units + st_units > s->arena_units) {
+        // snapshots only save time: with nothing in flight they give way
+        try {
+            GS_CUDA(cudaSetDevice(s->device));
+            if (cudaStreamQuery(s->run) == cudaErrorNotReady) server_stop_kernel(s);
+        } catch (CudaFail &f) {
+            s->lines.release(r.lb, n);
+            return fail_cuda(f.e);
+        }
+        s->snap_k = 0;
+        s->arena_units += s->snap_units;
+        s->arena.init(s->arena_units);
+    }
     if (!s->arena.alloc(r.g_units, &r.g_off)) {
         s->lines.release(r.lb, n);
         return GSOFA_ERR_BUSY;

@@ -89,6 +89,24 @@ __host__ __device__ inline int64_t pieces_per_pass(const Range &rg)
     return (top + rg.chunk - 1) / rg.chunk + ((int64_t)rg.tail + rg.small - 1) / rg.small;
 }
 
+// Shared pieces (paired passes with reuse, automatic piece length).  A CTA's
+// piece is a stretch of units of 8 sources of one range, which it claims from
+// below, an eighth of what is left at a time, while CTAs that have run out of
+// pieces take its upper part: a word per CTA holds {range, end, next unit}, and
+// a second one the costliest step so far beyond an average unit (a traversal
+// from nothing, which whoever takes a part has to run) and an average unit, in
+// 256 cycles.
+constexpr int UNIT = 8;
+constexpr int CLAIM_MAX = 8;   // units claimed at a time
+constexpr int UNIT_BITS = 20;
+constexpr unsigned long long UNIT_MASK = (1ull << UNIT_BITS) - 1;
+
+__device__ __forceinline__ unsigned long long piece_word(int range, int end, int next)
+{
+    return (unsigned long long)range << (2 * UNIT_BITS) | (unsigned long long)end << UNIT_BITS |
+           (unsigned long long)next;
+}
+
 // Error bits reported through JobArgs::status.
 enum : uint32_t {
     ERR_POOL_OVERFLOW = 1u,
@@ -102,6 +120,9 @@ struct JobArgs {
     const Range *ranges;
     int64_t npieces;
     unsigned long long *piece_counter; // dynamic fetch of work pieces
+    unsigned long long *shared_piece;  // shared pieces: a word per CTA (or null)
+    unsigned long long *shared_cost;   // ... and what its sources cost
+    unsigned *fresh_cost;      // ... and the first claims of pieces, by where they begin
     int32_t *queue;            // gridDim.x * qcap
     int64_t qcap;
     int32_t bitmap_words;      // shared-memory bitmap size (>= max n / 32, multiple of 128)
@@ -373,7 +394,6 @@ __device__ __forceinline__ void mark_word(const Bits<GBM> &b, int wi, bool on)
 struct Frontier {
     uint32_t ring;    // shared-window address
     int ring_size;
-    int32_t *spill;   // global memory, at least n entries
 };
 
 // Queues m at p where the bit was not in w and m < s.
@@ -393,11 +413,11 @@ __device__ __forceinline__ int32_t ring_get(const Frontier &f, int p)
     return v;
 }
 
-__device__ __forceinline__ void fr_put(const Frontier &f, int p, int w0, int32_t m, bool on)
+__device__ __forceinline__ void fr_put(const Frontier &f, int32_t *spill, int p, int w0, int32_t m, bool on)
 {
     const bool in = p - w0 < f.ring_size;
     ring_put(f, p, m, on && in ? 0u : 1u, 1u, INT32_MAX);
-    if (on && !in) f.spill[p] = m;
+    if (on && !in) spill[p] = m;
 }
 
 // The ring's entry at p where p < end, else `none`.
@@ -409,9 +429,9 @@ __device__ __forceinline__ int32_t ring_get(const Frontier &f, int p, int end, i
     return none;
 }
 
-__device__ __forceinline__ int32_t fr_get(const Frontier &f, int p, int w0)
+__device__ __forceinline__ int32_t fr_get(const Frontier &f, const int32_t *spill, int p, int w0)
 {
-    return p - w0 < f.ring_size ? ring_get(f, p) : f.spill[p];
+    return p - w0 < f.ring_size ? ring_get(f, p) : spill[p];
 }
 
 // Seeding window: the rows of up to SEED_WIN consecutive sources (SEED_ADJ
@@ -428,16 +448,40 @@ constexpr int SNAP_MAX = 8;
 constexpr int SNAP_REACH = 16;
 
 // Levels of at most this many vertices are run by a traversal's leader alone.
-constexpr int SOLO_MAX = 32;
+constexpr int SOLO_MAX = 16;
 
 // Work that a traversal's first warp (its leader) hands to its other warps, the
 // helpers.
 enum : int { OP_EXIT = 0, OP_LEVELS, OP_CLEAR, OP_LISTS, OP_SAVE, OP_MERGE };
 
+// A CTA's shared piece (word == nullptr: the piece is the CTA's alone).
+struct SharedPiece {
+    unsigned long long *word, *cost;
+    int32_t first, last;   // the range's sources [first, last)
+    int32_t s_lo;          // the piece's first source
+    volatile unsigned *fresh;   // where the cost of its first claim goes (JobArgs::fresh_cost)
+};
+
+// What a traversal needs now and then: kept in shared memory, since the
+// leader's registers are short.
+struct Home {
+    PassGraph g;             // the piece's pass graph
+    const int32_t *rawdeg;   // and input degrees
+    int32_t *spill;          // the frontier's entries past the ring
+    uint16_t *stamps;        // pattern mode: two stamp rows
+    int32_t *lists;          // pattern mode: a chain's vertices while its lists are written
+    uint32_t *snaps;         // snapshots
+    int64_t row;             // cnt / nxt / poff entry of the matrix's line 0 in this pass
+    int32_t *lrow;           // L row counts of the matrix's lines (pass G^T), or null
+    int32_t n;
+    int32_t pass;
+};
+
 // One traversal's shared state.  The leader warp runs the piece's sources and
 // alone touches the fields marked L; the other warps wait at the traversal's
 // barrier for an op, and the fields marked O are its arguments and results.
 struct SharedState {
+    Home home;
     int op;                 // O: OP_*
     int src, cidx;          // O: the source, its index in its chain
     int lv_start, lv_end, lv_wstart;   // O: OP_LEVELS: the level to start from
@@ -448,13 +492,20 @@ struct SharedState {
     int nh;                 // O: new vertices above the source that an op found
     int npush;              // O: queue entries that OP_MERGE made
     int seg[2];             // piece boundaries after chain alignment
+    SharedPiece own;        // (the first traversal's) the CTA's piece
+    volatile int next_end;  // shared pieces: where the claimed sources end
+    unsigned long long claim;   // ... the piece's word at the last claim
+    int claimed;            // ... units claimed there
+    int unit_done;          // ... sources done when it was made
+    unsigned unit_t, unit_sum, unit_mean, unit_most;   // ... when, what all units but the first took, a unit
+                            // takes on average, and the costliest step beyond that, in 256 cycles
     // list output (pattern mode): the chain -- consecutive sources sharing one
     // bitmap -- whose lists are written when it ends
     uint16_t *stamp;        // the chain's stamp row, or null (counts only)
     int chain_s0;           // its first source
-    int chain_len;          // its sources
+    int chain_first, chain_len;   // the lists to write: those of its sources [first, len)
     int chain_hi;           // no vertex above is set
-    int64_t chain_total;    // entries of its lists
+    int64_t chain_total;    // entries of those lists
     int64_t warp[32];       // per-warp counts of a chain's vertices
     long long pool_base;    // the chain's pool range (-1: pool short)
     // tallies, kept by the leader's first lane: levels, then cycles of the
@@ -483,6 +534,48 @@ __device__ __forceinline__ void init_state(SharedState &sh)
     sh.work[0] = sh.work[1] = sh.work[2] = 0;
     sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
     sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
+}
+
+// A traversal's home moves to pass `pass` of a matrix (its leader's first lane).
+__device__ __forceinline__ void settle(Home &h, const JobArgs &a, const MatDesc &md, int pass)
+{
+    h.g = md.g[pass];
+    h.rawdeg = md.rawdeg;
+    h.row = (int64_t)pass * a.L + md.line_base;
+    h.lrow = pass && a.want_pattern ? a.lrow + md.line_base : nullptr;
+    h.n = md.n;
+    h.pass = pass;
+}
+
+// A CTA's shared memory begins with this; bitmaps and rings follow.  It is at
+// the beginning of the dynamic part so that functions that are not inlined
+// reach it by a known shared address: the leader's and the helpers' code are
+// functions of their own, whose registers are allocated apart (as one body they
+// came out 20% slower or faster with every unrelated change).
+template <int NS, int HISTS>
+struct Cta {
+    JobArgs a;
+    SharedState t[NS];
+    volatile int pair_flag[2][2];   // [exchange parity][pass]: s+1 in hi(s), or a run's set sources
+    volatile long long piece;
+    volatile unsigned long long word;
+    int hist[HISTS][32];            // list output: a row a helper warp
+};
+
+template <int BLOCK, bool PAIRED, bool LISTS>
+using CtaOf = Cta<PAIRED ? 2 : 1, LISTS ? (PAIRED ? BLOCK / 32 - 2 : BLOCK / 32 - 1) : 1>;
+
+template <class C>
+__device__ __forceinline__ C &cta()
+{
+    extern __shared__ __align__(16) uint32_t smem_dyn[];
+    return *reinterpret_cast<C *>(smem_dyn);
+}
+
+// Bytes before the bitmaps (a multiple of 16).
+__host__ __device__ constexpr size_t cta_bytes(int ns, int hists)
+{
+    return ((ns == 2 ? sizeof(Cta<2, 1>) : sizeof(Cta<1, 1>)) + (size_t)(hists - 1) * 128 + 15) / 16 * 16;
 }
 
 // Barrier of the GT threads that work on one traversal: the whole CTA or one
@@ -560,19 +653,12 @@ __device__ __forceinline__ int32_t chain_start(const PassGraph &g, int32_t x, in
     return (y == 0 || !warp_has_prev(g, y)) ? y : x;
 }
 
-// What every warp of a traversal knows about it for one work piece.
+// What every warp of a traversal has in registers.
 template <bool GBM>
 struct Trav {
-    PassGraph g;
-    const int32_t *rawdeg;
-    int pass;
-    int32_t n;
     Bits<GBM> bits;
     Frontier f;
     uint16_t *stamp;       // the chain's stamps (pattern mode, else null)
-    uint16_t *stamps;      // this traversal's two stamp rows
-    int32_t *lists;        // pattern mode: a chain's vertices while its lists are written
-    uint32_t *snaps;       // this traversal's snapshots
 };
 
 // Per-thread tallies of one work piece (folded into SharedState::work when it
@@ -611,7 +697,7 @@ __device__ __forceinline__ void fold_work(SharedState &sh, const Tally &acc, int
 // here is counted: predicates are formed inside the memory operations, and a
 // lane without an id needs no test of its own.
 template <int U, bool GBM, class Alloc>
-__device__ __forceinline__ int visit(const Trav<GBM> &t, const int32_t (&m)[U], int32_t s, int cidx, int w0,
+__device__ __forceinline__ int visit(const Trav<GBM> &t, const SharedState &sh, const int32_t (&m)[U], int32_t s, int cidx, int w0,
                                      Alloc alloc)
 {
     const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
@@ -664,7 +750,7 @@ __device__ __forceinline__ int visit(const Trav<GBM> &t, const int32_t (&m)[U], 
 #pragma unroll
                 for (int k = 1; k < U; k++)
                     if (u == k) { mu = m[k]; lu = low[k]; }
-                fr_put(t.f, pos + __popc(lu & below), w0, mu, (lu >> (threadIdx.x & 31)) & 1u);
+                fr_put(t.f, sh.home.spill, pos + __popc(lu & below), w0, mu, (lu >> (threadIdx.x & 31)) & 1u);
                 pos += __popc(lu);
             }
         }
@@ -679,7 +765,7 @@ __device__ __forceinline__ int visit(const Trav<GBM> &t, const int32_t (&m)[U], 
 // id -- 32 rows' lines do not stay in the L1 that the bitmaps leave -- and ran
 // the 200,003-line power-law counts at 0.31 edges per SM cycle.)
 template <bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand_edges(const Trav<GBM> &t, int32_t b, int32_t d, int32_t s, int cidx, int w0,
+__device__ __forceinline__ int expand_edges(const Trav<GBM> &t, const SharedState &sh, int32_t b, int32_t d, int32_t s, int cidx, int w0,
                                             Alloc alloc)
 {
     const int lane = threadIdx.x & 31;
@@ -711,18 +797,18 @@ __device__ __forceinline__ int expand_edges(const Trav<GBM> &t, int32_t b, int32
             __reduce_or_sync(0xffffffffu, (unsigned)(excl - e0) < 32u ? 1u << (excl - e0) : 0u);
         const int row = before + __popc(begins & upto) - 1;
         const int32_t at = __shfl_sync(0xffffffffu, from, row & 31) + e0 + lane;
-        return e0 + lane < total ? ld<CG>(t.g.adj + at) : -1;
+        return e0 + lane < total ? ld<CG>(sh.home.g.adj + at) : -1;
     };
     int e0 = 0;
     for (; total - e0 > 32; e0 += 128) {   // 128 ids in flight
         int32_t m[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) m[u] = id(e0 + 32 * u);
-        nh += visit<4, GBM>(t, m, s, cidx, w0, alloc);
+        nh += visit<4, GBM>(t, sh, m, s, cidx, w0, alloc);
     }
     if (e0 < total) {
         const int32_t m[1] = {id(e0)};
-        nh += visit<1, GBM>(t, m, s, cidx, w0, alloc);
+        nh += visit<1, GBM>(t, sh, m, s, cidx, w0, alloc);
     }
     return nh;
 }
@@ -735,19 +821,19 @@ __device__ __forceinline__ int expand_edges(const Trav<GBM> &t, int32_t b, int32
 // level of a few vertices on the 80^3 matrix.)  Rows longer than a slot are
 // left to the caller: lane i gets the bounds (b, d) of vertex i, or d = 0.
 template <int U, bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand_slots(const Trav<GBM> &t, int first, int cnt, bool in_ring, int wstart, int32_t s,
+__device__ __forceinline__ int expand_slots(const Trav<GBM> &t, const SharedState &sh, int first, int cnt, bool in_ring, int wstart, int32_t s,
                                             int cidx, int w0, Tally &acc, Alloc alloc, int32_t &b, int32_t &d)
 {
     const int lane = threadIdx.x & 31;
     const int j = lane & 7;
-    const int32_t *const word = reinterpret_cast<const int32_t *>(t.g.slot) + j;
+    const int32_t *const word = reinterpret_cast<const int32_t *>(sh.home.g.slot) + j;
     int32_t v[U], m[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {   // past the last vertex: the empty slot behind the others
         const int p = first + 4 * u + (lane >> 3);
-        v[u] = t.n;
-        if (in_ring) v[u] = ring_get(t.f, p, first + cnt, t.n);
-        else if (p < first + cnt) v[u] = fr_get(t.f, p, wstart);
+        v[u] = sh.home.n;
+        if (in_ring) v[u] = ring_get(t.f, p, first + cnt, sh.home.n);
+        else if (p < first + cnt) v[u] = fr_get(t.f, sh.home.spill, p, wstart);
     }
 #pragma unroll
     for (int u = 0; u < U; u++) m[u] = ld<CG>(word + 8 * (int64_t)v[u]);
@@ -766,7 +852,7 @@ __device__ __forceinline__ int expand_slots(const Trav<GBM> &t, int first, int c
             const int off = __shfl_sync(0xffffffffu, m[u], ((lane & 3) << 3) + 1);
             if ((lane >> 2) == u && deg > SLOT_NB) { d = deg; b = off; }
             if (own > SLOT_NB) {
-                if (j == 1) acc.slot += (uint32_t)(ld<CG>(t.rawdeg + v[u]) - m[u]);
+                if (j == 1) acc.slot += (uint32_t)(ld<CG>(sh.home.rawdeg + v[u]) - m[u]);
                 m[u] = -1;
             }
         }
@@ -774,13 +860,15 @@ __device__ __forceinline__ int expand_slots(const Trav<GBM> &t, int first, int c
 #pragma unroll
     for (int u = 0; u < U; u++)
         if (j < 2) m[u] = -1;
-    return visit<U, GBM>(t, m, s, cidx, w0, alloc);
+    return visit<U, GBM>(t, sh, m, s, cidx, w0, alloc);
 }
 
 // Expands the frontier's entries [first, first + cnt), 0 < cnt <= 32, which were
-// written while the level starting at wstart ran.
-template <bool CG, bool GBM, class Alloc>
-__device__ __forceinline__ int expand(const Trav<GBM> &t, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
+// written while the level starting at wstart ran.  LEAD: the leader's small
+// levels, without the form for large ones, whose registers it would pay for all
+// the time.
+template <bool LEAD, bool CG, bool GBM, class Alloc>
+__device__ __forceinline__ int expand(const Trav<GBM> &t, const SharedState &sh, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
                                       Tally &acc, Alloc alloc)
 {
     const int lane = threadIdx.x & 31;
@@ -788,20 +876,20 @@ __device__ __forceinline__ int expand(const Trav<GBM> &t, int first, int cnt, in
     int32_t b = 0, d = 0;
     int nh = 0;
     if (lane == 0) acc.xcnt += cnt;
-    if (t.g.slot != nullptr) {
+    if (sh.home.g.slot != nullptr) {
         if (cnt <= 4) {
-            nh = expand_slots<1, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
+            nh = expand_slots<1, CG, GBM>(t, sh, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         } else if (cnt <= 8) {
-            nh = expand_slots<2, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
-        } else if (cnt <= 16) {
-            nh = expand_slots<4, CG, GBM>(t, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
+            nh = expand_slots<2, CG, GBM>(t, sh, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
+        } else if (LEAD || cnt <= 16) {
+            nh = expand_slots<4, CG, GBM>(t, sh, first, min(cnt, 16), in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         } else {
             // a lane a vertex, six ids a lane: fewer instructions a vertex,
             // for levels that keep every warp busy
             int32_t m[SLOT_NB] = {-1, -1, -1, -1, -1, -1};
             if (lane < cnt) {
-                const int32_t v = fr_get(t.f, first + lane, wstart);
-                const int4 sl0 = ld4<CG>(t.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(t.g.slot + 2 * (int64_t)v + 1);
+                const int32_t v = fr_get(t.f, sh.home.spill, first + lane, wstart);
+                const int4 sl0 = ld4<CG>(sh.home.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(sh.home.g.slot + 2 * (int64_t)v + 1);
                 d = sl0.x;
                 b = sl0.y;
                 acc.edges += (unsigned)d;
@@ -809,21 +897,21 @@ __device__ __forceinline__ int expand(const Trav<GBM> &t, int first, int cnt, in
                     acc.einsp += (unsigned)b;
                     m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
                     d = 0;
-                } else if (t.pass == 0) {
-                    acc.einsp += (unsigned)ld<CG>(t.rawdeg + v);
+                } else if (sh.home.pass == 0) {
+                    acc.einsp += (unsigned)ld<CG>(sh.home.rawdeg + v);
                 }
             }
-            nh = visit<SLOT_NB, GBM>(t, m, s, cidx, w0, alloc);
+            nh = visit<SLOT_NB, GBM>(t, sh, m, s, cidx, w0, alloc);
         }
         if (!__any_sync(0xffffffffu, d != 0)) return nh;
     } else if (lane < cnt) {
-        const int32_t v = fr_get(t.f, first + lane, wstart);
-        b = ld<CG>(t.g.ptr + v);
-        d = ld<CG>(t.g.ptr + v + 1) - b;
+        const int32_t v = fr_get(t.f, sh.home.spill, first + lane, wstart);
+        b = ld<CG>(sh.home.g.ptr + v);
+        d = ld<CG>(sh.home.g.ptr + v + 1) - b;
         acc.edges += (unsigned)d;
-        if (t.pass == 0) acc.einsp += (unsigned)ld<CG>(t.rawdeg + v);
+        if (sh.home.pass == 0) acc.einsp += (unsigned)ld<CG>(sh.home.rawdeg + v);
     }
-    return nh + expand_edges<CG, GBM>(t, b, d, s, cidx, w0, alloc);
+    return nh + expand_edges<CG, GBM>(t, sh, b, d, s, cidx, w0, alloc);
 }
 
 // The helper warps: levels from [start, end) on (entries written while the
@@ -848,7 +936,7 @@ __device__ __forceinline__ void run_levels(const Trav<GBM> &t, SharedState &sh, 
         const int cnt = end - start;
         // vertices a warp takes at a time: fewer than its lanes could, while
         // that keeps every warp busy
-        const int take = t.g.slot == nullptr ? min(32, max(1, (cnt + NW - 1) / NW))
+        const int take = sh.home.g.slot == nullptr ? min(32, max(1, (cnt + NW - 1) / NW))
                          : cnt <= 4 * NW     ? 4
                          : cnt <= 8 * NW     ? 8
                          : cnt <= 32 * NW    ? 16
@@ -861,7 +949,7 @@ __device__ __forceinline__ void run_levels(const Trav<GBM> &t, SharedState &sh, 
         int nh = 0;
         int base = wid * take;   // the first one by position, the others by demand
         while (base < cnt) {
-            nh += expand<CG, GBM>(t, start + base, min(take, cnt - base), wstart, s, cidx, start, acc, alloc);
+            nh += expand<false, CG, GBM>(t, sh, start + base, min(take, cnt - base), wstart, s, cidx, start, acc, alloc);
             if (cnt <= NW * take) break;
             if (lane == 0) base = atomicAdd(fetchp, take);
             base = __shfl_sync(0xffffffffu, base, 0) + NW * take;
@@ -962,7 +1050,7 @@ __device__ __forceinline__ void merge_state(const Trav<GBM> &t, const uint32_t *
                     uint32_t x = nb[q];
                     if (w == ws) x &= (1u << (s & 31)) - 1u;
                     if (w == (st >> 5)) x &= ~1u << (st & 31);
-                    for (; x; x &= x - 1u) fr_put(t.f, atomicAdd(&sh.npush, 1), 0, (w << 5) + __ffs(x) - 1, true);
+                    for (; x; x &= x - 1u) fr_put(t.f, sh.home.spill, atomicAdd(&sh.npush, 1), 0, (w << 5) + __ffs(x) - 1, true);
                 }
             }
         }
@@ -983,11 +1071,12 @@ __device__ __forceinline__ void merge_state(const Trav<GBM> &t, const uint32_t *
     if (lane == 0 && cnt) atomicAdd(&sh.nh, cnt);
 }
 
-// Writes the lists of the chain that just ended -- sources s0 .. s0 + len - 1,
-// which shared one bitmap -- by the helper warps, while the leader goes on with
-// the next sources: it waits only until the set vertices above s0 are out of
-// the bitmap (the barrier in the middle).  Bits are only ever added along a
-// chain, so list i is { v > s0 + i : v set, stamp(v) <= i }.  One exact pool
+// Writes lists first .. len - 1 of a chain -- sources s0, s0 + 1, .. which share
+// one bitmap -- by the helper warps, while the leader goes on with the next
+// sources: it waits only until the set vertices are out of the bitmap (the
+// barrier in the middle).  Bits are only ever added along a chain, so list i is
+// { v > s0 + i : v set, stamp(v) <= i } once source i is done; what later
+// sources add has larger stamps.  One exact pool
 // range holds all of the chain's lists (one global atomic per chain).
 //
 // First each warp extracts its share of the bitmap's chunks, in order, into
@@ -1003,19 +1092,19 @@ __device__ __forceinline__ void merge_state(const Trav<GBM> &t, const uint32_t *
 // Lists of pass G^T (columns of L) also count their entries into the L row
 // histogram, one reduction for the 32 lists.
 template <int GT, bool GBM>
-__device__ __forceinline__ void write_lists(const JobArgs &a, int64_t line_base, const Trav<GBM> &t, SharedState &sh, int (*hist)[32],
+__device__ __forceinline__ void write_lists(const JobArgs &a, const Trav<GBM> &t, SharedState &sh, int (*hist)[32],
                             int htid, int bar)
 {
     constexpr int NH = GT / 32 - 1;
     constexpr int UNR = 4;
     const int lane = htid & 31, wid = htid >> 5;
     const unsigned below = (1u << lane) - 1u;
-    const int s0 = sh.chain_s0, len = sh.chain_len, chain_hi = sh.chain_hi;
+    const int s0 = sh.chain_s0, first = sh.chain_first, len = sh.chain_len, chain_hi = sh.chain_hi;
     const int64_t total = sh.chain_total;
     const uint16_t *const stamp = sh.stamp;
-    int32_t *const scratch = t.lists;
-    const int64_t row0 = (int64_t)t.pass * a.L + line_base + s0;   // cnt / poff entry of s0
-    int32_t *const lrow = t.pass ? a.lrow + line_base : nullptr;
+    int32_t *const scratch = sh.home.lists;
+    const int64_t row0 = sh.home.row + s0;   // cnt / poff entry of s0
+    int32_t *const lrow = sh.home.lrow;
 
     // past the pool's capacity the chain's lists are not written, the tail
     // still advances, and its final value is the capacity the job needs
@@ -1026,11 +1115,11 @@ __device__ __forceinline__ void write_lists(const JobArgs &a, int64_t line_base,
         if (base < 0) atomicOr(a.status, ERR_POOL_OVERFLOW);
     }
 
-    // set bits above s0: words from w0 on (first_mask on w0)
-    const int w0 = (s0 + 1) >> 5;
-    const uint32_t first_mask = ~0u << ((s0 + 1) & 31);
+    // set bits above the first list's source: words from w0 on (first_mask on w0)
+    const int w0 = (s0 + first + 1) >> 5;
+    const uint32_t first_mask = ~0u << ((s0 + first + 1) & 31);
     const int c_lo = w0 >> 5;
-    const int c_hi = chain_hi > s0 ? (chain_hi >> 10) + 1 : c_lo;
+    const int c_hi = chain_hi > s0 + first ? (chain_hi >> 10) + 1 : c_lo;
     const int share = (max(c_hi - c_lo, 0) + NH - 1) / NH;
     const int my_lo = c_lo + wid * share, my_hi = min(c_hi, my_lo + share);
     auto word = [&](int cc) {
@@ -1084,7 +1173,7 @@ __device__ __forceinline__ void write_lists(const JobArgs &a, int64_t line_base,
     const int steps = (all + 31) >> 5, per = (steps + NH - 1) / NH;
     const int k_lo = min(all, wid * per * 32), k_hi = min(all, k_lo + per * 32);
     long long carry = 0;
-    for (int i0 = 0; i0 < len; i0 += 32) {
+    for (int i0 = first; i0 < len; i0 += 32) {
         const int nl = min(32, len - i0);
         // lane l: list i0 + l, its entries and its place
         const int c = lane < nl ? a.cnt[row0 + i0 + lane] : 0;
@@ -1199,7 +1288,7 @@ __device__ __forceinline__ void write_lists(const JobArgs &a, int64_t line_base,
 // them) behind the traversal's barrier; a second one tells the leader that it
 // is done.
 template <int GT, bool CG, bool GBM, bool LISTS>
-__device__ __forceinline__ void run_op(const JobArgs &a, int64_t line_base, Trav<GBM> &t, SharedState &sh,
+__device__ __forceinline__ void run_op(const JobArgs &a, Trav<GBM> &t, SharedState &sh,
                                        int (*hist)[32], int op, int htid, int bar, int &phase, Tally &acc)
 {
     if (LISTS) t.stamp = sh.stamp;
@@ -1208,12 +1297,12 @@ __device__ __forceinline__ void run_op(const JobArgs &a, int64_t line_base, Trav
     } else if (op == OP_CLEAR) {
         clear_state<GBM>(t.bits, htid >> 5, GT / 32 - 1, htid & 31);
     } else if (op == OP_SAVE) {
-        save_state<GT, GBM>(t.bits, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, htid);
+        save_state<GT, GBM>(t.bits, sh.home.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, htid);
     } else if (op == OP_MERGE) {
-        merge_state<GT, GBM>(t, t.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, sh.t, sh.src, sh.cidx, sh,
+        merge_state<GT, GBM>(t, sh.home.snaps + (int64_t)sh.snap * a.bitmap_words, sh.lo, sh.hi, sh.t, sh.src, sh.cidx, sh,
                              htid);
     } else if (LISTS && op == OP_LISTS) {
-        write_lists<GT, GBM>(a, line_base, t, sh, hist, htid, bar);   // the leader goes on from its middle
+        write_lists<GT, GBM>(a, t, sh, hist, htid, bar);   // the leader goes on from its middle
         return;
     }
     gsync<GT>(bar);
@@ -1240,6 +1329,117 @@ __device__ __forceinline__ int state_extent(const Bits<GBM> &b, int lane, int &l
     return (int)__reduce_add_sync(0xffffffffu, (unsigned)chunks);
 }
 
+// The CTA's next sources, from s on: those of the units that `claim` claimed
+// (lane 0 of the first leader).  Returns where they end: s when there are none.
+template <class C>
+__device__ __noinline__ int32_t next_units(int32_t s, int half)
+{
+    if (half == 0 && (threadIdx.x & 31) == 0) {
+        SharedState &sh = cta<C>().t[0];
+        const SharedPiece &own = sh.own;
+        const unsigned long long claim = sh.claim;
+        const int unit = (int)(claim & UNIT_MASK), end = (int)((claim >> UNIT_BITS) & UNIT_MASK);
+        if (unit < end) {
+            const int take = sh.claimed, next = min(unit + take, end);
+            sh.next_end = min(own.first + next * UNIT, own.last);
+            const int more = min(max((end - next) >> 3, 1), CLAIM_MAX);
+            sh.claimed = more;
+            const unsigned now = clock32() >> 8;   // in 256 cycles, 24 bits
+            const int done = s - own.s_lo;         // sources since the piece began
+            if (done > 0) {
+                const unsigned took = (now - sh.unit_t) & 0xffffffu;
+                if (sh.unit_done == 0) {   // the first unit
+                    sh.unit_most = took;
+                    own.fresh[0] = max(took, 1u);
+                    sh.unit_sum = 0u;
+                    sh.unit_mean = took;
+                } else {
+                    const int units = (done - sh.unit_done + UNIT - 1) / UNIT;
+                    const unsigned usual = (unsigned)units * sh.unit_mean;
+                    const bool spike = took > 4 * usual;   // not what the next units will take
+                    if (spike) sh.unit_most = max(sh.unit_most, took - usual);
+                    sh.unit_sum += spike ? usual : took;
+                    sh.unit_mean = max((unsigned)__fdividef((float)sh.unit_sum * (float)UNIT, (float)(done - UNIT)), 1u);
+                    *reinterpret_cast<volatile unsigned long long *>(own.cost) =
+                        (unsigned long long)sh.unit_most << 32 | sh.unit_mean;
+                }
+                sh.unit_done = done;
+            }
+            sh.unit_t = now;
+            // last: the store waits for the claim, which is needed a claim later
+            sh.claim = atomicAdd(own.word, (unsigned long long)more);
+        } else {
+            sh.next_end = s;
+        }
+    }
+    pair_sync();
+    return cta<C>().t[0].next_end;
+}
+
+// Where the cost of a piece that begins at `line` is noted.
+constexpr int FRESH_BUCKETS = 1024;
+
+__device__ __forceinline__ int fresh_bucket(int64_t line, int64_t lines)
+{
+    return (int)min(line * FRESH_BUCKETS / max(lines, (int64_t)1), (int64_t)FRESH_BUCKETS - 1);
+}
+
+// A part of another CTA's piece, as a piece word, or 0: of the parts of x units
+// from the top, half of what is left less half of what starting afresh costs,
+// the one that saves most.  While there is none but some CTA has yet to show
+// what its units cost, it looks again (a bounded number of times; every CTA of
+// the launch is resident and goes on).  One warp.
+template <class C>
+__device__ __noinline__ unsigned long long take_part(int ctas, int lane)
+{
+    const JobArgs &a = cta<C>().a;
+    for (int attempt = 0; attempt < (1 << 22); attempt++) {
+        bool wait = false;
+        unsigned best = 0u;
+        int from = -1, best_x = 0;
+        unsigned long long best_w = 0ull;
+        for (int c = lane; c < ctas; c += 32) {
+            const unsigned long long w = __ldcg(a.shared_piece + c), cost = __ldcg(a.shared_cost + c);
+            const long long left = (long long)((w >> UNIT_BITS) & UNIT_MASK) - (long long)(w & UNIT_MASK);
+            const long long mean = (long long)(cost & 0xffffffffull);
+            long long extra = (long long)(cost >> 32);
+            if (left <= 0) continue;
+            if (mean == 0) { wait = true; continue; }
+            if (left * mean <= extra) continue;
+            {   // a traversal from nothing above the middle: as the next piece there found it
+                const Range &rg = a.ranges[w >> (2 * UNIT_BITS)];
+                const int64_t line0 = a.mats[rg.mat].line_base + rg.offset;
+                const int64_t mid = line0 + ((int64_t)((w >> UNIT_BITS) & UNIT_MASK) - left / 2) * UNIT;
+                int b = fresh_bucket(mid, a.L);
+                const int b_end = min(fresh_bucket(line0 + rg.nj, a.L), b + 64);
+                unsigned f = 0u;
+                for (; b <= b_end && f == 0u; b++) f = __ldcg(a.fresh_cost + b);
+                extra = max(extra, (long long)f);
+            }
+            const long long x = (left * mean - extra) / (2 * mean);
+            if (x < 1) continue;
+            const unsigned gain = (unsigned)min(x * mean, 0x7fffffffll);
+            if (gain > best) { best = gain; from = c; best_x = (int)x; best_w = w; }
+        }
+        const unsigned top = __reduce_max_sync(0xffffffffu, best);
+        if (top == 0u) {
+            if (!__any_sync(0xffffffffu, wait)) return 0ull;
+            __nanosleep(1000);
+            continue;
+        }
+        const int who = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
+        unsigned long long got = 0ull;
+        if (lane == who) {
+            const int end = (int)((best_w >> UNIT_BITS) & UNIT_MASK), range = (int)(best_w >> (2 * UNIT_BITS));
+            const unsigned long long rest = piece_word(range, end - best_x, (int)(best_w & UNIT_MASK));
+            if (atomicCAS(a.shared_piece + from, best_w, rest) == best_w) got = piece_word(range, end, end - best_x);
+        }
+        got = __shfl_sync(0xffffffffu, got, who);
+        if (got) return got;   // else the owner, or another CTA, was there first
+    }
+    return 0ull;
+}
+
 // The sources s_lo, s_lo + stride, ... < s_hi of one work piece, in order,
 // each starting from the previous source's state whenever that is valid.
 //
@@ -1264,16 +1464,20 @@ __device__ __forceinline__ int state_extent(const Bits<GBM> &b, int lane, int &l
 // closure is most of the matrix: the 20,000-line one inspects 2.4e7 edges
 // instead of 2.7e8.
 template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
-__device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, Trav<GBM> &t, int32_t s_lo, int32_t s_hi,
-                           int32_t stride, SharedState *shs, volatile int (*pair_flag)[2], int half,
-                           int bar)
+__device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi, int32_t stride, bool shared, int half)
 {
+    using C = CtaOf<BLOCK, PAIRED, LISTS>;
     constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
     static_assert(GT >= 64, "a leader and at least one helper");
+    const JobArgs &a = cta<C>().a;
+    SharedState *const shs = cta<C>().t;
+    volatile int (*const pair_flag)[2] = cta<C>().pair_flag;
+    const int bar = 1 + half;
     SharedState &sh = shs[half];
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const int pass = t.pass;
+    const int pass = sh.home.pass;
+    const int32_t n = sh.home.n;
     Tally acc;
     const int nsnap = PAIRED ? a.snap_k : 0;
     auto collective = [&](int op) {   // arguments are in place
@@ -1307,7 +1511,8 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     unsigned xch = 0;         // exchanges with the other pass so far
     bool mine = false, other = false;   // this pass, the other pass reached s
     bool step = false;        // s is not for a run
-    long long total = 0;      // entries of the chain's lists
+    uint32_t total = 0;       // entries of the chain's lists from `pending` on
+    int pending = 0;          // the chain's first list that is not written
     // the seeding window: lane i holds row bounds and degree of source wlo + i
     int wlo = 0, whi = 0, wb = 0, we = 0, wraw = 0, wadj0 = 0;
     if (lane < SNAP_MAX) sh.snap_t[lane] = -1;
@@ -1315,29 +1520,36 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     // its words), and a copy is paid with as many vertices traversed or taken
     // over: where snapshots help, long traversals pay for them at once, and
     // where traversals are short they cost next to nothing.
-    const int heavy = max(64, md.n >> 8);
+    const int heavy = max(64, n >> 8);
     if (lane == 0) {
         sh.snaps = sh.weight = 0;
         if (sh.snap_credit < 0) sh.snap_credit = 4 * heavy;
     }
     __syncwarp();
 
+    auto lists_out = [&]() {   // of the chain's sources since `pending`
+        const long long c0 = clock64();
+        int lo, hi;
+        state_extent<GBM>(t.bits, lane, lo, hi);
+        if (lane == 0) {
+            sh.chain_s0 = prev - cidx;
+            sh.chain_first = pending;
+            sh.chain_len = cidx + 1;
+            sh.chain_total = total;
+            sh.chain_hi = min(hi << 5, n) - 1;
+        }
+        collective(OP_LISTS);
+        pending = cidx + 1;
+        total = 0;
+        spent(5, c0);
+    };
     auto end_chain = [&]() {
         int lo, hi;
-        if (LISTS && a.want_pattern && cidx >= 0) {
-            const long long c0 = clock64();
-            state_extent<GBM>(t.bits, lane, lo, hi);
-            if (lane == 0) {
-                sh.chain_s0 = prev - cidx;
-                sh.chain_len = cidx + 1;
-                sh.chain_total = total;
-                sh.chain_hi = min(hi << 5, md.n) - 1;
-            }
-            collective(OP_LISTS);
+        if (LISTS && a.want_pattern) {
+            if (pending <= cidx) lists_out();
             // the helpers read this chain's stamps on: the next chain takes
             // the traversal's other row
-            t.stamp = t.stamp == t.stamps ? t.stamps + a.stamp_stride : t.stamps;
-            spent(5, c0);
+            t.stamp = t.stamp == sh.home.stamps ? sh.home.stamps + a.stamp_stride : sh.home.stamps;
         }
         const long long c0 = clock64();
         const int chunks = state_extent<GBM>(t.bits, lane, lo, hi);
@@ -1353,21 +1565,40 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         spent(6, c0);
     };
 
+    if (PAIRED && shared && half == 0 && lane == 0) {
+        sh.claim = atomicAdd(sh.own.word, 1ull);   // a claim ahead of the sources
+        sh.claimed = 1;
+        sh.unit_t = clock32() >> 8;
+        sh.unit_done = 0;
+    }
+    if (lane == 0) sh.own.s_lo = s_lo;
     for (int32_t s = s_lo;;) {
+        if (PAIRED && s >= s_hi && shared) s_hi = next_units<C>(s, half);
         const bool more = s < s_hi;   // else: end the piece's last chain
+        // a long chain's lists go out as it grows, not all at its end
+        if (LISTS && a.want_pattern && cidx - pending >= 63 && total >= 1 << 15) lists_out();
         // a new seeding window when s is past the current one (consecutive
         // sources only): row bounds, then the rows themselves
         if (more && stride == 1 && s >= whi) {
             const int cnt = min(s_hi - s, SEED_WIN);
             const int i = min(lane, cnt - 1);
-            wb = ld<CG>(t.g.ptr + s + i);
-            we = ld<CG>(t.g.ptr + s + i + 1);
-            if (pass == 0) wraw = ld<CG>(t.rawdeg + s + i);
+            wb = ld<CG>(sh.home.g.ptr + s + i);
+            we = ld<CG>(sh.home.g.ptr + s + i + 1);
+            if (pass == 0) wraw = ld<CG>(sh.home.rawdeg + s + i);
             wadj0 = __shfl_sync(0xffffffffu, wb, 0);
             const int k = __popc(__ballot_sync(0xffffffffu, lane < cnt && we - wadj0 <= SEED_ADJ));   // rows that fit
             const int na = k ? __shfl_sync(0xffffffffu, we, k - 1) - wadj0 : 0;
             __syncwarp();
-            for (int q = lane; q < na; q += 32) sh.win_adj[q] = ld<CG>(t.g.adj + wadj0 + q);
+            const int32_t *const from = sh.home.g.adj + wadj0;
+#pragma unroll 1
+            for (int q0 = lane; q0 < na; q0 += 256) {   // 256 ids in flight: one round trip for most windows
+                int32_t x[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) x[u] = q0 + 32 * u < na ? ld<CG>(from + q0 + 32 * u) : 0;
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (q0 + 32 * u < na) sh.win_adj[q0 + 32 * u] = x[u];
+            }
             __syncwarp();
             wlo = s;
             whi = s + k;   // k == 0: a row too long for the window, read where it lies
@@ -1393,7 +1624,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             const int i0 = can ? s - wlo : 0;
             const int p0 = __shfl_sync(0xffffffffu, wb, i0) - wadj0;
             const int p1 = can ? __shfl_sync(0xffffffffu, we, i0 + k - 1) - wadj0 : p0;
-            const uint32_t ws = s + lane < md.n ? t.bits.get((s + lane) >> 5) : 0u;
+            const uint32_t ws = s + lane < n ? t.bits.get((s + lane) >> 5) : 0u;
             unsigned run_set = __ballot_sync(0xffffffffu, (ws >> ((s + lane) & 31)) & 1u);
             int ne = 0;
             for (int q0 = p0; q0 < p1 && ne <= 32; q0 += 128) {
@@ -1474,13 +1705,13 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 const int deg = __shfl_sync(0xffffffffu, we - wb, (i0 + lane) & 31);
                 const int raw = __shfl_sync(0xffffffffu, wraw, (i0 + lane) & 31);
                 if (lane < cut) {
-                    const int64_t slot = (int64_t)pass * a.L + md.line_base + s + lane;
+                    const int64_t slot = sh.home.row + s + lane;
                     a.cnt[slot] = c;
                     a.nxt[slot] = (uint8_t)((run_set >> (lane + 1)) & 1u);
                     acc.edges += (unsigned)deg;
                     if (pass == 0) acc.einsp += (unsigned)raw;
                 }
-                total += (long long)cut * hc - cut * (cut + 1) / 2 +
+                if (LISTS) total += cut * hc - cut * (cut + 1) / 2 +
                          (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < cut ? found : 0));
                 hc = __shfl_sync(0xffffffffu, c, cut - 1);
                 cidx += cut;
@@ -1501,8 +1732,8 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             b0 = __shfl_sync(0xffffffffu, wb, s - wlo);
             d0 = __shfl_sync(0xffffffffu, we, s - wlo) - b0;
         } else if (more) {
-            b0 = ld<CG>(t.g.ptr + s);
-            d0 = ld<CG>(t.g.ptr + s + 1) - b0;
+            b0 = ld<CG>(sh.home.g.ptr + s);
+            d0 = ld<CG>(sh.home.g.ptr + s + 1) - b0;
         }
 
         // take over the previous source's state, or end its chain; chain
@@ -1514,7 +1745,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             } else {
                 bool hit = false;
                 for (int k = lane; k < d0; k += 32)
-                    hit |= (in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(t.g.adj + b0 + k)) == s - 1;
+                    hit |= (in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(sh.home.g.adj + b0 + k)) == s - 1;
                 reuse = __any_sync(0xffffffffu, hit);
             }
         }
@@ -1522,11 +1753,15 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             cidx++;
         } else {
             if (cidx >= 0) end_chain();
-            if (!more) break;   // the next piece starts from an empty bitmap
+            if (!more) {   // the next piece starts from an empty bitmap
+                if (lane == 0) sh.nsrc += (unsigned)((s - sh.own.s_lo) / stride);
+                break;
+            }
             tally(sh.nfresh, 1u);
             cidx = 0;
             hc = 0;
             total = 0;
+            pending = 0;
             if (nsnap > 0 && lane == 0) sh.weight = 0;
         }
 
@@ -1539,7 +1774,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
         auto alloc = [&](int k) { const int p = tail; tail += k; return p; };
         if (lane == 0) {
             acc.edges += (unsigned)d0;
-            if (pass == 0 && !in_win) acc.einsp += (unsigned)ld<CG>(t.rawdeg + s);
+            if (pass == 0 && !in_win) acc.einsp += (unsigned)ld<CG>(sh.home.rawdeg + s);
         }
         if (in_win && lane == s - wlo) acc.einsp += (unsigned)wraw;
         if (nsnap > 0 && sh.snaps > 0) {
@@ -1559,7 +1794,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 const long long c0 = clock64();
                 if (!self) {   // before the merge, which leaves it out
                     const int32_t m[1] = {lane == 0 ? s : -1};
-                    nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
+                    nh += visit<1, GBM>(t, sh, m, s, cidx, 0, alloc);
                     self = true;
                 }
                 const int k = __ffs(__ballot_sync(0xffffffffu, st == best)) - 1;
@@ -1581,18 +1816,18 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
             }
         }
         {
-            auto id = [&](int k) { return in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(t.g.adj + b0 + k); };
+            auto id = [&](int k) { return in_win ? sh.win_adj[b0 - wadj0 + k] : ld<CG>(sh.home.g.adj + b0 + k); };
             const int32_t m[1] = {lane < d0 ? id(lane) : (lane == d0 && !self ? s : -1)};
-            nh += visit<1, GBM>(t, m, s, cidx, 0, alloc);
+            nh += visit<1, GBM>(t, sh, m, s, cidx, 0, alloc);
             for (int k0 = 32; k0 < d0; k0 += 128) {
                 int32_t x[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) x[u] = k0 + 32 * u + lane < d0 ? id(k0 + 32 * u + lane) : -1;
-                nh += visit<4, GBM>(t, x, s, cidx, 0, alloc);
+                nh += visit<4, GBM>(t, sh, x, s, cidx, 0, alloc);
             }
             if (d0 >= 32 && !self) {   // the row left no lane for s
                 const int32_t m1[1] = {lane == 0 ? s : -1};
-                nh += visit<1, GBM>(t, m1, s, cidx, 0, alloc);
+                nh += visit<1, GBM>(t, sh, m1, s, cidx, 0, alloc);
             }
         }
 
@@ -1604,7 +1839,7 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
                 if (end - start <= SOLO_MAX) {
                     __syncwarp();   // the level's queue entries, for every lane
                     n_levels++;
-                    nh += expand<CG, GBM>(t, start, end - start, wstart, s, cidx, start, acc, alloc);
+                    nh += expand<true, CG, GBM>(t, sh, start, end - start, wstart, s, cidx, start, acc, alloc);
                     wstart = start;
                     start = end;
                     end = tail;
@@ -1629,15 +1864,15 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
 
         // |hi(s)|: the bits above s; the link flag; both passes' exchange
         hc += nh - 1;
-        total += hc;
+        if (LISTS) total += hc;
         if (nsnap > 0 && end > 0 && lane == 0) {
             sh.weight = min(sh.weight + end, 1 << 28);
             sh.snap_credit = min(sh.snap_credit + end, 1 << 28);
         }
         __syncwarp();
-        mine = s + 1 < md.n && ((t.bits.get((s + 1) >> 5) >> ((s + 1) & 31)) & 1u);
+        mine = s + 1 < n && ((t.bits.get((s + 1) >> 5) >> ((s + 1) & 31)) & 1u);
         if (lane == 0) {
-            const int64_t slot = (int64_t)pass * a.L + md.line_base + s;
+            const int64_t slot = sh.home.row + s;
             a.cnt[slot] = hc;
             a.nxt[slot] = mine ? 1 : 0;
         }
@@ -1676,7 +1911,6 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     }
     fold_work(sh, acc, pass, lane);
     if (lane == 0) {
-        sh.nsrc += (unsigned)((s_hi - s_lo + stride - 1) / stride);
         sh.prof[0] += n_levels;
         sh.prof[2] += c_levels;
         sh.prof[7] += c_wait;
@@ -1687,24 +1921,38 @@ __device__ __forceinline__ void lead_piece(const JobArgs &a, const MatDesc &md, 
     gsync<GT>(bar);
 }
 
+// One work piece for a helper thread: the leader's ops until the piece ends.
+// Returns the phase of the level counters, which runs on.
+template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
+__device__ __noinline__ int help_piece(Trav<GBM> t, int half, int phase)
+{
+    using C = CtaOf<BLOCK, PAIRED, LISTS>;
+    constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
+    const int htid = (int)threadIdx.x - half * GT - 32;
+    const int bar = 1 + half;
+    SharedState &sh = cta<C>().t[half];
+    int (*const hist)[32] = cta<C>().hist + (LISTS ? half * (GT / 32 - 1) : 0);
+    Tally acc;
+    for (;;) {
+        gsync<GT>(bar);
+        const int op = sh.op;
+        if (op == OP_EXIT) break;
+        run_op<GT, CG, GBM, LISTS>(cta<C>().a, t, sh, hist, op, htid, bar, phase, acc);
+    }
+    fold_work(sh, acc, sh.home.pass, htid & 31);
+    return phase;
+}
+
 // One work piece: the first warp of every traversal leads, the others help.
 template <int BLOCK, bool PAIRED, bool CG, bool GBM, bool LISTS = true>
-__device__ __forceinline__ void run_piece(const JobArgs &a, const MatDesc &md, Trav<GBM> &t, int32_t s_lo,
-                                          int32_t s_hi, int32_t stride, SharedState *shs, int (*hist)[32],
-                                          volatile int (*pair_flag)[2], int half, int gtid, int bar, int &phase)
+__device__ __forceinline__ void run_piece(const Trav<GBM> &t, int32_t s_lo, int32_t s_hi, int32_t stride, bool shared,
+                                          int half, int gtid, int &phase)
 {
-    constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
     if (gtid < 32) {
-        lead_piece<BLOCK, PAIRED, CG, GBM, LISTS>(a, md, t, s_lo, s_hi, stride, shs, pair_flag, half, bar);
+        __syncwarp();   // the traversal's home, which the first lane has settled
+        lead_piece<BLOCK, PAIRED, CG, GBM, LISTS>(t, s_lo, s_hi, stride, shared, half);
     } else {
-        Tally acc;
-        for (;;) {
-            gsync<GT>(bar);
-            const int op = shs[half].op;
-            if (op == OP_EXIT) break;
-            run_op<GT, CG, GBM, LISTS>(a, md.line_base, t, shs[half], hist, op, gtid - 32, bar, phase, acc);
-        }
-        fold_work(shs[half], acc, t.pass, gtid & 31);
+        phase = help_piece<BLOCK, PAIRED, CG, GBM, LISTS>(t, half, phase);
     }
 }
 
@@ -1736,21 +1984,20 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
 {
     constexpr int GT = PAIRED ? BLOCK / 2 : BLOCK;
     constexpr int NS = PAIRED ? 2 : 1;
+    using C = CtaOf<BLOCK, PAIRED, LISTS>;
     extern __shared__ __align__(16) uint32_t smem_dyn[];
-    __shared__ SharedState shs[NS];
-    __shared__ volatile int pair_flag[2][2];   // [source parity][pass]: s+1 in hi(s)
-    __shared__ long long s_piece;
-    __shared__ int s_hist[LISTS ? NS * (GT / 32 - 1) : 1][32];   // list output: a row a helper warp
-    int (*const hist)[32] = s_hist + (LISTS ? (int)threadIdx.x / GT * (GT / 32 - 1) : 0);
+    C &ca = cta<C>();
+    SharedState *const shs = ca.t;
     cg::grid_group grid = cg::this_grid();
     const int tid = threadIdx.x;
     const int half = PAIRED ? tid / GT : 0;
     const int gtid = PAIRED ? tid % GT : tid;
-    const int bar = 1 + half;
     SharedState &sh = shs[half];
+    uint32_t *const smem = smem_dyn + (sizeof(C) + 15) / 16 * 4;
+    if (tid == 0) ca.a = a;
     const int64_t trav = (int64_t)blockIdx.x * NS + half;
-    uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * NS) * a.state_words : smem_dyn;
-    uint32_t *const ring = (GBM ? smem_dyn : smem_dyn + (size_t)NS * a.state_words) + (size_t)half * a.ring_size;
+    uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * NS) * a.state_words : smem;
+    uint32_t *const ring = (GBM ? smem : smem + (size_t)NS * a.state_words) + (size_t)half * a.ring_size;
 
     // ---- phase 1: traversals ------------------------------------------------
     unsigned long long t_start = 0;
@@ -1759,21 +2006,45 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
     if (gtid == 0) init_state(sh);
     Trav<GBM> t{};
     t.bits = bits_at<GBM>(state + (size_t)half * a.state_words + STATE_PAD, a.bitmap_words);
-    t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size, a.queue + trav * a.qcap};
-    if (LISTS && a.want_pattern) {
-        t.stamp = t.stamps = a.stamp + 2 * trav * a.stamp_stride;
-        t.lists = a.lists + trav * a.qcap;
+    t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size};
+    if (LISTS && a.want_pattern) t.stamp = a.stamp + 2 * trav * a.stamp_stride;
+    if (gtid == 0) {
+        sh.home.spill = a.queue + trav * a.qcap;
+        sh.home.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
+        if (LISTS && a.want_pattern) {
+            sh.home.stamps = t.stamp;
+            sh.home.lists = a.lists + trav * a.qcap;
+        }
     }
-    t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
     int phase = 0, last_mat = -1;
     __syncthreads();
     for (;;) {
-        if (tid == 0) s_piece = (long long)atomicAdd(a.piece_counter, 1ull);
+        const bool shared = PAIRED && a.shared_piece != nullptr;
+        if (tid < 32) {
+            long long pc = 0;
+            if (tid == 0) pc = (long long)atomicAdd(a.piece_counter, 1ull);
+            pc = __shfl_sync(0xffffffffu, pc, 0);
+            if (pc >= a.npieces) {
+                pc = -1;
+                if (shared) {   // no piece is left: a part of another CTA's
+                    const unsigned long long w = take_part<C>(gridDim.x, tid);
+                    if (tid == 0) ca.word = w;
+                }
+            }
+            if (tid == 0) ca.piece = pc;
+        }
         __syncthreads();
-        const int64_t pc = s_piece;
-        if (pc >= a.npieces) break;
+        const int64_t pc = ca.piece;
+        unsigned long long word = 0ull;
+        if (pc < 0) {
+            if (!shared) break;
+            word = ca.word;
+            if (word == 0ull) break;
+        }
         int r = 0;
-        {
+        if (pc < 0) {
+            r = (int)(word >> (2 * UNIT_BITS));
+        } else {
             int hi = a.nranges - 1;
             while (r < hi) {
                 const int mid = (r + hi + 1) >> 1;
@@ -1783,9 +2054,29 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
         const Range rg = a.ranges[r];
         const int64_t k = pc - rg.piece_base;
         const int pass = PAIRED ? half : (int)(k & 1);
-        const int64_t c = PAIRED ? k : (k >> 1);
         int64_t j0, j1;
-        piece_bounds(rg, c, j0, j1);
+        if (shared) {
+            if (pc >= 0) {   // the range's pieces from its top
+                const int units = (rg.nj + UNIT - 1) / UNIT, per = rg.chunk / UNIT;
+                const int end = units - (int)k * per;
+                word = piece_word(r, end, max(0, end - per));
+            }
+            j0 = (int64_t)(word & UNIT_MASK) * UNIT;
+            if (tid == 0) {   // the first unit is the CTA's own
+                SharedPiece &own = shs[0].own;
+                own.word = a.shared_piece + blockIdx.x;
+                own.cost = a.shared_cost + blockIdx.x;
+                own.first = rg.offset;
+                own.last = rg.offset + rg.nj;
+                own.fresh = a.fresh_cost + fresh_bucket(a.mats[rg.mat].line_base + rg.offset + j0, a.L);
+                *reinterpret_cast<volatile unsigned long long *>(own.cost) = 0ull;
+                __threadfence();
+                atomicExch(own.word, word + 1ull);
+            }
+            j1 = min(j0 + UNIT, (int64_t)rg.nj);
+        } else {
+            piece_bounds(rg, PAIRED ? k : (k >> 1), j0, j1);
+        }
         const MatDesc md = a.mats[rg.mat];
         const PassGraph g = md.g[pass];
         int32_t s_lo = rg.offset + (int32_t)j0 * rg.stride;
@@ -1805,13 +2096,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
         }
         if (rg.mat != last_mat && gtid == 0) sh.snap_credit = -1;
         last_mat = rg.mat;
-        t.g = g;
-        t.rawdeg = md.rawdeg;
-        t.pass = pass;
-        t.n = md.n;
-        run_piece<BLOCK, PAIRED, false, GBM, LISTS>(a, md, t, s_lo, s_hi, rg.stride, shs, hist, pair_flag, half, gtid,
-                                                    bar, phase);
-        __syncthreads();   // every thread is done with s_piece
+        if (gtid == 0) settle(sh.home, a, md, pass);
+        run_piece<BLOCK, PAIRED, false, GBM, LISTS>(t, s_lo, s_hi, rg.stride, shared, half, gtid, phase);
+        __syncthreads();   // every thread is done with the piece
     }
     {
         if (tid == 0) {   // this CTA's busy time, summed over CTAs (load balance)

@@ -70,26 +70,30 @@ template <int BLOCK, bool GBM>
 __global__ void __maxnreg__(64) serve_kernel(const __grid_constant__ ServeArgs sa)
 {
     constexpr int GT = BLOCK / 2;
+    using C = CtaOf<BLOCK, true, false>;
     const JobArgs &a = sa.job;
     extern __shared__ __align__(16) uint32_t smem_dyn[];
-    __shared__ SharedState shs[2];
-    __shared__ volatile int pair_flag[2][2];
+    C &ca = cta<C>();
+    SharedState *const shs = ca.t;
+    uint32_t *const smem = smem_dyn + (sizeof(C) + 15) / 16 * 4;
     __shared__ long long s_piece;
+    if (threadIdx.x == 0) ca.a = a;
     const int tid = threadIdx.x;
     const int half = tid / GT;
     const int gtid = tid % GT;
-    const int bar = 1 + half;
     SharedState &sh = shs[half];
-    uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * 2) * a.state_words : smem_dyn;
-    uint32_t *const ring = (GBM ? smem_dyn : smem_dyn + (size_t)2 * a.state_words) + (size_t)half * a.ring_size;
+    uint32_t *const state = GBM ? a.gbm + ((int64_t)blockIdx.x * 2) * a.state_words : smem;
+    uint32_t *const ring = (GBM ? smem : smem + (size_t)2 * a.state_words) + (size_t)half * a.ring_size;
     for (int w = tid; w < 2 * a.state_words; w += BLOCK) state[w] = w % a.state_words < STATE_PAD ? ~0u : 0u;
     if (gtid == 0) init_state(sh);   // counts only: no lists, no stamps
     const int64_t trav = (int64_t)blockIdx.x * 2 + half;
     Trav<GBM> t{};
     t.bits = bits_at<GBM>(state + (size_t)half * a.state_words + STATE_PAD, a.bitmap_words);
-    t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size, a.queue + trav * a.qcap};
-    t.stamp = nullptr;
-    t.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
+    t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size};
+    if (gtid == 0) {
+        sh.home.spill = a.queue + trav * a.qcap;
+        sh.home.snaps = a.snap + trav * a.snap_k * a.bitmap_words;
+    }
     int phase = 0;
     __shared__ int s_class;
     __syncthreads();
@@ -121,13 +125,9 @@ __global__ void __maxnreg__(64) serve_kernel(const __grid_constant__ ServeArgs s
         const ServePiece piece =
             load_cg(sa.pieces + (unsigned long long)s_class * sa.piece_cap + (pc % (long long)sa.piece_cap));
         const MatDesc md = load_cg(sa.slots + piece.slot);
-        t.g = md.g[half];
-        t.rawdeg = md.rawdeg;
-        t.pass = half;
-        t.n = md.n;
+        if (gtid == 0) settle(sh.home, a, md, half);
         if (gtid == 0) sh.snap_credit = -1;   // the piece may be another request's
-        run_piece<BLOCK, true, true, GBM, false>(a, md, t, piece.s_lo, piece.s_hi, 1, shs, nullptr, pair_flag, half, gtid,
-                                                 bar, phase);
+        run_piece<BLOCK, true, true, GBM, false>(t, piece.s_lo, piece.s_hi, 1, false, half, gtid, phase);
         __syncthreads();
         if (tid == 0) {
             __threadfence();
