@@ -420,23 +420,17 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
                       ((want_pair && pair_smem > ctx->smem_optin) || single_smem > ctx->smem_optin));
     const bool paired = want_pair && (gbm || pair_smem <= ctx->smem_optin);
     // Shared-state pairs past 8K lines hold one CTA per SM (1024 threads at
-    // 64 registers fill its register file): 768 threads with up to 80
-    // registers a thread run without register spills, measured faster than
-    // 1024 threads on the 80^3 stencil with and without the pattern.  Counts
-    // of matrices with long rows (no row slots: mean degree above SLOT_NB)
-    // take 1024 threads: their large frontiers keep every warp busy (9%
-    // faster on the 659K-line power-law matrix).  512 threads with up to 128
-    // registers -- GSOFA_FLAG_WIDE_REGS -- are faster still on latency-bound
-    // matrices, counts only, but slower where large frontiers keep many warps
-    // busy.
+    // 64 registers fill its register file).  768 threads with up to 80
+    // registers a thread are faster than 1024: counts of the 200K-line
+    // power-law matrix 19.7 and 20.7 ms, of the 659K-line one 81.5 and 88.8.
+    // GSOFA_FLAG_WIDE_REGS takes 512 threads with up to 128 registers, for
+    // matrices whose levels are too small for more warps.
     const bool wide = (p.flags & GSOFA_FLAG_WIDE_REGS) != 0;
-    bool long_rows = false;
-    for (int i = 0; i < count; i++) long_rows |= mats[i]->n > 0 && mats[i]->d_gslot == nullptr;
     int block = p.block_size;
     if (wide) block = 512;
     if (!block) {
         if (gbm) block = paired ? 512 : 128;
-        else if (paired && max_n > 8192) block = (!want_pattern && long_rows) ? 1024 : 768;
+        else if (paired && max_n > 8192) block = 768;
         else block = pick_block(max_n) * (paired ? 2 : 1);
     }
     if (wide && (!paired || gbm)) return GSOFA_ERR_INVALID_INPUT;

@@ -353,11 +353,19 @@ struct Bits<true> {
     __device__ __forceinline__ uint32_t peek(Place, int32_t m) const { return m < 0 ? ~0u : 0u; }
     __device__ __forceinline__ void add(Place at, uint32_t bit, uint32_t &w) const
     {
-        if (!(w & bit)) w = atomicOr(base + at, bit);
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b32 x;\n\tand.b32 x, %0, %2;\n\tsetp.eq.u32 p, x, 0;\n\t"
+            "@p atom.relaxed.gpu.global.or.b32 %0, [%1], %2;\n\t}"
+            : "+r"(w)
+            : "l"(base + at), "r"(bit)
+            : "memory");
     }
     __device__ __forceinline__ void add_or(int i, uint32_t m, bool on) const
     {
-        if (on) atomicOr(base + i, m);
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.relaxed.gpu.global.or.b32 [%0], %1;\n\t}" ::"l"(base + i),
+            "r"(m), "r"((uint32_t)on)
+            : "memory");
     }
 };
 
@@ -404,6 +412,15 @@ __device__ __forceinline__ void ring_put(const Frontier &f, int p, int32_t m, ui
         "setp.lt.and.s32 q, %1, %4, p;\n\t@q st.shared.u32 [%0], %1;\n\t}" ::"r"(
             f.ring + 4u * (uint32_t)(p & (f.ring_size - 1))),
         "r"(m), "r"(w), "r"(bit), "r"(s));
+}
+
+__device__ __forceinline__ void spill_put(int32_t *at, int32_t m, uint32_t w, uint32_t bit, int32_t s)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 x;\n\tand.b32 x, %2, %3;\n\tsetp.eq.u32 p, x, 0;\n\t"
+        "setp.lt.and.s32 q, %1, %4, p;\n\t@q st.global.u32 [%0], %1;\n\t}" ::"l"(at),
+        "r"(m), "r"(w), "r"(bit), "r"(s)
+        : "memory");
 }
 
 __device__ __forceinline__ int32_t ring_get(const Frontier &f, int p)
@@ -743,6 +760,12 @@ __device__ __forceinline__ int visit(const Trav<GBM> &t, const SharedState &sh, 
                 ring_put(t.f, pos + __popc(low[u] & below), m[u], w[u], bit[u], s);
                 pos += __popc(low[u]);
             }
+        } else if (pos - w0 >= t.f.ring_size) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                spill_put(sh.home.spill + pos + __popc(low[u] & below), m[u], w[u], bit[u], s);
+                pos += __popc(low[u]);
+            }
         } else {
 #pragma unroll 1
             for (int u = 0; u < U; u++) {
@@ -775,7 +798,10 @@ __device__ __forceinline__ int expand_edges(const Trav<GBM> &t, const SharedStat
     const unsigned some = __ballot_sync(0xffffffffu, d > 0);
     const int rows = __popc(some);
     if (some & (some + 1u)) {
-        const int from = __fns(some, 0, lane + 1) & 31;   // the lane of row `lane`
+        int from = 0;   // the lane of row `lane`: as many rows before it (a search; __fns is a loop)
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+            if (__popc(some & ((1u << (from + o)) - 1u)) <= lane) from += o;
         b = __shfl_sync(0xffffffffu, b, from);
         d = __shfl_sync(0xffffffffu, d, from);
         if (lane >= rows) d = 0;
@@ -863,11 +889,40 @@ __device__ __forceinline__ int expand_slots(const Trav<GBM> &t, const SharedStat
     return visit<U, GBM>(t, sh, m, s, cidx, w0, alloc);
 }
 
-// Expands the frontier's entries [first, first + cnt), 0 < cnt <= 32, which were
-// written while the level starting at wstart ran.  LEAD: the leader's small
-// levels, without the form for large ones, whose registers it would pay for all
-// the time.
-template <bool LEAD, bool CG, bool GBM, class Alloc>
+// Expands 32 vertices of a large level of a graph with row slots: a lane a
+// vertex, six ids a lane -- fewer instructions a vertex, where every warp is
+// busy.  v: the lane's vertex, or n, whose slot is empty.  next: its vertex of
+// the warp's next 32; that slot comes into L1 beside this step's bitmap
+// accesses.  A step is a chain of memory round trips (frontier, slot, bitmap
+// and, for long rows, ids and bitmap again) which only the warps of one
+// traversal share: with the frontier and the slot of the next step under way, no
+// ring arithmetic past the ring, and a search instead of a loop for the long
+// rows, the traversal of all of an 864,008-line bordered matrix takes 14.2 ms
+// and not 17.4 (80^3 counts 3.95 and 4.09).
+template <bool CG, bool GBM, class Alloc>
+__device__ __forceinline__ int expand_wide(const Trav<GBM> &t, const SharedState &sh, int32_t v, int32_t next, int32_t s, int cidx,
+                                           int w0, Tally &acc, Alloc alloc)
+{
+    const int4 sl0 = ld4<CG>(sh.home.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(sh.home.g.slot + 2 * (int64_t)v + 1);
+    int32_t b = sl0.y, d = sl0.x;
+    int32_t m[SLOT_NB] = {-1, -1, -1, -1, -1, -1};
+    acc.edges += (unsigned)d;
+    if (d <= SLOT_NB) {   // ids past the degree are -1 in the slot
+        acc.einsp += (unsigned)b;
+        m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
+        d = 0;
+    } else if (sh.home.pass == 0) {
+        acc.einsp += (unsigned)ld<CG>(sh.home.rawdeg + v);
+    }
+    if (!CG) asm volatile("prefetch.global.L1 [%0];" ::"l"(sh.home.g.slot + 2 * (int64_t)next));
+    int nh = visit<SLOT_NB, GBM>(t, sh, m, s, cidx, w0, alloc);
+    if (__any_sync(0xffffffffu, d != 0)) nh += expand_edges<CG, GBM>(t, sh, b, d, s, cidx, w0, alloc);
+    return nh;
+}
+
+// Expands the frontier's entries [first, first + cnt), 0 < cnt <= 32 (with row
+// slots, 16), which were written while the level starting at wstart ran.
+template <bool CG, bool GBM, class Alloc>
 __device__ __forceinline__ int expand(const Trav<GBM> &t, const SharedState &sh, int first, int cnt, int wstart, int32_t s, int cidx, int w0,
                                       Tally &acc, Alloc alloc)
 {
@@ -881,27 +936,8 @@ __device__ __forceinline__ int expand(const Trav<GBM> &t, const SharedState &sh,
             nh = expand_slots<1, CG, GBM>(t, sh, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         } else if (cnt <= 8) {
             nh = expand_slots<2, CG, GBM>(t, sh, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
-        } else if (LEAD || cnt <= 16) {
-            nh = expand_slots<4, CG, GBM>(t, sh, first, min(cnt, 16), in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         } else {
-            // a lane a vertex, six ids a lane: fewer instructions a vertex,
-            // for levels that keep every warp busy
-            int32_t m[SLOT_NB] = {-1, -1, -1, -1, -1, -1};
-            if (lane < cnt) {
-                const int32_t v = fr_get(t.f, sh.home.spill, first + lane, wstart);
-                const int4 sl0 = ld4<CG>(sh.home.g.slot + 2 * (int64_t)v), sl1 = ld4<CG>(sh.home.g.slot + 2 * (int64_t)v + 1);
-                d = sl0.x;
-                b = sl0.y;
-                acc.edges += (unsigned)d;
-                if (d <= SLOT_NB) {   // ids past the degree are -1 in the slot
-                    acc.einsp += (unsigned)b;
-                    m[0] = sl0.z; m[1] = sl0.w; m[2] = sl1.x; m[3] = sl1.y; m[4] = sl1.z; m[5] = sl1.w;
-                    d = 0;
-                } else if (sh.home.pass == 0) {
-                    acc.einsp += (unsigned)ld<CG>(sh.home.rawdeg + v);
-                }
-            }
-            nh = visit<SLOT_NB, GBM>(t, sh, m, s, cidx, w0, alloc);
+            nh = expand_slots<4, CG, GBM>(t, sh, first, cnt, in_ring, wstart, s, cidx, w0, acc, alloc, b, d);
         }
         if (!__any_sync(0xffffffffu, d != 0)) return nh;
     } else if (lane < cnt) {
@@ -948,11 +984,29 @@ __device__ __forceinline__ void run_levels(const Trav<GBM> &t, SharedState &sh, 
         };
         int nh = 0;
         int base = wid * take;   // the first one by position, the others by demand
-        while (base < cnt) {
-            nh += expand<false, CG, GBM>(t, sh, start + base, min(take, cnt - base), wstart, s, cidx, start, acc, alloc);
-            if (cnt <= NW * take) break;
-            if (lane == 0) base = atomicAdd(fetchp, take);
-            base = __shfl_sync(0xffffffffu, base, 0) + NW * take;
+        auto more = [&]() {
+            int p = 0;
+            if (lane == 0) p = atomicAdd(fetchp, take);
+            return __shfl_sync(0xffffffffu, p, 0) + NW * take;
+        };
+        if (sh.home.g.slot != nullptr && take == 32) {   // cnt > 32 * NW
+            auto vertex = [&](int at) {
+                return at + lane < cnt ? fr_get(t.f, sh.home.spill, start + at + lane, wstart) : sh.home.n;
+            };
+            int32_t v = vertex(base);
+            while (base < cnt) {
+                if (lane == 0) acc.xcnt += min(32, cnt - base);
+                base = more();
+                const int32_t next = vertex(base);
+                nh += expand_wide<CG, GBM>(t, sh, v, next, s, cidx, start, acc, alloc);
+                v = next;
+            }
+        } else {
+            while (base < cnt) {
+                nh += expand<CG, GBM>(t, sh, start + base, min(take, cnt - base), wstart, s, cidx, start, acc, alloc);
+                if (cnt <= NW * take) break;
+                base = more();
+            }
         }
         if (lane == 0 && nh) atomicAdd(&sh.nh, nh);
         helper_sync<GT>(bar);
@@ -1356,7 +1410,11 @@ __device__ __noinline__ int32_t next_units(int32_t s, int half)
                 } else {
                     const int units = (done - sh.unit_done + UNIT - 1) / UNIT;
                     const unsigned usual = (unsigned)units * sh.unit_mean;
-                    const bool spike = took > 4 * usual;   // not what the next units will take
+                    // a traversal from nothing in the middle of a piece of small ones is
+                    // not what the next units will take; up to sixteenfold they vary (a
+                    // limit of four hid what was left of the power-law matrices' pieces:
+                    // 200K lines 19.3 ms, now 17.1)
+                    const bool spike = took > 16 * usual;
                     if (spike) sh.unit_most = max(sh.unit_most, took - usual);
                     sh.unit_sum += spike ? usual : took;
                     sh.unit_mean = max((unsigned)__fdividef((float)sh.unit_sum * (float)UNIT, (float)(done - UNIT)), 1u);
@@ -1839,7 +1897,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
                 if (end - start <= SOLO_MAX) {
                     __syncwarp();   // the level's queue entries, for every lane
                     n_levels++;
-                    nh += expand<true, CG, GBM>(t, sh, start, end - start, wstart, s, cidx, start, acc, alloc);
+                    nh += expand<CG, GBM>(t, sh, start, end - start, wstart, s, cidx, start, acc, alloc);
                     wstart = start;
                     start = end;
                     end = tail;
