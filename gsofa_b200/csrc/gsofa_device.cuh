@@ -11,11 +11,19 @@
 //                 snind[L] uint8    -- line starts a supernode
 //   pool / out  : int32 pattern entries (the traversals write pool, one range
 //                 per chain of sources; compaction writes out in line order);
-//   stamp       : pattern mode, per traversal: n uint16, the chain index at
-//                 which each vertex was first set;
-//   per CTA     : frontier queue of qcap int32 (every vertex enters at most
-//                 once per source, so qcap >= n never overflows).
-// The per-source visited set is an n-bit bitmap in shared memory.
+//   per traversal (two a CTA, one a pass, in the paired kernels):
+//                 a frontier queue of qcap int32 (every vertex enters at most
+//                 once per source, so qcap >= n never overflows);
+//                 pattern mode: two rows of n uint16 stamps, the chain index at
+//                 which each vertex was first set (one row is being written
+//                 while the other's lists go out), and a chain's vertices;
+//                 up to SNAP_MAX bitmaps of finished traversals (snapshots).
+// The visited set is an n-bit bitmap with two summary levels, in shared memory
+// or, for large n, in global memory.
+//
+// A traversal is led by one warp: it seeds each source, runs its small levels
+// and decides what the source can reuse.  The other warps of its half of the
+// CTA wait for work from it: large levels, clearing, lists, snapshots.
 #pragma once
 
 #include <cooperative_groups.h>

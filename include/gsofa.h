@@ -63,8 +63,10 @@ typedef struct gsofa_matrix gsofa_matrix; /* device-resident G and G^T     */
 
 /* Tuning and output parameters; zero means "choose automatically". */
 typedef struct gsofa_params {
-    int32_t src_chunk;          /* consecutive sources per work item; 0: 32 to
-                                   512, about eight pieces per resident CTA  */
+    int32_t src_chunk;          /* consecutive sources per work item; 0: by the
+                                   shape (pieces that CTAs share, about two a
+                                   resident CTA; without reuse, or on a slice,
+                                   32 to 512 sources each)                    */
     int32_t block_size;         /* threads per CTA: 128, 256, 512, 768 (the
                                    two passes side by side only) or 1024      */
     int32_t threads_per_source; /* 0, 1, 4, 8, 16 or 32; chooses nothing any
@@ -112,9 +114,8 @@ typedef struct gsofa_params {
                                       traversals per SM, any n              */
 #define GSOFA_FLAG_WIDE_REGS 0x40  /* the two passes side by side in 512-thread
                                       CTAs with up to 128 registers a thread
-                                      (one CTA per SM): fastest on
-                                      latency-bound matrices (small frontiers),
-                                      slower on dense-fill ones               */
+                                      (one CTA per SM), for matrices whose
+                                      levels are too small for more warps     */
 #define GSOFA_FLAG_DIRECT_HOST 0x20 /* gsofa_symbfact_ranges into host memory:
                                       the kernel writes the lists there
                                       itself (no device pool; slower than the
