@@ -11,6 +11,7 @@
 #include "gsofa_supernodal.cuh"
 #include "gsofa_partition.hpp"
 #include "gsofa_order.cuh"
+#include "gsofa_scratch.hpp"
 
 #include <cuda_runtime.h>
 
@@ -65,11 +66,24 @@ std::mutex &kernel_attr_mutex()
     return m;
 }
 
-// Grow-only device buffer owned by a context.
-struct DevBuf {
-    void *p = nullptr;
-    size_t bytes = 0;
+struct DeviceMemory {
+    static void *alloc(size_t bytes)
+    {
+        void *p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        GS_CUDA(e);
+        return p;
+    }
+    static void free(void *p) { cudaFree(p); }
+    [[noreturn]] static void no_room() { throw CudaFail{cudaErrorMemoryAllocation}; }
 };
+
+using gsofa::DevBuf;
+using Scratch = gsofa::Scratch<DeviceMemory>;
 
 }  // namespace
 
@@ -83,12 +97,10 @@ struct GraphCache {
     cudaStream_t stream = nullptr;
 };
 
-struct gsofa_ctx {
+struct gsofa_ctx : Scratch {
     int device = 0;
     int sm_count = 0;
     size_t smem_optin = 0;
-    size_t budget = 0;
-    size_t held = 0;          // bytes of grow-only scratch currently held
     cudaStream_t stream = nullptr;      // stream all work is issued on
     cudaStream_t own_stream = nullptr;  // the context's own stream
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -116,39 +128,7 @@ struct gsofa_ctx {
     struct Shape { int block; int32_t words; bool paired; bool gbm; bool wide; bool lists; int ring; int occ; };
     std::vector<Shape> shapes;
 
-    void *grow(DevBuf &b, size_t bytes)
-    {
-        bytes = std::max<size_t>(bytes, 256);
-        if (b.bytes >= bytes) return b.p;
-        if (b.p) {
-            GS_CUDA(cudaFree(b.p));
-            held -= b.bytes;
-            b.p = nullptr;
-            b.bytes = 0;
-        }
-        // snapshots only save time: they give way to what a job needs
-        if (held + bytes > budget && &b != &snap) release(snap);
-        if (held + bytes > budget) throw CudaFail{cudaErrorMemoryAllocation};
-        cudaError_t e = cudaMalloc(&b.p, bytes);
-        if (e == cudaErrorMemoryAllocation && snap.p && &b != &snap) {
-            cudaGetLastError();
-            release(snap);
-            e = cudaMalloc(&b.p, bytes);
-        }
-        GS_CUDA(e);
-        b.bytes = bytes;
-        held += bytes;
-        return b.p;
-    }
-    void release(DevBuf &b)
-    {
-        if (b.p) {
-            cudaFree(b.p);
-            held -= b.bytes;
-        }
-        b.p = nullptr;
-        b.bytes = 0;
-    }
+    gsofa_ctx() { dispensable = {&snap}; }
 
     // Device slabs of freed matrices, kept for later uploads so that a caller
     // who uploads, factorizes and frees matrix after matrix pays no
@@ -588,20 +568,21 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
 
     ctx->job_id++;
     for (int attempt = 0; attempt < 2; attempt++) {
+        Scratch::Job job(*ctx);
         // scratch
-        int32_t *d_queue = (int32_t *)ctx->grow(ctx->queue, (size_t)grid * NS * qcap * sizeof(int32_t));
-        int32_t *d_cnt = (int32_t *)ctx->grow(ctx->cnt, (size_t)2 * L * sizeof(int32_t));
-        uint8_t *d_nxt = (uint8_t *)ctx->grow(ctx->nxt, (size_t)2 * L);
-        int64_t *d_poff = (int64_t *)ctx->grow(ctx->poff, (size_t)2 * L * sizeof(int64_t));
-        int64_t *d_gptr = (int64_t *)ctx->grow(ctx->gptr, (size_t)2 * (L + 1) * sizeof(int64_t));
-        int32_t *d_lrow = (int32_t *)ctx->grow(ctx->lrow, (size_t)L * sizeof(int32_t));
-        uint8_t *d_snind = (uint8_t *)ctx->grow(ctx->snind, (size_t)L);
-        int32_t *d_sn = (int32_t *)ctx->grow(ctx->snlist, (size_t)L * sizeof(int32_t));
-        int64_t *d_tiles = (int64_t *)ctx->grow(ctx->tiles, (size_t)4 * ntiles * sizeof(int64_t));
+        int32_t *d_queue = (int32_t *)job.take(ctx->queue, (size_t)grid * NS * qcap * sizeof(int32_t));
+        int32_t *d_cnt = (int32_t *)job.take(ctx->cnt, (size_t)2 * L * sizeof(int32_t));
+        uint8_t *d_nxt = (uint8_t *)job.take(ctx->nxt, (size_t)2 * L);
+        int64_t *d_poff = (int64_t *)job.take(ctx->poff, (size_t)2 * L * sizeof(int64_t));
+        int64_t *d_gptr = (int64_t *)job.take(ctx->gptr, (size_t)2 * (L + 1) * sizeof(int64_t));
+        int32_t *d_lrow = (int32_t *)job.take(ctx->lrow, (size_t)L * sizeof(int32_t));
+        uint8_t *d_snind = (uint8_t *)job.take(ctx->snind, (size_t)L);
+        int32_t *d_sn = (int32_t *)job.take(ctx->snlist, (size_t)L * sizeof(int32_t));
+        int64_t *d_tiles = (int64_t *)job.take(ctx->tiles, (size_t)4 * ntiles * sizeof(int64_t));
         // misc: piece counter, pool tail, counters[4], status
         // and shared pieces: two words a CTA, the costs of pieces' beginnings
         const size_t misc_bytes = 256 + (share ? (size_t)grid * 16 + FRESH_BUCKETS * 4 : 0);
-        char *d_misc = (char *)ctx->grow(ctx->misc, misc_bytes);
+        char *d_misc = (char *)job.take(ctx->misc, misc_bytes);
         unsigned long long *d_piece = (unsigned long long *)d_misc;
         unsigned long long *d_tail = (unsigned long long *)(d_misc + 8);
         unsigned long long *d_counters = (unsigned long long *)(d_misc + 16);   // 16 counters
@@ -612,38 +593,34 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
         // read off the bitmap when the chain ends
         const int64_t stamp_stride = (int64_t)bitmap_words * 32;
         if (pattern_form == 1) {
-            d_pool = (int32_t *)ctx->grow(ctx->pool, (size_t)pool_cap * sizeof(int32_t));
-            d_out = (int32_t *)ctx->grow(ctx->out, (size_t)pool_cap * sizeof(int32_t));
+            d_pool = (int32_t *)job.take(ctx->pool, (size_t)pool_cap * sizeof(int32_t));
+            d_out = (int32_t *)job.take(ctx->out, (size_t)pool_cap * sizeof(int32_t));
         } else if (pattern_form == 2) {
             d_pool = ext->dev;
         }
         int32_t *d_lists = nullptr;
         if (want_pattern) {
-            d_stamp = (uint16_t *)ctx->grow(ctx->stamp, (size_t)grid * NS * 2 * stamp_stride * sizeof(uint16_t));
-            d_lists = (int32_t *)ctx->grow(ctx->lists, (size_t)grid * NS * qcap * sizeof(int32_t));
+            d_stamp = (uint16_t *)job.take(ctx->stamp, (size_t)grid * NS * 2 * stamp_stride * sizeof(uint16_t));
+            d_lists = (int32_t *)job.take(ctx->lists, (size_t)grid * NS * qcap * sizeof(int32_t));
         }
-        uint32_t *d_gstate = gbm ? (uint32_t *)ctx->grow(ctx->gstate, (size_t)grid * NS * state_words * 4) : nullptr;
-        // Snapshots: paired passes with reuse, as many as a sixteenth of the
-        // budget holds, and none where the job leaves no room for them.
+        uint32_t *d_gstate = gbm ? (uint32_t *)job.take(ctx->gstate, (size_t)grid * NS * state_words * 4) : nullptr;
+        MatDesc *d_mats = (MatDesc *)job.take(ctx->mats, md.size() * sizeof(MatDesc));
+        int64_t *d_minfo = (int64_t *)job.take(ctx->matinfo, (size_t)3 * count * sizeof(int64_t));
+        Range *d_ranges = (Range *)job.take(ctx->ranges, std::max<size_t>(ranges.size(), 1) * sizeof(Range));
+
+        // Snapshots, after all that the job needs: paired passes with reuse, as
+        // many as a sixteenth of the budget holds, and none where the job
+        // leaves no room for them.
         uint32_t *d_snap = nullptr;
         int snap_k = 0;
         if (paired && reuse) {
             const size_t one = (size_t)grid * NS * bitmap_words * 4;
-            for (int k = SNAP_MAX; k >= 2 && !snap_k; k >>= 1) {
-                const size_t need = std::max<size_t>(one * k, 256);
-                if (need > ctx->budget / 16) continue;
-                if (ctx->snap.bytes < need && ctx->held - ctx->snap.bytes + need > ctx->budget) continue;
-                try {
-                    d_snap = (uint32_t *)ctx->grow(ctx->snap, need);
-                    snap_k = k;
-                } catch (CudaFail &) {
-                    cudaGetLastError();
-                }
+            for (int k = SNAP_MAX; k >= 2 && !d_snap; k >>= 1) {
+                if (one * k > ctx->budget / 16) continue;
+                d_snap = (uint32_t *)job.take_if_room(ctx->snap, one * k);
+                if (d_snap) snap_k = k;
             }
         }
-        MatDesc *d_mats = (MatDesc *)ctx->grow(ctx->mats, md.size() * sizeof(MatDesc));
-        int64_t *d_minfo = (int64_t *)ctx->grow(ctx->matinfo, (size_t)3 * count * sizeof(int64_t));
-        Range *d_ranges = (Range *)ctx->grow(ctx->ranges, std::max<size_t>(ranges.size(), 1) * sizeof(Range));
 
         cudaStream_t st = ctx->stream;
         JobArgs a{};

@@ -1,0 +1,103 @@
+// Host harness for gsofa_scratch.hpp: a device of `room` bytes behind it.
+#include "../gsofa_b200/csrc/gsofa_scratch.hpp"
+
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+
+struct NoRoom {};
+
+struct FakeDevice {
+    static inline size_t room = 0, used = 0;
+    static inline std::map<void *, size_t> live;
+    static void *alloc(size_t bytes)
+    {
+        if (used + bytes > room) return nullptr;
+        void *p = std::malloc(1);
+        live[p] = bytes;
+        used += bytes;
+        return p;
+    }
+    static void free(void *p)
+    {
+        used -= live.at(p);
+        live.erase(p);
+        std::free(p);
+    }
+    static void no_room() { throw NoRoom{}; }
+};
+
+using gsofa::DevBuf;
+using Scratch = gsofa::Scratch<FakeDevice>;
+
+#define CHECK(x)                                                              \
+    do {                                                                      \
+        if (!(x)) {                                                           \
+            std::printf("line %d: %s\n", __LINE__, #x);                       \
+            std::exit(1);                                                     \
+        }                                                                     \
+    } while (0)
+
+template <class F>
+bool refused(F f)
+{
+    try {
+        f();
+    } catch (NoRoom &) {
+        return true;
+    }
+    return false;
+}
+
+int main()
+{
+    // every budget and device size around what a job takes: the addresses that
+    // it holds are live when its last buffer is in place
+    for (size_t limit = 0; limit < 2; limit++)
+        for (size_t total = 9000; total <= 14000; total += 50) {
+            FakeDevice::room = limit ? total : 1 << 20;
+            Scratch s;
+            s.budget = limit ? 1 << 20 : total;
+            DevBuf queue, snap, mats, ranges, other;
+            s.dispensable = {&snap};
+            s.grow(other, 1000);
+            for (size_t batch = 300; batch <= 1500; batch += 300) {   // each job larger than the last
+                refused([&] {
+                    Scratch::Job job(s);
+                    void *q = job.take(queue, 8000);
+                    void *k = job.take_if_room(snap, 2000);
+                    void *m = job.take(mats, batch), *r = job.take(ranges, batch);
+                    CHECK(FakeDevice::live.count(q) && FakeDevice::live.count(m) && FakeDevice::live.count(r));
+                    CHECK(!k || (k == snap.p && FakeDevice::live.count(k)));
+                });
+                CHECK(s.held <= s.budget && s.held == FakeDevice::used);
+                CHECK(!queue.taken && !snap.taken && !mats.taken);
+            }
+            // with the job over, what only saves time gives way
+            if (total >= 12000) CHECK(!refused([&] { s.grow(other, total - 1000 - 8000 - 3000 + 900); }));
+            for (DevBuf *b : {&queue, &snap, &mats, &ranges, &other}) s.release(*b);
+            CHECK(FakeDevice::used == 0 && s.held == 0);
+        }
+    // a job that asks for its optional buffer last fits wherever its others do
+    for (size_t total = 9000; total <= 14000; total += 50) {
+        FakeDevice::room = 1 << 20;
+        Scratch s;
+        s.budget = total;
+        DevBuf queue, snap, mats;
+        s.dispensable = {&snap};
+        for (size_t batch = 300; batch <= 1500; batch += 300) {
+            bool live = true;
+            const bool no = refused([&] {
+                Scratch::Job job(s);
+                job.take(queue, 8000);
+                job.take(mats, batch);
+                void *k = job.take_if_room(snap, 2000);
+                live = !k || FakeDevice::live.count(k);
+            });
+            CHECK(live && no == (8000 + batch > total));
+        }
+        for (DevBuf *b : {&queue, &snap, &mats}) s.release(*b);
+    }
+    std::printf("ok\n");
+    return 0;
+}

@@ -1,0 +1,55 @@
+"""The rules of a context's device scratch (gsofa_scratch.hpp), on a fake
+device; and on a GPU, jobs whose budget ends just where their optional scratch
+does."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import gsofa_b200
+import oracle
+from gsofa_b200 import matgen
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def test_nothing_that_a_job_has_taken_is_freed(tmp_path):
+    exe = str(tmp_path / "scratch_rules")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-o", exe, os.path.join(HERE, "scratch_rules.cpp")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
+
+
+def _snapshots_used(g, budget):
+    """Whether a counts-only job under this budget keeps snapshots."""
+    with gsofa_b200.Context(0, mem_budget_bytes=budget) as ctx:
+        r = ctx.symbfact(ctx.upload(g), want_pattern=0)
+        return r.cycles[2] > 0
+
+
+@pytest.mark.gpu
+def test_jobs_whose_budget_ends_just_where_their_snapshots_do():
+    g = matgen.grid3d(32, 24, 16, seed=6)      # 12,288 lines: snapshots are a twentieth of the scratch
+    ref = oracle.symbfact(g.beg, g.end, g.adj, want_pattern=False)
+    tiny = [matgen.grid2d(3, seed=i) for i in range(40)]
+    tiny_refs = [oracle.symbfact(t.beg, t.end, t.adj, want_pattern=False) for t in tiny]
+    lo, hi = 10 << 20, 64 << 20
+    assert _snapshots_used(g, hi) and not _snapshots_used(g, lo)
+    while hi - lo > 64:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if _snapshots_used(g, mid) else (mid, hi)
+    for budget in [hi + d for d in range(-2048, 4096, 256)] + [hi + (1 << k) for k in range(13, 18)]:
+        with gsofa_b200.Context(0, mem_budget_bytes=budget) as ctx:
+            m = ctx.upload(g)
+            for _ in range(2):
+                r = ctx.symbfact(m, want_pattern=0)
+                assert r.fill_count == ref["fill_count"], budget
+                assert np.array_equal(r.u_row_count, ref["u_row_count"]), budget
+                assert np.array_equal(r.l_col_count, ref["l_col_count"]), budget
+            # a larger job, which needs more for its descriptors, where the
+            # first one's snapshots are still held
+            rs = ctx.symbfact_batch([m] + [ctx.upload(t) for t in tiny], want_pattern=0)
+            for r, want in zip(rs, [ref] + tiny_refs):
+                assert r.fill_count == want["fill_count"], budget
+                assert np.array_equal(r.l_col_count, want["l_col_count"]), budget
