@@ -1577,7 +1577,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
     unsigned xch = 0;         // exchanges with the other pass so far
     bool mine = false, other = false;   // this pass, the other pass reached s
     bool step = false;        // s is not for a run
-    uint32_t total = 0;       // entries of the chain's lists from `pending` on
+    long long total = 0;      // entries of the chain's lists from `pending` on (up to 94 lists of n)
     int pending = 0;          // the chain's first list that is not written
     // the seeding window: lane i holds row bounds and degree of source wlo + i
     int wlo = 0, whi = 0, wb = 0, we = 0, wraw = 0, wadj0 = 0;
@@ -1777,7 +1777,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
                     acc.edges += (unsigned)deg;
                     if (pass == 0) acc.einsp += (unsigned)raw;
                 }
-                if (LISTS) total += cut * hc - cut * (cut + 1) / 2 +
+                if (LISTS) total += (long long)cut * hc - cut * (cut + 1) / 2 +
                          (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < cut ? found : 0));
                 hc = __shfl_sync(0xffffffffu, c, cut - 1);
                 cidx += cut;
