@@ -539,6 +539,7 @@ struct SharedState {
     unsigned long long prof[8];
     unsigned long long nsrc, nfresh;
     unsigned long long work[3];   // edges, pass-G expansions, pass-G input degrees
+    uint32_t carry[3];            // ... and 2^31s of them
     int snaps;              // L: snapshots taken in this piece
     int snap_credit;        // L: what traversals and snapshots taken over have earned, in vertices (-1: none yet)
     int weight;             // L: vertices queued by the state's traversals
@@ -557,6 +558,7 @@ __device__ __forceinline__ void init_state(SharedState &sh)
     for (int q = 0; q < 8; q++) sh.prof[q] = 0;
     sh.nsrc = sh.nfresh = 0;
     sh.work[0] = sh.work[1] = sh.work[2] = 0;
+    sh.carry[0] = sh.carry[1] = sh.carry[2] = 0;
     sh.tailc[0] = sh.tailc[1] = sh.tailc[2] = 0;
     sh.fetch[0] = sh.fetch[1] = sh.fetch[2] = 0;
 }
@@ -628,6 +630,10 @@ __device__ __forceinline__ uint32_t clock32()
     return c;
 }
 
+// Since c0 (clock32), in 256s of cycles: right on average, for steps of up to
+// 2^32 cycles and sums of minutes.
+__device__ __forceinline__ uint32_t since(uint32_t c0) { return ((clock32() >> 8) - (c0 >> 8)) & 0xffffffu; }
+
 // Barrier of the two leader warps of a CTA that runs both passes of a source.
 __device__ __forceinline__ void pair_sync()
 {
@@ -693,6 +699,25 @@ struct Tally {
     uint32_t slot = 0;   // sums of slot words: lanes 0, 8, .. degrees, lanes 1, 9, .. input degrees
 };
 
+// Before a traversal, which adds less than 2^31 to any tally (it expands a
+// vertex once, and the input has less than 2^31 entries): 2^31 of each that has
+// them move to SharedState::carry.
+__device__ __forceinline__ void carry(SharedState &sh, Tally &acc, int lane)
+{
+    const uint32_t slot = (lane & 7) < 2 ? acc.slot : 0u;
+    if ((int)(acc.edges | acc.xcnt | acc.einsp | slot) < 0) {
+        const bool first = sh.home.pass == 0;   // the other pass counts edges only
+        if ((int)acc.edges < 0) atomicAdd(&sh.carry[0], 1u);
+        if ((int)acc.xcnt < 0 && first) atomicAdd(&sh.carry[1], 1u);
+        if ((int)acc.einsp < 0 && first) atomicAdd(&sh.carry[2], 1u);
+        if ((int)slot < 0 && ((lane & 7) == 0 || first)) atomicAdd(&sh.carry[(lane & 7) ? 2 : 0], 1u);
+        acc.edges &= 0x7fffffffu;
+        acc.xcnt &= 0x7fffffffu;
+        acc.einsp &= 0x7fffffffu;
+        acc.slot &= 0x7fffffffu;
+    }
+}
+
 // The sum of a 32-bit tally over a warp, and its addition to a 64-bit counter.
 __device__ __forceinline__ void fold_tally(unsigned long long *to, uint32_t v, int lane)
 {
@@ -701,8 +726,10 @@ __device__ __forceinline__ void fold_tally(unsigned long long *to, uint32_t v, i
     if (lane == 0) atomicAdd(to, lo + (hi << 16));
 }
 
-__device__ __forceinline__ void fold_work(SharedState &sh, const Tally &acc, int pass, int lane)
+__device__ __forceinline__ void fold_work(SharedState &sh, Tally acc, int pass, int lane)
 {
+    carry(sh, acc, lane);
+    __syncwarp();
     fold_tally(&sh.work[0], acc.edges + ((lane & 7) == 0 ? acc.slot : 0u), lane);
     if (pass) return;
     fold_tally(&sh.work[1], acc.xcnt, lane);
@@ -1355,6 +1382,8 @@ __device__ __forceinline__ void run_op(const JobArgs &a, Trav<GBM> &t, SharedSta
 {
     if (LISTS) t.stamp = sh.stamp;
     if (op == OP_LEVELS) {
+        carry(sh, acc, htid & 31);
+        __syncwarp();
         run_levels<GT, CG, GBM>(t, sh, htid, bar, phase, acc);
     } else if (op == OP_CLEAR) {
         clear_state<GBM>(t.bits, htid >> 5, GT / 32 - 1, htid & 31);
@@ -1569,7 +1598,8 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
         tally(sh.prof[1], 0ull - c);
     };
     tally(sh.prof[1], 0ull - (unsigned long long)clock64());
-    uint32_t n_levels = 0, c_levels = 0, c_wait = 0;
+    uint32_t n_levels = 0;                // 2^32 levels would be a piece of half an hour
+    uint32_t c_levels = 0, c_wait = 0;    // cycles in 256s
 
     int prev = -2;
     int cidx = -1;            // index of the last source in its chain (-1: none yet)
@@ -1901,6 +1931,8 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
         int start = 0, end = tail, wstart = 0;
         if (end > 0) {
             const uint32_t c0 = clock32();
+            carry(sh, acc, lane);
+            __syncwarp();
             do {
                 if (end - start <= SOLO_MAX) {
                     __syncwarp();   // the level's queue entries, for every lane
@@ -1925,7 +1957,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
                     nh += take_nh();
                 }
             } while (end > start);
-            c_levels += clock32() - c0;
+            c_levels += since(c0);
         }
 
         // |hi(s)|: the bits above s; the link flag; both passes' exchange
@@ -1952,7 +1984,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
             const uint32_t c0 = clock32();
             pair_sync();
             other = pair_flag[par][1 - half] != 0;
-            c_wait += clock32() - c0;
+            c_wait += since(c0);
             if (nsnap > 0 && end > 0 && sh.weight >= heavy && sh.snap_credit >= heavy) {
                 const long long c0 = clock64();
                 int lo, hi;
@@ -1977,10 +2009,11 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
     }
     fold_work(sh, acc, pass, lane);
     if (lane == 0) {
+        const unsigned long long levels = (unsigned long long)c_levels << 8, wait = (unsigned long long)c_wait << 8;
         sh.prof[0] += n_levels;
-        sh.prof[2] += c_levels;
-        sh.prof[7] += c_wait;
-        sh.prof[1] += (unsigned long long)clock64() - c_levels - c_wait;
+        sh.prof[2] += levels;
+        sh.prof[7] += wait;
+        sh.prof[1] += (unsigned long long)clock64() - levels - wait;
         sh.op = OP_EXIT;
     }
     __syncwarp();
@@ -2175,7 +2208,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
         if (tid == 0) {
             unsigned long long ns = 0, nr = 0, wk[3] = {0, 0, 0}, pv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int h = 0; h < NS; h++) {
-                for (int q = 0; q < 3; q++) wk[q] += shs[h].work[q];
+                for (int q = 0; q < 3; q++) wk[q] += shs[h].work[q] + ((unsigned long long)shs[h].carry[q] << 31);
                 ns += shs[h].nsrc;
                 nr += shs[h].nsrc - shs[h].nfresh;
                 for (int q = 0; q < 8; q++) pv[q] += shs[h].prof[q];

@@ -36,3 +36,40 @@ def test_a_chain_of_lists_with_more_than_2_32_entries():
             assert c == n - 1 - s and torch.equal(pool[u:u + c], line[s + 1:]), s
             assert r.l_col_count[s] == 1 and int(pool[int(r.l_beg[s])]) == s + 1, s
     assert bool((pool[entries:] == -1).all())
+
+
+def _inspected(n, rows, lengths):
+    """Input entries of every source's line and of the lines that its traversal expands."""
+    total = 0
+    for s in range(n):
+        seen, todo = {s}, [s]
+        while todo:
+            v = todo.pop()
+            total += lengths[v]
+            for u in rows[v]:
+                if u < s and u not in seen:
+                    seen.add(u)
+                    todo.append(u)
+    return total
+
+
+@pytest.mark.parametrize("flags", [0, gsofa_b200.FLAG_GLOBAL_STATE], ids=["shared", "global"])
+@pytest.mark.parametrize("level", [1, 21], ids=["leader", "helpers"])
+@pytest.mark.parametrize("longer", [0, 30], ids=["slot", "long_row"])
+def test_work_that_one_lane_counts_past_2_32(flags, level, longer):
+    """Line 0 repeats one id 2^25 times, and every other line's traversal
+    expands it: 260 of them in a piece are 8.7e9 input entries, all in the same
+    lane's count.  With `longer` line 0's row does not fit a slot; with a first
+    level of 21 vertices it is the helper warps that expand it."""
+    n, copies = 260, 1 << 25
+    rows = [sorted(set(range(1, longer + 1)) | {n - 1})] + [list(range(min(v, level))) for v in range(1, n)]
+    lengths = [longer + copies] + [len(r) for r in rows[1:]]
+    adj = [np.arange(1, longer + 1, dtype=np.int32), np.full(copies, n - 1, np.int32)]
+    adj += [np.array(r, np.int32) for r in rows[1:]]
+    end = np.cumsum(lengths, dtype=np.int64).astype(np.int32)
+    beg = np.concatenate([[0], end[:-1]]).astype(np.int32)
+    with gsofa_b200.Context(0) as ctx:
+        m = ctx.upload(Graph(n, beg, end, np.concatenate(adj), "copies"))
+        r = ctx.symbfact(m, want_pattern=0, reuse=0, src_chunk=512, flags=flags)
+        assert r.e_insp == _inspected(n, rows, lengths)
+        assert r.e_insp > 1 << 32
