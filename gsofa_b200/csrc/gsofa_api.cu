@@ -314,9 +314,16 @@ double now_ms()
     return duration<double, std::milli>(steady_clock::now().time_since_epoch()).count();
 }
 
-// On at most *grid_io CTAs (returns how many it asked for).
-gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
-                        const gsofa_params *pin, gsofa_result *out, const ExtPool *ext, int *grid_io)
+// What a job that has to be run again has learned.
+struct JobTry {
+    int grid = INT32_MAX;   // CTAs at most; out: those it was planned for
+    int64_t guess = (int64_t)1 << 31;   // pool entries at most, while the lists' are not known
+    int64_t pool = -1;      // entries of the lists (CSR form), once they are known
+    bool again = false;     // out: run it again
+};
+
+gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
+                          const gsofa_params *pin, gsofa_result *out, const ExtPool *ext, JobTry &job_try)
 {
     static const bool host_timing = std::getenv("GSOFA_HOST_TIMING") != nullptr;
     const double t_enter = now_ms();
@@ -455,28 +462,74 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
         if (occ <= 0) return GSOFA_ERR_UNSUPPORTED;
         ctx->shapes.push_back({block, bitmap_words, paired, gbm, wide, want_pattern != 0, ring, occ});
     }
-    int per_sm = p.ctas_per_sm > 0 ? std::min(p.ctas_per_sm, occ) : occ;
-    int grid = per_sm * ctx->sm_count;
+    const int per_sm = p.ctas_per_sm > 0 ? std::min(p.ctas_per_sm, occ) : occ;
+    int grid = std::min(per_sm * ctx->sm_count, job_try.grid);
+    const int64_t qcap = std::max<int64_t>(p.queue_capacity, max_n);
+    const int64_t ntiles = (L + TILE - 1) / TILE;
+    // a 16-bit chain index per vertex for every traversal: its lists are
+    // read off the bitmap when the chain ends
+    const int64_t stamp_stride = (int64_t)bitmap_words * 32;
+    // What the job takes of the context's scratch: a part that the CTAs do not
+    // change (with the pool and the compacted lists of `pool_cap` entries, in
+    // the CSR form), and what every CTA takes.
+    struct Need { DevBuf *buf; int64_t bytes; };
+    const std::vector<Need> fixed = {
+        {&ctx->cnt, 2 * L * 4},      {&ctx->nxt, 2 * L},       {&ctx->poff, 2 * L * 8},
+        {&ctx->gptr, 2 * (L + 1) * 8}, {&ctx->lrow, L * 4},    {&ctx->snind, L},
+        {&ctx->snlist, L * 4},       {&ctx->tiles, 4 * ntiles * 8},
+        {&ctx->misc, 256 + (int64_t)grid * 16 + FRESH_BUCKETS * 4},
+        {&ctx->mats, (int64_t)count * (int64_t)sizeof(MatDesc)}, {&ctx->matinfo, (int64_t)count * 24},
+        {&ctx->ranges, (int64_t)count * (int64_t)sizeof(Range)}};
+    const std::vector<Need> per_cta = {
+        {&ctx->queue, NS * qcap * 4},
+        {&ctx->stamp, want_pattern ? NS * 2 * stamp_stride * 2 : 0},
+        {&ctx->lists, want_pattern ? NS * qcap * 4 : 0},
+        {&ctx->gstate, gbm ? (int64_t)NS * state_words * 4 : 0}};
+    int64_t per_cta_bytes = 0, fixed_bytes = 0, others = (int64_t)ctx->held - (int64_t)ctx->snap.bytes;
+    for (const Need &x : per_cta) {
+        per_cta_bytes += x.bytes;
+        others -= (int64_t)x.buf->bytes;
+    }
+    for (const Need &x : fixed) {
+        fixed_bytes += std::max<int64_t>(x.bytes, 256);
+        others -= (int64_t)x.buf->bytes;
+    }
+    if (pattern_form == 1) others -= (int64_t)ctx->pool.bytes + (int64_t)ctx->out.bytes;
+
+    // pool sizing: the last run's exact need (every chain takes an exact
+    // range, so the pool holds the lists with no gaps), else a share of the
+    // budget that leaves the traversals theirs; the ranges form writes into
+    // the caller's pool
+    const int64_t avail = (int64_t)ctx->budget - others - fixed_bytes;   // for pool and traversals
+    int64_t pool_cap = 0;
+    if (pattern_form == 2) {
+        pool_cap = ext->cap;
+    } else if (want_pattern) {
+        int64_t known = 0;
+        for (int i = 0; i < count; i++)
+            known = known < 0 || mats[i]->last_pattern_total < 0 ? -1 : known + mats[i]->last_pattern_total;
+        if (job_try.pool >= 0) {
+            pool_cap = job_try.pool;
+        } else if (p.pool_capacity > 0) {
+            pool_cap = p.pool_capacity;
+        } else if (known >= 0) {
+            pool_cap = known;
+        } else {
+            const int64_t freeb = ctx->budget > ctx->held ? (int64_t)(ctx->budget - ctx->held) : 0;
+            pool_cap = std::min({freeb / 4 / 8, (avail - grid * per_cta_bytes) / 8, job_try.guess});
+            pool_cap = std::max<int64_t>(pool_cap, 1 << 20);
+            job_try.guess = pool_cap;
+        }
+        pool_cap = std::max<int64_t>(pool_cap, 1);
+    }
+    // Concurrent traversals within the memory budget (the reference shrinks
+    // its sources per pass until the state fits its pool,
+    // with_space_optimization/symbfact.cuh:1465-1507)
     {
-        // Concurrent traversals within the memory budget (the reference
-        // shrinks its sources per pass until the state fits its pool,
-        // with_space_optimization/symbfact.cuh:1465-1507): every traversal
-        // holds a frontier queue of n entries and, with the pattern, two rows
-        // of n chain stamps and n entries of list scratch; the per-line arrays
-        // and a minimal pool come first.
-        const int64_t q = std::max<int64_t>(p.queue_capacity, max_n);
-        const int64_t per_cta = (int64_t)NS * (q * 4 + (want_pattern ? (int64_t)words_needed * 32 * 4 + q * 4 : 0) +
-                                               (gbm ? (int64_t)state_words * 4 : 0));
-        // cnt, nxt, poff, gptr, lrow, snind, sn_list
-        const int64_t per_line = 2 * 4 + 2 + 2 * 8 + 2 * 8 + 4 + 1 + 4;
-        const int64_t fixed = L * per_line + ((L + TILE - 1) / TILE) * 32 + 64 * 1024 +
-                              (want_pattern ? (int64_t)2 * 4 * (1 << 20) : 0);
-        const int64_t others = (int64_t)ctx->held - (int64_t)ctx->queue.bytes - (int64_t)ctx->stamp.bytes -
-                               (int64_t)ctx->gstate.bytes - (int64_t)ctx->lists.bytes - (int64_t)ctx->snap.bytes;
-        const int64_t room = (int64_t)ctx->budget - others - fixed;
-        if (room < per_cta) return GSOFA_ERR_OOM;
-        grid = (int)std::min<int64_t>(std::min(grid, *grid_io), room / per_cta);
-        *grid_io = grid;
+        const int64_t room = avail - (pattern_form == 1 ? 8 * pool_cap : 0);
+        if (room < per_cta_bytes) return GSOFA_ERR_OOM;
+        grid = (int)std::min<int64_t>(grid, room / per_cta_bytes);
+        job_try.grid = grid;
     }
     // Sources per work piece.  A piece's first source cannot reuse state, and
     // its traversal from nothing costs as much as hundreds of later ones, so
@@ -536,38 +589,21 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
         ranges.push_back(r);
     }
 
-    const int64_t qcap = std::max<int64_t>(p.queue_capacity, max_n);
-    const int64_t ntiles = (L + TILE - 1) / TILE;
-
-    // pool sizing: the last run's exact need (every chain takes an exact
-    // range, so the pool holds the lists with no gaps), else a share of the
-    // budget; the ranges form writes into the caller's pool
-    auto pool_need = [&](int64_t entries) { return std::max<int64_t>(entries, 1); };
-    int64_t pool_cap = 0;
-    if (pattern_form == 2) {
-        pool_cap = ext->cap;
-    } else if (want_pattern) {
-        if (p.pool_capacity > 0) {
-            pool_cap = p.pool_capacity;
-        } else {
-            int64_t known = 0;
-            bool all_known = true;
-            for (int i = 0; i < count; i++) {
-                if (mats[i]->last_pattern_total < 0) all_known = false;
-                else known += mats[i]->last_pattern_total;
-            }
-            if (all_known) {
-                pool_cap = pool_need(known);
-            } else {
-                size_t freeb = ctx->budget > ctx->held ? ctx->budget - ctx->held : 0;
-                pool_cap = std::max<int64_t>((int64_t)(freeb / 4 / (2 * sizeof(int32_t))), 1 << 20);
-                pool_cap = std::min<int64_t>(pool_cap, (int64_t)1 << 31);
-            }
-        }
-    }
-
     ctx->job_id++;
-    for (int attempt = 0; attempt < 2; attempt++) {
+    {
+        // buffers that former jobs left larger than this one's go where all do
+        // not fit
+        int64_t all = others;
+        auto most = [&](const DevBuf &b, int64_t bytes) { all += std::max<int64_t>((int64_t)b.bytes, std::max<int64_t>(bytes, 256)); };
+        auto spare = [&](DevBuf &b, int64_t bytes) { if ((int64_t)b.bytes > std::max<int64_t>(bytes, 256)) ctx->release(b); };
+        for (const Need &x : fixed) most(*x.buf, x.bytes);
+        for (const Need &x : per_cta) most(*x.buf, grid * x.bytes);
+        if (pattern_form == 1) for (DevBuf *b : {&ctx->pool, &ctx->out}) most(*b, 4 * pool_cap);
+        if (all > (int64_t)ctx->budget) {
+            for (const Need &x : fixed) spare(*x.buf, x.bytes);
+            for (const Need &x : per_cta) spare(*x.buf, grid * x.bytes);
+            if (pattern_form == 1) for (DevBuf *b : {&ctx->pool, &ctx->out}) spare(*b, 4 * pool_cap);
+        }
         Scratch::Job job(*ctx);
         // scratch
         int32_t *d_queue = (int32_t *)job.take(ctx->queue, (size_t)grid * NS * qcap * sizeof(int32_t));
@@ -589,9 +625,6 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
         uint32_t *d_status = (uint32_t *)(d_misc + 192);
         int32_t *d_pool = nullptr, *d_out = nullptr;
         uint16_t *d_stamp = nullptr;
-        // a 16-bit chain index per vertex for every traversal: its lists are
-        // read off the bitmap when the chain ends
-        const int64_t stamp_stride = (int64_t)bitmap_words * 32;
         if (pattern_form == 1) {
             d_pool = (int32_t *)job.take(ctx->pool, (size_t)pool_cap * sizeof(int32_t));
             d_out = (int32_t *)job.take(ctx->out, (size_t)pool_cap * sizeof(int32_t));
@@ -777,9 +810,10 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
         // a property of the input
         if (status & ERR_COUNT_MISMATCH) return GSOFA_ERR_CUDA;
         if (want_pattern && (status & ERR_POOL_OVERFLOW)) {
-            if (attempt == 0 && pattern_form == 1) {
-                pool_cap = pool_need(tot[0] + tot[1]);
-                continue;   // rerun with the pool the counts ask for
+            if (job_try.pool < 0 && pattern_form == 1) {
+                job_try.pool = tot[0] + tot[1];
+                job_try.again = true;   // with the pool the counts ask for, if it fits
+                return GSOFA_ERR_QUEUE_OVERFLOW;
             }
             // the caller's pool is too small: report what the job needs
             for (int i = 0; i < count; i++) out[i].pool_used = (int64_t)h_misc[1];
@@ -890,29 +924,32 @@ gsofa_status run_job_on(gsofa_ctx *ctx, int count, const gsofa_matrix *const *ma
             for (int i = 0; i < count; i++) out[i].fill_count = out[i].nnz_u + out[i].nnz_l - processed_orig(i);
         return GSOFA_OK;
     }
-    return GSOFA_ERR_QUEUE_OVERFLOW;
 }
 
-// The job on as many CTAs as the budget holds: where it runs out of memory (the
-// lists' pool comes after the traversals' scratch), it is tried again on three
-// quarters of them.
+// A job is planned within the budget and run once; where its lists need more
+// than the pool it was given, once more with what the first run counted, or it
+// is refused.  Where the device has less memory than the budget says (nothing
+// has run then), it is planned smaller.
 gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
                      const gsofa_params *pin, gsofa_result *out, const ExtPool *ext = nullptr)
 {
-    int grid = INT32_MAX;
+    JobTry t;
     for (;;) {
+        t.again = false;
+        const int former = t.grid;
         gsofa_status s;
         try {
-            s = run_job_on(ctx, count, mats, pin, out, ext, &grid);
+            s = run_job_once(ctx, count, mats, pin, out, ext, t);
         } catch (CudaFail &f) {
-            if (f.e != cudaErrorMemoryAllocation || grid <= 1 || grid == INT32_MAX) throw;
+            if (f.e != cudaErrorMemoryAllocation || t.grid <= 1 || t.grid == INT32_MAX) throw;
             cudaGetLastError();
-            s = GSOFA_ERR_OOM;
+            for (DevBuf *b : {&ctx->queue, &ctx->stamp, &ctx->lists, &ctx->gstate, &ctx->snap}) ctx->release(*b);
+            t.grid = std::min(t.grid, former) * 3 / 4;
+            t.guess /= 2;
+            continue;
         }
-        if (s != GSOFA_ERR_OOM || grid <= 1 || grid == INT32_MAX) return s;
-        for (int i = 0; i < count; i++) free_result_arrays(&out[i]);
-        for (DevBuf *b : {&ctx->queue, &ctx->stamp, &ctx->lists, &ctx->gstate, &ctx->snap}) ctx->release(*b);
-        grid = grid * 3 / 4;
+        if (!t.again) return s;
+        t.grid = former;
     }
 }
 

@@ -3,6 +3,7 @@ device; and on a GPU, jobs whose budget ends just where their optional scratch
 does."""
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -10,6 +11,7 @@ import pytest
 import gsofa_b200
 import oracle
 from gsofa_b200 import matgen
+from tests.common import assert_same
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -53,3 +55,43 @@ def test_jobs_whose_budget_ends_just_where_their_snapshots_do():
             for r, want in zip(rs, [ref] + tiny_refs):
                 assert r.fill_count == want["fill_count"], budget
                 assert np.array_equal(r.l_col_count, want["l_col_count"]), budget
+
+
+@pytest.mark.gpu
+def test_a_pattern_that_fits_nowhere_is_refused_after_one_run():
+    """The lists of the 48^3 stencil take 708 MB with their compacted copy; a
+    context with less runs the job once to learn that, not once for every
+    number of CTAs."""
+    g = matgen.grid3d(48, seed=3)
+    with gsofa_b200.Context(0, mem_budget_bytes=600 << 20) as ctx:
+        m = ctx.upload(g)
+        took = []
+        for _ in range(3):
+            t = time.perf_counter()
+            with pytest.raises(gsofa_b200.GsofaError) as e:
+                ctx.symbfact(m)
+            took.append(time.perf_counter() - t)
+            assert e.value.status == 2
+        # a run at full width takes 1.3 ms; all numbers of CTAs some 700
+        assert min(took) < 0.1, took
+        # counts need no pool; and once they are known, nothing runs in vain
+        assert ctx.symbfact(m, want_pattern=0).nnz_lu > 88_000_000
+        with pytest.raises(gsofa_b200.GsofaError):
+            ctx.symbfact(m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mib", [200, 260, 320, 400, 600])
+def test_a_pattern_that_fits_beside_fewer_ctas(mib):
+    """Where lists and traversals do not fit together at full width, the job is
+    run on the CTAs that do, on a context that has met the matrix or not."""
+    g = matgen.grid3d(32, seed=4)              # 32,768 lines; lists 19.6M entries, 157 MB with their copy
+    ref = oracle.symbfact(g.beg, g.end, g.adj)
+    with gsofa_b200.Context(0, mem_budget_bytes=mib << 20) as ctx:
+        m = ctx.upload(g)
+        for _ in range(2):
+            assert_same(ctx.symbfact(m), ref, where=f"{mib} MiB")
+        assert_same(ctx.symbfact(ctx.upload(g)), ref, where=f"{mib} MiB, once more")
+        small = matgen.grid2d(20, seed=1)
+        assert_same(ctx.symbfact(ctx.upload(small)), oracle.symbfact(small.beg, small.end, small.adj), where="small")
+        assert_same(ctx.symbfact(m), ref, where=f"{mib} MiB, after a small one")
