@@ -480,16 +480,26 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         {&ctx->misc, 256 + (int64_t)grid * 16 + FRESH_BUCKETS * 4},
         {&ctx->mats, (int64_t)count * (int64_t)sizeof(MatDesc)}, {&ctx->matinfo, (int64_t)count * 24},
         {&ctx->ranges, (int64_t)count * (int64_t)sizeof(Range)}};
-    const std::vector<Need> per_cta = {
+    std::vector<Need> per_cta = {
         {&ctx->queue, NS * qcap * 4},
+        {&ctx->gstate, gbm ? (int64_t)NS * state_words * 4 : 0},
         {&ctx->stamp, want_pattern ? NS * 2 * stamp_stride * 2 : 0},
-        {&ctx->lists, want_pattern ? NS * qcap * 4 : 0},
-        {&ctx->gstate, gbm ? (int64_t)NS * state_words * 4 : 0}};
+        {&ctx->lists, want_pattern ? NS * qcap * 4 : 0}};
     int64_t per_cta_bytes = 0, fixed_bytes = 0, others = (int64_t)ctx->held - (int64_t)ctx->snap.bytes;
     for (const Need &x : per_cta) {
         per_cta_bytes += x.bytes;
         others -= (int64_t)x.buf->bytes;
     }
+    // The list output's own part of that is a second row of stamps and the
+    // scratch its lists are made in, which let it go on beside the traversal;
+    // a traversal can wait for its lists instead, with one row and its queue.
+    // That takes 8 to 14% longer on as many CTAs (80^3 ranges 8.5 ms and 7.5,
+    // 20,011-line power law 3.5 and 3.2), and half the scratch: where it puts
+    // an eighth more CTAs to work it is the faster one (80^3 with room for 114
+    // or 148: 10.4 and 8.5 ms; for 76 or 148: 12.2 and 10.3; power law with
+    // room for 117 or 148: 5.9 and 3.5).
+    const int64_t beside_bytes = want_pattern ? NS * (stamp_stride * 2 + qcap * 4) : 0;
+    bool beside = true;
     for (const Need &x : fixed) {
         fixed_bytes += std::max<int64_t>(x.bytes, 256);
         others -= (int64_t)x.buf->bytes;
@@ -516,7 +526,7 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
             pool_cap = known;
         } else {
             const int64_t freeb = ctx->budget > ctx->held ? (int64_t)(ctx->budget - ctx->held) : 0;
-            pool_cap = std::min({freeb / 4 / 8, (avail - grid * per_cta_bytes) / 8, job_try.guess});
+            pool_cap = std::min({freeb / 4 / 8, (avail - grid * (per_cta_bytes - beside_bytes)) / 8, job_try.guess});
             pool_cap = std::max<int64_t>(pool_cap, 1 << 20);
             job_try.guess = pool_cap;
         }
@@ -527,8 +537,15 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
     // with_space_optimization/symbfact.cuh:1465-1507)
     {
         const int64_t room = avail - (pattern_form == 1 ? 8 * pool_cap : 0);
-        if (room < per_cta_bytes) return GSOFA_ERR_OOM;
-        grid = (int)std::min<int64_t>(grid, room / per_cta_bytes);
+        const int64_t most = std::min<int64_t>(grid, room / per_cta_bytes);
+        const int64_t waiting = std::min<int64_t>(grid, room / (per_cta_bytes - beside_bytes));
+        if (waiting < 1) return GSOFA_ERR_OOM;
+        beside = most * 8 >= waiting * 7;
+        if (!beside) {
+            per_cta[2].bytes /= 2;
+            per_cta[3].bytes = 0;
+        }
+        grid = (int)(beside ? most : waiting);
         job_try.grid = grid;
     }
     // Sources per work piece.  A piece's first source cannot reuse state, and
@@ -633,8 +650,8 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         }
         int32_t *d_lists = nullptr;
         if (want_pattern) {
-            d_stamp = (uint16_t *)job.take(ctx->stamp, (size_t)grid * NS * 2 * stamp_stride * sizeof(uint16_t));
-            d_lists = (int32_t *)job.take(ctx->lists, (size_t)grid * NS * qcap * sizeof(int32_t));
+            d_stamp = (uint16_t *)job.take(ctx->stamp, (size_t)(grid * per_cta[2].bytes));
+            d_lists = beside ? (int32_t *)job.take(ctx->lists, (size_t)(grid * per_cta[3].bytes)) : d_queue;
         }
         uint32_t *d_gstate = gbm ? (uint32_t *)job.take(ctx->gstate, (size_t)grid * NS * state_words * 4) : nullptr;
         MatDesc *d_mats = (MatDesc *)job.take(ctx->mats, md.size() * sizeof(MatDesc));
@@ -702,6 +719,7 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         a.status = d_status;
         a.stamp = d_stamp;
         a.stamp_stride = stamp_stride;
+        a.stamp_other = beside ? stamp_stride : 0;
         a.lists = d_lists;
         a.gbm = d_gstate;
         a.blk_done = ext ? ext->blk_done : nullptr;

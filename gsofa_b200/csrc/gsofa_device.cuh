@@ -16,7 +16,8 @@
 //                 once per source, so qcap >= n never overflows);
 //                 pattern mode: two rows of n uint16 stamps, the chain index at
 //                 which each vertex was first set (one row is being written
-//                 while the other's lists go out), and a chain's vertices;
+//                 while the other's lists go out), and a chain's vertices
+//                 (where memory is short: one row, the vertices in the queue);
 //                 up to SNAP_MAX bitmaps of finished traversals (snapshots).
 // The visited set is an n-bit bitmap with two summary levels, in shared memory
 // or, for large n, in global memory.
@@ -171,7 +172,9 @@ struct JobArgs {
     uint32_t *status;
     uint16_t *stamp;           // pattern mode: per traversal, two rows of stamp_stride
     int64_t stamp_stride;      // entries: the chain index at which each vertex was first set
-    int32_t *lists;            // pattern mode: qcap entries per traversal
+    int64_t stamp_other;       // entries from a traversal's first row to its other one; 0: it has
+                               // one row, and no work goes on beside its list output
+    int32_t *lists;            // pattern mode: qcap entries per traversal (its queue, with one row)
     uint32_t *snap;            // snapshots: snap_k bitmaps per traversal slot
     uint32_t *gbm;             // global-state kernels: per traversal, state_words
                                // words (bitmap and its summaries) in global memory
@@ -1163,7 +1166,8 @@ __device__ __forceinline__ void merge_state(const Trav<GBM> &t, const uint32_t *
 // Writes lists first .. len - 1 of a chain -- sources s0, s0 + 1, .. which share
 // one bitmap -- by the helper warps, while the leader goes on with the next
 // sources: it waits only until the set vertices are out of the bitmap (the
-// barrier in the middle).  Bits are only ever added along a chain, so list i is
+// barrier in the middle), unless the traversal has no scratch for both
+// (JobArgs::stamp_other).  Bits are only ever added along a chain, so list i is
 // { v > s0 + i : v set, stamp(v) <= i } once source i is done; what later
 // sources add has larger stamps.  One exact pool
 // range holds all of the chain's lists (one global atomic per chain).
@@ -1394,7 +1398,7 @@ __device__ __forceinline__ void run_op(const JobArgs &a, Trav<GBM> &t, SharedSta
                              htid);
     } else if (LISTS && op == OP_LISTS) {
         write_lists<GT, GBM>(a, t, sh, hist, htid, bar);   // the leader goes on from its middle
-        return;
+        if (a.stamp_other != 0) return;
     }
     gsync<GT>(bar);
 }
@@ -1635,6 +1639,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
             sh.chain_hi = min(hi << 5, n) - 1;
         }
         collective(OP_LISTS);
+        if (a.stamp_other == 0) gsync<GT>(bar);   // its stamps and its queue are free again
         pending = cidx + 1;
         total = 0;
         spent(5, c0);
@@ -1645,7 +1650,7 @@ __device__ __noinline__ void lead_piece(Trav<GBM> t, int32_t s_lo, int32_t s_hi,
             if (pending <= cidx) lists_out();
             // the helpers read this chain's stamps on: the next chain takes
             // the traversal's other row
-            t.stamp = t.stamp == sh.home.stamps ? sh.home.stamps + a.stamp_stride : sh.home.stamps;
+            t.stamp = t.stamp == sh.home.stamps ? sh.home.stamps + a.stamp_other : sh.home.stamps;
         }
         const long long c0 = clock64();
         const int chunks = state_extent<GBM>(t.bits, lane, lo, hi);
@@ -2106,7 +2111,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) factor_kernel(const __grid_consta
     Trav<GBM> t{};
     t.bits = bits_at<GBM>(state + (size_t)half * a.state_words + STATE_PAD, a.bitmap_words);
     t.f = Frontier{(uint32_t)__cvta_generic_to_shared(ring), a.ring_size};
-    if (LISTS && a.want_pattern) t.stamp = a.stamp + 2 * trav * a.stamp_stride;
+    if (LISTS && a.want_pattern) t.stamp = a.stamp + trav * (a.stamp_stride + a.stamp_other);
     if (gtid == 0) {
         sh.home.spill = a.queue + trav * a.qcap;
         sh.home.snaps = a.snap + trav * a.snap_k * a.bitmap_words;

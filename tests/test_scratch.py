@@ -1,6 +1,7 @@
 """The rules of a context's device scratch (gsofa_scratch.hpp), on a fake
 device; and on a GPU, jobs whose budget ends just where their optional scratch
 does."""
+import functools
 import os
 import subprocess
 import time
@@ -11,6 +12,7 @@ import pytest
 import gsofa_b200
 import oracle
 from gsofa_b200 import matgen
+from gsofa_b200.matgen import Graph
 from tests.common import assert_same
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -95,3 +97,59 @@ def test_a_pattern_that_fits_beside_fewer_ctas(mib):
         small = matgen.grid2d(20, seed=1)
         assert_same(ctx.symbfact(ctx.upload(small)), oracle.symbfact(small.beg, small.end, small.adj), where="small")
         assert_same(ctx.symbfact(m), ref, where=f"{mib} MiB, after a small one")
+
+
+def _least_budget(g, **kw):
+    """The smallest budget, to a KiB, under which the job runs."""
+    lo, hi = 1 << 20, 1 << 30
+    while hi - lo > 1024:
+        mid = (lo + hi) // 2
+        with gsofa_b200.Context(0, mem_budget_bytes=mid) as ctx:
+            try:
+                ctx.symbfact(ctx.upload(g), **kw)
+                hi = mid
+            except gsofa_b200.GsofaError as e:
+                assert e.status == 2
+                lo = mid
+    return hi
+
+
+@pytest.mark.gpu
+def test_lists_need_a_row_of_stamps_and_no_more():
+    """Beside what counts take, the least that a job with lists runs in is its
+    pool and one row of stamps for each of two traversals."""
+    n = 100_000
+    end = np.concatenate([np.arange(2, 2 * n, 2), [2 * n - 2]]).astype(np.int32)
+    end[0] = 1
+    end[1:-1] = np.arange(3, 2 * n - 2, 2)
+    beg = np.concatenate([[0], end[:-1]]).astype(np.int32)
+    adj = np.concatenate([[1], np.stack([np.arange(n - 2), np.arange(2, n)], 1).ravel(), [n - 2]]).astype(np.int32)
+    g = Graph(n, beg, end, adj, "path")
+    row = 2 * ((n + 4095) // 4096 * 4096)
+    assert _least_budget(g) - _least_budget(g, want_pattern=0) <= 2 * row + (8 << 20) + 4096
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [functools.partial(matgen.grid2d, 37, drop_frac=0.1, seed=5),
+                                  functools.partial(matgen.grid3d, 23, 21, 19, seed=6),
+                                  functools.partial(matgen.powerlaw, 3001, seed=4),
+                                  functools.partial(matgen.bordered_blocks, 100, seed=2)],
+                         ids=["grid2d", "nd3d", "powerlaw", "bordered"])
+@pytest.mark.parametrize("flags", [0, gsofa_b200.FLAG_GLOBAL_STATE], ids=["shared", "global"])
+def test_lists_at_every_budget(make, flags):
+    """From the least budget on: one row of stamps a traversal, then two, and
+    few CTAs to all."""
+    g = make()
+    ref = oracle.symbfact(g.beg, g.end, g.adj)
+    ctas = set()
+    budget = _least_budget(g, flags=flags)
+    while budget < 256 << 20:
+        for reuse in (-1, 2):
+            with gsofa_b200.Context(0, mem_budget_bytes=budget) as ctx:
+                m = ctx.upload(g)
+                for _ in range(2):
+                    r = ctx.symbfact(m, flags=flags, reuse=reuse)
+                    assert_same(r, ref, where=f"{g.name} budget {budget} reuse {reuse}")
+            ctas.add(r.ctas)
+        budget += budget // 12
+    assert len(ctas) > 4
