@@ -128,7 +128,7 @@ struct gsofa_ctx : Scratch {
     struct Shape { int block; int32_t words; bool paired; bool gbm; bool wide; bool lists; int ring; int occ; };
     std::vector<Shape> shapes;
 
-    gsofa_ctx() { dispensable = {&snap}; }
+    gsofa_ctx() { dispensable = {&snap, &lists, &stamp, &gstate, &queue}; }
 
     // Device slabs of freed matrices, kept for later uploads so that a caller
     // who uploads, factorizes and frees matrix after matrix pays no
@@ -151,10 +151,8 @@ struct gsofa_ctx : Scratch {
             *got = b.bytes;
             return b.p;
         }
-        void *p = nullptr;
-        GS_CUDA(cudaMalloc(&p, bytes));
         *got = bytes;
-        return p;
+        return alloc(bytes);
     }
     void slab_give(void *p, size_t bytes)
     {
@@ -1463,12 +1461,12 @@ gsofa_status gsofa_symbfact_ranges(gsofa_ctx *c, int count, const gsofa_matrix *
                 return GSOFA_ERR_INVALID_INPUT;
             }
             // Staged through device memory when a device pool of the same
-            // capacity fits the budget (the copy engine moves it at full
+            // capacity fits the budget beside what cannot give way (the copy engine moves it at full
             // PCIe speed); else, or with GSOFA_FLAG_DIRECT_HOST, the kernel
             // writes the lists into host memory itself, so the pattern needs
             // no device memory at all.
             const size_t bytes = (size_t)pool_capacity * 4;
-            const bool staged = !(p.flags & GSOFA_FLAG_DIRECT_HOST) && c->held - c->pool.bytes + bytes <= c->budget / 2;
+            const bool staged = !(p.flags & GSOFA_FLAG_DIRECT_HOST) && c->held - c->idle() - c->pool.bytes + bytes <= c->budget / 2;
             if (staged) {
                 ext.dev = (int32_t *)c->grow(c->pool, bytes);
                 host_dst = pool;

@@ -2,8 +2,9 @@
 // (host only; the device allocator is a parameter, so the rules can be tested
 // without one).
 //
-// Every buffer grows and is kept for the next job.  Buffers that only save time
-// give way to what a job needs, but never while a job that is being set up or
+// Every buffer grows and is kept for the next job.  Dispensable buffers -- those
+// that only save time, and a job's own, which the next one can make again -- give
+// way to whatever needs the room, but never while a job that is being set up or
 // is running has taken them: what a job has its addresses from stays.
 #pragma once
 
@@ -38,6 +39,14 @@ struct Scratch {
         b.bytes = 0;
     }
 
+    // Bytes that can give way now.
+    size_t idle() const
+    {
+        size_t bytes = 0;
+        for (const DevBuf *d : dispensable) bytes += d->taken ? 0 : d->bytes;
+        return bytes;
+    }
+
     // Frees one dispensable buffer other than b that no job has taken; false
     // when there is none.
     bool give_way(const DevBuf *b)
@@ -50,6 +59,15 @@ struct Scratch {
         return false;
     }
 
+    // Device memory outside the budget (b: not to be freed for it).
+    void *alloc(size_t bytes, const DevBuf *b = nullptr)
+    {
+        void *p;
+        while (!(p = Memory::alloc(bytes)))
+            if (!give_way(b)) Memory::no_room();
+        return p;
+    }
+
     // At least `bytes` in b (contents are not kept).
     void *grow(DevBuf &b, size_t bytes)
     {
@@ -58,13 +76,10 @@ struct Scratch {
         release(b);
         while (held + bytes > budget)
             if (!give_way(&b)) Memory::no_room();
-        void *p;
-        while (!(p = Memory::alloc(bytes)))
-            if (!give_way(&b)) Memory::no_room();
-        b.p = p;
+        b.p = alloc(bytes, &b);
         b.bytes = bytes;
         held += bytes;
-        return p;
+        return b.p;
     }
 
     // The buffers of one job, from the first one taken until the job ends.

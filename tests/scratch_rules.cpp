@@ -98,6 +98,36 @@ int main()
         }
         for (DevBuf *b : {&queue, &snap, &mats}) s.release(*b);
     }
+    // what a job left gives way to anything else, in order, whether the budget
+    // or the device is short; not to a buffer that holds it itself, nor while
+    // a job has it
+    for (size_t limit = 0; limit < 2; limit++) {
+        FakeDevice::room = limit ? 10000 : 1 << 20;
+        Scratch s;
+        s.budget = limit ? 1 << 20 : 10000;
+        DevBuf snap, lists, order;
+        s.dispensable = {&snap, &lists};
+        {
+            Scratch::Job job(s);
+            job.take(lists, 6000);
+            CHECK(job.take_if_room(snap, 3000) && !job.take_if_room(order, 3000) && s.idle() == 0);
+            CHECK(refused([&] { s.grow(order, 3000); }));
+            if (limit) CHECK(refused([&] { s.alloc(3000); }));
+        }
+        CHECK(s.idle() == 9000);
+        CHECK(!refused([&] { s.grow(order, 3000); }) && !snap.p && lists.p);
+        CHECK(!refused([&] { s.grow(order, 9000); }) && !lists.p);
+        CHECK(!refused([&] { s.grow(snap, 1000); }) && refused([&] { s.grow(snap, 1001 + 1000); }));
+        s.release(order);
+        if (limit) {
+            s.grow(lists, 5000);
+            void *p = s.alloc(6000);
+            CHECK(p && !lists.p);
+            FakeDevice::free(p);
+        }
+        for (DevBuf *b : {&snap, &lists, &order}) s.release(*b);
+        CHECK(FakeDevice::used == 0);
+    }
     std::printf("ok\n");
     return 0;
 }

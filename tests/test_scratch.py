@@ -153,3 +153,30 @@ def test_lists_at_every_budget(make, flags):
             ctas.add(r.ctas)
         budget += budget // 12
     assert len(ctas) > 4
+
+
+@pytest.mark.gpu
+def test_what_a_job_left_gives_way_to_other_calls():
+    """A job takes all the CTAs that a small budget holds; an ordering, a larger
+    upload and the streamed form find room on the same context all the same."""
+    import torch
+    g = matgen.grid3d(21, seed=3)
+    ref = oracle.symbfact(g.beg, g.end, g.adj)
+    # the ordering takes about 5 MiB (two arrays of 141,000 keys, columns, sort
+    # space); the job's traversals fill what its lists (19 MiB with their copy) leave
+    big = matgen.powerlaw(8000, seed=1, ordering="random")
+    with gsofa_b200.Context(0) as ctx:
+        perm = ctx.order_rcm(big)
+    for mib in (32, 36, 44):
+        with gsofa_b200.Context(0, mem_budget_bytes=mib << 20) as ctx:
+            m = ctx.upload(g)
+            assert_same(ctx.symbfact(m), ref, where=f"{mib} MiB")
+            assert np.array_equal(ctx.order_rcm(big), perm)
+            assert_same(ctx.symbfact(m), ref, where=f"{mib} MiB, after an ordering")
+            ctx.upload(big).free()
+            pool = torch.zeros(ref["u_idx"].size + ref["l_idx"].size, dtype=torch.int32).pin_memory().numpy()
+            for _ in range(2):
+                r = ctx.symbfact_ranges(m, pool)
+                assert np.array_equal(r.u_row_count, ref["u_row_count"])
+                for v in (0, 100, 5000, 9000):
+                    assert np.array_equal(r.u_row(v), ref["u_idx"][ref["u_ptr"][v]:ref["u_ptr"][v + 1]])
