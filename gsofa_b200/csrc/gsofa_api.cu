@@ -105,10 +105,9 @@ struct gsofa_ctx : Scratch {
     cudaStream_t own_stream = nullptr;  // the context's own stream
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // job scratch
-    DevBuf queue, cnt, nxt, poff, gptr, lrow, snind, snlist, tiles, misc, pool, out, mats, ranges, stamp;
-    DevBuf lists;             // list output: a chain's vertices, per traversal
-    DevBuf snap;              // snapshots of finished traversals
-    DevBuf gstate;            // visited bitmaps of the global-state kernels
+    DevBuf cnt, nxt, poff, gptr, lrow, snind, snlist, tiles, misc, pool, out, mats, ranges;
+    DevBuf trav;              // of the traversals: queues, bitmaps in global memory, stamps, list
+                              // scratch, snapshots of finished traversals
     DevBuf blk;               // streaming: written entries per pool block
     DevBuf order;             // gsofa_order_rcm: symmetric structure, levels, sort space
     unsigned int *h_blk = nullptr;   // page-locked mirror of blk
@@ -128,7 +127,7 @@ struct gsofa_ctx : Scratch {
     struct Shape { int block; int32_t words; bool paired; bool gbm; bool wide; bool lists; int ring; int occ; };
     std::vector<Shape> shapes;
 
-    gsofa_ctx() { dispensable = {&snap, &lists, &stamp, &gstate, &queue}; }
+    gsofa_ctx() { dispensable = {&trav}; }
 
     // Device slabs of freed matrices, kept for later uploads so that a caller
     // who uploads, factorizes and frees matrix after matrix pays no
@@ -315,6 +314,7 @@ double now_ms()
 // What a job that has to be run again has learned.
 struct JobTry {
     int grid = INT32_MAX;   // CTAs at most; out: those it was planned for
+    bool snaps = true;      // with snapshots where the budget has room
     int64_t guess = (int64_t)1 << 31;   // pool entries at most, while the lists' are not known
     int64_t pool = -1;      // entries of the lists (CSR form), once they are known
     bool again = false;     // out: run it again
@@ -478,26 +478,20 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         {&ctx->misc, 256 + (int64_t)grid * 16 + FRESH_BUCKETS * 4},
         {&ctx->mats, (int64_t)count * (int64_t)sizeof(MatDesc)}, {&ctx->matinfo, (int64_t)count * 24},
         {&ctx->ranges, (int64_t)count * (int64_t)sizeof(Range)}};
-    std::vector<Need> per_cta = {
-        {&ctx->queue, NS * qcap * 4},
-        {&ctx->gstate, gbm ? (int64_t)NS * state_words * 4 : 0},
-        {&ctx->stamp, want_pattern ? NS * 2 * stamp_stride * 2 : 0},
-        {&ctx->lists, want_pattern ? NS * qcap * 4 : 0}};
-    int64_t per_cta_bytes = 0, fixed_bytes = 0, others = (int64_t)ctx->held - (int64_t)ctx->snap.bytes;
-    for (const Need &x : per_cta) {
-        per_cta_bytes += x.bytes;
-        others -= (int64_t)x.buf->bytes;
-    }
-    // The list output's own part of that is a second row of stamps and the
-    // scratch its lists are made in, which let it go on beside the traversal;
-    // a traversal can wait for its lists instead, with one row and its queue.
-    // That takes 8 to 14% longer on as many CTAs (80^3 ranges 8.5 ms and 7.5,
-    // 20,011-line power law 3.5 and 3.2), and half the scratch: where it puts
-    // an eighth more CTAs to work it is the faster one (80^3 with room for 114
-    // or 148: 10.4 and 8.5 ms; for 76 or 148: 12.2 and 10.3; power law with
+    const int64_t queue_bytes = NS * qcap * 4, gstate_bytes = gbm ? (int64_t)NS * state_words * 4 : 0,
+                  row_bytes = NS * stamp_stride * 2;
+    // The list output's own part of a CTA's scratch is a second row of stamps
+    // and the scratch its lists are made in, which let it go on beside the
+    // traversal; a traversal can wait for its lists instead, with one row and
+    // its queue.  That takes 8 to 14% longer on as many CTAs (80^3 ranges 8.5 ms
+    // and 7.5, 20,011-line power law 3.5 and 3.2), and half the scratch: where it
+    // puts an eighth more CTAs to work it is the faster one (80^3 with room for
+    // 114 or 148: 10.4 and 8.5 ms; for 76 or 148: 12.2 and 10.3; power law with
     // room for 117 or 148: 5.9 and 3.5).
-    const int64_t beside_bytes = want_pattern ? NS * (stamp_stride * 2 + qcap * 4) : 0;
+    const int64_t beside_bytes = want_pattern ? row_bytes + queue_bytes : 0;
+    const int64_t per_cta_bytes = queue_bytes + gstate_bytes + (want_pattern ? row_bytes : 0) + beside_bytes;
     bool beside = true;
+    int64_t fixed_bytes = 4 * 256, others = (int64_t)ctx->held - (int64_t)ctx->trav.bytes;
     for (const Need &x : fixed) {
         fixed_bytes += std::max<int64_t>(x.bytes, 256);
         others -= (int64_t)x.buf->bytes;
@@ -533,19 +527,35 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
     // Concurrent traversals within the memory budget (the reference shrinks
     // its sources per pass until the state fits its pool,
     // with_space_optimization/symbfact.cuh:1465-1507)
+    const int64_t room = avail - (pattern_form == 1 ? 8 * pool_cap : 0);
     {
-        const int64_t room = avail - (pattern_form == 1 ? 8 * pool_cap : 0);
         const int64_t most = std::min<int64_t>(grid, room / per_cta_bytes);
         const int64_t waiting = std::min<int64_t>(grid, room / (per_cta_bytes - beside_bytes));
         if (waiting < 1) return GSOFA_ERR_OOM;
         beside = most * 8 >= waiting * 7;
-        if (!beside) {
-            per_cta[2].bytes /= 2;
-            per_cta[3].bytes = 0;
-        }
         grid = (int)(beside ? most : waiting);
         job_try.grid = grid;
     }
+    // The traversals' scratch in one buffer (a first call pays for every
+    // allocation: 31 x 29 x 27 with its lists 5.0 ms, in one 3.9), every part
+    // 256-byte aligned.
+    int64_t trav_bytes = 0;
+    auto part = [&](int64_t per_cta) {
+        const int64_t at = trav_bytes;
+        trav_bytes += (grid * per_cta + 255) / 256 * 256;
+        return at;
+    };
+    const int64_t at_queue = part(queue_bytes), at_gstate = part(gstate_bytes),
+                  at_stamp = part(want_pattern ? (beside ? 2 : 1) * row_bytes : 0),
+                  at_lists = want_pattern && beside ? part(queue_bytes) : at_queue;
+    // Snapshots: paired passes with reuse, as many as a sixteenth of the budget
+    // holds, and none where the rest of the job leaves no room for them.
+    int snap_k = 0;
+    const int64_t one_snap = NS * (int64_t)bitmap_words * 4;
+    if (paired && reuse && job_try.snaps)
+        for (int k = SNAP_MAX; k >= 2 && !snap_k; k >>= 1)
+            if (grid * one_snap * k <= (int64_t)(ctx->budget / 16) && trav_bytes + grid * one_snap * k <= room) snap_k = k;
+    const int64_t at_snap = part(snap_k * one_snap);
     // Sources per work piece.  A piece's first source cannot reuse state, and
     // its traversal from nothing costs as much as hundreds of later ones, so
     // pieces should be few and long, and yet the launch must not wait for the
@@ -612,16 +622,17 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         auto most = [&](const DevBuf &b, int64_t bytes) { all += std::max<int64_t>((int64_t)b.bytes, std::max<int64_t>(bytes, 256)); };
         auto spare = [&](DevBuf &b, int64_t bytes) { if ((int64_t)b.bytes > std::max<int64_t>(bytes, 256)) ctx->release(b); };
         for (const Need &x : fixed) most(*x.buf, x.bytes);
-        for (const Need &x : per_cta) most(*x.buf, grid * x.bytes);
+        most(ctx->trav, trav_bytes);
         if (pattern_form == 1) for (DevBuf *b : {&ctx->pool, &ctx->out}) most(*b, 4 * pool_cap);
         if (all > (int64_t)ctx->budget) {
             for (const Need &x : fixed) spare(*x.buf, x.bytes);
-            for (const Need &x : per_cta) spare(*x.buf, grid * x.bytes);
+            spare(ctx->trav, trav_bytes);
             if (pattern_form == 1) for (DevBuf *b : {&ctx->pool, &ctx->out}) spare(*b, 4 * pool_cap);
         }
         Scratch::Job job(*ctx);
         // scratch
-        int32_t *d_queue = (int32_t *)job.take(ctx->queue, (size_t)grid * NS * qcap * sizeof(int32_t));
+        char *d_trav = (char *)job.take(ctx->trav, (size_t)trav_bytes);
+        int32_t *d_queue = (int32_t *)(d_trav + at_queue);
         int32_t *d_cnt = (int32_t *)job.take(ctx->cnt, (size_t)2 * L * sizeof(int32_t));
         uint8_t *d_nxt = (uint8_t *)job.take(ctx->nxt, (size_t)2 * L);
         int64_t *d_poff = (int64_t *)job.take(ctx->poff, (size_t)2 * L * sizeof(int64_t));
@@ -639,36 +650,19 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         unsigned long long *d_counters = (unsigned long long *)(d_misc + 16);   // 16 counters
         uint32_t *d_status = (uint32_t *)(d_misc + 192);
         int32_t *d_pool = nullptr, *d_out = nullptr;
-        uint16_t *d_stamp = nullptr;
         if (pattern_form == 1) {
             d_pool = (int32_t *)job.take(ctx->pool, (size_t)pool_cap * sizeof(int32_t));
             d_out = (int32_t *)job.take(ctx->out, (size_t)pool_cap * sizeof(int32_t));
         } else if (pattern_form == 2) {
             d_pool = ext->dev;
         }
-        int32_t *d_lists = nullptr;
-        if (want_pattern) {
-            d_stamp = (uint16_t *)job.take(ctx->stamp, (size_t)(grid * per_cta[2].bytes));
-            d_lists = beside ? (int32_t *)job.take(ctx->lists, (size_t)(grid * per_cta[3].bytes)) : d_queue;
-        }
-        uint32_t *d_gstate = gbm ? (uint32_t *)job.take(ctx->gstate, (size_t)grid * NS * state_words * 4) : nullptr;
+        uint16_t *d_stamp = want_pattern ? (uint16_t *)(d_trav + at_stamp) : nullptr;
+        int32_t *d_lists = want_pattern ? (int32_t *)(d_trav + at_lists) : nullptr;
+        uint32_t *d_gstate = gbm ? (uint32_t *)(d_trav + at_gstate) : nullptr;
+        uint32_t *d_snap = snap_k ? (uint32_t *)(d_trav + at_snap) : nullptr;
         MatDesc *d_mats = (MatDesc *)job.take(ctx->mats, md.size() * sizeof(MatDesc));
         int64_t *d_minfo = (int64_t *)job.take(ctx->matinfo, (size_t)3 * count * sizeof(int64_t));
         Range *d_ranges = (Range *)job.take(ctx->ranges, std::max<size_t>(ranges.size(), 1) * sizeof(Range));
-
-        // Snapshots, after all that the job needs: paired passes with reuse, as
-        // many as a sixteenth of the budget holds, and none where the job
-        // leaves no room for them.
-        uint32_t *d_snap = nullptr;
-        int snap_k = 0;
-        if (paired && reuse) {
-            const size_t one = (size_t)grid * NS * bitmap_words * 4;
-            for (int k = SNAP_MAX; k >= 2 && !d_snap; k >>= 1) {
-                if (one * k > ctx->budget / 16) continue;
-                d_snap = (uint32_t *)job.take_if_room(ctx->snap, one * k);
-                if (d_snap) snap_k = k;
-            }
-        }
 
         cudaStream_t st = ctx->stream;
         JobArgs a{};
@@ -957,11 +951,14 @@ gsofa_status run_job(gsofa_ctx *ctx, int count, const gsofa_matrix *const *mats,
         try {
             s = run_job_once(ctx, count, mats, pin, out, ext, t);
         } catch (CudaFail &f) {
-            if (f.e != cudaErrorMemoryAllocation || t.grid <= 1 || t.grid == INT32_MAX) throw;
+            if (f.e != cudaErrorMemoryAllocation || t.grid == INT32_MAX || (t.grid <= 1 && !t.snaps)) throw;
             cudaGetLastError();
-            for (DevBuf *b : {&ctx->queue, &ctx->stamp, &ctx->lists, &ctx->gstate, &ctx->snap}) ctx->release(*b);
-            t.grid = std::min(t.grid, former) * 3 / 4;
-            t.guess /= 2;
+            ctx->release(ctx->trav);
+            if (!t.snaps) {
+                t.grid = t.grid * 3 / 4;
+                t.guess /= 2;
+            }
+            t.snaps = false;
             continue;
         }
         if (!t.again) return s;
@@ -1060,10 +1057,10 @@ void gsofa_destroy(gsofa_ctx *c)
     if (!c) return;
     cudaSetDevice(c->device);
     while (!c->matrices.empty()) gsofa_matrix_free(c->matrices.back());
-    DevBuf *bufs[] = {&c->queue, &c->cnt, &c->nxt, &c->poff, &c->gptr, &c->lrow, &c->snind,
+    DevBuf *bufs[] = {&c->trav, &c->cnt, &c->nxt, &c->poff, &c->gptr, &c->lrow, &c->snind,
                       &c->snlist, &c->tiles, &c->misc, &c->pool, &c->out, &c->mats, &c->ranges,
-                      &c->st_beg, &c->st_end, &c->st_adj, &c->st_tmp, &c->matinfo, &c->stamp,
-                      &c->sn_head, &c->sn_data, &c->gstate, &c->blk, &c->order, &c->snap, &c->lists};
+                      &c->st_beg, &c->st_end, &c->st_adj, &c->st_tmp, &c->matinfo,
+                      &c->sn_head, &c->sn_data, &c->blk, &c->order};
     for (DevBuf *b : bufs) c->release(*b);
     for (DevBuf &b : c->slabs) cudaFree(b.p);
     c->slabs.clear();

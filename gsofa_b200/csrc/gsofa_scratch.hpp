@@ -2,10 +2,10 @@
 // (host only; the device allocator is a parameter, so the rules can be tested
 // without one).
 //
-// Every buffer grows and is kept for the next job.  Dispensable buffers -- those
-// that only save time, and a job's own, which the next one can make again -- give
-// way to whatever needs the room, but never while a job that is being set up or
-// is running has taken them: what a job has its addresses from stays.
+// Every buffer grows and is kept for the next job.  Dispensable buffers, which
+// the next job can make again, give way to whatever needs the room, but never
+// while a job that is being set up or is running has taken them: what a job has
+// its addresses from stays.
 #pragma once
 
 #include <algorithm>
@@ -99,22 +99,6 @@ struct Scratch {
             if (!b.taken) bufs.push_back(&b);
             b.taken = true;
             return p;
-        }
-        // Same, for a buffer that the job can do without: null where the budget
-        // or the device has no room (nothing gives way for it).
-        void *take_if_room(DevBuf &b, size_t bytes)
-        {
-            bytes = std::max<size_t>(bytes, 256);
-            if (b.bytes < bytes) {
-                of.release(b);
-                if (of.held + bytes > of.budget) return nullptr;
-                void *p = Memory::alloc(bytes);
-                if (!p) return nullptr;
-                b.p = p;
-                b.bytes = bytes;
-                of.held += bytes;
-            }
-            return take(b, bytes);
         }
     };
 };

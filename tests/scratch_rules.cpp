@@ -52,52 +52,31 @@ bool refused(F f)
 int main()
 {
     // every budget and device size around what a job takes: the addresses that
-    // it holds are live when its last buffer is in place
+    // it holds are live when its last buffer is in place, whichever buffers of
+    // it are dispensable
     for (size_t limit = 0; limit < 2; limit++)
         for (size_t total = 9000; total <= 14000; total += 50) {
             FakeDevice::room = limit ? total : 1 << 20;
             Scratch s;
             s.budget = limit ? 1 << 20 : total;
-            DevBuf queue, snap, mats, ranges, other;
-            s.dispensable = {&snap};
+            DevBuf trav, snap, mats, ranges, other;
+            s.dispensable = {&snap, &trav};
             s.grow(other, 1000);
             for (size_t batch = 300; batch <= 1500; batch += 300) {   // each job larger than the last
-                refused([&] {
+                const bool no = refused([&] {
                     Scratch::Job job(s);
-                    void *q = job.take(queue, 8000);
-                    void *k = job.take_if_room(snap, 2000);
+                    void *t = job.take(trav, 6000), *k = job.take(snap, 2000);
                     void *m = job.take(mats, batch), *r = job.take(ranges, batch);
-                    CHECK(FakeDevice::live.count(q) && FakeDevice::live.count(m) && FakeDevice::live.count(r));
-                    CHECK(!k || (k == snap.p && FakeDevice::live.count(k)));
+                    for (void *p : {t, k, m, r}) CHECK(FakeDevice::live.count(p));
+                    CHECK(t == trav.p && k == snap.p && m == mats.p && r == ranges.p && s.idle() == 0);
                 });
+                CHECK(no == (9000 + 2 * batch > total));
                 CHECK(s.held <= s.budget && s.held == FakeDevice::used);
-                CHECK(!queue.taken && !snap.taken && !mats.taken);
+                CHECK(!trav.taken && !snap.taken && !mats.taken);
             }
-            // with the job over, what only saves time gives way
-            if (total >= 12000) CHECK(!refused([&] { s.grow(other, total - 1000 - 8000 - 3000 + 900); }));
-            for (DevBuf *b : {&queue, &snap, &mats, &ranges, &other}) s.release(*b);
+            for (DevBuf *b : {&trav, &snap, &mats, &ranges, &other}) s.release(*b);
             CHECK(FakeDevice::used == 0 && s.held == 0);
         }
-    // a job that asks for its optional buffer last fits wherever its others do
-    for (size_t total = 9000; total <= 14000; total += 50) {
-        FakeDevice::room = 1 << 20;
-        Scratch s;
-        s.budget = total;
-        DevBuf queue, snap, mats;
-        s.dispensable = {&snap};
-        for (size_t batch = 300; batch <= 1500; batch += 300) {
-            bool live = true;
-            const bool no = refused([&] {
-                Scratch::Job job(s);
-                job.take(queue, 8000);
-                job.take(mats, batch);
-                void *k = job.take_if_room(snap, 2000);
-                live = !k || FakeDevice::live.count(k);
-            });
-            CHECK(live && no == (8000 + batch > total));
-        }
-        for (DevBuf *b : {&queue, &snap, &mats}) s.release(*b);
-    }
     // what a job left gives way to anything else, in order, whether the budget
     // or the device is short; not to a buffer that holds it itself, nor while
     // a job has it
@@ -105,27 +84,28 @@ int main()
         FakeDevice::room = limit ? 10000 : 1 << 20;
         Scratch s;
         s.budget = limit ? 1 << 20 : 10000;
-        DevBuf snap, lists, order;
-        s.dispensable = {&snap, &lists};
+        DevBuf snap, trav, order;
+        s.dispensable = {&snap, &trav};
         {
             Scratch::Job job(s);
-            job.take(lists, 6000);
-            CHECK(job.take_if_room(snap, 3000) && !job.take_if_room(order, 3000) && s.idle() == 0);
+            job.take(trav, 6000);
+            job.take(snap, 3000);
+            CHECK(s.idle() == 0);
             CHECK(refused([&] { s.grow(order, 3000); }));
             if (limit) CHECK(refused([&] { s.alloc(3000); }));
         }
         CHECK(s.idle() == 9000);
-        CHECK(!refused([&] { s.grow(order, 3000); }) && !snap.p && lists.p);
-        CHECK(!refused([&] { s.grow(order, 9000); }) && !lists.p);
+        CHECK(!refused([&] { s.grow(order, 3000); }) && !snap.p && trav.p);
+        CHECK(!refused([&] { s.grow(order, 9000); }) && !trav.p);
         CHECK(!refused([&] { s.grow(snap, 1000); }) && refused([&] { s.grow(snap, 1001 + 1000); }));
         s.release(order);
         if (limit) {
-            s.grow(lists, 5000);
+            s.grow(trav, 5000);
             void *p = s.alloc(6000);
-            CHECK(p && !lists.p);
+            CHECK(p && !trav.p);
             FakeDevice::free(p);
         }
-        for (DevBuf *b : {&snap, &lists, &order}) s.release(*b);
+        for (DevBuf *b : {&snap, &trav, &order}) s.release(*b);
         CHECK(FakeDevice::used == 0);
     }
     std::printf("ok\n");
