@@ -2728,26 +2728,37 @@ gsofa_status gsofa_server_submit(gsofa_server *s, int32_t n, int64_t nnz, const 
     const int64_t st_units = units(server_staging_bytes(n, nnz));
     r.g_units = units(server_graph_bytes(n, nnz));
     if (!s->lines.alloc(n, &r.lb)) return GSOFA_ERR_BUSY;
-    if (s->snap_k && s->reqs.empty() && r.g_units + st_units > s->arena_units) {
-        // snapshots only save time: with nothing in flight they give way
-        try {
-            GS_CUDA(cudaSetDevice(s->device));
-            if (cudaStreamQuery(s->run) == cudaErrorNotReady) server_stop_kernel(s);
-        } catch (CudaFail &f) {
-            s->lines.release(r.lb, n);
-            return fail_cuda(f.e);
+    auto place = [&](RangeAlloc &arena) {
+        if (!arena.alloc(r.g_units, &r.g_off)) return false;
+        if (arena.alloc(st_units, &st_off)) return true;
+        arena.release(r.g_off, r.g_units);
+        return false;
+    };
+    bool placed = place(s->arena);
+    if (!placed && s->snap_k) {
+        // snapshots only save time: they give way where that makes the request
+        // fit and no traversal is using them
+        bool idle = true;
+        for (const auto &kv : s->reqs) idle &= kv.second.done;
+        RangeAlloc with = s->arena;
+        with.release(s->arena_units, s->snap_units);
+        if (idle && place(with)) {
+            try {
+                GS_CUDA(cudaSetDevice(s->device));
+                if (cudaStreamQuery(s->run) == cudaErrorNotReady) server_stop_kernel(s);
+            } catch (CudaFail &f) {
+                s->lines.release(r.lb, n);
+                return fail_cuda(f.e);
+            }
+            s->arena = with;
+            s->arena_units += s->snap_units;
+            s->snap_units = 0;
+            s->snap_k = 0;
+            placed = true;
         }
-        s->snap_k = 0;
-        s->arena_units += s->snap_units;
-        s->arena.init(s->arena_units);
     }
-    if (!s->arena.alloc(r.g_units, &r.g_off)) {
+    if (!placed) {
         s->lines.release(r.lb, n);
-        return GSOFA_ERR_BUSY;
-    }
-    if (!s->arena.alloc(st_units, &st_off)) {
-        s->lines.release(r.lb, n);
-        s->arena.release(r.g_off, r.g_units);
         return GSOFA_ERR_BUSY;
     }
     r.slot = s->free_slots.back();
