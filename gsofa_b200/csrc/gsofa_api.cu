@@ -210,7 +210,8 @@ struct ExtPool {
 
 // Shared memory of the factorization kernel beside bitmaps and rings.
 // lists: the instance has the list output (factor_kernel_for).
-constexpr int kMinRing = 512;
+constexpr int kMinRing = 512;    // frontier ring entries
+constexpr int kTightRing = 256;  // ... where the bitmaps leave no room for more
 constexpr size_t kStaticShared = 1024;   // the runtime's own and some slack
 size_t cta_shared(int block, int ns, bool lists) { return cta_bytes(ns, lists ? block / 32 - ns : 1); }
 
@@ -396,9 +397,12 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
     // paired kernel) up to ~850K lines and one up to ~1.7M; global memory
     // holds any number of any size.  GSOFA_FLAG_GLOBAL_STATE /
     // GSOFA_FLAG_SHARED_STATE choose; else shared memory while the pair fits.
-    const size_t pair_smem = (size_t)2 * state_needed * 4 + 2 * kMinRing * 4 + cta_shared(768, 2, want_pattern) + kStaticShared;
+    // (The pair with a ring of 256 is faster than global memory: 95 x 94 x 94
+    // ranges 13.6 and 15.2 ms, 95 x 95 x 94 counts 7.5 and 10.0, 839,368-line
+    // bordered ranges 18.4 and 21.5.)
+    const size_t pair_smem = (size_t)2 * state_needed * 4 + 2 * kTightRing * 4 + cta_shared(768, 2, want_pattern) + kStaticShared;
     if ((p.flags & GSOFA_FLAG_GLOBAL_STATE) && (p.flags & GSOFA_FLAG_SHARED_STATE)) return GSOFA_ERR_INVALID_INPUT;
-    const size_t single_smem = (size_t)state_needed * 4 + kMinRing * 4 + cta_shared(512, 1, true) + kStaticShared;
+    const size_t single_smem = (size_t)state_needed * 4 + kTightRing * 4 + cta_shared(512, 1, true) + kStaticShared;
     const bool want_pair = reuse && p.reuse != 2;
     const bool gbm = (p.flags & GSOFA_FLAG_GLOBAL_STATE) ||
                      (!(p.flags & GSOFA_FLAG_SHARED_STATE) &&
@@ -422,6 +426,17 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
     void *kfn = factor_kernel_for(block, paired, gbm, wide, want_pattern != 0);
     if (!kfn) return GSOFA_ERR_INVALID_INPUT;
     const int NS = paired ? 2 : 1;
+    // shared memory per traversal: its bitmap and summaries (unless in global
+    // memory) and its frontier ring; and beside them a row of counters a helper
+    // warp, for which a large block gives way where the bitmaps leave no room
+    const size_t smem_state = gbm ? 0 : (size_t)state_needed * 4;
+    size_t fixed_smem = 0;
+    for (;; block -= 256) {
+        fixed_smem = cta_shared(block, NS, want_pattern || !has_counts_form(block, paired, gbm, wide));
+        if ((size_t)NS * (smem_state + kTightRing * 4) + fixed_smem + kStaticShared <= ctx->smem_optin) break;
+        if (block <= 512) return GSOFA_ERR_UNSUPPORTED;
+    }
+    kfn = factor_kernel_for(block, paired, gbm, wide, want_pattern != 0);
     // accepted as ever; a warp's lanes share its vertices' rows by their
     // lengths, so the value chooses nothing any more
     const int lanes = p.threads_per_source ? p.threads_per_source : 1;
@@ -430,13 +445,9 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
 
     const int32_t bitmap_words = words_needed;
     const int32_t state_words = state_needed;
-    const size_t fixed_smem = cta_shared(block, NS, want_pattern || !has_counts_form(block, paired, gbm, wide));
-    // shared memory per traversal: its bitmap and summaries (unless in global
-    // memory) and its frontier ring
-    const size_t smem_state = gbm ? 0 : (size_t)state_words * 4;
-    if ((size_t)NS * (smem_state + kMinRing * 4) + fixed_smem + kStaticShared > ctx->smem_optin) return GSOFA_ERR_UNSUPPORTED;
     // frontier ring: the largest of 8K down to 512 entries that keeps the most
-    // CTAs (each with its own bitmap) resident on an SM; sized once per shape
+    // CTAs (each with its own bitmap) resident on an SM, or of 256 where no larger
+    // one fits; sized once per shape
     int ring = 0, occ = 0;
     size_t smem = 0;
     bool cached = false;
@@ -449,7 +460,7 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
         smem = fixed_smem + (size_t)NS * (smem_state + (size_t)ring * 4);
     } else {
         std::lock_guard<std::mutex> lk(kernel_attr_mutex());
-        for (int cand = 8192; cand >= kMinRing; cand >>= 1) {
+        for (int cand = 8192; cand >= (occ ? kMinRing : kTightRing); cand >>= 1) {
             const size_t sm = fixed_smem + (size_t)NS * (smem_state + (size_t)cand * 4);
             if (sm + kStaticShared > ctx->smem_optin) continue;
             GS_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -2563,7 +2574,7 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         // the global-state form unless shared memory is asked for
         s->gbm = !(cfg->flags & GSOFA_FLAG_SHARED_STATE);
         s->block = s->gbm ? kServeBlockG : kServeBlock;
-        const int64_t per_half_words = ((int64_t)(s->optin - static_smem - fixed_smem) / 2 - 1024 * 4) / 4;
+        const int64_t per_half_words = ((int64_t)(s->optin - static_smem - fixed_smem) / 2 - kMinRing * 4) / 4;
         const int32_t limit_n =
             s->gbm ? (int32_t)(1 << 26)
                    : (int32_t)std::min<int64_t>((per_half_words - 64) * 32 / 33 / 128 * 128 * 32, INT32_MAX);
@@ -2581,7 +2592,7 @@ gsofa_status gsofa_server_create(gsofa_server **out, gsofa_server_config *cfg)
         const int per_sm = s->gbm ? kServeCtasG : 1;
         const size_t smem_state = s->gbm ? 0 : (size_t)s->state_words * 4;
         s->ring = 0;
-        for (int cand = 8192; cand >= 1024; cand >>= 1) {
+        for (int cand = 8192; cand >= kMinRing; cand >>= 1) {
             const size_t sm = fixed_smem + 2 * (smem_state + (size_t)cand * 4);
             if ((sm + static_smem - reserve) * per_sm + reserve <= (size_t)prop.sharedMemPerMultiprocessor &&
                 sm + static_smem <= s->optin) {
