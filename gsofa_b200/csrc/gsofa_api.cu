@@ -213,6 +213,7 @@ struct ExtPool {
 constexpr int kMinRing = 512;    // frontier ring entries
 constexpr int kTightRing = 256;  // ... where the bitmaps leave no room for more
 constexpr size_t kStaticShared = 1024;   // the runtime's own and some slack
+constexpr int32_t kPairLines = 843776;   // whose two bitmaps fit with the list output's counters
 size_t cta_shared(int block, int ns, bool lists) { return cta_bytes(ns, lists ? block / 32 - ns : 1); }
 
 // Launch shapes whose counts-only jobs run an instantiation without the list
@@ -1823,13 +1824,22 @@ size_t gsofa_predict_scratch_bytes(const gsofa_ctx *c, int32_t n, int64_t nnz,
     const size_t grid = (size_t)per_sm * c->sm_count;
     const size_t qcap = (size_t)std::max<int64_t>(p.queue_capacity, n);
     const size_t L = (size_t)n;
-    size_t b = grid * qcap * 4;                 // frontier queues
+    size_t b = 0;
+    if (p.want_pattern) {
+        // Traversals come in pairs: a queue, list scratch, two rows of stamps and,
+        // past what shared memory holds, a bitmap each.  (Snapshots, at most
+        // another n bytes each, are taken where there is room only.)
+        const bool global = n > kPairLines;
+        const int most = n <= 8192 || global ? 2 : 1;
+        const size_t pairs = (size_t)(p.ctas_per_sm > 0 ? std::min(p.ctas_per_sm, most) : most) * c->sm_count;
+        b += pairs * 2 * (2 * qcap * 4 + 2 * ((size_t)(n + 4095) / 4096 * 4096) * 2 + (global ? (size_t)n / 31 * 4 : 0));
+    } else {
+        b += grid * qcap * 4;                   // frontier queues
+    }
     b += L * (2 * 4 + 2 + 2 * 8 + 4 + 1 + 4);   // cnt, nxt, poff, lrow, snind, sn list
     b += 2 * (L + 1) * 8;                       // gptr
     b += (size_t)(n + 1) * 8 + (size_t)nnz * 8; // G and G^T
     b += (size_t)n * 64;                        // their 32-byte row slots
-    if (p.want_pattern)                         // chain stamps, two traversals a CTA
-        b += grid * 2 * ((size_t)(n + 4095) / 4096 * 4096) * 2;
     return b;
 }
 

@@ -180,3 +180,22 @@ def test_what_a_job_left_gives_way_to_other_calls():
                 assert np.array_equal(r.u_row_count, ref["u_row_count"])
                 for v in (0, 100, 5000, 9000):
                     assert np.array_equal(r.u_row(v), ref["u_idx"][ref["u_ptr"][v]:ref["u_ptr"][v + 1]])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [8000, 50_000, 200_000, 800_000, 1_000_000])
+def test_predicted_scratch_covers_a_job_with_lists(n):
+    import torch
+    v = np.arange(n, dtype=np.int32)
+    g = Graph(n, v, v + 1, (v ^ 1).astype(np.int32), "pairs")
+    pool = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+    with gsofa_b200.Context(0) as ctx:
+        m = ctx.upload(g)
+        predicted = ctx.predict_scratch_bytes(n, g.nnz)
+        free = torch.cuda.mem_get_info()[0]
+        ctx.symbfact_ranges(m, pool)
+        used = free - torch.cuda.mem_get_info()[0]
+    # beside it: snapshots, one byte in thirteen, and the 2 MiB that each of a
+    # dozen allocations is rounded to
+    assert used <= predicted * 13 / 12 + (28 << 20)
+    assert predicted <= used * 2 + (28 << 20)
