@@ -1,10 +1,11 @@
 """Autotuner for the factorization launch parameters.
 
-Chooses (threads per CTA, lanes per frontier vertex, sources per work piece)
-from measured kernel times on the caller's own matrices, and caches the
-choice per workload signature (size buckets of n and nnz, matrix count) in a
-JSON file, so later runs skip the search.  The parameters only change speed:
-every choice returns bit-identical results.
+Chooses (threads per CTA, threads_per_source, sources per work piece) from
+measured kernel times on the caller's own matrices, and caches the choice per
+workload signature (size buckets of n and nnz, matrix count) in a JSON file, so
+later runs skip the search.  A choice holds for the kernels it was measured
+with (REVISION).  The parameters only change speed: every choice returns
+bit-identical results.
 """
 from __future__ import annotations
 
@@ -16,9 +17,14 @@ from typing import Dict, Iterable, List, Optional, Sequence, Tuple
 from . import Context, Matrix, Params
 
 DEFAULT_CANDIDATES: Tuple[Tuple[int, int, int], ...] = (
-    # (block_size, threads_per_source, src_chunk)
-    (0, 1, 0), (1024, 1, 128), (1024, 1, 512), (512, 1, 0), (256, 1, 0), (1024, 8, 0),
+    # (block_size, threads_per_source, src_chunk); the second chooses nothing
+    # any more, and a src_chunk keeps CTAs from sharing their pieces
+    (0, 1, 0), (1024, 1, 0), (1024, 1, 128), (1024, 1, 512), (512, 1, 0), (256, 1, 0),
 )
+
+# Of the kernels: a cached choice of another revision is measured anew (entries
+# without one are from before pieces were shared).
+REVISION = 2
 
 _CACHE_ENV = "GSOFA_AUTOTUNE_CACHE"
 
@@ -93,7 +99,7 @@ def autotune(ctx: Context, mats: Sequence[Matrix], base: Optional[Params] = None
     key = signature(mats)
     path = _cache_path(cache_path)
     table = _load(path) if use_cache else {}
-    if use_cache and key in table:
+    if use_cache and table.get(key, {}).get("revision") == REVISION:
         c = table[key]["choice"]
         return _params(base, *c), {"signature": key, "choice": c, "cached": True}
     timings: List[dict] = []
@@ -106,6 +112,6 @@ def autotune(ctx: Context, mats: Sequence[Matrix], base: Optional[Params] = None
             best, best_ms = (block, lanes, chunk), ms
     report = {"signature": key, "choice": list(best), "timings": timings, "cached": False}
     if use_cache:
-        table[key] = {"choice": list(best), "kernel_ms": best_ms}
+        table[key] = {"choice": list(best), "kernel_ms": best_ms, "revision": REVISION}
         _store(path, table)
     return _params(base, *best), report
