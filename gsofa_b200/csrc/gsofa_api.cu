@@ -395,7 +395,8 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
     const int32_t words_needed = ((max_n + 31) / 32 + 127) / 128 * 128;
     const int32_t state_needed = STATE_PAD + words_needed + words_needed / 32 + ((words_needed / 32 + 31) / 32 + 3) / 4 * 4;
     // Where the visited bitmaps live: shared memory holds two of them (the
-    // paired kernel) up to ~850K lines and one up to ~1.7M; global memory
+    // paired kernel) up to 843,776 lines (856,064 for counts) and one up to
+    // 1,736,704; global memory
     // holds any number of any size.  GSOFA_FLAG_GLOBAL_STATE /
     // GSOFA_FLAG_SHARED_STATE choose; else shared memory while the pair fits.
     // (The pair with a ring of 256 is faster than global memory: 95 x 94 x 94
@@ -413,8 +414,11 @@ gsofa_status run_job_once(gsofa_ctx *ctx, int count, const gsofa_matrix *const *
     // 64 registers fill its register file).  768 threads with up to 80
     // registers a thread are faster than 1024: counts of the 200K-line
     // power-law matrix 19.7 and 20.7 ms, of the 659K-line one 81.5 and 88.8.
+    // A caller's block_size may still ask for 1024, which are faster where many
+    // short levels are wide (300 x 300 grid 2.2 and 2.5 ms).
     // GSOFA_FLAG_WIDE_REGS takes 512 threads with up to 128 registers, for
-    // matrices whose levels are too small for more warps.
+    // matrices whose levels are too small for more warps (20^3 counts 0.28 ms
+    // and 0.33 with two CTAs of 64; 300 x 300 2.75 and 2.46 with 768 threads).
     const bool wide = (p.flags & GSOFA_FLAG_WIDE_REGS) != 0;
     int block = p.block_size;
     if (wide) block = 512;
@@ -2406,7 +2410,9 @@ constexpr int32_t kSmallRequest = 65536;   // lines below which a request is cla
 // per SM: two 256-thread upload blocks still run beside the persistent kernel.
 constexpr int kServeBlock = 768;
 // Global-state form: 256-thread CTAs, three per SM (768 threads, 48K of the
-// 64K registers), six traversals per SM.
+// 64K registers), six traversals per SM, for many small requests side by side.
+// (One traversal alone is faster with more helper warps; larger CTAs have not
+// been measured here.)
 constexpr int kServeBlockG = 256;
 constexpr int kServeCtasG = 3;
 

@@ -183,7 +183,6 @@ struct JobArgs {
 };
 
 constexpr int TILE = 2048;     // lines per tile in the post-traversal phases
-constexpr int HEAVY_ROW = 32;  // rows longer than this are expanded by a whole warp
 
 __device__ __forceinline__ int64_t warp_incl_scan(int64_t x)
 {
@@ -1545,8 +1544,8 @@ __device__ __noinline__ unsigned long long take_part(int ctas, int lane)
 // A traversal's first warp, its leader, runs the sources by itself: nine of
 // ten on nested-dissection matrices add no vertex below the source and need no
 // other warp.  The other warps wait at the traversal's barrier and join only
-// for large steps: a level of more than 32 vertices (and the levels after it
-// while they stay large), clearing or copying a wide bitmap, a chain's list
+// for large steps: a level of more than SOLO_MAX vertices (and the levels after
+// it while they stay large), clearing or copying a wide bitmap, a chain's list
 // output.  With all warps at a barrier two or three times a source, the 80^3
 // counts spent 4,600 cycles a source and pass.
 //
@@ -2073,10 +2072,12 @@ __device__ __forceinline__ void run_piece(const Trav<GBM> &t, int32_t s_lo, int3
 //
 // GBM = true: every traversal's visited bitmap and summaries live in global
 // memory (a.gbm, resident in L2 for the sizes that matter) instead of shared
-// memory, which then holds only the frontier rings.  A traversal's state no
-// longer bounds how many traversals an SM runs (shared memory holds two
-// bitmaps of at most ~850K lines each), so small CTAs run many traversals per
-// SM side by side, and n is bounded only by device memory.
+// memory, which then holds only the frontier rings: n is bounded only by device
+// memory (shared memory holds two bitmaps of at most 844K lines each, 856K for counts).  Two
+// CTAs of 512 threads an SM run four traversals side by side; smaller CTAs would
+// run more of them, but the one traversal of a whole matrix that a separator
+// line needs takes as long as its own helper warps are few (864,008-line
+// bordered matrix: 17 ms with seven of them, 39 with three).
 //
 // MINB: resident CTAs per SM the registers are budgeted for (the default
 // fills the SM with 1024 threads; 1 gives a 512-thread CTA up to 128

@@ -26,15 +26,18 @@
 namespace gsofa {
 namespace part {
 
-// Per-traversal, per-list-entry and per-edge costs (SM cycles, from the
-// factorization kernel's own tallies on the 80^3 nested-dissection matrix:
-// ~7K cycles per source and pass, ~2.6 cycles per list entry, ~3.2 cycles per
-// inspected edge of a traversal that starts afresh).  A traversal starts
-// afresh at the first source of every work piece and then expands all of
-// X(s), whose size is bounded by s's descendants in the elimination tree of
-// A + A^T.  Work pieces of a range of r lines of an n-line matrix are
-// max(r / 8G, min(n / 8G, r / 4G)) sources long on a GPU of G = 148 SMs,
-// between 32 and 512.
+// Per-traversal, per-list-entry and per-edge costs: weights in SM cycles, as a
+// kernel that took a step of all its warps for every source spent them on the
+// 80^3 nested-dissection matrix (~7K cycles per source and pass, ~2.6 per list
+// entry, ~3.2 per inspected edge of a traversal that starts afresh).  Sources
+// that go in runs take some 150 cycles now, so lines without lists weigh too
+// much: the slowest of four ranges takes 1.37 times their mean on that matrix,
+// 1.06 times on the 659,033-line power law.  Other weights would move the cuts
+// that callers get.  A traversal starts afresh at the first source of every
+// work piece and then expands all of X(s), whose size is bounded by s's
+// descendants in the elimination tree of A + A^T; a piece is taken to be
+// max(r / 8G, min(n / 8G, r / 4G)) sources long in a range of r lines of an
+// n-line matrix on a GPU of G = 148 SMs, between 32 and 512.
 constexpr double kCostPerSource = 7000.0;
 constexpr double kCostPerEntry = 2.6;
 constexpr double kCostPerEdge = 3.2;
