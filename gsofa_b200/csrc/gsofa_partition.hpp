@@ -32,7 +32,7 @@ namespace part {
 // entry, ~3.2 per inspected edge of a traversal that starts afresh).  Sources
 // that go in runs take some 150 cycles now, so lines without lists weigh too
 // much: the slowest of four ranges takes 1.37 times their mean on that matrix,
-// 1.06 times on the 659,033-line power law.  Other weights would move the cuts
+// 1.07 times on the 659,033-line power law.  Other weights would move the cuts
 // that callers get.  A traversal starts afresh at the first source of every
 // work piece and then expands all of X(s), whose size is bounded by s's
 // descendants in the elimination tree of A + A^T; a piece is taken to be
